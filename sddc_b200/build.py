@@ -39,6 +39,13 @@ CUDA_UNITS = {
     "adjoint_exact.cu": ["-fmad=false"],
     "output.cu": ["-fmad=false"],
 }
+# the line kernel's units: one object per N (0: the dispatch over N), with
+# the flags of the form's stage kernel
+LINE_N = (0, 2, 3, 4, 5, 6)
+OBJECTS = {name[:-3]: (name, flags) for name, flags in CUDA_UNITS.items()}
+for _form in ("exact", "fp64", "mixed"):
+    for _n in LINE_N:
+        OBJECTS[f"line_{_form}_n{_n}"] = (f"line_{_form}.cu", [*CUDA_UNITS[f"stage_{_form}.cu"], f"-DSDDC_N={_n}"])
 
 
 def _nvcc() -> str:
@@ -77,20 +84,21 @@ def build_host(force: bool = False) -> str:
     return out
 
 
-def build_gpu(force: bool = False, jobs: int = 4) -> str:
+def build_gpu(force: bool = False, jobs: int = os.cpu_count() or 4) -> str:
     os.makedirs(OBJ, exist_ok=True)
     out = os.path.join(LIB, "libsddc_b200.so")
     dep = _newest_dep()
     nvcc = _nvcc()
 
     def compile_unit(name):
-        obj = os.path.join(OBJ, name.replace(".cu", ".o"))
+        obj = os.path.join(OBJ, name + ".o")
+        source, flags = OBJECTS[name]
         if force or _stale(obj, dep):
-            _run([nvcc, *ARCH, *NVCC_COMMON, *CUDA_UNITS[name], "-c", os.path.join(CSRC, name), "-o", obj])
+            _run([nvcc, *ARCH, *NVCC_COMMON, *flags, "-c", os.path.join(CSRC, source), "-o", obj])
         return obj
 
     with cf.ThreadPoolExecutor(max_workers=jobs) as ex:
-        objs = list(ex.map(compile_unit, CUDA_UNITS))
+        objs = list(ex.map(compile_unit, OBJECTS))
     if force or _stale(out, max(os.path.getmtime(o) for o in objs)):
         _run([nvcc, *ARCH, "-shared", "-o", out, *objs, "-lcudart"])
     return out

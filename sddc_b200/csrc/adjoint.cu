@@ -156,7 +156,7 @@ int ensure_ws(sddc_ctx *ctx)
     const size_t nc = ctx->ncell, N = ctx->N;
     w->grid = (ctx->ncell + kAdjCpb - 1) / kAdjCpb;
     w->rec_cap = (int)std::min<size_t>(nc * 4 * N, (size_t)1 << 24);
-    const size_t tr = nc * 4 * N * 9;
+    const size_t tr = nc * 4 * trace_stride(ctx->N, 8);
     int rc;
     if ((rc = alloc(ctx, (void **)&w->at, nc * 4 * N * 12 * sizeof(double), "adjoint traces")) ||
         (rc = alloc(ctx, (void **)&w->at2, nc * 4 * N * 12 * sizeof(double), "adjoint traces")) ||
@@ -342,6 +342,7 @@ int forward_steps(sddc_ctx *ctx, double dt, int step0, int nsteps, double *const
             a.rk_kind = f.kind;
             a.q_in = S[5 * m + f.in];
             a.t_in = T[5 * m + f.in];
+            a.tfs = trace_stride(ctx->N, 8);
             a.q_out = S[5 * m + f.out];
             a.t_out = T[5 * m + f.out];
             a.reg_a = f.ra >= 0 ? S[5 * m + f.ra] : nullptr;
@@ -396,7 +397,7 @@ extern "C" int sddc_vjp_resid(sddc_ctx *ctx, const double *Rbar, double *Qbar, d
     if (rc) return rc;
     AdjWs *w = ctx->adj;
     CKA(cudaMemcpyAsync(w->lam, Rbar, ctx->nq * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
-    CKA(launch_trace_exact(ctx->N, ctx->ncell, ctx->reg[0], w->tq, ctx->ops, ctx->stream));
+    CKA(launch_trace_exact(ctx->N, ctx->ncell, ctx->reg[0], w->tq, trace_stride(ctx->N, 8), ctx->ops, ctx->stream));
     CKA(cudaMemcpyAsync(w->host, ctx->maxima + 2 * ctx->slot, 2 * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
     CKA(cudaMemsetAsync(w->acc, 0, sizeof(AdjScalars), ctx->stream));
     CKA(cudaStreamSynchronize(ctx->stream));
@@ -443,7 +444,7 @@ extern "C" int sddc_adjoint_run(sddc_ctx *ctx, const sddc_adjoint_opts *o, doubl
     const int ns = o->nsteps, K = o->checkpoint_every ? o->checkpoint_every : 20;
     const int nseg = (ns + K - 1) / K;
     const int segmax = std::min(K, ns);
-    const size_t nq = ctx->nq, tr = (size_t)ctx->ncell * 4 * ctx->N * 9;
+    const size_t nq = ctx->nq, tr = (size_t)ctx->ncell * 4 * trace_stride(ctx->N, 8);
     const double D = o->diameter > 0.0 ? o->diameter : 1.0;
 
     RunBufs rb;
@@ -512,7 +513,7 @@ extern "C" int sddc_adjoint_run(sddc_ctx *ctx, const sddc_adjoint_opts *o, doubl
     for (int s = 0; s < nseg; s++) {
         const int step0 = s * K, nst = std::min(K, ns - step0);
         CKA(cudaMemcpyAsync(S[0], ckpt[s], nq * sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream));
-        CKA(launch_trace_exact(ctx->N, ctx->ncell, S[0], T[0], ctx->ops, ctx->stream));
+        CKA(launch_trace_exact(ctx->N, ctx->ncell, S[0], T[0], trace_stride(ctx->N, 8), ctx->ops, ctx->stream));
         if (s == 0 && o->n1 == 0) CKA(wall_force(ctx, T[0], force));
         if ((rc = forward_steps(ctx, o->dt, step0, nst, S.data(), T.data(), hist, o->n1, o->n2, force, cmax,
                                 ctx->stream)))
@@ -596,7 +597,7 @@ extern "C" int sddc_adjoint_run(sddc_ctx *ctx, const sddc_adjoint_opts *o, doubl
         auto recompute = [&](int seg, int buf, cudaStream_t st) -> int {
             const int s0 = seg * K, n = std::min(K, ns - s0);
             CKA(cudaMemcpyAsync((*SS[buf])[0], ckpt[seg], nq * sizeof(double), cudaMemcpyDeviceToDevice, st));
-            CKA(launch_trace_exact(ctx->N, ctx->ncell, (*SS[buf])[0], (*TT[buf])[0], ctx->ops, st));
+            CKA(launch_trace_exact(ctx->N, ctx->ncell, (*SS[buf])[0], (*TT[buf])[0], trace_stride(ctx->N, 8), ctx->ops, st));
             return forward_steps(ctx, o->dt, s0, n, SS[buf]->data(), TT[buf]->data(), hist, 0, -1, nullptr, CM[buf], st);
         };
         for (int s = nseg - 1; s >= 0; s--) {
@@ -698,7 +699,7 @@ extern "C" int sddc_adjoint_run(sddc_ctx *ctx, const sddc_adjoint_opts *o, doubl
         if (grad && nseg > 1) {  // the stage store now holds the first segment: rerun the last one
             const int step0 = (nseg - 1) * K;
             CKA(cudaMemcpyAsync(S[0], ckpt[nseg - 1], nq * sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream));
-            CKA(launch_trace_exact(ctx->N, ctx->ncell, S[0], T[0], ctx->ops, ctx->stream));
+            CKA(launch_trace_exact(ctx->N, ctx->ncell, S[0], T[0], trace_stride(ctx->N, 8), ctx->ops, ctx->stream));
             if ((rc = forward_steps(ctx, o->dt, step0, last, S.data(), T.data(), hist, 0, -1, nullptr, cmax,
                                     ctx->stream)))
                 return rc;

@@ -402,8 +402,8 @@ __global__ void __launch_bounds__(adj_threads(N, CPB), 4) vjp_kernel(const VjpAr
                 const int pc = rec.x, plf = (rec.y >> 8) & 0xff;
                 // the face's 9N trace values, widened to 16-byte bounds (the
                 // buffer, 288N bytes per cell, starts and ends on one)
-                const uintptr_t t0 = (uintptr_t)(a.t_in + trace_at<N>(pc, plf, 0, 0)) & ~(uintptr_t)15;
-                const uintptr_t t1 = ((uintptr_t)(a.t_in + trace_at<N>(pc, plf, 0, 9)) + 15) & ~(uintptr_t)15;
+                const uintptr_t t0 = (uintptr_t)(a.t_in + trace_at<N>(trace_stride<N, double>(), pc, plf, 0, 0)) & ~(uintptr_t)15;
+                const uintptr_t t1 = ((uintptr_t)(a.t_in + trace_at<N>(trace_stride<N, double>(), pc, plf, 0, 9)) + 15) & ~(uintptr_t)15;
                 if (((uintptr_t)a.t_in & 15) == 0) bulk_prefetch_l2((const void *)t0, (unsigned)(t1 - t0));
                 if (a.xbar && ((uintptr_t)a.at & 15) == 0)
                     bulk_prefetch_l2(a.at + adj_trace_at<N>(pc, plf, 0, 0), 12 * N * sizeof(double));
@@ -511,7 +511,7 @@ __global__ void __launch_bounds__(adj_threads(N, CPB), 4) vjp_kernel(const VjpAr
         if (kind == kFaceLeft || own_right) {
             const int pc = rec.x, plf = (rec.y >> 8) & 0xff;
 #pragma unroll
-            for (int k = 0; k < 9; k++) oth[k] = a.t_in[trace_at<N>(pc, plf, N - nfp, k)];
+            for (int k = 0; k < 9; k++) oth[k] = a.t_in[trace_at<N>(trace_stride<N, double>(), pc, plf, N - nfp, k)];
         } else {
             const double *nrm = sNrm + c * NM + ML::normal(fam, line, r);
             bc_ghost<double, true>(kind, own, nrm[0], nrm[1], a.vismode, a.fs, oth);
@@ -992,7 +992,7 @@ __device__ void locate_tile(const LocateArgs &a, const Ops &ops, int tile, bool 
                 const int pc = rec.x, plf = (rec.y >> 8) & 0xff;
                 int pfam, pline, pr;
                 face_point<N>(plf, N - nfp + 1, pfam, pline, pr);
-                for (int k = 0; k < 9; k++) oth[k] = a.t_in[trace_at<N>(pc, plf, N - nfp, k)];
+                for (int k = 0; k < 9; k++) oth[k] = a.t_in[trace_at<N>(trace_stride<N, double>(), pc, plf, N - nfp, k)];
                 if (!own_right) {
                     sign_r = pr == N ? -1 : 1;
                 } else {
@@ -1076,7 +1076,7 @@ __global__ void __launch_bounds__(256) wall_force_kernel(int nw, const int2 *__r
         const int nfp = 1 + e % N, lf = wf.y;
         int fam, line, r;
         face_point<N>(lf, nfp, fam, line, r);
-        const size_t own = trace_at<N>(wf.x, lf, nfp - 1, 0);  // variable k at own + k*N
+        const size_t own = trace_at<N>(trace_stride<N, double>(), wf.x, lf, nfp - 1, 0);  // variable k at own + k*N
         const double *nr = met + (size_t)wf.x * ML::kSize + ML::normal(fam, line, r);
         const int sign_l = r == 0 ? -1 : 1;
         double ql[9], gh[9], Fl[9], Fr[9], eig, um = 0.0;

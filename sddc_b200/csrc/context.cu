@@ -208,7 +208,10 @@ extern "C" int sddc_create(sddc_ctx **out, const sddc_params *p)
         return bad("cells_per_cta must be 0, 4, 6, 8 or 16");
     ctx->N = p->N;
     ctx->ncell = p->ncell;
-    ctx->cpb = p->cells_per_cta ? p->cells_per_cta : 8;
+    // time steps run by lines, or (exact form) by tiles: see small_exact_mesh
+    const bool tiles = p->precision == SDDC_FP64_EXACT &&
+                       (p->cells_per_cta ? p->cells_per_cta == kTileCpb : small_exact_mesh(p->N, p->ncell));
+    ctx->cpb = tiles ? kTileCpb : line_tile_cells(p->N);
     if (!ctx->p.ncellglob) ctx->p.ncellglob = p->ncell;
     ctx->msize = met_size(p->N);
     ctx->nq = (size_t)9 * p->N * p->N * p->ncell;
@@ -217,13 +220,15 @@ extern "C" int sddc_create(sddc_ctx **out, const sddc_params *p)
     CK(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
     const int nreg = p->k_stage == 5 ? 6 : 4;
     int rc;
-    ctx->trace_bytes = (size_t)p->ncell * 4 * p->N * 9 * (p->precision == SDDC_MIXED ? sizeof(float) : sizeof(double));
+    const size_t elem = p->precision == SDDC_MIXED ? sizeof(float) : sizeof(double);
+    ctx->tfs = trace_stride(p->N, (int)elem);
+    ctx->trace_bytes = (size_t)p->ncell * 4 * ctx->tfs * elem;
     for (int r = 0; r < nreg; r++) {
         if ((rc = alloc(ctx, (void **)&ctx->reg[r], ctx->nq * sizeof(double), "state register"))) return rc;
         if ((rc = alloc(ctx, &ctx->trace[r], ctx->trace_bytes, "face traces"))) return rc;
     }
     const size_t nc = p->ncell;
-    const int diag_grid = (p->ncell + 7) / 8;
+    const int diag_grid = (p->ncell + kResidCpb - 1) / kResidCpb;
     const int mon_blocks = std::max(ctx->grid, diag_grid);
     ctx->nrm_double = p->precision != SDDC_MIXED;
     ctx->jac_inv = p->precision != SDDC_FP64_EXACT;
@@ -284,10 +289,7 @@ extern "C" int sddc_set_tables(sddc_ctx *ctx, const double *Lmat, const double *
     const int N = ctx->N, N1 = N + 1, NC = ctx->ncell;
     for (int r = 0; r < N1; r++)
         for (int s = 0; s < N; s++) {
-            ctx->ops.L[r * N + s] = Lmat[r + N1 * s];
-            ctx->ops.M[r * N + s] = Mmat[r + N1 * s];
-            ctx->ops.Lf[r * N + s] = (float)Lmat[r + N1 * s];
-            ctx->ops.Mf[r * N + s] = (float)Mmat[r + N1 * s];
+            ctx->ops.set(r * N + s, Lmat[r + N1 * s], Mmat[r + N1 * s]);
         }
     // packed metrics: S1(1,1:2,r,j), S2(2,1:2,i,r), Jac(i,j)
     std::vector<double> met((size_t)NC * ctx->msize, 0.0);
@@ -411,14 +413,14 @@ namespace {
 // send[slot][nfp][k] = trace of the slot's own (cell, local face), the
 // reference's SBUFC order (procintflux_all.f90:49-70)
 template <typename T>
-__global__ void proc_pack_kernel(int nproc, int N, const int2 *__restrict__ pc, const T *__restrict__ tr,
+__global__ void proc_pack_kernel(int nproc, int N, int tfs, const int2 *__restrict__ pc, const T *__restrict__ tr,
                                  T *__restrict__ send)
 {
     const int n = nproc * N * 9;
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
         const int k = e % 9, nfp0 = (e / 9) % N, b = e / (9 * N);
         const int2 c = pc[b];
-        send[e] = tr[((size_t)c.x * 4 + (c.y - 1)) * 9 * N + (size_t)k * N + nfp0];  // trace_at
+        send[e] = tr[((size_t)c.x * 4 + (c.y - 1)) * tfs + (size_t)k * N + nfp0];  // trace_at
     }
 }
 }  // namespace
@@ -437,11 +439,11 @@ static int exchange(sddc_ctx *ctx, int reg, int slot)
         const int n = nproc * ctx->N * 9, nb = std::min((n + 255) / 256, 4096);
         if (ctx->p.precision == SDDC_MIXED)
             proc_pack_kernel<float><<<nb, 256, 0, ctx->stream>>>(
-                nproc, ctx->N, ctx->proc_cells, reinterpret_cast<const float *>(ctx->trace[reg]),
+                nproc, ctx->N, ctx->tfs, ctx->proc_cells, reinterpret_cast<const float *>(ctx->trace[reg]),
                 reinterpret_cast<float *>(ctx->proc_send));
         else
             proc_pack_kernel<double><<<nb, 256, 0, ctx->stream>>>(
-                nproc, ctx->N, ctx->proc_cells, reinterpret_cast<const double *>(ctx->trace[reg]),
+                nproc, ctx->N, ctx->tfs, ctx->proc_cells, reinterpret_cast<const double *>(ctx->trace[reg]),
                 reinterpret_cast<double *>(ctx->proc_send));
         CK(cudaGetLastError());
     }
@@ -459,9 +461,9 @@ static int refresh_traces(sddc_ctx *ctx)
 {
     cudaError_t e;
     switch (ctx->p.precision) {
-    case SDDC_FP64_EXACT: e = launch_trace_exact(ctx->N, ctx->ncell, ctx->reg[0], ctx->trace[0], ctx->ops, ctx->stream); break;
-    case SDDC_FP64: e = launch_trace_fp64(ctx->N, ctx->ncell, ctx->reg[0], ctx->trace[0], ctx->ops, ctx->stream); break;
-    default: e = launch_trace_mixed(ctx->N, ctx->ncell, ctx->reg[0], ctx->trace[0], ctx->ops, ctx->stream); break;
+    case SDDC_FP64_EXACT: e = launch_trace_exact(ctx->N, ctx->ncell, ctx->reg[0], ctx->trace[0], ctx->tfs, ctx->ops, ctx->stream); break;
+    case SDDC_FP64: e = launch_trace_fp64(ctx->N, ctx->ncell, ctx->reg[0], ctx->trace[0], ctx->tfs, ctx->ops, ctx->stream); break;
+    default: e = launch_trace_mixed(ctx->N, ctx->ncell, ctx->reg[0], ctx->trace[0], ctx->tfs, ctx->ops, ctx->stream); break;
     }
     if (e != cudaSuccess) return cuda_err(ctx, e, "trace kernel");
     ctx->traces_stale = false;
@@ -506,6 +508,7 @@ StageArgs sddc::base_args(sddc_ctx *ctx)
     a.jac = ctx->jac;
     a.jac_inv = ctx->jac_inv ? 1 : 0;
     a.faces = ctx->faces;
+    a.tfs = ctx->tfs;
     a.proc_recv = ctx->proc_recv;
     a.maxima = ctx->maxima;
     a.sm_ind = ctx->sm_ind;
@@ -525,6 +528,7 @@ static cudaError_t launch_visc(sddc_ctx *ctx, const double *q_in, const void *t_
     v.fs = Freestream{ctx->p.rinf, ctx->p.pinf, ctx->p.uinf, ctx->p.vinf, ctx->p.bxinf, ctx->p.byinf};
     v.q = q_in;
     v.t_in = t_in;
+    v.tfs = ctx->tfs;
     v.met = ctx->met;
     v.met2 = ctx->met2;
     v.faces = ctx->faces;
@@ -623,7 +627,7 @@ extern "C" int sddc_compresid(sddc_ctx *ctx)
     if ((rc = exchange(ctx, 0, a.slot_w))) return rc;
     ctx->slot = a.slot_w;
     ctx->sensor_stale = false;
-    ctx->mon_nblk = ctx->ncase ? ctx->ntiles_diag : (ctx->ncell + 7) / 8;
+    ctx->mon_nblk = ctx->ncase ? ctx->ntiles_diag : (ctx->ncell + kResidCpb - 1) / kResidCpb;
     CK(cudaStreamSynchronize(ctx->stream));
     return check_flags(ctx);
 }
@@ -915,6 +919,7 @@ extern "C" int sddc_set_cases(sddc_ctx *ctx, int ncase, const sddc_case *cases)
         next += cases[c].ncell;
     }
     if (next != ctx->ncell) return set_err(ctx, SDDC_EINVAL, "the cases do not cover the context's cells");
+    ctx->cpb = line_tile_cells(ctx->N);  // batches run by lines
     ctx->ncase = ncase;
     ctx->cases.assign(cases, cases + ncase);
     std::vector<CaseParams> cp(ncase);
@@ -930,7 +935,7 @@ extern "C" int sddc_set_cases(sddc_ctx *ctx, int ncase, const sddc_case *cases)
     if ((rc = alloc(ctx, (void **)&ctx->case_dev, ncase * sizeof(CaseParams), "case table"))) return rc;
     CK(cudaMemcpyAsync(ctx->case_dev, cp.data(), ncase * sizeof(CaseParams), cudaMemcpyHostToDevice, ctx->stream));
     if ((rc = build_tiles(ctx, ctx->cpb, &ctx->tiles_rk, &ctx->ntiles_rk))) return rc;
-    if ((rc = build_tiles(ctx, 8, &ctx->tiles_diag, &ctx->ntiles_diag))) return rc;
+    if ((rc = build_tiles(ctx, kResidCpb, &ctx->tiles_diag, &ctx->ntiles_diag))) return rc;
     // per-case running maxima and per-tile monitor partials
     cudaFree(ctx->maxima);
     cudaFree(ctx->mon_part);
@@ -960,7 +965,7 @@ extern "C" int sddc_set_persistent(sddc_ctx *ctx, int on)
     if (ctx->ncase) {  // the tile tables in the launch's order
         int rc;
         if ((rc = build_tiles(ctx, ctx->cpb, &ctx->tiles_rk, &ctx->ntiles_rk)) ||
-            (rc = build_tiles(ctx, 8, &ctx->tiles_diag, &ctx->ntiles_diag)))
+            (rc = build_tiles(ctx, kResidCpb, &ctx->tiles_diag, &ctx->ntiles_diag)))
             return rc;
     }
     for (auto &g : ctx->graph)

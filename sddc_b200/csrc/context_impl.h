@@ -19,9 +19,9 @@ struct Output;
 cudaError_t launch_stage_exact(int N, int cpb, bool diag, const StageArgs &a, const Ops &ops, cudaStream_t st);
 cudaError_t launch_stage_fp64(int N, int cpb, bool diag, const StageArgs &a, const Ops &ops, cudaStream_t st);
 cudaError_t launch_stage_mixed(int N, int cpb, bool diag, const StageArgs &a, const Ops &ops, cudaStream_t st);
-cudaError_t launch_trace_exact(int N, int ncell, const double *q, void *t, const Ops &ops, cudaStream_t st);
-cudaError_t launch_trace_fp64(int N, int ncell, const double *q, void *t, const Ops &ops, cudaStream_t st);
-cudaError_t launch_trace_mixed(int N, int ncell, const double *q, void *t, const Ops &ops, cudaStream_t st);
+cudaError_t launch_trace_exact(int N, int ncell, const double *q, void *t, int tfs, const Ops &ops, cudaStream_t st);
+cudaError_t launch_trace_fp64(int N, int ncell, const double *q, void *t, int tfs, const Ops &ops, cudaStream_t st);
+cudaError_t launch_trace_mixed(int N, int ncell, const double *q, void *t, int tfs, const Ops &ops, cudaStream_t st);
 struct ViscArgs;
 cudaError_t launch_visc_exact(int N, const ViscArgs &a, const Ops &ops, cudaStream_t st);
 cudaError_t launch_visc_fp64(int N, const ViscArgs &a, const Ops &ops, cudaStream_t st);
@@ -61,6 +61,7 @@ struct sddc_ctx {
     double *reg[sddc::kRegs] = {};
     void *trace[sddc::kRegs] = {};  // face traces of each register (float in the mixed form)
     size_t trace_bytes = 0;
+    int tfs = 0;  // stride of a face's trace record
     double *met = nullptr;
     // the metrics split for the stage kernel's staging copies: normals in the
     // form's arithmetic type [NCELL][4N(N+1)] and Jac [NCELL][kJacPad]

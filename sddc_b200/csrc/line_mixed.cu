@@ -1,0 +1,6 @@
+// The mixed form of the line kernel; one object per N (SDDC_N), SDDC_N = 0 for
+// the dispatch.
+#define SDDC_R float
+#define SDDC_EXACT_FORM false
+#define SDDC_LINE launch_line_mixed
+#include "line_launch.inc"

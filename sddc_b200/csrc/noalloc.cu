@@ -27,9 +27,9 @@ namespace sddc {
 cudaError_t launch_stage_exact(int N, int cpb, bool diag, const StageArgs &a, const Ops &ops, cudaStream_t st);
 cudaError_t launch_stage_fp64(int N, int cpb, bool diag, const StageArgs &a, const Ops &ops, cudaStream_t st);
 cudaError_t launch_stage_mixed(int N, int cpb, bool diag, const StageArgs &a, const Ops &ops, cudaStream_t st);
-cudaError_t launch_trace_exact(int N, int ncell, const double *q, void *t, const Ops &ops, cudaStream_t st);
-cudaError_t launch_trace_fp64(int N, int ncell, const double *q, void *t, const Ops &ops, cudaStream_t st);
-cudaError_t launch_trace_mixed(int N, int ncell, const double *q, void *t, const Ops &ops, cudaStream_t st);
+cudaError_t launch_trace_exact(int N, int ncell, const double *q, void *t, int tfs, const Ops &ops, cudaStream_t st);
+cudaError_t launch_trace_fp64(int N, int ncell, const double *q, void *t, int tfs, const Ops &ops, cudaStream_t st);
+cudaError_t launch_trace_mixed(int N, int ncell, const double *q, void *t, int tfs, const Ops &ops, cudaStream_t st);
 }  // namespace sddc
 
 using namespace sddc;
@@ -152,10 +152,7 @@ extern "C" int sddc_compresid_noalloc(const sddc_params *p, const double *Lmat, 
     Ops ops{};
     for (int r = 0; r < N1; r++)
         for (int s = 0; s < N; s++) {
-            ops.L[r * N + s] = Lmat[r + N1 * s];
-            ops.M[r * N + s] = Mmat[r + N1 * s];
-            ops.Lf[r * N + s] = (float)Lmat[r + N1 * s];
-            ops.Mf[r * N + s] = (float)Mmat[r + N1 * s];
+            ops.set(r * N + s, Lmat[r + N1 * s], Mmat[r + N1 * s]);
         }
     double Xs[kMaxN], Xf[kMaxN + 1], Xl[kMaxN], Xlf[kMaxN + 1];
     sd_points(N, Xs, Xf);
@@ -179,9 +176,9 @@ extern "C" int sddc_compresid_noalloc(const sddc_params *p, const double *Lmat, 
 
     void *trace = scratch + L.trace;
     switch (p->precision) {
-    case SDDC_FP64_EXACT: e = launch_trace_exact(N, p->ncell, q_dev, trace, ops, st); break;
-    case SDDC_FP64: e = launch_trace_fp64(N, p->ncell, q_dev, trace, ops, st); break;
-    default: e = launch_trace_mixed(N, p->ncell, q_dev, trace, ops, st); break;
+    case SDDC_FP64_EXACT: e = launch_trace_exact(N, p->ncell, q_dev, trace, 9 * N, ops, st); break;
+    case SDDC_FP64: e = launch_trace_fp64(N, p->ncell, q_dev, trace, 9 * N, ops, st); break;
+    default: e = launch_trace_mixed(N, p->ncell, q_dev, trace, 9 * N, ops, st); break;
     }
     if (e != cudaSuccess) return fail(SDDC_ECUDA, std::string("trace kernel: ") + cudaGetErrorString(e));
 
@@ -194,6 +191,7 @@ extern "C" int sddc_compresid_noalloc(const sddc_params *p, const double *Lmat, 
     a.rk_kind = kRkNone;
     a.q_in = q_dev;
     a.t_in = trace;
+    a.tfs = 9 * N;
     a.met = met_dev;
     a.faces = reinterpret_cast<const int2 *>(faces_dev);
     a.maxima = maxima;
@@ -205,9 +203,9 @@ extern "C" int sddc_compresid_noalloc(const sddc_params *p, const double *Lmat, 
     a.mon_part = nullptr;
     a.err_flags = flags;
     switch (p->precision) {
-    case SDDC_FP64_EXACT: e = launch_stage_exact(N, 8, true, a, ops, st); break;
-    case SDDC_FP64: e = launch_stage_fp64(N, 8, true, a, ops, st); break;
-    default: e = launch_stage_mixed(N, 8, true, a, ops, st); break;
+    case SDDC_FP64_EXACT: e = launch_stage_exact(N, kResidCpb, true, a, ops, st); break;
+    case SDDC_FP64: e = launch_stage_fp64(N, kResidCpb, true, a, ops, st); break;
+    default: e = launch_stage_mixed(N, kResidCpb, true, a, ops, st); break;
     }
     if (e != cudaSuccess) return fail(SDDC_ECUDA, std::string("stage kernel: ") + cudaGetErrorString(e));
 

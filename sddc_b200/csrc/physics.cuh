@@ -26,6 +26,45 @@ SDDC_HD double Abs(double x) { return fabs(x); }
 SDDC_HD float Abs(float x) { return fabsf(x); }
 template <typename R> SDDC_HD R Max(R a, R b) { return a > b ? a : b; }
 
+// Quotients a[i] / b of one divisor, each rounded to nearest as the division
+// itself rounds it.  On the device, in double, from y, the correctly rounded
+// reciprocal of b: q0 = RN(a y) is within 1.5 ulp of a / b, the step
+// RN(q0 + RN(a - b q0) y) makes it a neighbour of a / b, and a second step
+// rounds it correctly (Markstein, IBM J. Res. Dev. 34, 1990: a faithful
+// quotient, its exact remainder and a correctly rounded reciprocal).  The
+// steps need exponents far from the format's ends; other operands go through
+// the division.  Divisions are branches of their own, one after the other;
+// these overlap.
+SDDC_HD double quotient_from(double a, double b, double y)
+{
+    const double q0 = a * y;
+    const double q1 = fma(fma(-b, q0, a), y, q0);
+    return copysign(fma(fma(-b, q1, a), y, q1), q0);  // a zero keeps its sign
+}
+// whether |x| lies in [2^-500, 2^500): hi is the upper half of its bits
+SDDC_HD bool mid_range(unsigned hi) { return (hi & 0x7fffffffu) - ((1023u - 500u) << 20) < (1000u << 20); }
+template <int n, typename R> SDDC_HD void quotients(const R *a, R b, R *q)
+{
+#pragma unroll
+    for (int i = 0; i < n; i++) q[i] = a[i] / b;
+}
+#ifdef __CUDA_ARCH__
+template <int n> __device__ __forceinline__ void quotients(const double *a, double b, double *q)
+{
+    bool ok = mid_range(__double2hiint(b));
+#pragma unroll
+    for (int i = 0; i < n; i++) ok = ok && (mid_range(__double2hiint(a[i])) || a[i] == 0.0);
+    if (ok) {
+        const double y = __drcp_rn(b);
+#pragma unroll
+        for (int i = 0; i < n; i++) q[i] = quotient_from(a[i], b, y);
+    } else {
+#pragma unroll
+        for (int i = 0; i < n; i++) q[i] = a[i] / b;
+    }
+}
+#endif
+
 struct Freestream {
     double rinf, pinf, uinf, vinf, bxinf, byinf;
 };
@@ -52,34 +91,37 @@ SDDC_HD void iflux(const R *Q, R c_h, R &umax, R *F, R *G)
     const R Bx = Q[5], By = Q[6], Bz = Q[7], psi = Q[8];
     const R NORM_B = (Bx * Bx + By * By) + Bz * Bz;
     if constexpr (EX) {
-        const R pr = (R)(kGam - 1.0) *
-                     (((rhoE - (R)0.5 * ((rhou * rhou + rhov * rhov) + rhow * rhow) / rho) - (R)0.5 * NORM_B) -
-                      (R)0.5 * (psi * psi));
+        // the nine quotients by rho of both fluxes
+        const R num[9] = {rhou, rhov, rhow, rhou * rhou, rhou * rhov, rhou * rhow, rhov * rhov, rhow * rhov,
+                          (R)0.5 * ((rhou * rhou + rhov * rhov) + rhow * rhow)};
+        R d[9];
+        quotients<9>(num, rho, d);
+        const R u = d[0], v = d[1], w = d[2];
+        const R pr = (R)(kGam - 1.0) * (((rhoE - d[8]) - (R)0.5 * NORM_B) - (R)0.5 * (psi * psi));
         F[0] = rhou;
-        F[1] = ((rhou * rhou) / rho + pr) + ((R)0.5 * NORM_B - Bx * Bx);
-        F[2] = rhou * rhov / rho - Bx * By;
-        F[3] = rhou * rhow / rho - Bx * Bz;
-        const R ub = (rhou / rho * Bx + rhov / rho * By) + rhow / rho * Bz;
+        F[1] = (d[3] + pr) + ((R)0.5 * NORM_B - Bx * Bx);
+        F[2] = d[4] - Bx * By;
+        F[3] = d[5] - Bx * Bz;
+        const R ub = (u * Bx + v * By) + w * Bz;
         const R eb = ((rhoE - (R)0.5 * (psi * psi)) + pr) + (R)0.5 * NORM_B;
-        F[4] = (rhou / rho) * eb - ub * Bx;
+        F[4] = u * eb - ub * Bx;
         F[5] = (R)0;
-        F[6] = rhou / rho * By - rhov / rho * Bx;
-        F[7] = rhou / rho * Bz - rhow / rho * Bx;
+        F[6] = u * By - v * Bx;
+        F[7] = u * Bz - w * Bx;
         G[0] = rhov;
-        G[1] = rhou * rhov / rho - Bx * By;
-        G[2] = ((rhov * rhov) / rho + pr) + ((R)0.5 * NORM_B - By * By);
-        G[3] = rhow * rhov / rho - By * Bz;
-        G[4] = (rhov / rho) * eb - ub * By;
-        G[5] = rhov / rho * Bx - rhou / rho * By;
+        G[1] = d[4] - Bx * By;
+        G[2] = (d[6] + pr) + ((R)0.5 * NORM_B - By * By);
+        G[3] = d[7] - By * Bz;
+        G[4] = v * eb - ub * By;
+        G[5] = v * Bx - u * By;
         G[6] = (R)0;
-        G[7] = rhov / rho * Bz - rhow / rho * By;
+        G[7] = v * Bz - w * By;
         F[4] = F[4] + c_h * psi * Bx;
         G[4] = G[4] + c_h * psi * By;
         F[5] = F[5] + c_h * psi;
         G[6] = G[6] + c_h * psi;
         F[8] = c_h * Bx;
         G[8] = c_h * By;
-        const R u = rhou / rho, v = rhov / rho, w = rhow / rho;
         const R um = Max(Max(Abs(u), Abs(v)), Abs(w));
         if (um > umax) umax = um;
     } else {
@@ -157,8 +199,11 @@ SDDC_HD void rusanov(const R *Qfl, const R *Qfr, R *Fnl, R *Fnr, R n0, R n1, int
     const R NORM_Bl = (Bxl * Bxl + Byl * Byl) + Bzl * Bzl;
     const R NORM_Br = (Bxr * Bxr + Byr * Byr) + Bzr * Bzr;
     if constexpr (EX) {
-        unit_x = n0 / magnorm * (R)sign_l;
-        unit_y = n1 / magnorm * (R)sign_l;
+        const R nn[2] = {n0, n1};
+        R un[2];
+        quotients<2>(nn, magnorm, un);
+        unit_x = un[0] * (R)sign_l;
+        unit_y = un[1] * (R)sign_l;
         R rhoi = (R)1 / Qfl[0];
         ul = rhoi * Qfl[1]; vl = rhoi * Qfl[2]; wl = rhoi * Qfl[3];
         pl = (R)(kGam - 1.0) * (((Qfl[4] - (R)0.5 * Qfl[0] * ((ul * ul + vl * vl) + wl * wl)) - NORM_Bl * (R)0.5) -
@@ -189,9 +234,14 @@ SDDC_HD void rusanov(const R *Qfl, const R *Qfr, R *Fnl, R *Fnr, R n0, R n1, int
     const R bn = Bx * unit_x + By * unit_y;
     R c_a, c_d, c_n;
     if constexpr (EX) {
-        c_a = (R)kGam * (pgl + pgr) / (Qfl[0] + Qfr[0]);
-        c_d = ((Bx * Bx + By * By) + Bz * Bz) / ((R)0.5 * (Qfl[0] + Qfr[0]));
-        c_n = bn * bn / ((R)0.5 * (Qfl[0] + Qfr[0]));
+        const R rs = Qfl[0] + Qfr[0];
+        // by rs, and twice by rs / 2: doubling the numerators instead is exact
+        const R num[3] = {(R)kGam * (pgl + pgr), (R)2 * ((Bx * Bx + By * By) + Bz * Bz), (R)2 * (bn * bn)};
+        R c[3];
+        quotients<3>(num, rs, c);
+        c_a = c[0];
+        c_d = c[1];
+        c_n = c[2];
     } else {
         const R rs = (R)1 / (Qfl[0] + Qfr[0]);
         c_a = (R)kGam * (pgl + pgr) * rs;
@@ -208,7 +258,7 @@ SDDC_HD void rusanov(const R *Qfl, const R *Qfr, R *Fnl, R *Fnr, R n0, R n1, int
         R f = (R)0.5 * ((fl + fr) - eigv * (Qfr[k] - Qfl[k]));
         f = sl * f;
         Fnl[k] = f;
-        Fnr[k] = slr * f;
+        if (Fnr) Fnr[k] = slr * f;  // null: the left slot alone
     };
     put(0, Qfl[0] * Vn_l, Qfr[0] * Vn_r);
     put(1, (Qfl[1] * Vn_l + pl * unit_x) - Bxl * Bn_l, (Qfr[1] * Vn_r + pr * unit_x) - Bxr * Bn_r);

@@ -1,17 +1,20 @@
-// The fused residual + RK stage kernel of the SDDC drop-in.
+// The fused residual (+ RK stage) kernel of the SDDC drop-in, by tiles.
 //
 // One launch evaluates compresid (compresid.f90:1-80, compflux.f90:1-104,
 // interfaceflux_all.f90:1-112, cyclocflux_all.f90:1-112, bcflux.f90:1-377,
-// nablaQsp compflux.f90:107-157, the AV sensor AV.f90:1-142) for every cell
-// and applies one RK stage update (iterations.f90:88-213) to it, so a stage
-// reads the state once and writes it once.
+// nablaQsp compflux.f90:107-157, the AV sensor AV.f90:1-142) for every cell.
+// It serves residual evaluations in every form, with the gradients of all
+// nine variables and the sensor, and the time step's stages of the exact
+// form on small meshes (small_exact_mesh), where it also applies the RK
+// stage update (iterations.f90:88-213).  All other stages run in line_kernel
+// (line_kernel.cuh), which keeps a line's values in registers.
 //
 // Work split: one CTA owns CPB consecutive cells and stages them in shared
 // memory.  Phases, separated by __syncthreads:
 //   A  Lagrange interpolation of every line of solution points to its N+1
 //      flux points (one thread per cell x line index x variable: the xi-
 //      and eta-line of one index share the operator row, so their sums go
-//      through paired FMAs, FFMA2 in the mixed form);
+//      through paired FMAs);
 //   B1 physical flux at the interior flux points (thread per point; the
 //      FP64 and mixed forms form F n0 + G n1 directly along the normal);
 //   B2 Rusanov flux at the 4N face points of each cell (thread per point).
@@ -21,10 +24,10 @@
 //      reference's left/right assignment, so both get the value the
 //      reference scatters to them.  Its loads from global memory are issued
 //      early in the FP64 and mixed forms: the face record before the
-//      staging wait, the neighbour's trace and the normals before B1 (all
-//      after B1 in the exact form);
-//   C  divergence of the flux, gradient of (Bx, By) from the face-averaged
-//      flux-point states, Powell and GLM sources (thread per solution point);
+//      staging wait, the neighbour's trace before B1 (all after B1 in the
+//      exact form);
+//   C  divergence of the flux, gradients from the face-averaged flux-point
+//      states, Powell and GLM sources (thread per solution point);
 //   D  the AV smoothness sensor per cell (residual evaluations only);
 //   E  in a time step, the RK stage update of each point by the thread of
 //      phase C: the RK register slice was staged by TMA with the state, the
@@ -45,13 +48,28 @@ namespace sddc {
 
 constexpr int kMaxN = 6;
 
-// threads per cell: one per face point (4N); the 6-cell tile gives each
-// solution point its own thread where there are more of those (N*N > 4N, N
-// >= 5), so that the residual phase takes one round (the fastest tile of all
-// three forms at N = 5: 64 registers and 6 CTAs per SM in the mixed form)
-__host__ __device__ constexpr int stage_tpc(int n, int cpb) { return cpb == 6 && n * n > 4 * n ? n * n : 4 * n; }
-// threads of a CTA owning cpb cells, rounded up to whole warps
-__host__ __device__ constexpr int stage_threads(int n, int cpb) { return (stage_tpc(n, cpb) * cpb + 31) / 32 * 32; }
+// threads of a CTA owning cpb cells: one per face point (4N a cell), rounded
+// up to whole warps
+__host__ __device__ constexpr int stage_threads(int n, int cpb) { return (4 * n * cpb + 31) / 32 * 32; }
+
+// Cells per CTA of a time step's stages (line_kernel.cuh, 2N threads per
+// cell): one or two warps with few idle lanes.
+__host__ __device__ constexpr int line_tile_cells(int n)
+{
+    return n == 2 ? 8 : n == 3 ? 10 : n == 4 ? 8 : n == 5 ? 6 : 2;
+}
+
+constexpr int kResidCpb = 8;  // cells per CTA of a residual evaluation
+// Time steps of the exact form on meshes of fewer cells than this take the
+// tile kernel with kTileCpb cells per CTA: a line's 2N+2 dependent point
+// fluxes, in unfused operations, are a longer chain than the tile's phases,
+// which shows while the mesh leaves SMs idle.  us per step, tile kernel and
+// line kernel: N = 4, 48^2 cells 58 and 66, 64^2 cells 76 and 74; N = 5,
+// 64^2 cells 152 and 169, 96^2 cells 299 and 290; N = 6, 32^2 cells 78 and 88,
+// 48^2 cells 146 and 103.  (The FP64 and mixed forms are no slower by lines at
+// 8^2 cells: 41 and 41, 38 and 31 at N = 4.)
+constexpr int kTileCpb = 4;
+__host__ __device__ constexpr bool small_exact_mesh(int n, int ncell) { return ncell < (n == 5 ? 5000 : n == 6 ? 1500 : 3500); }
 
 // operators in kernel parameter space (row-major)
 struct Ops {
@@ -61,6 +79,19 @@ struct Ops {
     double HL[kMaxN * (kMaxN - 1)];  // HL[s*(N-1) + l] = hhval_low(l+1, Xs(s+1))
     float Lf[(kMaxN + 1) * kMaxN];
     float Mf[(kMaxN + 1) * kMaxN];
+    // (L, L) and (M, M): operands of paired FMAs as they are read
+    float2 Lp[(kMaxN + 1) * kMaxN];
+    float2 Mp[(kMaxN + 1) * kMaxN];
+    // element k = r*N + s of both operators, in every type
+    __host__ __device__ void set(int k, double l, double m)
+    {
+        L[k] = l;
+        M[k] = m;
+        Lf[k] = (float)l;
+        Mf[k] = (float)m;
+        Lp[k] = make_float2(Lf[k], Lf[k]);
+        Mp[k] = make_float2(Mf[k], Mf[k]);
+    }
 };
 
 // how the stage output is formed from the residual r of the stage input q
@@ -103,8 +134,9 @@ struct StageArgs {
     const CaseParams *cases;
     const double *__restrict__ q_in;   // (9,N,N,NCELL), never written during the stage
     double *q_out;                     // RK output (may be reg_a: FiveStageRk stage 5)
-    const void *__restrict__ t_in;     // face traces of q_in, R[NCELL][4][9][N] (trace_at)
+    const void *__restrict__ t_in;     // face traces of q_in, R[NCELL][4][tfs] (trace_at)
     void *t_out;                       // face traces of q_out (null: not produced)
+    int tfs;                           // stride of a face's record in both
     const double *reg_a;               // RK registers read by this stage
     const double *reg_b;
     const double *reg_c;
@@ -210,13 +242,7 @@ __device__ __forceinline__ void bulk_prefetch_l2(const void *src, unsigned bytes
 template <int N, typename R, bool DIAG> struct Smem {
     static constexpr int NQ = 9 * N * N;
     static constexpr int NP = N + 1;
-    static constexpr int NG = DIAG ? 9 : (sizeof(R) == 4 ? 1 : 2);  // variables of the face-averaged state kept
-    // normals staged in shared memory (the mixed form's time step reads them
-    // from global memory where used)
-    static constexpr bool kStageNrm = DIAG || sizeof(R) == 8;
-    // the mixed form's time step also keeps the block reductions at one slot
-    // per warp and no AV operators (6 CTAs per SM at the 6-cell tile, N = 5)
-    static constexpr bool kLean = !DIAG && sizeof(R) == 4;
+    static constexpr int NG = DIAG ? 9 : 2;  // variables of the face-averaged state kept
     static constexpr int kF = 2 * N * NP * 9;   // R per cell: state then flux at every flux point
     static constexpr int kV = 2 * N * NP * NG;  // R per cell: face-averaged state at every flux point
     static constexpr int kLow = 2 * (N - 1) * (N - 1);
@@ -251,8 +277,12 @@ template <typename R> __device__ __forceinline__ P2<R> splat2(R v)
     return p;
 }
 
-template <typename R> __device__ __forceinline__ P2<R> opL2(const Ops &o, int i) { return splat2<R>(opL<R>(o, i)); }
-template <typename R> __device__ __forceinline__ P2<R> opM2(const Ops &o, int i) { return splat2<R>(opM<R>(o, i)); }
+template <typename R> __device__ __forceinline__ P2<R> opL2(const Ops &o, int i);
+template <> __device__ __forceinline__ P2<double> opL2<double>(const Ops &o, int i) { return splat2<double>(o.L[i]); }
+template <> __device__ __forceinline__ P2<float> opL2<float>(const Ops &o, int i) { return o.Lp[i]; }
+template <typename R> __device__ __forceinline__ P2<R> opM2(const Ops &o, int i);
+template <> __device__ __forceinline__ P2<double> opM2<double>(const Ops &o, int i) { return splat2<double>(o.M[i]); }
+template <> __device__ __forceinline__ P2<float> opM2<float>(const Ops &o, int i) { return o.Mp[i]; }
 
 // local face lf (1..4), face point nfp (1..N) -> flux point (family, line, point)
 // (face2fpconnec, initsetup.f90:347-383)
@@ -269,11 +299,18 @@ __device__ __forceinline__ void face_point(int lf, int nfp, int &fam, int &line,
 
 // face traces of a state, [cell][local face][variable][face point]: the N
 // points of one face, which consecutive lanes read and write, are adjacent.
-// lf is 1-based, nfp0 0-based.
-template <int N> __host__ __device__ __forceinline__ size_t trace_at(size_t cell, int lf, int nfp0, int k)
+// tfs is the face record's stride; lf is 1-based, nfp0 0-based.
+template <int N>
+__host__ __device__ __forceinline__ size_t trace_at(int tfs, size_t cell, int lf, int nfp0, int k)
 {
-    return ((cell * 4 + (size_t)(lf - 1)) * 9 + (size_t)k) * N + (size_t)nfp0;
+    return (cell * 4 + (size_t)(lf - 1)) * tfs + (size_t)(k * N + nfp0);
 }
+// the stride of a context's records in values of elem bytes: 9N rounded up to
+// whole 16-byte units, so that asynchronous copies move a face at a time
+// (6.7% more at N = 5 in the mixed form, none at N = 4).  The allocation-free
+// entry packs its records (stride 9N): its scratch array is fixed.
+__host__ __device__ constexpr int trace_stride(int n, int elem) { return (9 * n * elem + 15) / 16 * 16 / elem; }
+template <int N, typename R> __host__ __device__ constexpr int trace_stride() { return trace_stride(N, sizeof(R)); }
 
 template <typename T> __device__ __forceinline__ T warp_max(T v)
 {
@@ -295,28 +332,21 @@ __device__ __forceinline__ double warp_sum(double v)
 template <int N, int CPB, typename R, bool DIAG> constexpr size_t stage_smem_bytes()
 {
     using S = Smem<N, R, DIAG>;
-    // sQ, sA, sJac; the sensor's sJz and sLow in residual evaluations only
-    size_t d = (size_t)CPB * (2 * S::NQ + MetLayout<N>::kJacPad + (DIAG ? N * N + S::kLow : 0)) +
-               4 * (S::kLean ? stage_threads(N, CPB) / 32 : 32) + (S::kLean ? 0 : 2 * (N - 1) * N);
-    size_t r = (size_t)CPB * (S::kF + S::kV + (S::kStageNrm ? 2 * MetLayout<N>::kFam : 0)) + 2 * (N + 1) * N;
+    // sQ, sA, sJac, the AV operators; the sensor's sJz and sLow in residual
+    // evaluations only
+    size_t d = (size_t)CPB * (2 * S::NQ + MetLayout<N>::kJacPad + (DIAG ? N * N + S::kLow : 0)) + 4 * 32 + 2 * (N - 1) * N;
+    size_t r = (size_t)CPB * (S::kF + S::kV + 2 * MetLayout<N>::kFam) + 2 * (N + 1) * N;
     return d * sizeof(double) + r * sizeof(R);
 }
 
 // CTAs per SM the kernel is compiled for: as many as the 228 KB of shared
 // memory per SM hold (1 KB per CTA is the driver's), but no fewer than 96
-// registers per thread (64 for the 6-cell tile: 6 CTAs of 160 threads at
-// N = 5 in the mixed form, measured faster than 5 CTAs with 80 registers),
-// and at most 8, except for the mixed form's 6-cell tile at N >= 4, which
-// may take what shared memory allows up to the SM's 32 CTAs and 2048
-// threads: 9 CTAs of 96 threads at N = 4 (70 registers; compiled for 8 it
-// took 74, allocated as 80, and held 8; measured 5% faster)
+// registers per thread, and at most 8
 template <int N, int CPB, typename R, bool DIAG> constexpr int stage_min_blocks()
 {
-    constexpr bool kWide = CPB == 6 && sizeof(R) == sizeof(float) && N >= 4;
-    const int bmax = kWide ? (2048 / stage_threads(N, CPB) < 32 ? 2048 / stage_threads(N, CPB) : 32) : 8;
     int b = (int)((228 * 1024) / (stage_smem_bytes<N, CPB, R, DIAG>() + 1024));
-    b = b < 1 ? 1 : (b > bmax ? bmax : b);
-    while (b > 1 && 65536 / (stage_threads(N, CPB) * b) < (CPB == 6 ? 64 : 96)) b--;
+    b = b < 1 ? 1 : (b > 8 ? 8 : b);
+    while (b > 1 && 65536 / (stage_threads(N, CPB) * b) < 96) b--;
     return b;
 }
 
@@ -328,12 +358,7 @@ template <int N, int CPB, typename R, bool DIAG, bool EXACT>
 __device__ __forceinline__ bool stage_tile(const StageArgs &a, const Ops &ops, const int tile)
 {
     constexpr bool EX = EXACT && (sizeof(R) == sizeof(double));
-    // a time step of the forms other than the exact one needs only div B:
-    // the face-averaged state is kept as its contravariant component
-    // Bn = Bx n0 + By n1 at each flux point (this cell's normal), and div B
-    // is the SD divergence of Bn (the same sum as the exact form's
-    // d(Bx)/dx + d(By)/dy, associated differently)
-    constexpr bool kBn = !DIAG && !EX;
+    static_assert(DIAG || EX, "time steps of the other forms run in line_kernel");
     using S = Smem<N, R, DIAG>;
     using ML = MetLayout<N>;
     constexpr int NT = stage_threads(N, CPB);  // whole warps: the reductions use full-warp masks
@@ -347,14 +372,14 @@ __device__ __forceinline__ bool stage_tile(const StageArgs &a, const Ops &ops, c
     double *sJac = sQ + CPB * NQ;                                // [CPB][NJ]
     double *sJz = sJac + CPB * NJ;                               // [CPB][NN]  Jz^2 for the sensor (DIAG)
     double *sLow = sJz + (DIAG ? CPB * NN : 0);                  // [CPB][kLow] (DIAG)
-    constexpr int NWR = S::kLean ? NT / 32 : 32;
+    constexpr int NWR = 32;
     double *sRed = sLow + (DIAG ? CPB * S::kLow : 0);            // [4][NWR] block reductions
     // residual (DIAG); in a time step the RK register, then the output
     double *sA = sRed + 4 * NWR;                                 // [CPB][NQ]
     double *sOpH = sA + CPB * NQ;                                // [N-1][N]  AV projection
-    double *sOpHL = sOpH + (S::kLean ? 0 : (N - 1) * N);         // [N][N-1]  AV prolongation (DIAG)
-    R *sNrm = reinterpret_cast<R *>(sOpHL + (S::kLean ? 0 : N * (N - 1)));  // [CPB][NM] flux-point normals
-    R *sF = sNrm + (S::kStageNrm ? CPB * NM : 0);                // [CPB][2][N][NP][9]
+    double *sOpHL = sOpH + (N - 1) * N;         // [N][N-1]  AV prolongation (DIAG)
+    R *sNrm = reinterpret_cast<R *>(sOpHL + N * (N - 1));  // [CPB][NM] flux-point normals
+    R *sF = sNrm + CPB * NM;                // [CPB][2][N][NP][9]
     R *sV = sF + CPB * S::kF;                                    // [CPB][2][N][NP][NG]
     // operators read with lane-dependent indices live in shared memory
     // (divergent reads of kernel parameters serialise per address)
@@ -381,8 +406,8 @@ __device__ __forceinline__ bool stage_tile(const StageArgs &a, const Ops &ops, c
     // the face record of this thread's face point (a cell has 4N face points
     // and at least 4N threads: one face point per thread at most), loaded
     // before the staging wait (in the exact form with the rest of the face
-    // point's inputs, after B1: measured faster there)
-    static_assert(stage_tpc(N, CPB) >= 4 * N, "one face point per thread at most");
+    // point's inputs, after B1: measured faster there); a thread has one face
+    // point at most
     const bool has_fp = tid < ncl * 4 * N;
     int2 frec = make_int2(0, 0);
     if (!EX && has_fp) frec = __ldg(a.faces + (size_t)c0 * 4 + tid / N);
@@ -416,10 +441,10 @@ __device__ __forceinline__ bool stage_tile(const StageArgs &a, const Ops &ops, c
         sAbort = 0;
         if (bulk) {
             mbar_init(&sBar, 1);
-            mbar_expect_tx(&sBar, (unsigned)(qbytes + mbytes + (S::kStageNrm ? nbytes : 0) + jbytes + (want_ra ? qbytes : 0)));
+            mbar_expect_tx(&sBar, (unsigned)(qbytes + mbytes + nbytes + jbytes + (want_ra ? qbytes : 0)));
             bulk_g2s(sQ, qsrc, (unsigned)qbytes, &sBar);
             if (split) {
-                if (S::kStageNrm) bulk_g2s(sNrm, nsrc, (unsigned)nbytes, &sBar);
+                bulk_g2s(sNrm, nsrc, (unsigned)nbytes, &sBar);
                 bulk_g2s(sJac, jsrc, (unsigned)jbytes, &sBar);
             } else {
                 bulk_g2s(sMetRaw, msrc0, (unsigned)mbytes, &sBar);
@@ -431,7 +456,7 @@ __device__ __forceinline__ bool stage_tile(const StageArgs &a, const Ops &ops, c
         sOpL[k] = opL<R>(ops, k);
         sOpM[k] = opM<R>(ops, k);
     }
-    if constexpr (!S::kLean)
+    if constexpr (DIAG)
         for (int k = tid; k < (N - 1) * N; k += NT) {
             sOpH[k] = ops.H[k];
             sOpHL[k] = ops.HL[k];
@@ -452,7 +477,7 @@ __device__ __forceinline__ bool stage_tile(const StageArgs &a, const Ops &ops, c
         };
         stage_copy(sQ, qsrc, ncl * NQ);
         if (split) {
-            if (S::kStageNrm) stage_copy(sNrm, nsrc, ncl * NM);
+            stage_copy(sNrm, nsrc, ncl * NM);
             stage_copy(sJac, jsrc, ncl * NJ);
         } else {
             stage_copy(sMetRaw, msrc0, ncl * ML::kSize);
@@ -476,7 +501,7 @@ __device__ __forceinline__ bool stage_tile(const StageArgs &a, const Ops &ops, c
         for (int k = tid; k < ncl * ML::kSize; k += NT) {
             const int c = k / ML::kSize, o = k - c * ML::kSize;
             const double v = sMetRaw[k];
-            if (o < NM) { if (S::kStageNrm) sNrm[c * NM + o] = (R)v; }
+            if (o < NM) sNrm[c * NM + o] = (R)v;
             else if (o < NM + NN) sJac[c * NJ + (o - NM)] = v;
         }
         __syncthreads();
@@ -525,16 +550,8 @@ __device__ __forceinline__ bool stage_tile(const StageArgs &a, const Ops &ops, c
             int fam, line, r;
             face_point<N>(lf, nfp, fam, line, r);
             const int kind = frec.y & 0xff;
-            if constexpr (S::kStageNrm) {
-                const R *nrm = sNrm + c * NM + ML::normal(fam, line, r);
-                on0 = nrm[0]; on1 = nrm[1];
-            } else if (split) {
-                const R *gn = reinterpret_cast<const R *>(a.nrm) + (size_t)(c0 + c) * NM + ML::normal(fam, line, r);
-                on0 = __ldg(gn); on1 = __ldg(gn + 1);
-            } else {
-                const double *gn = a.met + (size_t)(c0 + c) * ML::kSize + ML::normal(fam, line, r);
-                on0 = (R)__ldg(gn); on1 = (R)__ldg(gn + 1);
-            }
+            const R *nrm = sNrm + c * NM + ML::normal(fam, line, r);
+            on0 = nrm[0]; on1 = nrm[1];
             if (kind == kFaceProc) {
                 // the received trace, remote point N+1-nfp (procintflux_all.f90:83-99)
                 const R *rv = reinterpret_cast<const R *>(a.proc_recv) + ((size_t)frec.x * N + (N - nfp)) * 9;
@@ -546,7 +563,7 @@ __device__ __forceinline__ bool stage_tile(const StageArgs &a, const Ops &ops, c
                 const int pc = frec.x, plf = (frec.y >> 8) & 0xff;
                 const R *tp = reinterpret_cast<const R *>(a.t_in);
 #pragma unroll
-                for (int k = 0; k < 9; k++) other[k] = tp[trace_at<N>(pc, plf, N - nfp, k)];
+                for (int k = 0; k < 9; k++) other[k] = tp[trace_at<N>(a.tfs, pc, plf, N - nfp, k)];
                 if (kind == kFaceRight) {
                     // the left (partner) cell's normal, from the split array or
                     // the packed record
@@ -570,16 +587,8 @@ __device__ __forceinline__ bool stage_tile(const StageArgs &a, const Ops &ops, c
     // ---- B1: interior flux points (inviscid_flux_interior) ---------------------
     // the normal of family f, line l, flux point r of cell c
     auto normal_at = [&](int c, int f, int l, int r, R &n0, R &n1) {
-        if constexpr (S::kStageNrm) {
-            const R *nrm = sNrm + c * NM + ML::normal(f, l, r);
-            n0 = nrm[0]; n1 = nrm[1];
-        } else if (split) {
-            const R *gn = reinterpret_cast<const R *>(a.nrm) + (size_t)(c0 + c) * NM + ML::normal(f, l, r);
-            n0 = __ldg(gn); n1 = __ldg(gn + 1);
-        } else {
-            const double *gn = a.met + (size_t)(c0 + c) * ML::kSize + ML::normal(f, l, r);
-            n0 = (R)__ldg(gn); n1 = (R)__ldg(gn + 1);
-        }
+        const R *nrm = sNrm + c * NM + ML::normal(f, l, r);
+        n0 = nrm[0]; n1 = nrm[1];
     };
     for (int t = tid; t < ncl * 2 * N * (N - 1); t += NT) {
         const int r = 1 + t % (N - 1), l = (t / (N - 1)) % N, f = (t / ((N - 1) * N)) % 2,
@@ -608,12 +617,8 @@ __device__ __forceinline__ bool stage_tile(const StageArgs &a, const Ops &ops, c
 #pragma unroll
             for (int k = 0; k < 9; k++) vs[k] = q[k];
         } else {
-            if constexpr (kBn) {
-                vs[0] = q[5] * n0 + q[6] * n1;
-            } else {
-                vs[0] = q[5];
-                vs[1] = q[6];
-            }
+            vs[0] = q[5];
+            vs[1] = q[6];
         }
     }
 
@@ -677,13 +682,8 @@ __device__ __forceinline__ bool stage_tile(const StageArgs &a, const Ops &ops, c
 #pragma unroll
             for (int k = 0; k < 9; k++) vs[k] = (R)0.5 * Ql[k] + (R)0.5 * Qr[k];
         } else {
-            const R bxa = (R)0.5 * Ql[5] + (R)0.5 * Qr[5], bya = (R)0.5 * Ql[6] + (R)0.5 * Qr[6];
-            if constexpr (kBn) {
-                vs[0] = bxa * on0 + bya * on1;  // this cell's normal
-            } else {
-                vs[0] = bxa;
-                vs[1] = bya;
-            }
+            vs[0] = (R)0.5 * Ql[5] + (R)0.5 * Qr[5];
+            vs[1] = (R)0.5 * Ql[6] + (R)0.5 * Qr[6];
         }
     }
     __syncthreads();
@@ -724,7 +724,7 @@ __device__ __forceinline__ bool stage_tile(const StageArgs &a, const Ops &ops, c
     for (int t = tid; t < ncl * NN; t += NT) {
         const int i = t % N, j = (t / N) % N, c = t / NN;
         const int cell = c0 + c;
-        const R *met = S::kStageNrm ? sNrm + c * NM : nullptr;  // used only where the normals are staged
+        const R *met = sNrm + c * NM;
         // Jac, or its reciprocal when the split array holds reciprocals (the
         // exact form divides by Jac, as the reference does; the others multiply
         // by 1/Jac, rounded once, on the host or here)
@@ -747,21 +747,9 @@ __device__ __forceinline__ bool stage_tile(const StageArgs &a, const Ops &ops, c
                 for (int k = 0; k < 18; k++) go[k] = 0.0;
             }
         }
-        double divB = 0.0;
-        if constexpr (kBn) {
-            // div B from the contravariant component Bn at the flux points
-            if (a.vismode == 1) {
-                R sx = (R)0, sy = (R)0;
-#pragma unroll
-                for (int r = 0; r < NP; r++) sx = sx + Vx[r * NG] * sOpM[r * N + i];
-#pragma unroll
-                for (int r = 0; r < NP; r++) sy = sy + Vy[r * NG] * sOpM[r * N + j];
-                divB = (double)(sx + sy) * rJ;
-            }
-        }
 #pragma unroll
         for (int g = 0; g < NG; g++) {
-            if (kBn || a.vismode != 1) break;
+            if (a.vismode != 1) break;
             R ax = (R)0, ay = (R)0, bx = (R)0, by = (R)0;
 #pragma unroll
             for (int r = 0; r < NP; r++) {
@@ -794,7 +782,7 @@ __device__ __forceinline__ bool stage_tile(const StageArgs &a, const Ops &ops, c
                 }
             }
         }
-        if constexpr (!kBn) divB = gB[0][0] + gB[1][1];
+        const double divB = gB[0][0] + gB[1][1];
         if constexpr (DIAG) {
             const double d = gB[1][0] - gB[0][1];
             sJz[c * NN + i + N * j] = d * d;
@@ -818,8 +806,7 @@ __device__ __forceinline__ bool stage_tile(const StageArgs &a, const Ops &ops, c
         // compresid.f90:53-78: 1/Jac, Powell 8-wave and GLM sources
         const double *q = sQ + c * NQ + 9 * (i + N * j);
         if constexpr (EX) {
-#pragma unroll
-            for (int k = 0; k < 9; k++) res[k] = res[k] / J;
+            quotients<9>(res, J, res);
         } else {
 #pragma unroll
             for (int k = 0; k < 9; k++) res[k] = res[k] * rJ;
@@ -827,7 +814,9 @@ __device__ __forceinline__ bool stage_tile(const StageArgs &a, const Ops &ops, c
         const double Bx = q[5], By = q[6], Bz = q[7], psi = q[8];
         double ux, uy, uz;
         if constexpr (EX) {
-            ux = q[1] / q[0]; uy = q[2] / q[0]; uz = q[3] / q[0];
+            double uu[3];
+            quotients<3>(q + 1, q[0], uu);
+            ux = uu[0]; uy = uu[1]; uz = uu[2];
         } else {
             const double ri = 1.0 / q[0];
             ux = q[1] * ri; uy = q[2] * ri; uz = q[3] * ri;
@@ -853,13 +842,9 @@ __device__ __forceinline__ bool stage_tile(const StageArgs &a, const Ops &ops, c
         } else {
             // ---- E: the RK stage update of this point (iterations.f90:88-213);
             // the point's state and RK register slot are read by this thread
-            // only, so the output goes to the register slot in place, and in
-            // the float form a float copy over the state slot for phase F
-            // element by element in order: float copy k overwrites bytes of
-            // state element k/2 <= k, already read
+            // only, so the output goes to the register slot in place
             const size_t g = (size_t)cell * NQ + 9 * (i + N * j);
             const int kind = a.rk_kind;
-            R *qf = reinterpret_cast<R *>(sQ + c * NQ + 9 * (i + N * j));
 #pragma unroll
             for (int k = 0; k < 9; k++) {
                 const double qk = q[k], r = res[k];
@@ -876,7 +861,6 @@ __device__ __forceinline__ bool stage_tile(const StageArgs &a, const Ops &ops, c
                 }
                 ap[k] = o;
                 if (a.resid_w) a.resid_w[g + k] = r;
-                if constexpr (sizeof(R) != sizeof(double)) qf[k] = (R)o;
             }
             fence_proxy_async();  // sA is the source of the bulk store below
         }
@@ -996,64 +980,30 @@ __device__ __forceinline__ bool stage_tile(const StageArgs &a, const Ops &ops, c
     // time step nothing between them writes shared memory)
     if (!DIAG && a.t_out) {
         R *to = reinterpret_cast<R *>(a.t_out);
-        // the output state: sA (double), or its float copy over the state
-        // slots (9 floats at the start of each point's 9 doubles)
-        constexpr int PS = sizeof(R) == sizeof(double) ? 9 : 18;  // R per point
-        const R *qo = sizeof(R) == sizeof(double) ? reinterpret_cast<const R *>(qout_src)
-                                                  : reinterpret_cast<const R *>(sQ);
-        if constexpr (sizeof(R) == sizeof(double)) {
-            // one thread per (cell, family, variable, line): the line's N
-            // values give the traces at both of its ends (r = 0 and r = N),
-            // each summed in order as phase A sums them (measured faster than
-            // one thread per face point in the FP64 forms, slower in the mixed)
-            for (int t = tid; t < ncl * 2 * 9 * N; t += NT) {
-                const int line = t % N, k = (t / N) % 9, fam = (t / (9 * N)) % 2, c = t / (18 * N);
-                const R *q = qo + c * (PS * NN) + (fam == 0 ? PS * N * line : PS * line) + k;
-                const int stride = fam == 0 ? PS : PS * N;
-                R qs[N];
+        const R *qo = reinterpret_cast<const R *>(qout_src);
+        // one thread per (cell, family, variable, line): the line's N values
+        // give the traces at both of its ends (r = 0 and r = N), each summed
+        // in order as phase A sums them
+        for (int t = tid; t < ncl * 2 * 9 * N; t += NT) {
+            const int line = t % N, k = (t / N) % 9, fam = (t / (9 * N)) % 2, c = t / (18 * N);
+            const R *q = qo + c * NQ + (fam == 0 ? 9 * N * line : 9 * line) + k;
+            const int stride = fam == 0 ? 9 : 9 * N;
+            R qs[N];
 #pragma unroll
-                for (int s = 0; s < N; s++) qs[s] = q[stride * s];
-                R a0 = (R)0, aN = (R)0;
+            for (int s = 0; s < N; s++) qs[s] = q[stride * s];
+            R a0 = (R)0, aN = (R)0;
 #pragma unroll
-                for (int s = 0; s < N; s++) {
-                    a0 = a0 + qs[s] * sOpL[s];
-                    aN = aN + qs[s] * sOpL[N * N + s];
-                }
-                // the faces at the line's ends (face_point inverted): xi line j
-                // ends on local faces 4 (point N-j) and 2 (point j+1), eta
-                // line i on local faces 1 (point i+1) and 3 (point N-i)
-                const int lf0 = fam == 0 ? 4 : 1, nfp0 = fam == 0 ? N - line : line + 1;
-                const int lfN = fam == 0 ? 2 : 3, nfpN = fam == 0 ? line + 1 : N - line;
-                to[trace_at<N>(c0 + c, lf0, nfp0 - 1, k)] = a0;
-                to[trace_at<N>(c0 + c, lfN, nfpN - 1, k)] = aN;
+            for (int s = 0; s < N; s++) {
+                a0 = a0 + qs[s] * sOpL[s];
+                aN = aN + qs[s] * sOpL[N * N + s];
             }
-        } else {
-            for (int t = tid; t < ncl * 4 * N; t += NT) {  // one thread per face point
-                const int nfp = 1 + t % N, lf = 1 + (t / N) % 4, c = t / (4 * N);
-                int fam, line, r;
-                face_point<N>(lf, nfp, fam, line, r);
-                const R *q = qo + c * (PS * NN) + (fam == 0 ? PS * N * line : PS * line);
-                const int stride = fam == 0 ? PS : PS * N;
-                // variables in pairs (8-byte loads of the float copy, paired FMAs)
-                P2<R> Ls[N];
-#pragma unroll
-                for (int s = 0; s < N; s++) Ls[s] = splat2<R>(sOpL[r * N + s]);
-#pragma unroll
-                for (int k = 0; k < 8; k += 2) {
-                    P2<R> acc = splat2<R>((R)0);
-#pragma unroll
-                    for (int s = 0; s < N; s++)
-                        acc = fma2(*reinterpret_cast<const P2<R> *>(q + k + stride * s), Ls[s], acc);
-                    to[trace_at<N>(c0 + c, lf, nfp - 1, k)] = acc.x;
-                    to[trace_at<N>(c0 + c, lf, nfp - 1, k + 1)] = acc.y;
-                }
-                {
-                    R acc = (R)0;
-#pragma unroll
-                    for (int s = 0; s < N; s++) acc = acc + q[8 + stride * s] * Ls[s].x;
-                    to[trace_at<N>(c0 + c, lf, nfp - 1, 8)] = acc;
-                }
-            }
+            // the faces at the line's ends (face_point inverted): xi line j
+            // ends on local faces 4 (point N-j) and 2 (point j+1), eta
+            // line i on local faces 1 (point i+1) and 3 (point N-i)
+            const int lf0 = fam == 0 ? 4 : 1, nfp0 = fam == 0 ? N - line : line + 1;
+            const int lfN = fam == 0 ? 2 : 3, nfpN = fam == 0 ? line + 1 : N - line;
+            to[trace_at<N>(a.tfs, c0 + c, lf0, nfp0 - 1, k)] = a0;
+            to[trace_at<N>(a.tfs, c0 + c, lfN, nfpN - 1, k)] = aN;
         }
     }
 
@@ -1117,19 +1067,6 @@ __device__ __forceinline__ bool stage_tile(const StageArgs &a, const Ops &ops, c
     return true;
 }
 
-// a batch's stage as a persistent launch: each CTA walks the tile table with
-// a grid stride
-template <int N, int CPB, typename R, bool DIAG, bool EXACT>
-__device__ __forceinline__ void stage_tiles_persistent(const StageArgs &a, const Ops &ops)
-{
-    for (int t = blockIdx.x; t < a.ntiles; t += gridDim.x) {
-        if (!stage_tile<N, CPB, R, DIAG, EXACT>(a, ops, t)) return;
-        __syncthreads();  // tile t's last shared-memory reads before tile t+grid stages
-    }
-}
-
-// One CTA per tile.  The persistent walk is a kernel of its own, so that the
-// one-tile kernel carries no loop state.
 template <int N, int CPB, typename R, bool DIAG, bool EXACT>
 __global__ void __launch_bounds__(stage_threads(N, CPB), (stage_min_blocks<N, CPB, R, DIAG>()))
     stage_kernel(const StageArgs a, const Ops ops)
@@ -1137,22 +1074,14 @@ __global__ void __launch_bounds__(stage_threads(N, CPB), (stage_min_blocks<N, CP
     stage_tile<N, CPB, R, DIAG, EXACT>(a, ops, blockIdx.x);
 }
 
-template <int N, int CPB, typename R, bool DIAG, bool EXACT>
-__global__ void __launch_bounds__(stage_threads(N, CPB), (stage_min_blocks<N, CPB, R, DIAG>()))
-    stage_kernel_persistent(const StageArgs a, const Ops ops)
-{
-    stage_tiles_persistent<N, CPB, R, DIAG, EXACT>(a, ops);
-}
-
-// Face traces of a state: T[trace_at(cell, lf, nfp, k)] = sum_s Q(k, line
+// Face traces of a state: T[trace_at(tfs, cell, lf, nfp, k)] = sum_s Q(k, line
 // points) * L(r, s) at the flux point of local face lf, face point nfp -- the
 // same interpolation, in the same order and type, as phase A and phase F.
 template <int N, typename R, bool EXACT>  // EXACT: compiled with -fmad=false, like phase A
-__global__ void trace_kernel(int ncell, const double *__restrict__ q, R *__restrict__ t, const Ops ops)
+__global__ void trace_kernel(int ncell, const double *__restrict__ q, R *__restrict__ t, int tfs, const Ops ops)
 {
     const size_t n = (size_t)ncell * 4 * N * 9;
     for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
-        // e = trace_at(c, lf, nfp - 1, k)
         const int nfp = 1 + (int)(e % N), k = (int)((e / N) % 9), lf = 1 + (int)((e / (9 * N)) % 4);
         const size_t c = e / (36 * N);
         int fam, line, r;
@@ -1164,7 +1093,7 @@ __global__ void trace_kernel(int ncell, const double *__restrict__ q, R *__restr
             const double x = fam == 0 ? qc[k + 9 * (s + N * line)] : qc[k + 9 * (line + N * s)];
             acc = acc + (R)x * opL<R>(ops, r * N + s);
         }
-        t[e] = acc;
+        t[trace_at<N>(tfs, c, lf, nfp - 1, k)] = acc;
     }
 }
 

@@ -1,0 +1,93 @@
+"""The stage kernel that works by lines (csrc/line_kernel.cuh) at the edges of
+its tiles, and the quotients its exact form takes from one reciprocal."""
+import os
+import shutil
+import subprocess
+
+import numpy as np
+import pytest
+
+import sddc_oracle as O
+from helpers import channel_physics, rel_l2, smooth_state
+from sddc_b200 import cases, host, mesh
+from sddc_b200.solver import Solver
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+NVCC = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+TILE = {2: 8, 3: 10, 4: 8, 5: 6, 6: 2}  # cells per CTA
+
+
+@pytest.mark.skipif(not os.path.exists(NVCC), reason="nvcc not available")
+def test_quotients_round_as_division(tmp_path):
+    exe = str(tmp_path / "quotients_check")
+    subprocess.run([NVCC, "-std=c++17", "-O2", "-gencode", "arch=compute_100a,code=sm_100a", "-Xcompiler",
+                    "-ffp-contract=off", f"-I{os.path.join(os.path.dirname(HERE), 'sddc_b200', 'csrc')}",
+                    os.path.join(HERE, "native", "quotients_check.cu"), "-o", exe], check=True, capture_output=True)
+    r = subprocess.run([exe], capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
+def _case(N, ncell):
+    """A jittered channel with a boundary of another kind on each side."""
+    m = mesh.channel_box(ncell, 1, sides=("WALL", "OUTL", "FREE", "INLE"), jitter=0.0, seed=N)
+    if ncell % 2 == 0:
+        m = mesh.channel_box(ncell // 2, 2, sides=("SYMP", "OUTL", "WALL", "INLE"), jitter=0.2, seed=N)
+    t = host.build_tables(m, N)
+    ph = channel_physics()
+    return t, ph, smooth_state(t, ph, seed=ncell), 0.2 * m.min_edge() / N
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("N", sorted(TILE))
+@pytest.mark.parametrize("k_stage", [3, 5])
+def test_lines_match_oracle_at_tile_edges(N, k_stage):
+    for ncell in sorted({1, 2, TILE[N] - 1, TILE[N], TILE[N] + 1, 3 * TILE[N] + 1}):
+        if ncell < 1:
+            continue
+        t, ph, Q, dt = _case(N, ncell)
+        o = O.Oracle(t, ph)
+        o.set_state(Q)
+        (o.rk_s5p3 if k_stage == 3 else o.five_stage_rk)(dt, 2)
+        ref = o.state()["Q"]
+        mo = o.maxima()
+        # the bars of the parity tests: exact bit for bit, FP64 1e-12, mixed 1e-6
+        for form, bar in (("fp64_exact", 0.0), ("fp64", 1e-12), ("mixed", 1e-6)):
+            s = Solver(t, ph, precision=form, k_stage=k_stage, cells_per_cta=8)
+            s.set_state(Q)
+            s.rk_s5p3(dt, 2)
+            g = s.state()["Q"]
+            if bar:
+                assert rel_l2(g, ref) <= bar, (form, ncell)
+            else:
+                assert np.array_equal(g, ref), ncell
+                mg = s.maxima()
+                assert (mg["eigvmax"], mg["umax"]) == (mo["eigvmax"], mo["umax"])
+            s.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("N", [3, 5])
+def test_both_exact_kernels_agree_with_zeros_and_fault(N):
+    """A state with zero components (their quotients keep the zero), and the
+    step at which the configured Mach number faults: by lines and by tiles
+    the same bits."""
+    c = cases.cylinder_case(8, 16, N, ms=1.5, ma=2.0, noise=0.0)
+    t = host.build_tables(c.mesh, N)
+    Q = c.initial_state(t)
+    dt = cases.cfl_dt(c.mesh, Q, N)
+    out = []
+    for cpb in (4, 8):
+        s = Solver(t, c.physics, precision="fp64_exact", cells_per_cta=cpb)
+        s.set_state(Q)
+        seen = []
+        for _ in range(12):
+            try:
+                s.rk_s5p3(dt, 1)
+                fault = False
+            except RuntimeError:
+                fault = True
+            seen.append((fault, s.state()["Q"].copy()))
+        s.close()
+        out.append(seen)
+    for (fa, qa), (fb, qb) in zip(*out):
+        assert fa == fb and np.array_equal(qa, qb, equal_nan=True)
