@@ -25,6 +25,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <utility>
 #include <vector>
 
 #include "adjoint_kernel.cuh"
@@ -369,22 +370,30 @@ int forward_steps(sddc_ctx *ctx, double dt, int step0, int nsteps, double *const
     return SDDC_OK;
 }
 
-// device buffers of one run, released on every exit path
+// device buffers of one run: named first, then carved from one allocation,
+// which is released on every exit path (a run names several hundred buffers;
+// one cudaMalloc and cudaFree each took nine tenths of a 40-step run at 64x128
+// cells)
 struct RunBufs {
-    std::vector<void *> p;
+    std::vector<std::pair<double **, size_t>> named;  // buffer, doubles
+    void *slab = nullptr;
     size_t bytes = 0;
-    ~RunBufs()
+    ~RunBufs() { cudaFree(slab); }
+    void name(double **out, size_t n)
     {
-        for (void *x : p) cudaFree(x);
+        named.push_back({out, n});
+        bytes += (n * sizeof(double) + 255) / 256 * 256;
     }
-    int get(sddc_ctx *ctx, double **out, size_t n, const char *what)
+    int get(sddc_ctx *ctx, const char *what)
     {
-        int rc = alloc(ctx, (void **)out, n * sizeof(double), what);
-        if (rc == SDDC_OK) {
-            p.push_back(*out);
-            bytes += n * sizeof(double);
+        const int rc = alloc(ctx, &slab, bytes, what);
+        if (rc) return rc;
+        unsigned char *at = static_cast<unsigned char *>(slab);
+        for (auto &b : named) {
+            *b.first = reinterpret_cast<double *>(at);
+            at += (b.second * sizeof(double) + 255) / 256 * 256;
         }
-        return rc;
+        return SDDC_OK;
     }
 };
 
@@ -450,17 +459,17 @@ extern "C" int sddc_adjoint_run(sddc_ctx *ctx, const sddc_adjoint_opts *o, doubl
     RunBufs rb;
     std::vector<double *> ckpt(nseg), S(5 * segmax + 1), T(5 * segmax + 1);
     double *hist = nullptr, *force = nullptr, *cmax = nullptr, *A[6] = {};
-    for (int s = 0; s < nseg; s++)
-        if ((rc = rb.get(ctx, &ckpt[s], nq, "checkpoint"))) return rc;
-    for (int i = 0; i <= 5 * segmax; i++)
-        if ((rc = rb.get(ctx, &S[i], nq, "stage state")) || (rc = rb.get(ctx, &T[i], tr, "stage traces"))) return rc;
-    if ((rc = rb.get(ctx, &hist, 2 * ((size_t)5 * ns + 1), "running maxima")) ||
-        (rc = rb.get(ctx, &force, 2 * ((size_t)ns + 1), "wall force")) ||
-        (rc = rb.get(ctx, &cmax, (size_t)5 * segmax * 2 * ((ctx->ncell + ctx->cpb - 1) / ctx->cpb), "CTA maxima")))
-        return rc;
+    const size_t ncmax = (size_t)5 * segmax * 2 * ((ctx->ncell + ctx->cpb - 1) / ctx->cpb);
+    for (auto &c : ckpt) rb.name(&c, nq);
+    for (int i = 0; i <= 5 * segmax; i++) {
+        rb.name(&S[i], nq);
+        rb.name(&T[i], tr);
+    }
+    rb.name(&hist, 2 * ((size_t)5 * ns + 1));
+    rb.name(&force, 2 * ((size_t)ns + 1));
+    rb.name(&cmax, ncmax);
     if (grad)
-        for (auto &a : A)
-            if ((rc = rb.get(ctx, &a, nq, "adjoint register"))) return rc;
+        for (auto &a : A) rb.name(&a, nq);
     // the reverse sweep recomputes segment s - 1 into a second stage store
     // (with its own per-CTA maxima) on a second stream while it reverses
     // segment s from the first
@@ -468,11 +477,13 @@ extern "C" int sddc_adjoint_run(sddc_ctx *ctx, const sddc_adjoint_opts *o, doubl
     std::vector<double *> S2(overlap ? 5 * segmax + 1 : 0), T2(overlap ? 5 * segmax + 1 : 0);
     double *cmax2 = nullptr;
     if (overlap) {
-        for (int i = 0; i <= 5 * segmax; i++)
-            if ((rc = rb.get(ctx, &S2[i], nq, "stage state")) || (rc = rb.get(ctx, &T2[i], tr, "stage traces"))) return rc;
-        if ((rc = rb.get(ctx, &cmax2, (size_t)5 * segmax * 2 * ((ctx->ncell + ctx->cpb - 1) / ctx->cpb), "CTA maxima")))
-            return rc;
+        for (int i = 0; i <= 5 * segmax; i++) {
+            rb.name(&S2[i], nq);
+            rb.name(&T2[i], tr);
+        }
+        rb.name(&cmax2, ncmax);
     }
+    if ((rc = rb.get(ctx, "checkpoints and stage states"))) return rc;
 
     // streams and events of the overlapped reverse sweep; on every exit the
     // streams are drained (before the run buffers go) and the context's
