@@ -528,13 +528,13 @@ static cudaError_t launch_visc(sddc_ctx *ctx, const double *q_in, const void *t_
     v.fs = Freestream{ctx->p.rinf, ctx->p.pinf, ctx->p.uinf, ctx->p.vinf, ctx->p.bxinf, ctx->p.byinf};
     v.q = q_in;
     v.t_in = t_in;
-    v.tfs = ctx->tfs;
     v.met = ctx->met;
     v.met2 = ctx->met2;
     v.faces = ctx->faces;
     v.grad = ctx->visc_grad;
     v.gt = ctx->visc_gt;
     v.rv = ctx->visc_rv;
+    v.err_flags = ctx->err_flags;
     switch (ctx->p.precision) {
     case SDDC_FP64_EXACT: return launch_visc_exact(ctx->N, v, ctx->ops, ctx->stream);
     case SDDC_FP64: return launch_visc_fp64(ctx->N, v, ctx->ops, ctx->stream);

@@ -103,7 +103,7 @@ struct sddc_ctx {
     // viscous / resistive chain (vismode = 1 with mu or eta0 nonzero)
     bool visc = false;
     double *visc_grad = nullptr;  // nablaQs (9,2,N,N,NCELL)
-    double *visc_gt = nullptr;    // gradient traces [cell][lf][nfp][18]
+    double *visc_gt = nullptr;    // gradient traces [cell][lf][18][nfp]
     double *visc_rv = nullptr;    // dFv + dGv (9,N,N,NCELL)
     double *met2 = nullptr;       // [cell][lf][nfp][2]: the other normal row at each face point
     // restart / Tecplot output (output.cu), created on first use

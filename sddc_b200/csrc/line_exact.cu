@@ -1,6 +1,7 @@
-// The exact FP64 form of the line kernel; one object per N (SDDC_N), SDDC_N = 0 for
+// The exact FP64 form of the kernels by lines; one object per N (SDDC_N), SDDC_N = 0 for
 // the dispatch.
 #define SDDC_R double
 #define SDDC_EXACT_FORM true
 #define SDDC_LINE launch_line_exact
+#define SDDC_VISC launch_visc_exact
 #include "line_launch.inc"

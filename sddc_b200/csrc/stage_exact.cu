@@ -4,6 +4,5 @@
 #define SDDC_EXACT_FORM true
 #define SDDC_LAUNCH launch_stage_exact
 #define SDDC_TRACE launch_trace_exact
-#define SDDC_VISC launch_visc_exact
 #define SDDC_LINE launch_line_exact
 #include "stage_launch.inc"

@@ -1,8 +1,9 @@
 // The viscous / resistive chain of the SDDC residual (vismode = 1 with
 // mu or eta0 nonzero): compflux.f90:36-50 and what it calls.
 //
-// Two launches before each stage launch, both per tile of cells staged in
-// shared memory:
+// Two launches before each stage launch, both with one thread per line of
+// solution points as in line_kernel.cuh (sums in registers, one exchange
+// between the lines that cross at a point):
 //   visc_grad_kernel  face-averaged states at every flux point (interior:
 //                     the interpolated state; faces: (left + right)/2 with
 //                     the neighbour's trace or the boundary ghost state, as
@@ -23,11 +24,20 @@
 //                     the stage kernel adds to the inviscid residual.
 // The AV viscous flux (getVfluxvectors_AV) has its coefficients hard-coded
 // to zero (getrusanov.f90:326,328); it is not formed (it could only change
-// the sign of a zero).  Every expression keeps the reference's order; the
-// exact instantiation is compiled without FMA.
+// the sign of a zero), nor are the first and last viscous flux components,
+// which are zero.  Every sum keeps the reference's order; the exact
+// instantiation is compiled without FMA.
+//
+// What bounds them: latency at 1.4 to 1.8 warps per scheduler (232 and 224
+// registers at N = 4 hold the sums of 18 and 7 values per point of the line;
+// the states and gradients are read from shared memory at every flux point,
+// which keeps the L1 pipe 59% and 49% busy).  At 128x128 cells, N = 4, FP64,
+// they take 38 and 58 us cold; one thread per point and variable, with every
+// operand from shared memory and an IEEE division per quotient, took about
+// 215 together (a step of the chain: 1253 us then, 725 now).
 #pragma once
 
-#include "stage_kernel.cuh"
+#include "line_kernel.cuh"
 
 namespace sddc {
 
@@ -38,71 +48,89 @@ struct ViscArgs {
     int ncell, vismode;
     double mu, eta0;
     Freestream fs;
-    const double *__restrict__ q;     // stage input state
+    const double *q;                  // stage input state
     const void *t_in;                 // its face traces (layout trace_at), in the form's type
-    int tfs;                          // their face record's stride
     const double *__restrict__ met;   // packed metrics
     const double *__restrict__ met2;  // [cell][lf][nfp][2]: S1(2,1:2) or S2(1,1:2) at the face point
     const int2 *__restrict__ faces;
     double *grad;  // nablaQs (9,2,N,N,NCELL)
-    double *gt;    // gradient traces [cell][lf][nfp][18]: (9 x-derivatives, 9 y-derivatives)
+    double *gt;    // gradient traces [cell][lf][18][nfp]: (9 x-derivatives, 9 y-derivatives)
     double *rv;    // dFv + dGv (9,N,N,NCELL)
+    unsigned *err_flags;
 };
 
-constexpr int kViscCpb = 4;
-constexpr int kViscThreads = 128;
-
-// getVfluxvectors (getrusanov.f90:197-294) with viscosity mu and resistivity
-// eta0; nQ = (9 x-derivatives, 9 y-derivatives)
-__device__ __forceinline__ void vflux(const double *Qv, const double *nQ, double mu, double eta0, double *Fv,
-                                      double *Gv)
+// o[k-1] = Fv(k) n0 + Gv(k) n1, k = 1..7, of getVfluxvectors
+// (getrusanov.f90:197-294) with viscosity mu and resistivity eta0; nQ =
+// (9 x-derivatives, 9 y-derivatives)
+template <bool EX>
+__device__ __forceinline__ void vflux(const double *Qv, const double *nQ, double mu, double eta0, double n0, double n1,
+                                      double *o)
 {
-    const double rho = Qv[0], rhou = Qv[1], rhov = Qv[2], rhow = Qv[3], rhoE = Qv[4];
+    const double rho = Qv[0], rhoE = Qv[4];
     const double Bx = Qv[5], By = Qv[6], Bz = Qv[7], psi = Qv[8];
-    const double u = rhou / rho, v = rhov / rho, w = rhow / rho;
+    const double ri = EX ? 0.0 : 1.0 / rho;
+    // quotients by rho
+    auto over_rho = [&](auto &x) {
+        constexpr int n = sizeof(x) / sizeof(double);
+        if constexpr (EX) {
+            quotients<n>(x, rho, x);
+        } else {
+#pragma unroll
+            for (int k = 0; k < n; k++) x[k] = x[k] * ri;
+        }
+    };
+    double vel[3] = {Qv[1], Qv[2], Qv[3]};
+    over_rho(vel);
+    const double u = vel[0], v = vel[1], w = vel[2];
     const double NORM_U = (u * u + v * v) + w * w;
     const double NORM_B = (Bx * Bx + By * By) + Bz * Bz;
-    const double inte = (((rhoE - 0.5 * NORM_U * rho) - 0.5 * NORM_B) - 0.5 * (psi * psi)) / rho;
-    double du[2], dv[2], dw[2], de[2], dBx[2], dBy[2], dBz[2];
+    // the internal energy and the velocity gradients
+    double a[7];
+    a[6] = ((rhoE - 0.5 * NORM_U * rho) - 0.5 * NORM_B) - 0.5 * (psi * psi);
 #pragma unroll
     for (int d = 0; d < 2; d++) {
         const double *g = nQ + 9 * d;
-        const double drho = g[0];
-        du[d] = (g[1] - drho * u) / rho;
-        dv[d] = (g[2] - drho * v) / rho;
-        dw[d] = (g[3] - drho * w) / rho;
-        dBx[d] = g[5];
-        dBy[d] = g[6];
-        dBz[d] = g[7];
-        const double dpsi = g[8];
-        const double dKE = 0.5 * NORM_U * drho + rho * ((u * du[d] + v * dv[d]) + w * dw[d]);
-        const double dpre_B = (Bx * dBx[d] + By * dBy[d]) + Bz * dBz[d];
-        const double dpsi2 = psi * dpsi;
-        de[d] = ((((g[4] - dKE) - dpre_B) - drho * inte) - dpsi2) / rho;
+        a[3 * d] = g[1] - g[0] * u;
+        a[3 * d + 1] = g[2] - g[0] * v;
+        a[3 * d + 2] = g[3] - g[0] * w;
     }
-    const double ux = du[0], uy = du[1], vx = dv[0], vy = dv[1], wx = dw[0], wy = dw[1], ex = de[0], ey = de[1];
-    const double Bxy = dBx[1], Byx = dBy[0], Bzx = dBz[0], Bzy = dBz[1];
-    Fv[0] = 0.0;
-    Fv[1] = mu * (2.0 * ux + kLambdaVisc * (ux + vy));
-    Fv[2] = mu * (vx + uy);
-    Fv[3] = mu * wx;
-    Fv[4] = ((u * Fv[1] + v * Fv[2]) + w * Fv[3]) + mu * kGam * ex / kPrandtl;
-    Gv[0] = 0.0;
-    Gv[1] = mu * (vx + uy);
-    Gv[2] = mu * (2.0 * vy + kLambdaVisc * (ux + vy));
-    Gv[3] = mu * wy;
-    Gv[4] = ((Gv[1] * u + Gv[2] * v) + Gv[3] * w) + mu * kGam * ey / kPrandtl;
+    over_rho(a);
+    const double inte = a[6];
+    double e[2];
+#pragma unroll
+    for (int d = 0; d < 2; d++) {
+        const double *g = nQ + 9 * d;
+        const double dKE = 0.5 * NORM_U * g[0] + rho * ((u * a[3 * d] + v * a[3 * d + 1]) + w * a[3 * d + 2]);
+        const double dpre_B = (Bx * g[5] + By * g[6]) + Bz * g[7];
+        const double dpsi2 = psi * g[8];
+        e[d] = (((g[4] - dKE) - dpre_B) - g[0] * inte) - dpsi2;
+    }
+    over_rho(e);
+    const double ux = a[0], uy = a[3], vx = a[1], vy = a[4], wx = a[2], wy = a[5];
+    const double Bxy = nQ[14], Byx = nQ[6], Bzx = nQ[7], Bzy = nQ[16];
+    const double F1 = mu * (2.0 * ux + kLambdaVisc * (ux + vy)), F2 = mu * (vx + uy), F3 = mu * wx;
+    const double G2 = mu * (2.0 * vy + kLambdaVisc * (ux + vy)), G3 = mu * wy;
+    double h[2] = {mu * kGam * e[0], mu * kGam * e[1]};
+    if constexpr (EX) {
+        quotients<2>(h, kPrandtl, h);
+    } else {
+        h[0] = h[0] * (1.0 / kPrandtl);
+        h[1] = h[1] * (1.0 / kPrandtl);
+    }
+    double F4 = ((u * F1 + v * F2) + w * F3) + h[0];
+    double G4 = ((F2 * u + G2 * v) + G3 * w) + h[1];
     const double Jx = Bzy - 0.0, Jy = 0.0 - Bzx, Jz = Byx - Bxy;
-    Fv[5] = 0.0;
-    Fv[6] = eta0 * Jz;
-    Fv[7] = -(eta0 * Jy);
-    Fv[4] = (Fv[4] + Fv[6] * By) + Fv[7] * Bz;
-    Gv[5] = -(eta0 * Jz);
-    Gv[6] = 0.0;
-    Gv[7] = eta0 * Jx;
-    Gv[4] = (Gv[4] + Gv[5] * Bx) + Gv[7] * Bz;
-    Fv[8] = 0.0;
-    Gv[8] = 0.0;
+    const double F6 = eta0 * Jz, F7 = -(eta0 * Jy);
+    F4 = (F4 + F6 * By) + F7 * Bz;
+    const double G5 = -(eta0 * Jz), G7 = eta0 * Jx;
+    G4 = (G4 + G5 * Bx) + G7 * Bz;
+    o[0] = F1 * n0 + F2 * n1;
+    o[1] = F2 * n0 + G2 * n1;
+    o[2] = F3 * n0 + G3 * n1;
+    o[3] = F4 * n0 + G4 * n1;
+    o[4] = G5 * n1;
+    o[5] = F6 * n0;
+    o[6] = F7 * n0 + G7 * n1;
 }
 
 // internal energy at a face-averaged state (compflux.f90:272-277)
@@ -113,302 +141,497 @@ __device__ __forceinline__ double enei_of(const double *q)
            0.5 * (((q[5] * q[5] + q[6] * q[6]) + q[7] * q[7]) + q[8] * q[8]) / q[0];
 }
 
-template <int N> struct ViscSmem {
-    static constexpr int NQ = 9 * N * N, NP = N + 1, NN = N * N;
-    static constexpr int kF = 2 * N * NP * 9;   // a state or flux at every flux point
-    static constexpr int kG = 2 * N * NP * 18;  // a gradient at every flux point
-    static constexpr int NM = 2 * MetLayout<N>::kFam;
+// Shared memory of both kernels, in doubles: the state slice, the packed
+// metric records, the neighbours' traces (type T), then in the gradient
+// kernel the exchanged sums, which become the gradients, and over the
+// earlier regions the gradients' traces; in the flux kernel the gradients,
+// the neighbours' gradient traces (then the exchanged sums) and, for cells
+// at a wall, the internal-energy gradient.
+template <int N, int CPB, typename T> struct ViscSmem {
+    static constexpr int NQ = 9 * N * N, NN = N * N;
+    static constexpr bool kPad = N % 2 == 0;  // two doubles per cell against bank conflicts
+    static constexpr int QS = kPad ? NQ + 2 : NQ;
+    static constexpr int MS = MetLayout<N>::kSize;
+    static constexpr int TFS = trace_stride<N, T>();
+    static constexpr int TS = 4 * TFS + 16 / (int)sizeof(T);  // in T
+    static constexpr int GF = 18 * N;                          // a face's gradient trace record
+    static constexpr int GTS = 4 * GF + 2;                     // per cell
+    static constexpr int GS = 18 * NN + 2;                     // gradients per cell
+    static constexpr int NX = 7;                               // flux sums exchanged per point
+    static constexpr int kIn = CPB * (QS + MS) + CPB * TS * (int)sizeof(T) / 8;  // doubles of the first three regions
+    static constexpr int kGradIn = kIn > CPB * GTS ? kIn : CPB * GTS;
+    static constexpr size_t kGradBytes = 8 * (size_t)(kGradIn + CPB * GS);
+    static constexpr size_t kFluxBytes = 8 * (size_t)(kIn + CPB * (GS + GTS + 2 * NN));
+    static_assert(NX * NN <= GTS, "the exchanged sums fit the gradient traces' region");
 };
-
-// the staging both kernels share: the state, Jac, the normals, the
-// operators, and the face-averaged state at every flux point (in sV)
-template <int N, typename T>
-__device__ __forceinline__ void visc_stage_states(const ViscArgs &a, const Ops &ops, int c0, int ncl, double *sQ,
-                                                  double *sJac, double *sNrm, double *sL, double *sM, double *sV)
+// cells per CTA: the stage's (at N = 4, 8 cells leave 6 warps per SM and 4
+// cells 7, but with twice the bank conflicts: 38 and 41 us, 58 and 60)
+__host__ __device__ constexpr int visc_cells(int n) { return line_tile_cells(n); }
+template <int N, int CPB, size_t SMEM> constexpr int visc_min_blocks()
 {
-    using ML = MetLayout<N>;
-    using S = ViscSmem<N>;
-    constexpr int NQ = S::NQ, NP = S::NP, NN = S::NN, NM = S::NM, kF = S::kF;
-    const int tid = threadIdx.x;
-    for (int k = tid; k < NP * N; k += kViscThreads) {
-        sL[k] = ops.L[k];
-        sM[k] = ops.M[k];
-    }
-    for (int k = tid; k < ncl * NQ; k += kViscThreads) sQ[k] = __ldg(a.q + (size_t)c0 * NQ + k);
-    for (int k = tid; k < ncl * ML::kSize; k += kViscThreads) {
-        const int c = k / ML::kSize, o = k - c * ML::kSize;
-        const double v = __ldg(a.met + (size_t)c0 * ML::kSize + k);
-        if (o < NM) sNrm[c * NM + o] = v;
-        else if (o < NM + NN) sJac[c * NN + (o - NM)] = v;
-    }
-    __syncthreads();
-    // interpolation to every flux point (inviscid_flux_interior's Qf)
-    for (int t = tid; t < ncl * 2 * N * 9; t += kViscThreads) {
-        const int v = t % 9, l = (t / 9) % N, f = (t / (9 * N)) % 2, c = t / (18 * N);
-        const double *q = sQ + c * NQ;
-        double qs[N];
-#pragma unroll
-        for (int s = 0; s < N; s++) qs[s] = f == 0 ? q[v + 9 * (s + N * l)] : q[v + 9 * (l + N * s)];
-        double *o = sV + c * kF + (f * N + l) * NP * 9 + v;
-#pragma unroll
-        for (int r = 0; r < NP; r++) {
-            double acc = 0.0;
-#pragma unroll
-            for (int s = 0; s < N; s++) acc = acc + qs[s] * sL[r * N + s];
-            o[r * 9] = acc;
-        }
-    }
-    __syncthreads();
-    // face points: (left + right)/2 with the neighbour's trace or the ghost
-    for (int t = tid; t < ncl * 4 * N; t += kViscThreads) {
-        const int nfp = 1 + t % N, lf = 1 + (t / N) % 4, c = t / (4 * N);
-        int fam, line, r;
-        face_point<N>(lf, nfp, fam, line, r);
-        double *slot = sV + c * kF + ((fam * N + line) * NP + r) * 9;
-        double own[9], oth[9];
-#pragma unroll
-        for (int k = 0; k < 9; k++) own[k] = slot[k];
-        const int2 rec = a.faces[(size_t)(c0 + c) * 4 + (lf - 1)];
-        const int kind = rec.y & 0xff;
-        const bool own_right = kind == kFaceRight;
-        if (kind == kFaceLeft || own_right) {
-            const int pc = rec.x, plf = (rec.y >> 8) & 0xff;
-            const T *tp = reinterpret_cast<const T *>(a.t_in);
-#pragma unroll
-            for (int k = 0; k < 9; k++) oth[k] = (double)tp[trace_at<N>(a.tfs, pc, plf, N - nfp, k)];
-        } else {
-            const double *nrm = sNrm + c * NM + ML::normal(fam, line, r);
-            bc_ghost<double, true>(kind, own, nrm[0], nrm[1], a.vismode, a.fs, oth);
-        }
-#pragma unroll
-        for (int k = 0; k < 9; k++) slot[k] = own_right ? 0.5 * oth[k] + 0.5 * own[k] : 0.5 * own[k] + 0.5 * oth[k];
-    }
-    __syncthreads();
+    // 8 warps of 255 registers per SM, more where fewer registers hold a line
+    const int w = (N >= 4 ? 8 : N == 3 ? 12 : 16) / (line_threads(N, CPB) / 32), m = (int)(228 * 1024 / (SMEM + 1280));
+    const int b = w < m ? w : m;
+    return b < 1 ? 1 : b;
 }
+
+// the 18 gradient components of a point in shared memory (16-byte aligned),
+// two at a time
+__device__ __forceinline__ void load18(const double *p, double *g)
+{
+#pragma unroll
+    for (int k = 0; k < 9; k++) {
+        const double2 v = reinterpret_cast<const double2 *>(p)[k];
+        g[2 * k] = v.x;
+        g[2 * k + 1] = v.y;
+    }
+}
+__device__ __forceinline__ void store18(double *p, const double *g)
+{
+#pragma unroll
+    for (int k = 0; k < 9; k++) reinterpret_cast<double2 *>(p)[k] = make_double2(g[2 * k], g[2 * k + 1]);
+}
+
+// what both kernels share: a thread's line, the staging, and the
+// face-averaged state at a flux point of the line
+template <int N, int CPB, typename T> struct ViscTile {
+    using S = ViscSmem<N, CPB, T>;
+    using ML = MetLayout<N>;
+    static constexpr int NT = line_threads(N, CPB);
+    const ViscArgs &a;
+    const Ops &ops;
+    double *sQ, *sMet;
+    T *sT;
+    int c0, ncl, fam, c, l, lf0, lfN, np0, npN;
+    bool act;
+    int2 rec0, recN;
+    unsigned cbytes;
+
+    __device__ __forceinline__ ViscTile(const ViscArgs &a_, const Ops &o_, double *base)
+        : a(a_), ops(o_), sQ(base), sMet(base + CPB * S::QS), sT(reinterpret_cast<T *>(base + CPB * (S::QS + S::MS)))
+    {
+        const int tid = threadIdx.x;
+        c0 = blockIdx.x * CPB;
+        ncl = min(CPB, a.ncell - c0);
+        fam = tid >= N * CPB ? 1 : 0;
+        const int lt = tid - fam * N * CPB, lc = lt % CPB;
+        act = tid < 2 * N * CPB && lc < ncl;
+        c = act ? lc : 0;
+        l = act ? lt / CPB : 0;
+        lf0 = fam == 0 ? 4 : 1;
+        lfN = fam == 0 ? 2 : 3;
+        np0 = fam == 0 ? N - 1 - l : l;
+        npN = fam == 0 ? l : N - 1 - l;
+        rec0 = recN = make_int2(0, 0);
+        if (act) {
+            rec0 = __ldg(a.faces + (size_t)(c0 + c) * 4 + lf0 - 1);
+            recN = __ldg(a.faces + (size_t)(c0 + c) * 4 + lfN - 1);
+        }
+        cbytes = (unsigned)((S::kPad ? 1 : ncl) * S::NQ * sizeof(double));
+    }
+    // bytes of each pair face's record of PER values of type V from src to dst
+    // (cell stride DS), by asynchronous copies
+    template <typename V, int PER, int DS> __device__ __forceinline__ void fetch_faces(V *dst, const V *src)
+    {
+        constexpr int CH = PER * (int)sizeof(V) / 16, E = 16 / (int)sizeof(V), IT = (CPB * 4 * CH + NT - 1) / NT;
+        static_assert(PER * sizeof(V) % 16 == 0, "whole 16-byte units");
+        constexpr int B = IT < 9 ? IT : 9;  // records loaded ahead of their copies
+#pragma unroll 1
+        for (int m0 = 0; m0 < IT; m0 += B) {
+            int2 r[B];
+#pragma unroll
+            for (int m = 0; m < B; m++) {
+                const int f = ((int)threadIdx.x + (m0 + m) * NT) / CH;
+                r[m] = f < ncl * 4 ? __ldg(a.faces + (size_t)c0 * 4 + f) : make_int2(0, 0);
+            }
+#pragma unroll
+            for (int m = 0; m < B; m++) {
+                const int e = (int)threadIdx.x + (m0 + m) * NT, f = e / CH, ch = e - f * CH, kd = r[m].y & 0xff;
+                if (kd == kFaceLeft || kd == kFaceRight)
+                    cp_async16(dst + (f >> 2) * DS + (f & 3) * PER + ch * E,
+                               src + ((size_t)r[m].x * 4 + ((r[m].y >> 8) & 0xff) - 1) * PER + ch * E);
+            }
+        }
+    }
+    // stages the state, the metrics, the traces and (g null: not) the
+    // gradients and their neighbours' traces; false if the copies timed out
+    __device__ __forceinline__ bool stage(const double *g, double *sG, const double *gt, double *sGT)
+    {
+        __shared__ __align__(8) unsigned long long sBar;
+        __shared__ int sAbort;
+        const int tid = threadIdx.x;
+        const double *qsrc = a.q + (size_t)c0 * S::NQ;
+        const bool bulk = (((uintptr_t)qsrc | cbytes) & 15) == 0;
+        if (tid < 32) {
+            if (tid == 0) {
+                sAbort = 0;
+                mbar_init(&sBar, 1);
+                mbar_expect_tx(&sBar, (unsigned)(ncl * (S::MS + (bulk ? S::NQ : 0) + (g ? 18 * S::NN : 0)) * sizeof(double)));
+                bulk_g2s(sMet, a.met + (size_t)c0 * S::MS, (unsigned)(ncl * S::MS * sizeof(double)), &sBar);
+            }
+            __syncwarp();
+            grid_dependency_wait();
+            if (bulk && tid < (S::kPad ? ncl : 1)) bulk_g2s(sQ + tid * S::QS, qsrc + (size_t)tid * S::NQ, cbytes, &sBar);
+            if (g && tid < ncl)
+                bulk_g2s(sG + tid * S::GS, g + (size_t)(c0 + tid) * 18 * S::NN, 18 * S::NN * sizeof(double), &sBar);
+        }
+        grid_dependency_wait();
+        grid_launch_dependents();
+        fetch_faces<T, S::TFS, S::TS>(sT, reinterpret_cast<const T *>(a.t_in));
+        if (g) fetch_faces<double, S::GF, S::GTS>(sGT, gt);
+        if (!bulk)
+            for (int k = tid; k < ncl * S::NQ; k += NT) {
+                const int cc = k / S::NQ;
+                sQ[cc * S::QS + (k - cc * S::NQ)] = qsrc[k];
+            }
+        cp_async_wait_all();
+        if (tid == 0 && !mbar_wait_bounded(&sBar, 0)) {
+            atomicOr(a.err_flags, kErrStagingTimeout);
+            sAbort = 1;
+            mbar_wait_bounded(&sBar, 0);
+        }
+        __syncthreads();
+        return !sAbort;
+    }
+    __device__ __forceinline__ void normal(int r, double &n0, double &n1) const
+    {
+        const double2 n = *reinterpret_cast<const double2 *>(sMet + c * S::MS + ML::normal(fam, l, r));
+        n0 = n.x;
+        n1 = n.y;
+    }
+    // the interpolated state at flux point r
+    __device__ __forceinline__ void own_state(int r, double *q) const
+    {
+        int q0 = c * S::QS + (fam == 0 ? 9 * N * l : 9 * l);
+        asm volatile("" : "+r"(q0));  // read anew at every point: the registers hold sums
+        const int str = fam == 0 ? 9 : 9 * N;
+#pragma unroll
+        for (int k = 0; k < 9; k++) q[k] = 0.0;
+#pragma unroll
+        for (int s = 0; s < N; s++) {
+            const double L = ops.L[r * N + s];
+#pragma unroll
+            for (int k = 0; k < 9; k++) q[k] = q[k] + sQ[q0 + str * s + k] * L;
+        }
+    }
+    // the face-averaged state from the own trace, at the line's end r (0 or N)
+    __device__ __forceinline__ void face_average(int r, double *q) const
+    {
+        const int2 rec = r == 0 ? rec0 : recN;
+        const int lf = r == 0 ? lf0 : lfN, np = r == 0 ? np0 : npN, kind = rec.y & 0xff;
+        double oth[9];
+        if (kind == kFaceLeft || kind == kFaceRight) {
+            const T *tp = sT + c * S::TS + (lf - 1) * S::TFS + (N - 1 - np);
+#pragma unroll
+            for (int k = 0; k < 9; k++) oth[k] = (double)tp[k * N];
+        } else {
+            double n0, n1;
+            normal(r, n0, n1);
+            bc_ghost<double, true>(kind, q, n0, n1, a.vismode, a.fs, oth);
+        }
+#pragma unroll
+        for (int k = 0; k < 9; k++) q[k] = 0.5 * q[k] + 0.5 * oth[k];
+    }
+    // point t of the line, and the parity of the points this thread finishes
+    __device__ __forceinline__ int point(int t) const { return (fam == 0 ? N * l : l) + (fam == 0 ? 1 : N) * t; }
+    __device__ __forceinline__ int parity() const { return (l ^ fam) & 1; }
+};
 
 // ---- gradients at the solution points and their face traces ------------------------
 // T: the trace type of the form (EX and T keep the instantiations of the
 // translation units apart)
-template <int N, bool EX, typename T>
-__global__ void __launch_bounds__(kViscThreads) visc_grad_kernel(const ViscArgs a, const Ops ops)
+template <int N, bool EX, typename T, int CPB>
+__global__ void __launch_bounds__(line_threads(N, CPB), (visc_min_blocks<N, CPB, ViscSmem<N, CPB, T>::kGradBytes>()))
+    visc_grad_kernel(const ViscArgs a, const Ops ops)
 {
+    using S = ViscSmem<N, CPB, T>;
     using ML = MetLayout<N>;
-    using S = ViscSmem<N>;
-    constexpr int NQ = S::NQ, NP = S::NP, NN = S::NN, NM = S::NM, kF = S::kF, CPB = kViscCpb;
+    constexpr int NH = (N + 1) / 2;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    double *sQ = reinterpret_cast<double *>(smem_raw);  // [CPB][NQ]
-    double *sV = sQ + CPB * NQ;                         // [CPB][kF] face-averaged states
-    double *sG = sV + CPB * kF;                         // [CPB][NN][18] gradients
-    double *sJac = sG + CPB * NN * 18;                  // [CPB][NN]
-    double *sNrm = sJac + CPB * NN;                     // [CPB][NM]
-    double *sL = sNrm + CPB * NM;
-    double *sM = sL + NP * N;
-    const int tid = threadIdx.x, c0 = blockIdx.x * CPB, ncl = min(CPB, a.ncell - c0);
-    visc_stage_states<N, T>(a, ops, c0, ncl, sQ, sJac, sNrm, sL, sM, sV);
-    // nablaQsp (compflux.f90:107-157), one thread per (cell, point, variable)
-    for (int t = tid; t < ncl * NN * 9; t += kViscThreads) {
-        const int v = t % 9, i = (t / 9) % N, j = (t / (9 * N)) % N, c = t / (9 * NN);
-        const double *met = sNrm + c * NM;
-        const double J = sJac[c * NN + i + N * j];
-        const double *Vx = sV + c * kF + (0 * N + j) * NP * 9;
-        const double *Vy = sV + c * kF + (1 * N + i) * NP * 9;
-        double g[2];
+    double *base = reinterpret_cast<double *>(smem_raw);
+    double *sX = base + S::kGradIn;  // [CPB][GS]
+    ViscTile<N, CPB, T> t(a, ops, base);
+    if (!t.stage(nullptr, nullptr, nullptr, nullptr)) return;
+
+    // nablaQsp (compflux.f90:107-157): this line's sums
+    double gx[N][9], gy[N][9];
 #pragma unroll
-        for (int d = 0; d < 2; d++) {
-            double aa = 0.0, bb = 0.0;
+    for (int i = 0; i < N; i++)
 #pragma unroll
-            for (int r = 0; r < NP; r++) aa = aa + Vx[r * 9 + v] * sM[r * N + i] * met[ML::normal(0, j, r) + d];
+        for (int k = 0; k < 9; k++) gx[i][k] = gy[i][k] = 0.0;
+    if (t.act) {
+        auto add = [&](int r) {
+            double V[9], n0, n1;
+            t.own_state(r, V);
+            t.normal(r, n0, n1);
+            if (r == 0 || r == N) t.face_average(r, V);
 #pragma unroll
-            for (int r = 0; r < NP; r++) bb = bb + Vy[r * 9 + v] * sM[r * N + j] * met[ML::normal(1, i, r) + d];
-            g[d] = (aa + bb) / J;
+            for (int i = 0; i < N; i++) {
+                const double M = ops.M[r * N + i];
+#pragma unroll
+                for (int k = 0; k < 9; k++) {
+                    const double m = V[k] * M;
+                    gx[i][k] = gx[i][k] + m * n0;
+                    gy[i][k] = gy[i][k] + m * n1;
+                }
+            }
+        };
+        add(0);
+#pragma unroll 1
+        for (int r = 1; r < N; r++) add(r);
+        add(N);
+    }
+    const int par = t.parity();
+    if (t.act) {
+#pragma unroll
+        for (int m = 0; m < NH; m++) {
+            const int i0 = 2 * m, i1 = 2 * m + 1 < N ? 2 * m + 1 : 2 * m;
+            if (2 * m + 1 < N || par) {
+                double o[18];
+#pragma unroll
+                for (int k = 0; k < 9; k++) {
+                    o[k] = par ? gx[i0][k] : gx[i1][k];
+                    o[9 + k] = par ? gy[i0][k] : gy[i1][k];
+                }
+                store18(sX + t.c * S::GS + t.point(2 * m + 1 - par) * 18, o);
+            }
         }
-        sG[(c * NN + i + N * j) * 18 + v] = g[0];
-        sG[(c * NN + i + N * j) * 18 + 9 + v] = g[1];
-        double *go = a.grad + ((size_t)(c0 + c) * NN + i + N * j) * 18;
-        go[v] = g[0];
-        go[9 + v] = g[1];
     }
     __syncthreads();
-    // gradient traces at the face points (grad_trace: the same interpolation)
-    for (int t = tid; t < ncl * 4 * N * 18; t += kViscThreads) {
-        const int k = t % 18, fpt = (t / 18) % (4 * N), c = t / (72 * N);
-        const int nfp = 1 + fpt % N, lf = 1 + fpt / N;
-        int fam, line, r;
-        face_point<N>(lf, nfp, fam, line, r);
-        double acc = 0.0;
+    if (t.act) {
+#pragma unroll
+        for (int m = 0; m < NH; m++) {
+            const int i0 = 2 * m, i1 = 2 * m + 1 < N ? 2 * m + 1 : 2 * m;
+            if (!(2 * m + 1 < N) && par) continue;
+            const int pt = t.point(2 * m + par);
+            double *x = sX + t.c * S::GS + pt * 18;
+            const double J = t.sMet[t.c * S::MS + ML::kJac + pt];
+            double g[18];
+            load18(x, g);
+#pragma unroll
+            for (int k = 0; k < 9; k++) {
+                g[k] = (par ? gx[i1][k] : gx[i0][k]) + g[k];
+                g[9 + k] = (par ? gy[i1][k] : gy[i0][k]) + g[9 + k];
+            }
+            if constexpr (EX) {
+                quotients<18>(g, J, g);
+            } else {
+                const double rJ = 1.0 / J;
+#pragma unroll
+                for (int k = 0; k < 18; k++) g[k] = g[k] * rJ;
+            }
+            store18(x, g);
+        }
+    }
+    fence_proxy_async();
+    __syncthreads();
+    if ((int)threadIdx.x < t.ncl)
+        bulk_s2g(a.grad + (size_t)(t.c0 + threadIdx.x) * 18 * S::NN, sX + threadIdx.x * S::GS, 18 * S::NN * sizeof(double));
+    // the gradients' traces at the line's ends (the same interpolation)
+    if (t.act) {
+        double e0[18], eN[18];
+#pragma unroll
+        for (int k = 0; k < 18; k++) e0[k] = eN[k] = 0.0;
 #pragma unroll
         for (int s = 0; s < N; s++) {
-            const int sp = fam == 0 ? s + N * line : line + N * s;
-            acc = acc + sG[(c * NN + sp) * 18 + k] * sL[r * N + s];
+            double g[18];
+            load18(sX + t.c * S::GS + t.point(s) * 18, g);
+            const double L0 = ops.L[s], LN = ops.L[N * N + s];
+#pragma unroll
+            for (int k = 0; k < 18; k++) {
+                e0[k] = e0[k] + g[k] * L0;
+                eN[k] = eN[k] + g[k] * LN;
+            }
         }
-        a.gt[((size_t)(c0 + c) * 4 * N + fpt) * 18 + k] = acc;
+        double *o0 = base + t.c * S::GTS + (t.lf0 - 1) * S::GF + t.np0, *oN = base + t.c * S::GTS + (t.lfN - 1) * S::GF + t.npN;
+#pragma unroll
+        for (int k = 0; k < 18; k++) {
+            o0[k * N] = e0[k];
+            oN[k * N] = eN[k];
+        }
+    }
+    fence_proxy_async();
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        if ((int)threadIdx.x < t.ncl)
+            bulk_s2g(a.gt + (size_t)(t.c0 + threadIdx.x) * 4 * S::GF, base + threadIdx.x * S::GTS, 4 * S::GF * sizeof(double));
+        bulk_wait_read();
     }
 }
 
 // ---- the viscous flux and its divergence ---------------------------------------------
-template <int N, bool EX, typename T>
-__global__ void __launch_bounds__(kViscThreads) visc_flux_kernel(const ViscArgs a, const Ops ops)
+template <int N, bool EX, typename T, int CPB>
+__global__ void __launch_bounds__(line_threads(N, CPB), (visc_min_blocks<N, CPB, ViscSmem<N, CPB, T>::kFluxBytes>()))
+    visc_flux_kernel(const ViscArgs a, const Ops ops)
 {
-    using ML = MetLayout<N>;
-    using S = ViscSmem<N>;
-    constexpr int NQ = S::NQ, NP = S::NP, NN = S::NN, NM = S::NM, kF = S::kF, kG = S::kG, CPB = kViscCpb;
+    using S = ViscSmem<N, CPB, T>;
+    constexpr int NN = S::NN, NH = (N + 1) / 2, NX = S::NX;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    double *sQ = reinterpret_cast<double *>(smem_raw);  // [CPB][NQ]
-    double *sV = sQ + CPB * NQ;                         // [CPB][kF] face-averaged states
-    double *sFv = sV + CPB * kF;                        // [CPB][kF] viscous flux
-    double *sGf = sFv + CPB * kF;                       // [CPB][kG] gradient at the flux points
-    double *sG = sGf + CPB * kG;                        // [CPB][NN][18] gradients at the solution points
-    double *sDE = sG + CPB * NN * 18;                   // [CPB][NN][2] internal-energy gradient
-    double *sJac = sDE + CPB * NN * 2;                  // [CPB][NN]
-    double *sNrm = sJac + CPB * NN;                     // [CPB][NM]
-    double *sL = sNrm + CPB * NM;
-    double *sM = sL + NP * N;
-    __shared__ int sWall[CPB];
-    const int tid = threadIdx.x, c0 = blockIdx.x * CPB, ncl = min(CPB, a.ncell - c0);
-    if (tid < CPB) {
-        int w = 0;
-        if (tid < ncl)
-            for (int lf = 0; lf < 4; lf++) w |= (a.faces[(size_t)(c0 + tid) * 4 + lf].y & 0xff) == kFaceWall;
-        sWall[tid] = w;
-    }
-    for (int k = tid; k < ncl * NN * 18; k += kViscThreads) sG[k] = __ldg(a.grad + (size_t)c0 * NN * 18 + k);
-    visc_stage_states<N, T>(a, ops, c0, ncl, sQ, sJac, sNrm, sL, sM, sV);
+    double *base = reinterpret_cast<double *>(smem_raw);
+    double *sG = base + S::kIn;         // [CPB][GS] gradients
+    double *sGT = sG + CPB * S::GS;     // [CPB][GTS] neighbours' gradient traces, then exchanged sums
+    double *sDE = sGT + CPB * S::GTS;   // [CPB][NN][2] internal-energy gradient of cells at a wall
+    ViscTile<N, CPB, T> t(a, ops, base);
+    if (!t.stage(a.grad, sG, a.gt, sGT)) return;
+
     // comp_grad_internal_energy (compflux.f90:260-298) for cells with a wall
     // face (the only ones whose values are read)
-    for (int t = tid; t < ncl * NN; t += kViscThreads) {
-        const int i = t % N, j = (t / N) % N, c = t / NN;
-        if (!sWall[c]) continue;
-        double x = 0.0, y = 0.0;
+    bool wall = false;
+    if (t.act)
+        for (int f = 0; f < 4; f++) wall |= (__ldg(a.faces + (size_t)(t.c0 + t.c) * 4 + f).y & 0xff) == kFaceWall;
+    if (__syncthreads_or(wall)) {
+        if (wall) {
+            double de[N];
 #pragma unroll
-        for (int r = 0; r < NP; r++) x = x + enei_of(sV + c * kF + ((0 * N + j) * NP + r) * 9) * sM[r * N + i];
+            for (int i = 0; i < N; i++) de[i] = 0.0;
+#pragma unroll 1
+            for (int r = 0; r <= N; r++) {
+                double V[9];
+                t.own_state(r, V);
+                if (r == 0 || r == N) t.face_average(r, V);
+                const double e = enei_of(V);
 #pragma unroll
-        for (int r = 0; r < NP; r++) y = y + enei_of(sV + c * kF + ((1 * N + i) * NP + r) * 9) * sM[r * N + j];
-        sDE[(c * NN + i + N * j) * 2] = x;
-        sDE[(c * NN + i + N * j) * 2 + 1] = y;
-    }
-    __syncthreads();
-    // the gradient at the interior flux points (nablaQ_interior_FP)
-    for (int t = tid; t < ncl * 2 * N * (N - 1) * 18; t += kViscThreads) {
-        const int k = t % 18, r = 1 + (t / 18) % (N - 1), l = (t / (18 * (N - 1))) % N,
-                  f = (t / (18 * (N - 1) * N)) % 2, c = t / (36 * (N - 1) * N);
-        double acc = 0.0;
-#pragma unroll
-        for (int s = 0; s < N; s++) {
-            const int sp = f == 0 ? s + N * l : l + N * s;
-            acc = acc + sG[(c * NN + sp) * 18 + k] * sL[r * N + s];
-        }
-        sGf[c * kG + ((f * N + l) * NP + r) * 18 + k] = acc;
-    }
-    // the gradient at the face points: the average of both sides' traces
-    // (interfaceVISflux, CYCLOCVISFLUX) or of the trace and the boundary
-    // state (BCVISFLUX)
-    for (int t = tid; t < ncl * 4 * N; t += kViscThreads) {
-        const int nfp = 1 + t % N, lf = 1 + (t / N) % 4, c = t / (4 * N);
-        int fam, line, r;
-        face_point<N>(lf, nfp, fam, line, r);
-        double g[18], o[18];
-#pragma unroll
-        for (int k = 0; k < 18; k++) {
-            double acc = 0.0;
-#pragma unroll
-            for (int s = 0; s < N; s++) {
-                const int sp = fam == 0 ? s + N * line : line + N * s;
-                acc = acc + sG[(c * NN + sp) * 18 + k] * sL[r * N + s];
+                for (int i = 0; i < N; i++) de[i] = de[i] + e * ops.M[r * N + i];
             }
-            g[k] = acc;
+#pragma unroll
+            for (int i = 0; i < N; i++) sDE[(t.c * NN + t.point(i)) * 2 + t.fam] = de[i];
         }
-        const int2 rec = a.faces[(size_t)(c0 + c) * 4 + (lf - 1)];
-        const int kind = rec.y & 0xff;
-        const bool own_right = kind == kFaceRight;
-        double *dst = sGf + c * kG + ((fam * N + line) * NP + r) * 18;
-        if (kind == kFaceLeft || own_right) {
-            const int pc = rec.x, plf = (rec.y >> 8) & 0xff;
-            const double *tp = a.gt + (((size_t)pc * 4 + (plf - 1)) * N + (N - nfp)) * 18;
-#pragma unroll
-            for (int k = 0; k < 18; k++) {
-                const double p = tp[k];
-                dst[k] = own_right ? 0.5 * p + 0.5 * g[k] : 0.5 * g[k] + 0.5 * p;
-            }
-            continue;
-        }
-#pragma unroll
-        for (int k = 0; k < 18; k++) o[k] = g[k];
-        if (kind == kFaceWall) {
-            // adiabatic wall: the boundary energy gradient (bcflux.f90:469-583)
-            const double *q = sQ + c * NQ;
-            double Qfo[9], dxi = 0.0, deta = 0.0;
-#pragma unroll
-            for (int k = 0; k < 9; k++) Qfo[k] = 0.0;
-#pragma unroll
-            for (int s = 0; s < N; s++) {
-                const int sp = fam == 0 ? s + N * line : line + N * s;
-                const double l = sL[r * N + s];
-#pragma unroll
-                for (int k = 0; k < 9; k++) Qfo[k] = Qfo[k] + q[9 * sp + k] * l;
-                dxi = dxi + sDE[(c * NN + sp) * 2] * l;
-                deta = deta + sDE[(c * NN + sp) * 2 + 1] * l;
-            }
-            const double *m2 = a.met2 + (((size_t)(c0 + c) * 4 + (lf - 1)) * N + (nfp - 1)) * 2;
-            const double ur = Qfo[1] / Qfo[0], vr = Qfo[2] / Qfo[0], wr = Qfo[3] / Qfo[0];
-            const double inte = (Qfo[4] / Qfo[0] - 0.5 * ((ur * ur + vr * vr) + wr * wr)) -
-                                0.5 * (((Qfo[5] * Qfo[5] + Qfo[6] * Qfo[6]) + Qfo[7] * Qfo[7]) + Qfo[8] * Qfo[8]) /
-                                    Qfo[0];
-            // dBp of both directions is the first direction's (bcflux.f90:563)
-            const double dBp = ((Qfo[5] * g[5] + Qfo[6] * g[6]) + Qfo[7] * g[7]) + Qfo[8] * g[8];
-#pragma unroll
-            for (int d = 0; d < 2; d++) {
-                const double *gd = g + 9 * d;
-                const double dur = (gd[1] - ur * gd[0]) / Qfo[0];
-                const double dvr = (gd[2] - vr * gd[0]) / Qfo[0];
-                const double dwr = (gd[3] - wr * gd[0]) / Qfo[0];
-                const double dKE =
-                    0.5 * ((ur * ur + vr * vr) + wr * wr) * o[9 * d] + Qfo[0] * ((ur * dur + vr * dvr) + wr * dwr);
-                // the ghost family's other normal row: S1(2,d) on xi faces,
-                // S2(1,d) on eta faces; the energy gradient along it
-                const double tw = fam == 0 ? 2.0 * deta * m2[d] * Qfo[0] : 2.0 * dxi * m2[d] * Qfo[0];
-                o[9 * d + 4] = (((-gd[4] + 2.0 * inte * o[9 * d]) + 2.0 * dKE) + dBp) + tw;
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < 18; k++) dst[k] = 0.5 * g[k] + 0.5 * o[k];
+        __syncthreads();
     }
-    __syncthreads();
-    // the viscous flux at every flux point (comp_viscous_flux)
-    for (int t = tid; t < ncl * 2 * N * NP; t += kViscThreads) {
-        const int r = t % NP, l = (t / NP) % N, f = (t / (NP * N)) % 2, c = t / (2 * N * NP);
-        const int slot = (f * N + l) * NP + r;
-        double Fv[9], Gv[9];
-        vflux(sV + c * kF + slot * 9, sGf + c * kG + slot * 18, a.mu, a.eta0, Fv, Gv);
-        const double *nr = sNrm + c * NM + ML::normal(f, l, r);
-        double *o = sFv + c * kF + slot * 9;
-#pragma unroll
-        for (int k = 0; k < 9; k++) o[k] = Fv[k] * nr[0] + Gv[k] * nr[1];
-    }
-    __syncthreads();
-    // dFv + dGv at the solution points (compresid.f90:14-32)
-    for (int t = tid; t < ncl * NQ; t += kViscThreads) {
-        const int k = t % 9, i = (t / 9) % N, j = (t / (9 * N)) % N, c = t / NQ;
-        const double *Fx = sFv + c * kF + (0 * N + j) * NP * 9 + k;
-        const double *Fy = sFv + c * kF + (1 * N + i) * NP * 9 + k;
-        double dF = 0.0, dG = 0.0;
-#pragma unroll
-        for (int r = 0; r < NP; r++) dF = dF + Fx[r * 9] * sM[r * N + i];
-#pragma unroll
-        for (int r = 0; r < NP; r++) dG = dG + Fy[r * 9] * sM[r * N + j];
-        a.rv[(size_t)c0 * NQ + t] = dF + dG;
-    }
-}
 
-template <int N> constexpr size_t visc_grad_smem()
-{
-    using S = ViscSmem<N>;
-    return sizeof(double) * ((size_t)kViscCpb * (S::NQ + S::kF + 18 * S::NN + S::NN + S::NM) + 2 * S::NP * N);
-}
-template <int N> constexpr size_t visc_flux_smem()
-{
-    using S = ViscSmem<N>;
-    return sizeof(double) *
-           ((size_t)kViscCpb * (S::NQ + 2 * S::kF + S::kG + 18 * S::NN + 2 * S::NN + S::NN + S::NM) + 2 * S::NP * N);
+    double d[N][NX];
+#pragma unroll
+    for (int i = 0; i < N; i++)
+#pragma unroll
+        for (int k = 0; k < NX; k++) d[i][k] = 0.0;
+    if (t.act) {
+        auto add = [&](int r) {
+            double V[9], g[18], n0, n1;
+            t.own_state(r, V);
+            t.normal(r, n0, n1);
+            {
+                int g0 = t.c * S::GS + t.point(0) * 18;
+                asm volatile("" : "+r"(g0));  // read anew at every point
+                const int str = t.fam == 0 ? 18 : 18 * N;
+#pragma unroll
+                for (int k = 0; k < 18; k++) g[k] = 0.0;
+#pragma unroll
+                for (int s = 0; s < N; s++) {
+                    const double L = ops.L[r * N + s];
+                    double x[18];
+                    load18(sG + g0 + str * s, x);
+#pragma unroll
+                    for (int k = 0; k < 18; k++) g[k] = g[k] + x[k] * L;
+                }
+            }
+            if (r == 0 || r == N) {
+                // the average of both sides' gradients (interfaceVISflux,
+                // CYCLOCVISFLUX), or of the own and the boundary's (BCVISFLUX)
+                const int2 rec = r == 0 ? t.rec0 : t.recN;
+                const int lf = r == 0 ? t.lf0 : t.lfN, np = r == 0 ? t.np0 : t.npN, kind = rec.y & 0xff;
+                if (kind == kFaceLeft || kind == kFaceRight) {
+                    const double *tp = sGT + t.c * S::GTS + (lf - 1) * S::GF + (N - 1 - np);
+#pragma unroll
+                    for (int k = 0; k < 18; k++) g[k] = 0.5 * g[k] + 0.5 * tp[k * N];
+                } else {
+                    double o4[2] = {g[4], g[13]};
+                    if (kind == kFaceWall) {
+                        // adiabatic wall: the boundary energy gradient
+                        // (bcflux.f90:469-583); V is still the own trace
+                        double dxi = 0.0, deta = 0.0;
+#pragma unroll
+                        for (int s = 0; s < N; s++) {
+                            const double *de = sDE + (t.c * NN + t.point(s)) * 2;
+                            dxi = dxi + de[0] * ops.L[r * N + s];
+                            deta = deta + de[1] * ops.L[r * N + s];
+                        }
+                        const double *m2 = a.met2 + (((size_t)(t.c0 + t.c) * 4 + (lf - 1)) * N + np) * 2;
+                        const double ur = V[1] / V[0], vr = V[2] / V[0], wr = V[3] / V[0];
+                        const double inte = (V[4] / V[0] - 0.5 * ((ur * ur + vr * vr) + wr * wr)) -
+                                            0.5 * (((V[5] * V[5] + V[6] * V[6]) + V[7] * V[7]) + V[8] * V[8]) / V[0];
+                        // dBp of both directions is the first direction's (bcflux.f90:563)
+                        const double dBp = ((V[5] * g[5] + V[6] * g[6]) + V[7] * g[7]) + V[8] * g[8];
+#pragma unroll
+                        for (int e = 0; e < 2; e++) {
+                            const double *gd = g + 9 * e;
+                            const double dur = (gd[1] - ur * gd[0]) / V[0];
+                            const double dvr = (gd[2] - vr * gd[0]) / V[0];
+                            const double dwr = (gd[3] - wr * gd[0]) / V[0];
+                            const double dKE =
+                                0.5 * ((ur * ur + vr * vr) + wr * wr) * gd[0] + V[0] * ((ur * dur + vr * dvr) + wr * dwr);
+                            // the ghost family's other normal row: S1(2,e) on xi
+                            // faces, S2(1,e) on eta faces; the energy gradient along it
+                            const double tw = t.fam == 0 ? 2.0 * deta * m2[e] * V[0] : 2.0 * dxi * m2[e] * V[0];
+                            o4[e] = (((-gd[4] + 2.0 * inte * gd[0]) + 2.0 * dKE) + dBp) + tw;
+                        }
+                    }
+                    // the other components' boundary gradients are the own ones
+                    const double g4 = g[4], g13 = g[13];
+#pragma unroll
+                    for (int k = 0; k < 18; k++) g[k] = 0.5 * g[k] + 0.5 * g[k];
+                    g[4] = 0.5 * g4 + 0.5 * o4[0];
+                    g[13] = 0.5 * g13 + 0.5 * o4[1];
+                }
+                t.face_average(r, V);
+            }
+            double o[NX];
+            vflux<EX>(V, g, a.mu, a.eta0, n0, n1, o);
+#pragma unroll
+            for (int i = 0; i < N; i++) {
+                const double M = ops.M[r * N + i];
+#pragma unroll
+                for (int k = 0; k < NX; k++) d[i][k] = d[i][k] + o[k] * M;
+            }
+        };
+        add(0);
+#pragma unroll 1
+        for (int r = 1; r < N; r++) add(r);
+        add(N);
+    }
+    __syncthreads();  // the gradient traces and the states are read
+    const int par = t.parity();
+    double *sX = sGT;
+    if (t.act) {
+#pragma unroll
+        for (int m = 0; m < NH; m++) {
+            const int i0 = 2 * m, i1 = 2 * m + 1 < N ? 2 * m + 1 : 2 * m;
+            if (2 * m + 1 < N || par) {
+                double *o = sX + t.c * S::GTS + t.point(2 * m + 1 - par) * NX;
+#pragma unroll
+                for (int k = 0; k < NX; k++) o[k] = par ? d[i0][k] : d[i1][k];
+            }
+        }
+    }
+    __syncthreads();
+    if (t.act) {
+#pragma unroll
+        for (int m = 0; m < NH; m++) {
+            const int i0 = 2 * m, i1 = 2 * m + 1 < N ? 2 * m + 1 : 2 * m;
+            if (!(2 * m + 1 < N) && par) continue;
+            const int pt = t.point(2 * m + par);
+            const double *x = sX + t.c * S::GTS + pt * NX;
+            double *o = t.sQ + t.c * S::QS + 9 * pt;
+            o[0] = 0.0;
+#pragma unroll
+            for (int k = 0; k < NX; k++) o[1 + k] = (par ? d[i1][k] : d[i0][k]) + x[k];
+            o[8] = 0.0;
+        }
+    }
+    fence_proxy_async();
+    __syncthreads();
+    double *dst = a.rv + (size_t)t.c0 * S::NQ;
+    if ((((uintptr_t)dst | t.cbytes) & 15) == 0) {
+        if (threadIdx.x < 32) {
+            if ((int)threadIdx.x < (S::kPad ? t.ncl : 1))
+                bulk_s2g(dst + (size_t)threadIdx.x * S::NQ, t.sQ + threadIdx.x * S::QS, t.cbytes);
+            bulk_wait_read();
+        }
+    } else {
+        for (int k = threadIdx.x; k < t.ncl * S::NQ; k += line_threads(N, CPB)) {
+            const int cc = k / S::NQ;
+            dst[k] = t.sQ[cc * S::QS + (k - cc * S::NQ)];
+        }
+    }
 }
 
 }  // namespace sddc
