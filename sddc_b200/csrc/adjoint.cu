@@ -302,13 +302,10 @@ int reverse_stage(sddc_ctx *ctx, const RevStage &s)
 
 int adjoint_flags(sddc_ctx *ctx)
 {
-    CKA(cudaMemcpyAsync(ctx->adj->host, ctx->err_flags, sizeof(unsigned), cudaMemcpyDeviceToHost, ctx->stream));
     CKA(cudaStreamSynchronize(ctx->stream));
-    unsigned f;
-    std::memcpy(&f, ctx->adj->host, sizeof(unsigned));
+    const unsigned f = *(volatile unsigned *)ctx->err_flags;
     if (f & (kErrAdjointMaxLost | kErrAdjointRecords)) {
-        CKA(cudaMemsetAsync(ctx->err_flags, 0, sizeof(unsigned), ctx->stream));
-        CKA(cudaStreamSynchronize(ctx->stream));
+        take_flags(ctx);
         if (f & kErrAdjointRecords) return set_err(ctx, SDDC_ENUMERIC, "adjoint: more points attain a running maximum than the record buffer holds");
         return set_err(ctx, SDDC_ENUMERIC, "adjoint: no point reproduces a recorded running maximum");
     }

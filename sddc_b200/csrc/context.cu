@@ -148,22 +148,29 @@ int sddc::cuda_err(sddc_ctx *c, cudaError_t e, const char *what)
 
 extern "C" const char *sddc_last_error(const sddc_ctx *ctx) { return ctx ? ctx->err.c_str() : "NULL context"; }
 
+static void drop_graphs(sddc_ctx *ctx)
+{
+    for (auto &slot : ctx->graph)
+        for (auto &g : slot) {
+            if (g.exec) cudaGraphExecDestroy(g.exec);
+            g = {};
+        }
+    ctx->stepped_dt = -1.0;
+}
+
 static void free_all(sddc_ctx *ctx)
 {
     output_free(ctx);
-    for (auto &g : ctx->graph)
-        if (g) {
-            cudaGraphExecDestroy(g);
-            g = nullptr;
-        }
+    drop_graphs(ctx);
     for (auto &r : ctx->reg) cudaFree(r), r = nullptr;
     for (auto &t : ctx->trace) cudaFree(t), t = nullptr;
     void *bufs[] = {ctx->met, ctx->nrm, ctx->jac, ctx->faces, ctx->maxima, ctx->sm_ind, ctx->muav, ctx->resid, ctx->grad,
-                    ctx->mon_part, ctx->mon_out, ctx->int_part, ctx->wq, ctx->err_flags,
+                    ctx->mon_part, ctx->mon_out, ctx->int_part, ctx->wq,
                     ctx->case_dev, ctx->tiles_rk, ctx->tiles_diag, ctx->visc_grad, ctx->visc_gt,
                     ctx->visc_rv, ctx->met2, ctx->max_scratch, ctx->proc_cells};
     for (void *b : bufs) cudaFree(b);
     if (ctx->host_small) cudaFreeHost(ctx->host_small);
+    if (ctx->err_flags) cudaFreeHost(ctx->err_flags);
     adjoint_free(ctx);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
 }
@@ -243,8 +250,7 @@ extern "C" int sddc_create(sddc_ctx **out, const sddc_params *p)
         (rc = alloc(ctx, (void **)&ctx->mon_part, (size_t)mon_blocks * 2 * sizeof(double), "monitor")) ||
         (rc = alloc(ctx, (void **)&ctx->mon_out, 4 * sizeof(double), "monitor")) ||
         (rc = alloc(ctx, (void **)&ctx->int_part, 1024 * 2 * sizeof(double), "integrals")) ||
-        (rc = alloc(ctx, (void **)&ctx->wq, kMaxN * sizeof(double), "weights")) ||
-        (rc = alloc(ctx, (void **)&ctx->err_flags, sizeof(unsigned), "flags")))
+        (rc = alloc(ctx, (void **)&ctx->wq, kMaxN * sizeof(double), "weights")))
         return rc;
     // the viscous chain runs only with vismode = 1 (compflux.f90:36)
     ctx->visc = p->vismode == 1 && (p->mu != 0.0 || p->eta0 != 0.0);
@@ -256,8 +262,9 @@ extern "C" int sddc_create(sddc_ctx **out, const sddc_params *p)
             return rc;
     }
     CK(cudaMallocHost((void **)&ctx->host_small, 64 * sizeof(double)));
+    CK(cudaMallocHost((void **)&ctx->err_flags, sizeof(unsigned)));
+    *ctx->err_flags = 0;
     CK(cudaMemsetAsync(ctx->maxima, 0, kSlots * 2 * sizeof(double), ctx->stream));
-    CK(cudaMemsetAsync(ctx->err_flags, 0, sizeof(unsigned), ctx->stream));
     CK(cudaMemsetAsync(ctx->sm_ind, 0, nc * 2 * sizeof(double), ctx->stream));
     CK(cudaMemsetAsync(ctx->mon_part, 0, (size_t)mon_blocks * 2 * sizeof(double), ctx->stream));
 
@@ -374,6 +381,7 @@ extern "C" int sddc_set_tables(sddc_ctx *ctx, const double *Lmat, const double *
     CK(cudaMemcpyAsync(ctx->jac, jac.data(), jac.size() * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(ctx->faces, fr.data(), fr.size() * sizeof(int2), cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
+    drop_graphs(ctx);  // their launches hold the operators
     ctx->tables = true;
     ctx->traces_stale = true;
     ctx->proc_stale = true;
@@ -583,15 +591,17 @@ static int proc_ready(sddc_ctx *ctx)
     return SDDC_OK;
 }
 
+unsigned sddc::take_flags(sddc_ctx *ctx)
+{
+    const unsigned f = *(volatile unsigned *)ctx->err_flags;
+    if (f) *ctx->err_flags = 0;
+    return f;
+}
+
 int sddc::check_flags(sddc_ctx *ctx)
 {
-    CK(cudaMemcpyAsync(ctx->host_small, ctx->err_flags, sizeof(unsigned), cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
-    unsigned f;
-    std::memcpy(&f, ctx->host_small, sizeof(unsigned));
-    if (f) {
-        CK(cudaMemsetAsync(ctx->err_flags, 0, sizeof(unsigned), ctx->stream));
-        CK(cudaStreamSynchronize(ctx->stream));
+    if (const unsigned f = take_flags(ctx)) {
         std::string m = "device numerics:";
         if (f & kErrNonPositiveDensity) m += " non-positive density";
         if (f & kErrNonFiniteWaveSpeed) m += " non-finite wave speed";
@@ -628,7 +638,6 @@ extern "C" int sddc_compresid(sddc_ctx *ctx)
     ctx->slot = a.slot_w;
     ctx->sensor_stale = false;
     ctx->mon_nblk = ctx->ncase ? ctx->ntiles_diag : (ctx->ncell + kResidCpb - 1) / kResidCpb;
-    CK(cudaStreamSynchronize(ctx->stream));
     return check_flags(ctx);
 }
 
@@ -726,36 +735,47 @@ static int run_steps(sddc_ctx *ctx, double dt, int nsteps)
         CK(cudaStreamSynchronize(ctx->stream));
         return check_flags(ctx);
     }
-    for (int s = 0; s < nsteps; s++) {
+    // Steps replay a graph of 1 or of kGraphSteps steps.  The first step with a
+    // dt runs eagerly (kernel attributes, warm-up; a dt that changes from call
+    // to call never pays for a capture); a graph is captured when its steps
+    // come a second time, in the same call or in a later one.
+    const double seen = ctx->stepped_dt;
+    for (int s = 0; s < nsteps;) {
         const int s0 = ctx->slot;
-        cudaGraphExec_t &g = ctx->graph[s0];
-        if (g && ctx->graph_dt[s0] != dt) {
-            cudaGraphExecDestroy(g);
-            g = nullptr;
+        const bool warm = s > 0 || seen == dt;
+        const int many = warm && nsteps - s >= kGraphSteps ? 1 : 0;
+        const int n = many ? kGraphSteps : 1;
+        sddc_ctx::StepGraph &g = ctx->graph[s0][many];
+        if (g.exec && g.dt != dt) {
+            cudaGraphExecDestroy(g.exec);
+            g = {};
         }
-        if (!g && s > 0) {  // first step of a call runs eagerly (kernel attributes, warm-up)
+        if (!g.exec && warm) {
             cudaGraph_t graph;
             CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
-            cudaError_t e = enqueue_step(ctx, dt, s0);
+            cudaError_t e = cudaSuccess;
+            for (int k = 0; k < n && e == cudaSuccess; k++) e = enqueue_step(ctx, dt, s0);
             cudaError_t e2 = cudaStreamEndCapture(ctx->stream, &graph);
             if (e != cudaSuccess) return cuda_err(ctx, e, "stage launch (capture)");
             if (e2 != cudaSuccess) return cuda_err(ctx, e2, "cudaStreamEndCapture");
-            e = cudaGraphInstantiate(&g, graph, 0);
+            e = cudaGraphInstantiate(&g.exec, graph, 0);
             cudaGraphDestroy(graph);
             if (e != cudaSuccess) return cuda_err(ctx, e, "cudaGraphInstantiate");
-            ctx->graph_dt[s0] = dt;
+            g.dt = dt;
         }
-        if (g) {
-            CK(cudaGraphLaunch(g, ctx->stream));
+        if (g.exec) {
+            CK(cudaGraphLaunch(g.exec, ctx->stream));
         } else {
             cudaError_t e = enqueue_step(ctx, dt, s0);
             if (e != cudaSuccess) return cuda_err(ctx, e, "stage launch");
         }
-        ctx->ctime += dt;  // ctime = ctime0 + dt after the last stage (iterations.f90:211)
+        // ctime = ctime0 + dt after the last stage (iterations.f90:211)
+        for (int k = 0; k < n; k++) ctx->ctime += dt;
+        s += n;
+        ctx->stepped_dt = dt;
         ctx->sensor_stale = true;
         ctx->mon_nblk = ctx->ncase ? ctx->ntiles_rk : ctx->grid;
     }
-    CK(cudaStreamSynchronize(ctx->stream));
     return check_flags(ctx);
 }
 
@@ -947,11 +967,7 @@ extern "C" int sddc_set_cases(sddc_ctx *ctx, int ncase, const sddc_case *cases)
         return rc;
     CK(cudaMemsetAsync(ctx->maxima, 0, (size_t)ncase * kSlots * 2 * sizeof(double), ctx->stream));
     CK(cudaMemsetAsync(ctx->mon_part, 0, (size_t)nmon * 2 * sizeof(double), ctx->stream));
-    for (auto &g : ctx->graph)
-        if (g) {
-            cudaGraphExecDestroy(g);
-            g = nullptr;
-        }
+    drop_graphs(ctx);
     CK(cudaStreamSynchronize(ctx->stream));
     ctx->state = false;  // the maxima were reset: set the state again
     ctx->mon_nblk = 0;
@@ -968,11 +984,7 @@ extern "C" int sddc_set_persistent(sddc_ctx *ctx, int on)
             (rc = build_tiles(ctx, kResidCpb, &ctx->tiles_diag, &ctx->ntiles_diag)))
             return rc;
     }
-    for (auto &g : ctx->graph)
-        if (g) {
-            cudaGraphExecDestroy(g);
-            g = nullptr;
-        }
+    drop_graphs(ctx);
     CK(cudaStreamSynchronize(ctx->stream));
     return SDDC_OK;
 }

@@ -32,6 +32,7 @@ cudaError_t launch_visc_mixed(int N, const ViscArgs &a, const Ops &ops, cudaStre
 namespace sddc {
 
 constexpr int kSlots = 5;     // rotating running-max slots
+constexpr int kGraphSteps = 8;  // time steps of the longer graph (a small mesh's step takes about 35 us)
 constexpr int kRegs = 6;      // RK registers (FiveStageRk needs six)
 constexpr int kMonThreads = 256;
 
@@ -73,6 +74,8 @@ struct sddc_ctx {
     double *maxima = nullptr;  // [sddc::kSlots][2]
     double *sm_ind = nullptr, *muav = nullptr, *resid = nullptr, *grad = nullptr;
     double *mon_part = nullptr, *mon_out = nullptr, *int_part = nullptr, *wq = nullptr;
+    // numerical faults, OR-ed by the kernels: pinned host memory, so that the
+    // host reads them after a synchronisation without a copy
     unsigned *err_flags = nullptr;
     double *host_small = nullptr;  // pinned scratch for small read-backs
     Ops ops{};
@@ -89,8 +92,12 @@ struct sddc_ctx {
     bool tables = false, state = false;
     bool traces_stale = true;  // trace[0] does not match reg[0] yet
     double ctime = 0.0;
-    cudaGraphExec_t graph[sddc::kSlots] = {};
-    double graph_dt[sddc::kSlots] = {};
+    struct StepGraph {
+        cudaGraphExec_t exec = nullptr;
+        double dt = 0.0;
+    };
+    StepGraph graph[sddc::kSlots][2];  // by the slot a step starts from: one step, kGraphSteps steps
+    double stepped_dt = -1.0;          // dt of the last step run (-1: none since the graphs were dropped)
     // batch of independent cases (sddc_set_cases); ncase == 0 for one case
     int ncase = 0;
     std::vector<sddc_case> cases;
@@ -124,7 +131,8 @@ SDDC_INTERNAL int set_err(sddc_ctx *c, int code, const std::string &m);
 SDDC_INTERNAL int cuda_err(sddc_ctx *c, cudaError_t e, const char *what);
 SDDC_INTERNAL int alloc(sddc_ctx *ctx, void **p, size_t bytes, const char *what);
 SDDC_INTERNAL int ready(sddc_ctx *ctx);
-SDDC_INTERNAL int check_flags(sddc_ctx *ctx);
+SDDC_INTERNAL int check_flags(sddc_ctx *ctx);  // synchronises the stream
+SDDC_INTERNAL unsigned take_flags(sddc_ctx *ctx);  // reads and clears, after a synchronisation
 SDDC_INTERNAL int met_size(int N);
 SDDC_INTERNAL StageArgs base_args(sddc_ctx *ctx);
 SDDC_INTERNAL void adjoint_free(sddc_ctx *ctx);

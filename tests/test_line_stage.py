@@ -1,5 +1,6 @@
 """The stage kernel that works by lines (csrc/line_kernel.cuh) at the edges of
 its tiles, and the quotients its exact form takes from one reciprocal."""
+import dataclasses
 import os
 import shutil
 import subprocess
@@ -63,6 +64,46 @@ def test_lines_match_oracle_at_tile_edges(N, k_stage):
                 mg = s.maxima()
                 assert (mg["eigvmax"], mg["umax"]) == (mo["eigvmax"], mo["umax"])
             s.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("N", sorted(TILE))
+def test_viscous_lines_match_oracle_at_tile_edges(N):
+    for ncell in sorted({1, 2, TILE[N] + 1, 2 * TILE[N]}):
+        t, ph, Q, dt = _case(N, ncell)
+        ph = dataclasses.replace(ph, mu=0.02, eta0=0.015)
+        o = O.Oracle(t, ph)
+        o.set_state(Q)
+        o.rk_s5p3(0.2 * dt, 1)
+        ref = o.state()["Q"]
+        for form, bar in (("fp64_exact", 0.0), ("fp64", 1e-12), ("mixed", 1e-6)):
+            s = Solver(t, ph, precision=form, cells_per_cta=8)
+            s.set_state(Q)
+            s.rk_s5p3(0.2 * dt, 1)
+            g = s.state()["Q"]
+            assert np.array_equal(g, ref) if not bar else rel_l2(g, ref) <= bar, (form, ncell)
+            s.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("form", ["fp64_exact", "fp64", "mixed"])
+def test_steps_in_any_grouping_are_the_same(form):
+    """Single steps (eager, then a graph), a graph of several steps, and a dt
+    that changes in between: the same states, maxima and time."""
+    t, ph, Q, dt = _case(4, 40)
+    out = []
+    for groups in ([1] * 23, [23], [2, 11, 1, 9]):
+        s = Solver(t, ph, precision=form)
+        s.set_state(Q)
+        for n in groups:
+            s.rk_s5p3(dt, n)
+        s.rk_s5p3(0.5 * dt, 1)
+        s.rk_s5p3(0.5 * dt, 2)
+        s.rk_s5p3(dt, 1)
+        out.append((s.state()["Q"].copy(), s.maxima(), s.monitor()["mass"]))
+        s.close()
+    for q, mx, mass in out[1:]:
+        assert np.array_equal(q, out[0][0]) and mx == out[0][1] and mass == out[0][2]
 
 
 @pytest.mark.gpu
