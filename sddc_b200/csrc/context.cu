@@ -170,7 +170,6 @@ static void free_all(sddc_ctx *ctx)
                     ctx->visc_rv, ctx->met2, ctx->max_scratch, ctx->proc_cells};
     for (void *b : bufs) cudaFree(b);
     if (ctx->host_small) cudaFreeHost(ctx->host_small);
-    if (ctx->err_flags) cudaFreeHost(ctx->err_flags);
     adjoint_free(ctx);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
 }
@@ -261,8 +260,8 @@ extern "C" int sddc_create(sddc_ctx **out, const sddc_params *p)
             (rc = alloc(ctx, (void **)&ctx->met2, nc * 4 * p->N * 2 * sizeof(double), "face metrics")))
             return rc;
     }
-    CK(cudaMallocHost((void **)&ctx->host_small, 64 * sizeof(double)));
-    CK(cudaMallocHost((void **)&ctx->err_flags, sizeof(unsigned)));
+    CK(cudaMallocHost((void **)&ctx->host_small, 65 * sizeof(double)));
+    ctx->err_flags = reinterpret_cast<unsigned *>(ctx->host_small + 64);
     *ctx->err_flags = 0;
     CK(cudaMemsetAsync(ctx->maxima, 0, kSlots * 2 * sizeof(double), ctx->stream));
     CK(cudaMemsetAsync(ctx->sm_ind, 0, nc * 2 * sizeof(double), ctx->stream));

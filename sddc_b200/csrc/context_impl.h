@@ -74,8 +74,8 @@ struct sddc_ctx {
     double *maxima = nullptr;  // [sddc::kSlots][2]
     double *sm_ind = nullptr, *muav = nullptr, *resid = nullptr, *grad = nullptr;
     double *mon_part = nullptr, *mon_out = nullptr, *int_part = nullptr, *wq = nullptr;
-    // numerical faults, OR-ed by the kernels: pinned host memory, so that the
-    // host reads them after a synchronisation without a copy
+    // numerical faults, OR-ed by the kernels: pinned host memory behind
+    // host_small, so that the host reads them after a synchronisation without a copy
     unsigned *err_flags = nullptr;
     double *host_small = nullptr;  // pinned scratch for small read-backs
     Ops ops{};

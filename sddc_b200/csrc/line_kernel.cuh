@@ -77,18 +77,40 @@ template <int N, int CPB, typename R, bool EX> __host__ __device__ constexpr siz
            (S::kTOwn ? (size_t)CPB * S::TS * sizeof(R) : 0);
 }
 
+// Whether a thread holds its line's states in registers beside the sums.  In
+// double at N = 6 they do not fit (exact form, 121x87 cells: 638 us a step
+// with spills, 465 read from shared memory), and at N = 4 there is a second
+// kernel without them (WIDE): 168 registers instead of 240 let a scheduler
+// hold 3 warps instead of 2.  (At N = 5 the sums alone leave no third warp: 363
+// us a stage held, 423 read.)
+template <int N, typename R, bool WIDE> __host__ __device__ constexpr bool line_hold()
+{
+    return sizeof(R) == sizeof(float) || (N <= 5 && !WIDE);
+}
+__host__ __device__ constexpr bool line_has_wide(int n, int elem) { return n == 4 && elem == 8; }
+// Which of the two takes a stage of the given tiles, by the waves it needs
+// (CTAs resident at once: 592 held, 888 wide) and what a wave costs: one wave
+// of a small mesh takes 9.4 us held and 12.2 wide.  us per step, held and
+// wide: FP64, 64x64 cells (1 wave each) 47 and 61, 96x96 (2 and 2) 96 and 109,
+// 128x128 (4 and 3) 178 and 172, 256x256 (14 and 10) 630 and 573; exact,
+// 256x256 cells 922 and 852.
+__host__ __device__ constexpr bool line_use_wide(int tiles, int resident_held, int resident_wide)
+{
+    return (tiles + resident_wide - 1) / resident_wide * 13 < (tiles + resident_held - 1) / resident_held * 10;
+}
+
 // CTAs per SM the kernel is compiled for: as many as shared memory holds, up
 // to the warps whose registers hold a line (a scheduler's 512 registers per
 // lane go to whole warps: 4 warps of 128 registers, 3 of 168, 2 of 255)
-template <int N, typename R> constexpr int line_warps()
+template <int N, typename R, bool WIDE> constexpr int line_warps()
 {
     if (sizeof(R) == 4) return N >= 6 ? 12 : N >= 4 ? 16 : N == 3 ? 20 : 24;
-    return N >= 4 ? 8 : N == 3 ? 12 : 16;
+    return N >= 4 ? (WIDE ? 12 : 8) : N == 3 ? 12 : 16;
 }
-template <int N, int CPB, typename R, bool EX> constexpr int line_min_blocks()
+template <int N, int CPB, typename R, bool EX, bool WIDE> constexpr int line_min_blocks()
 {
     int b = (int)((228 * 1024) / (line_smem_bytes<N, CPB, R, EX>() + 1024 + 256));
-    const int br = line_warps<N, R>() / (line_threads(N, CPB) / 32);
+    const int br = line_warps<N, R, WIDE>() / (line_threads(N, CPB) / 32);
     b = b < br ? b : br;
     return b < 1 ? 1 : b;
 }
@@ -112,7 +134,7 @@ __device__ __forceinline__ void cp_async_wait_all()
     asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
-template <int N, int CPB, typename R, bool EXACT, int KIND>
+template <int N, int CPB, typename R, bool EXACT, int KIND, bool WIDE>
 __device__ __forceinline__ bool line_tile(const StageArgs &a, const Ops &ops, const int tile)
 {
     constexpr bool EX = EXACT && sizeof(R) == sizeof(double);
@@ -182,7 +204,7 @@ __device__ __forceinline__ bool line_tile(const StageArgs &a, const Ops &ops, co
 
     // ---- 1: staging -------------------------------------------------------------
     // first what no earlier launch writes: normals and Jac (the split arrays,
-    // or the packed records, in double), and the partners' normals
+    // or the packed records, in double)
     const int kind = KIND >= 0 ? KIND : a.rk_kind;
     const bool want_ra = kind == kRkTwoReg || kind == kRkTwoRegT;
     const double *qsrc = a.q_in + (size_t)c0 * NQ;
@@ -215,10 +237,6 @@ __device__ __forceinline__ bool line_tile(const StageArgs &a, const Ops &ops, co
         face_point<N>((rec.y >> 8) & 0xff, N - np, pfam, pline, pr);
         cp_async_pair(dst, reinterpret_cast<const P2<R> *>(nbase + (size_t)rec.x * nstride + ML::normal(pfam, pline, pr)));
     };
-    if (act) {
-        fetch_pn(rec0, np0, sP + tid);
-        fetch_pn(recN, npN, sP + NT + tid);
-    }
     // what the previous launch wrote: the states, the neighbours' traces and
     // the running maxima.  Its end is awaited here; the next launch's CTAs may
     // start as soon as every CTA of this one has.
@@ -236,6 +254,11 @@ __device__ __forceinline__ bool line_tile(const StageArgs &a, const Ops &ops, co
         if (kd == kFaceLeft || kd == kFaceRight)
             cp_async16(sX + (f >> 2) * TS + (f & 3) * TFS + ch * CE,
                        tin + ((size_t)frec[m].x * 4 + ((frec[m].y >> 8) & 0xff) - 1) * TFS + ch * CE);
+    }
+    // the left (partner) cell's normal where this cell is the right one
+    if (act) {
+        fetch_pn(rec0, np0, sP + tid);
+        fetch_pn(recN, npN, sP + NT + tid);
     }
     if (!bulk)
         for (int k = tid; k < ncl * NQ; k += NT) {
@@ -268,11 +291,10 @@ __device__ __forceinline__ bool line_tile(const StageArgs &a, const Ops &ops, co
         dy[i] = (R)0;
     }
     if (act) {
-        // the line's states: in registers, or, where the sums leave no room
-        // (double, N = 6), read from shared memory at every flux point (exact
-        // form, 121x87 cells: 638 us a step with spills, 530 so; at N = 5, where
-        // they fit, 363 us a stage held and 423 read)
-        constexpr bool kHold = sizeof(R) == sizeof(float) || N <= 5;
+        // the line's states: in registers, or read from shared memory at every
+        // flux point (line_hold); then both ends' fluxes are formed first, while
+        // the sums' registers are still free
+        constexpr bool kHold = line_hold<N, R, WIDE>();
         P2<R> q2[kHold ? N : 1][K2];
         R q8[kHold ? N : 1];
         const int q0 = c * QS + (fam == 0 ? 9 * N * l : 9 * l);
@@ -289,9 +311,11 @@ __device__ __forceinline__ bool line_tile(const StageArgs &a, const Ops &ops, co
             }
         }
         const P2<R> *nl = reinterpret_cast<const P2<R> *>(sN + c * NM + ML::normal(fam, l, 0));
-        auto point = [&](const int r) {
-            const P2<R> nn = nl[r];
-            const R n0 = nn.x, n1 = nn.y;
+        // the flux along the normal at flux point r (F), the normal (n), and
+        // what div B sums there (V): Bn, or in the exact form Bx and By
+        auto flux_at = [&](const int r, R (&F)[9], R (&V)[2], P2<R> &n) {
+            n = nl[r];
+            const R n0 = n.x, n1 = n.y;
             // the state at flux point r
             R q[9];
             int qi = q0;
@@ -325,7 +349,6 @@ __device__ __forceinline__ bool line_tile(const StageArgs &a, const Ops &ops, co
                 }
                 q[8] = acc8;
             }
-            R F[9], V[2];  // flux along the normal; Bn, or (exact) Bx and By
             if (r > 0 && r < N) {
                 // interior flux point (inviscid_flux_interior)
                 if (!(q[0] > (R)0)) err |= kErrNonPositiveDensity;
@@ -393,7 +416,9 @@ __device__ __forceinline__ bool line_tile(const StageArgs &a, const Ops &ops, co
                     V[1] = bya;
                 }
             }
-            // its share of the derivatives (compresid.f90:14-32) and of div B
+        };
+        // its share of the derivatives (compresid.f90:14-32) and of div B
+        auto accumulate = [&](const int r, const R (&F)[9], const R (&V)[2], const P2<R> &n) {
 #pragma unroll
             for (int i = 0; i < N; i++) {
                 const P2<R> M2 = opM2<R>(ops, r * N + i);
@@ -411,15 +436,23 @@ __device__ __forceinline__ bool line_tile(const StageArgs &a, const Ops &ops, co
                     d[i][K2] = fma2(f2, M2, d[i][K2]);
                 } else {
                     d[i][K2].x = d[i][K2].x + F[8] * M2.x;
-                    d[i][K2].y = d[i][K2].y + V[0] * M2.x * n0;
-                    dy[i] = dy[i] + V[1] * M2.x * n1;
+                    d[i][K2].y = d[i][K2].y + V[0] * M2.x * n.x;
+                    dy[i] = dy[i] + V[1] * M2.x * n.y;
                 }
             }
         };
-        point(0);
+        R F[9], V[2], G[9], W[2];
+        P2<R> n, m;
+        flux_at(0, F, V, n);
+        if constexpr (!kHold) flux_at(N, G, W, m);
+        accumulate(0, F, V, n);
 #pragma unroll 1
-        for (int r = 1; r < N; r++) point(r);
-        point(N);
+        for (int r = 1; r < N; r++) {
+            flux_at(r, F, V, n);
+            accumulate(r, F, V, n);
+        }
+        if constexpr (kHold) flux_at(N, G, W, m);
+        accumulate(N, G, W, m);
     }
     __syncthreads();  // the neighbours' traces are read: sX is free
 
@@ -711,21 +744,21 @@ __device__ __forceinline__ bool line_tile(const StageArgs &a, const Ops &ops, co
 }
 
 // KIND: the stage's RkKind, or -1 for any (read from the arguments)
-template <int N, int CPB, typename R, bool EXACT, int KIND>
-__global__ void __launch_bounds__(line_threads(N, CPB), (line_min_blocks<N, CPB, R, EXACT>()))
+template <int N, int CPB, typename R, bool EXACT, int KIND, bool WIDE>
+__global__ void __launch_bounds__(line_threads(N, CPB), (line_min_blocks<N, CPB, R, EXACT, WIDE>()))
     line_kernel(const StageArgs a, const Ops ops)
 {
-    line_tile<N, CPB, R, EXACT, KIND>(a, ops, blockIdx.x);
+    line_tile<N, CPB, R, EXACT, KIND, WIDE>(a, ops, blockIdx.x);
 }
 
 // a batch's stage as a persistent launch: each CTA walks the tile table with
 // a grid stride
-template <int N, int CPB, typename R, bool EXACT>
-__global__ void __launch_bounds__(line_threads(N, CPB), (line_min_blocks<N, CPB, R, EXACT>()))
+template <int N, int CPB, typename R, bool EXACT, bool WIDE>
+__global__ void __launch_bounds__(line_threads(N, CPB), (line_min_blocks<N, CPB, R, EXACT, WIDE>()))
     line_kernel_persistent(const StageArgs a, const Ops ops)
 {
     for (int t = blockIdx.x; t < a.ntiles; t += gridDim.x) {
-        if (!line_tile<N, CPB, R, EXACT, -1>(a, ops, t)) return;
+        if (!line_tile<N, CPB, R, EXACT, -1, WIDE>(a, ops, t)) return;
         __syncthreads();  // tile t's last shared-memory reads before tile t+grid stages
     }
 }

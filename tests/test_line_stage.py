@@ -86,6 +86,28 @@ def test_viscous_lines_match_oracle_at_tile_edges(N):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("N,nx,ny", [(4, 76, 75), (4, 64, 65), (6, 37, 41)])
+def test_lines_match_oracle_over_several_waves(N, nx, ny):
+    """More tiles than CTAs are resident: at N = 4 in double 713 tiles take the
+    kernel of three warps per scheduler, 520 the other one."""
+    m = mesh.channel_box(nx, ny, sides=("SYMP", "OUTL", "WALL", "INLE"), jitter=0.2, seed=N)
+    t = host.build_tables(m, N)
+    ph = channel_physics()
+    Q, dt = smooth_state(t, ph, seed=nx), 0.2 * m.min_edge() / N
+    o = O.Oracle(t, ph)
+    o.set_state(Q)
+    o.rk_s5p3(dt, 1)
+    ref = o.state()["Q"]
+    for form, bar in (("fp64_exact", 0.0), ("fp64", 1e-12), ("mixed", 1e-6)):
+        s = Solver(t, ph, precision=form, cells_per_cta=8)
+        s.set_state(Q)
+        s.rk_s5p3(dt, 1)
+        g = s.state()["Q"]
+        assert np.array_equal(g, ref) if not bar else rel_l2(g, ref) <= bar, form
+        s.close()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("form", ["fp64_exact", "fp64", "mixed"])
 def test_steps_in_any_grouping_are_the_same(form):
     """Single steps (eager, then a graph), a graph of several steps, and a dt
