@@ -277,6 +277,18 @@ __device__ __forceinline__ bool line_tile(const StageArgs &a, const Ops &ops, co
     }
     __syncthreads();
     if (sAbort) return false;
+    // into L2: the face records and traces of the tile that takes this CTA's
+    // place, the two loads in a row that its start waits for (with its state,
+    // register and metrics too it was no faster; us per stage at 256x512 cells,
+    // N = 5: FP64 362 before, 345 after; mixed 227 and 226; N = 4, 512x512 cells
+    // 274 and 270)
+    if (tid == NT - 1) {
+        const int nc0 = c0 + a.ahead * CPB;
+        if (nc0 + CPB <= a.ncell && (N % 2 == 0 || !(nc0 & 1))) {
+            bulk_prefetch_l2(a.faces + (size_t)nc0 * 4, CPB * 4 * sizeof(int2));
+            bulk_prefetch_l2(tin + (size_t)nc0 * 4 * TFS, CPB * 4 * TFS * sizeof(R));
+        }
+    }
 
     // ---- 2: the line ------------------------------------------------------------
     R eigmax = (R)0, umax = (R)0;

@@ -131,6 +131,7 @@ struct StageArgs {
     // batch launched persistently: each CTA walks the tile table with a grid
     // stride (the table is ordered largest case first); 0: one CTA per tile
     int persistent;
+    int ahead;  // tiles resident at once (set by the launch)
     const CaseParams *cases;
     const double *__restrict__ q_in;   // (9,N,N,NCELL), never written during the stage
     double *q_out;                     // RK output (may be reg_a: FiveStageRk stage 5)
