@@ -95,11 +95,16 @@ cudaError_t launch_adj_trace(sddc_ctx *ctx, const double *xbar, double scale, co
 
 template <int N> cudaError_t launch_vjp_n(sddc_ctx *ctx, const VjpArgs &a)
 {
-    constexpr int CPB = kAdjCpb;
-    const size_t smem = vjp_smem_doubles<N, CPB>() * sizeof(double);
-    cudaError_t e = cudaFuncSetAttribute(vjp_kernel<N, CPB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    vjp_kernel<N, CPB><<<(ctx->ncell + CPB - 1) / CPB, adj_threads(N, CPB), smem, ctx->stream>>>(a, ctx->ops);
+    constexpr int CPB = VjpSmem<N>::CPB;
+    constexpr size_t smem = VjpSmem<N>::kBytes;
+    static bool configured = false;
+    if (!configured) {
+        cudaError_t e = cudaFuncSetAttribute(vjp_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(vjp_kernel<N>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+        if (e != cudaSuccess) return e;
+        configured = true;
+    }
+    vjp_kernel<N><<<(ctx->ncell + CPB - 1) / CPB, line_threads(N, CPB), smem, ctx->stream>>>(a, ctx->ops);
     return cudaGetLastError();
 }
 
@@ -155,7 +160,7 @@ int ensure_ws(sddc_ctx *ctx)
     auto *w = new AdjWs();
     ctx->adj = w;
     const size_t nc = ctx->ncell, N = ctx->N;
-    w->grid = (ctx->ncell + kAdjCpb - 1) / kAdjCpb;
+    w->grid = (ctx->ncell + line_tile_cells(ctx->N) - 1) / line_tile_cells(ctx->N);
     w->rec_cap = (int)std::min<size_t>(nc * 4 * N, (size_t)1 << 24);
     const size_t tr = nc * 4 * trace_stride(ctx->N, 8);
     int rc;
@@ -242,10 +247,6 @@ int reverse_stage(sddc_ctx *ctx, const RevStage &s)
     a.lam_scale = s.scale;
     a.at = w->at;
     a.met = ctx->met;
-    if (ctx->nrm_double && !ctx->jac_inv) {  // an exact context holds double normals and Jac
-        a.nrm = static_cast<const double *>(ctx->nrm);
-        a.jac = ctx->jac;
-    }
     a.faces = ctx->faces;
     a.ra = s.ra;
     a.rb = s.rb;
@@ -455,7 +456,7 @@ extern "C" int sddc_adjoint_run(sddc_ctx *ctx, const sddc_adjoint_opts *o, doubl
 
     RunBufs rb;
     std::vector<double *> ckpt(nseg), S(5 * segmax + 1), T(5 * segmax + 1);
-    double *hist = nullptr, *force = nullptr, *cmax = nullptr, *A[6] = {};
+    double *hist = nullptr, *force = nullptr, *cmax = nullptr, *fin = nullptr, *A[6] = {};
     const size_t ncmax = (size_t)5 * segmax * 2 * ((ctx->ncell + ctx->cpb - 1) / ctx->cpb);
     for (auto &c : ckpt) rb.name(&c, nq);
     for (int i = 0; i <= 5 * segmax; i++) {
@@ -474,6 +475,7 @@ extern "C" int sddc_adjoint_run(sddc_ctx *ctx, const sddc_adjoint_opts *o, doubl
     std::vector<double *> S2(overlap ? 5 * segmax + 1 : 0), T2(overlap ? 5 * segmax + 1 : 0);
     double *cmax2 = nullptr;
     if (overlap) {
+        rb.name(&fin, nq);  // the final state: the sweep overwrites the stores
         for (int i = 0; i <= 5 * segmax; i++) {
             rb.name(&S2[i], nq);
             rb.name(&T2[i], tr);
@@ -530,6 +532,13 @@ extern "C" int sddc_adjoint_run(sddc_ctx *ctx, const sddc_adjoint_opts *o, doubl
             CKA(cudaMemcpyAsync(ckpt[s + 1], S[5 * nst], nq * sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream));
     }
     CKA(cudaEventRecord(ev[1], ctx->stream));
+    {
+        double *last = S[5 * (ns - (nseg - 1) * K)];
+        if (overlap)
+            CKA(cudaMemcpyAsync(fin, last, nq * sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream));
+        else
+            fin = last;
+    }
     std::vector<double> H(2 * ((size_t)5 * ns + 1)), Fh(2 * ((size_t)ns + 1));
     CKA(cudaMemcpyAsync(H.data(), hist, H.size() * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
     CKA(cudaMemcpyAsync(Fh.data(), force, Fh.size() * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
@@ -702,16 +711,6 @@ extern "C" int sddc_adjoint_run(sddc_ctx *ctx, const sddc_adjoint_opts *o, doubl
 
     // ---- the context continues from the final state -------------------------------
     {
-        const int last = ns - (nseg - 1) * K;
-        double *fin = S[5 * last];
-        if (grad && nseg > 1) {  // the stage store now holds the first segment: rerun the last one
-            const int step0 = (nseg - 1) * K;
-            CKA(cudaMemcpyAsync(S[0], ckpt[nseg - 1], nq * sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream));
-            CKA(launch_trace_exact(ctx->N, ctx->ncell, S[0], T[0], trace_stride(ctx->N, 8), ctx->ops, ctx->stream));
-            if ((rc = forward_steps(ctx, o->dt, step0, last, S.data(), T.data(), hist, 0, -1, nullptr, cmax,
-                                    ctx->stream)))
-                return rc;
-        }
         CKA(cudaMemcpyAsync(ctx->reg[0], fin, nq * sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream));
         const double *hl = &H[2 * (size_t)5 * ns];
         std::vector<double> mx(2 * kSlots);

@@ -32,7 +32,7 @@
 #pragma once
 
 #include "adjoint_point.cuh"
-#include "stage_kernel.cuh"
+#include "line_kernel.cuh"
 
 namespace sddc {
 
@@ -66,9 +66,6 @@ struct VjpArgs {
     double lam_scale;                 // lambda = lam_scale * xbar
     const double *__restrict__ at;    // adjoint traces, layout adj_trace_at
     const double *__restrict__ met;
-    // the split metrics of an exact context (double normals [NCELL][4N(N+1)],
-    // Jac [NCELL][MetLayout::kJacPad]), staged directly; null: the packed record
-    const double *__restrict__ nrm, *__restrict__ jac;
     const int2 *__restrict__ faces;
     // epilogue: out = (wa*ra + wb*rb) + qbar;  out2 = wc*rc + wd*xbar
     const double *ra, *rb;
@@ -89,44 +86,6 @@ struct VjpArgs {
     double scale_next;
     double *at_next;
 };
-
-constexpr int kAdjCpb = 4;
-__host__ __device__ constexpr int adj_threads(int n, int cpb) { return (4 * n * cpb > 128 ? (4 * n * cpb + 31) / 32 * 32 : 128); }
-
-// Warps of vjp_kernel given to the face points (the rest take the interior
-// flux points): the count that minimises the slower side's rounds, with a
-// face point's Rusanov adjoint costing about kFaceCost interior points' flux
-// adjoints (measured on the B200 at N = 4); ties go to fewer face warps.
-constexpr int kFaceCost = 7;
-__host__ __device__ constexpr int adj_face_warps(int n, int cpb)
-{
-    const int nw = adj_threads(n, cpb) / 32, nf = cpb * 4 * n, ni = cpb * 2 * n * (n - 1);
-    int best = 1, cost = 1 << 30;
-    for (int w = 1; w < nw; w++) {
-        const int cf = (nf + 32 * w - 1) / (32 * w) * kFaceCost, ci = (ni + 32 * (nw - w) - 1) / (32 * (nw - w));
-        const int c = cf > ci ? cf : ci;
-        if (c < cost) {
-            cost = c;
-            best = w;
-        }
-    }
-    return best;
-}
-
-template <int N, int CPB> constexpr size_t vjp_smem_doubles()
-{
-    constexpr int NQ = 9 * N * N, NP = N + 1, NN = N * N;
-    constexpr int kF = 2 * N * NP * 9, kV = 2 * N * NP * 2, kO = 4 * N * 9, kP = 4 * N * 13;
-    constexpr int NM = 2 * MetLayout<N>::kFam;
-    return (size_t)CPB * (2 * NQ + 2 * kF + kV + kO + kP + MetLayout<N>::kJacPad + NN + NM) + 2 * NP * N + 8 * 32;
-}
-
-// the tile fits a CTA's shared memory (227 KB) at every N; at N = 4 four
-// CTAs fit an SM (228 KB, 1 KB reserved per CTA), which the 128-register cap
-// of vjp_kernel's launch bounds assumes
-static_assert(vjp_smem_doubles<6, kAdjCpb>() * sizeof(double) <= 227 * 1024, "VJP tile exceeds shared memory");
-static_assert(4 * (vjp_smem_doubles<4, kAdjCpb>() * sizeof(double) + 1024) <= 228 * 1024,
-              "VJP tile at N = 4 no longer fits four CTAs per SM");
 
 // ---- adjoint traces ----------------------------------------------------------
 // at(cell, lf, nfp) = (Fbar(9), Vbar_Bx, Vbar_By, 0): the adjoint of this
@@ -323,416 +282,419 @@ static __device__ __noinline__ void adj_record_face(RecSink rs, Freestream fs, i
 }
 
 // ---- the stage VJP -------------------------------------------------------------
-template <int N, int CPB>
-__global__ void __launch_bounds__(adj_threads(N, CPB), 4) vjp_kernel(const VjpArgs a, const Ops ops)
+// One thread per line of solution points, as the forward stage works
+// (line_kernel.cuh).  At every flux point of its line, one after the other,
+// the thread forms the primal state and the flux adjoint (the transposed flux
+// derivative) from the states and -lambda/J of the line, applies the point
+// adjoint and adds its share of the transposed interpolation to N*9 sums in
+// registers; the two lines through a point exchange their sums once.
+//
+// What bounds it: latency, at 2 warps of up to 255 registers per scheduler
+// (a line's sums, a point's state, flux adjoint and state adjoint, and the
+// Rusanov adjoint's own values); the states are read from shared memory at
+// every flux point.  One thread per point and variable, every operand through
+// shared memory, 4 CTAs of 4 warps per SM: 64 us at 64x128 cells, N = 4, and
+// 144 ms for the reverse sweep of 100 steps at 128x256; by lines 53 us and
+// 122 ms.
+template <int N> struct VjpSmem {
+    static constexpr int CPB = line_tile_cells(N);
+    static constexpr int NQ = 9 * N * N, NN = N * N;
+    static constexpr bool kPad = N % 2 == 0;  // two doubles per cell against bank conflicts
+    static constexpr int QS = kPad ? NQ + 2 : NQ;
+    static constexpr int MS = MetLayout<N>::kSize;
+    static constexpr int TFS = trace_stride<N, double>();
+    static constexpr int TS = 4 * TFS + 2;
+    static constexpr int AF = 12 * N;          // a face's adjoint trace record
+    static constexpr int AS = 4 * AF + 2;      // per cell
+    static constexpr int XS = 9 * NN + 1;      // exchanged sums per cell, over the traces
+    static_assert(XS <= TS + AS, "the exchanged sums fit the traces' region");
+    static constexpr size_t kBytes =
+        8 * ((size_t)CPB * (2 * QS + MS + TS + AS + NN) + 2 * 2 * line_threads(N, CPB) + 8 * 32);
+};
+template <int N> constexpr int vjp_min_blocks()
 {
+    const int w = (N >= 4 ? 8 : N == 3 ? 9 : 12) / (line_threads(N, VjpSmem<N>::CPB) / 32);
+    const int m = (int)(228 * 1024 / (VjpSmem<N>::kBytes + 1280));
+    const int b = w < m ? w : m;
+    return b < 1 ? 1 : b;
+}
+
+// a boundary face point (rare): the own trace's adjoint of its flux and
+// average, through the ghost state, and the free stream's; out of line
+static __device__ __noinline__ double vjp_boundary(int kind, const double *own, const double *oth, double n0, double n1,
+                                                   int sign_l, int vismode, Freestream fs, double c_h, const double *fbar,
+                                                   const double *fown, double vbx, double vby, double *qown, double *pb)
+{
+    double qgb[9] = {0, 0, 0, 0, 0, 0.5 * vbx, 0.5 * vby, 0, 0}, eig, um;
+    const double wdc =
+        rusanov_vjp(own, oth, n0, n1, sign_l, c_h, fbar, 0.0, 0.0, qown, qgb, eig, um, nullptr, fown);
+    bc_ghost_vjp(kind, own, n0, n1, vismode, fs, qgb, qown, pb);
+    return wdc;
+}
+static __device__ __noinline__ void vjp_ghost(int kind, const double *own, double n0, double n1, int vismode, Freestream fs,
+                                              double *oth)
+{
+    bc_ghost<double, true>(kind, own, n0, n1, vismode, fs, oth);
+}
+
+template <int N>
+__global__ void __launch_bounds__(line_threads(N, VjpSmem<N>::CPB), (vjp_min_blocks<N>()))
+    vjp_kernel(const VjpArgs a, const Ops ops)
+{
+    using S = VjpSmem<N>;
     using ML = MetLayout<N>;
-    constexpr int NT = adj_threads(N, CPB);
-    constexpr int NQ = 9 * N * N, NP = N + 1, NN = N * N;
-    constexpr int kF = 2 * N * NP * 9, kV = 2 * N * NP * 2, kO = 4 * N * 9, kP = 4 * N * 13, NM = 2 * ML::kFam;
+    constexpr int CPB = S::CPB, NT = line_threads(N, CPB), NQ = S::NQ, NN = S::NN, QS = S::QS, NH = (N + 1) / 2;
 
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    double *sQ = reinterpret_cast<double *>(smem_raw);  // [CPB][NQ] q, then qbar of the sources, then qbar
-    double *sA = sQ + CPB * NQ;                         // [CPB][NQ] lambda, then -lambda/J
-    double *sQf = sA + CPB * NQ;                        // [CPB][2][N][NP][9] flux-point states
-    double *sFb = sQf + CPB * kF;                       // [CPB][2][N][NP][9] flux adjoint, then state adjoint
-    double *sVb = sFb + CPB * kF;                       // [CPB][2][N][NP][2] face-averaged Bx,By, then adjoint
-    double *sQo = sVb + CPB * kV;                       // [CPB][4N][9] neighbour / ghost trace
-    // [CPB][4N][13] per face point: the partner's signed flux adjoint (9) and
-    // face-average adjoints (2), zero on boundary faces; the face's normal (2)
-    double *sPa = sQo + CPB * kO;
-    constexpr int NJ = ML::kJacPad;
-    double *sJac = sPa + CPB * kP;                      // [CPB][NJ]
-    double *sBeta = sJac + CPB * NJ;                    // [CPB][NN] adjoint of divB, over Jac
-    double *sNrm = sBeta + CPB * NN;                    // [CPB][NM]
-    double *sL = sNrm + CPB * NM;                       // [NP][N]
-    double *sM = sL + NP * N;                           // [NP][N]
-    double *sRed = sM + NP * N;                         // [8][32]
-
-    const int tid = threadIdx.x;
-    const int c0 = blockIdx.x * CPB;
-    const int ncl = min(CPB, a.ncell - c0);
-
-    // the tile's state, lambda source and metric slices by TMA bulk copies
-    // when they are 16-byte aligned, else by loads: the split normals and Jac
-    // straight into place, or the packed metric records into sQf (free until
-    // the primal phase) for conversion
-    __shared__ __align__(8) unsigned long long sBar;
+    double *sQ = reinterpret_cast<double *>(smem_raw);  // [CPB][QS] q, then qbar, then out
+    double *sA = sQ + CPB * QS;                         // [CPB][QS] lambda, then -lambda/J, then the next stage's q
+    double *sMet = sA + CPB * QS;                       // [CPB][MS] normals, Jac
+    double *sT = sMet + CPB * S::MS;                    // [CPB][TS] neighbours' (or ghost) traces
+    double *sAT = sT + CPB * S::TS;                     // [CPB][AS] neighbours' adjoint traces
+    double *sX = sT;                                    // [CPB][XS] exchanged sums, over both
+    double *sBeta = sAT + CPB * S::AS;                  // [CPB][NN] div B sums, then the adjoint of div B over J
+    double2 *sP = reinterpret_cast<double2 *>(sBeta + CPB * NN);  // [2][NT] partners' normals at the line's ends
+    double *sRed = reinterpret_cast<double *>(sP + 2 * NT);       // [8][32]
+    __shared__ __align__(8) unsigned long long sBar, sBarN;
     __shared__ int sAbort;
-    const bool split = a.nrm != nullptr;  // uniform
-    {
-        const double *qsrc = a.q + (size_t)c0 * NQ, *msrc = a.met + (size_t)c0 * ML::kSize;
-        const double *nsrc = split ? a.nrm + (size_t)c0 * NM : nullptr, *jsrc = split ? a.jac + (size_t)c0 * NJ : nullptr;
-        const double *xsrc = a.xbar ? a.xbar + (size_t)c0 * NQ : nullptr;
-        const size_t qbytes = (size_t)ncl * NQ * sizeof(double);
-        const size_t mbytes = split ? 0 : (size_t)ncl * ML::kSize * sizeof(double);
-        const size_t nbytes = split ? (size_t)ncl * NM * sizeof(double) : 0;
-        const size_t jbytes = split ? (size_t)ncl * NJ * sizeof(double) : 0;
-        const bool bulk = (((uintptr_t)qsrc | (uintptr_t)msrc | (uintptr_t)nsrc | (uintptr_t)jsrc | (uintptr_t)xsrc |
-                            qbytes | mbytes | nbytes | jbytes) & 15) == 0;
+
+    const int tid = threadIdx.x, c0 = blockIdx.x * CPB, ncl = min(CPB, a.ncell - c0);
+    // this thread's line (as in line_kernel) and the records of its end faces
+    const int fam = tid >= N * CPB ? 1 : 0;
+    const int lt = tid - fam * N * CPB, lc = lt % CPB;
+    const bool act = tid < 2 * N * CPB && lc < ncl;
+    const int c = act ? lc : 0, l = act ? lt / CPB : 0;
+    const int lf0 = fam == 0 ? 4 : 1, lfN = fam == 0 ? 2 : 3;
+    const int np0 = fam == 0 ? N - 1 - l : l, npN = fam == 0 ? l : N - 1 - l;  // 0-based
+    int2 rec0 = make_int2(0, 0), recN = make_int2(0, 0);
+    if (act) {
+        rec0 = __ldg(a.faces + (size_t)(c0 + c) * 4 + lf0 - 1);
+        recN = __ldg(a.faces + (size_t)(c0 + c) * 4 + lfN - 1);
+    }
+    const int pt0 = fam == 0 ? N * l : l, pts = fam == 0 ? 1 : N;  // point t of the line: pt0 + pts*t
+    const int par = (l ^ fam) & 1;                                 // this thread finishes points t with t + par even
+
+    // ---- staging --------------------------------------------------------------------
+    const double *qsrc = a.q + (size_t)c0 * NQ, *xsrc = a.xbar ? a.xbar + (size_t)c0 * NQ : nullptr;
+    const unsigned cbytes = (unsigned)((S::kPad ? 1 : ncl) * NQ * sizeof(double));
+    const bool bulk = (((uintptr_t)qsrc | (uintptr_t)xsrc | cbytes) & 15) == 0;
+    if (tid < 32) {
         if (tid == 0) {
             sAbort = 0;
-            if (bulk) {
-                mbar_init(&sBar, 1);
-                mbar_expect_tx(&sBar, (unsigned)(qbytes + mbytes + nbytes + jbytes + (xsrc ? qbytes : 0)));
-                bulk_g2s(sQ, qsrc, (unsigned)qbytes, &sBar);
-                if (split) {
-                    bulk_g2s(sNrm, nsrc, (unsigned)nbytes, &sBar);
-                    bulk_g2s(sJac, jsrc, (unsigned)jbytes, &sBar);
-                } else {
-                    bulk_g2s(sQf, msrc, (unsigned)mbytes, &sBar);
-                }
-                if (xsrc) bulk_g2s(sA, xsrc, (unsigned)qbytes, &sBar);
+            mbar_init(&sBar, 1);
+            mbar_init(&sBarN, 1);
+            mbar_expect_tx(&sBar, (unsigned)((ncl * S::MS + (bulk ? ncl * NQ * (xsrc ? 2 : 1) : 0)) * sizeof(double)));
+            bulk_g2s(sMet, a.met + (size_t)c0 * S::MS, (unsigned)(ncl * S::MS * sizeof(double)), &sBar);
+        }
+        __syncwarp();
+        if (bulk && tid < (S::kPad ? ncl : 1)) {
+            bulk_g2s(sQ + tid * QS, qsrc + (size_t)tid * NQ, cbytes, &sBar);
+            if (xsrc) bulk_g2s(sA + tid * QS, xsrc + (size_t)tid * NQ, cbytes, &sBar);
+        }
+        // L2 prefetches of the RK registers the epilogue reads
+        if (tid < 3) {
+            const double *r = tid == 0 ? a.ra : tid == 1 ? a.rb : a.out2 ? a.rc : nullptr;
+            const unsigned n = (unsigned)((size_t)ncl * NQ * sizeof(double));
+            if (r && (((uintptr_t)(r + (size_t)c0 * NQ) | n) & 15) == 0) bulk_prefetch_l2(r + (size_t)c0 * NQ, n);
+        }
+    }
+    // the neighbours' traces and adjoint traces, 16 bytes of a face at a time
+    {
+        constexpr int CT = S::TFS / 2, CA = S::AF / 2, IT = (CPB * 4 * (CT + CA) + NT - 1) / NT, B = IT < 8 ? IT : 8;
+#pragma unroll 1
+        for (int m0 = 0; m0 < IT; m0 += B) {
+            int2 r[B];
+#pragma unroll
+            for (int m = 0; m < B; m++) {
+                const int f = (tid + (m0 + m) * NT) / (CT + CA);
+                r[m] = f < ncl * 4 ? __ldg(a.faces + (size_t)c0 * 4 + f) : make_int2(0, 0);
+            }
+#pragma unroll
+            for (int m = 0; m < B; m++) {
+                const int e = tid + (m0 + m) * NT, f = e / (CT + CA), ch = e - f * (CT + CA), kd = r[m].y & 0xff;
+                if (kd != kFaceLeft && kd != kFaceRight) continue;
+                const size_t pf = (size_t)r[m].x * 4 + ((r[m].y >> 8) & 0xff) - 1;
+                if (ch < CT)
+                    cp_async16(sT + (f >> 2) * S::TS + (f & 3) * S::TFS + 2 * ch, a.t_in + pf * S::TFS + 2 * ch);
+                else if (a.xbar)
+                    cp_async16(sAT + (f >> 2) * S::AS + (f & 3) * S::AF + 2 * (ch - CT), a.at + pf * S::AF + 2 * (ch - CT));
             }
         }
-        // L2 prefetches of what later phases load from global memory: the RK
-        // registers of the epilogue, and per shared face the partner's trace
-        // and adjoint trace (each face's values are contiguous)
-        if (tid == 0) {
-            const size_t g0 = (size_t)c0 * NQ;
-            const double *regs[3] = {a.ra, a.rb, a.out2 ? a.rc : nullptr};
-            for (int m = 0; m < 3; m++)
-                if (regs[m] && (((uintptr_t)(regs[m] + g0) | qbytes) & 15) == 0)
-                    bulk_prefetch_l2(regs[m] + g0, (unsigned)qbytes);
-        } else if (tid >= 32 && tid < 32 + ncl * 4) {
-            const int c = (tid - 32) >> 2, lf = 1 + ((tid - 32) & 3);
-            const int2 rec = a.faces[(size_t)(c0 + c) * 4 + (lf - 1)];
-            const int kind = rec.y & 0xff;
-            if (kind == kFaceLeft || kind == kFaceRight) {
-                const int pc = rec.x, plf = (rec.y >> 8) & 0xff;
-                // the face's 9N trace values, widened to 16-byte bounds (the
-                // buffer, 288N bytes per cell, starts and ends on one)
-                const uintptr_t t0 = (uintptr_t)(a.t_in + trace_at<N>(trace_stride<N, double>(), pc, plf, 0, 0)) & ~(uintptr_t)15;
-                const uintptr_t t1 = ((uintptr_t)(a.t_in + trace_at<N>(trace_stride<N, double>(), pc, plf, 0, 9)) + 15) & ~(uintptr_t)15;
-                if (((uintptr_t)a.t_in & 15) == 0) bulk_prefetch_l2((const void *)t0, (unsigned)(t1 - t0));
-                if (a.xbar && ((uintptr_t)a.at & 15) == 0)
-                    bulk_prefetch_l2(a.at + adj_trace_at<N>(pc, plf, 0, 0), 12 * N * sizeof(double));
-            }
+    }
+    auto fetch_pn = [&](const int2 rec, int np, double2 *dst) {
+        if ((rec.y & 0xff) != kFaceRight) return;
+        int pfam, pline, pr;
+        face_point<N>((rec.y >> 8) & 0xff, N - np, pfam, pline, pr);
+        cp_async_pair(dst, reinterpret_cast<const double2 *>(a.met + (size_t)rec.x * S::MS + ML::normal(pfam, pline, pr)));
+    };
+    if (act) {
+        fetch_pn(rec0, np0, sP + tid);
+        fetch_pn(recN, npN, sP + NT + tid);
+    }
+    if (!bulk)
+        for (int k = tid; k < ncl * NQ; k += NT) {
+            const int cc = k / NQ, o = cc * QS + (k - cc * NQ);
+            sQ[o] = qsrc[k];
+            if (xsrc) sA[o] = xsrc[k];
         }
-        for (int k = tid; k < NP * N; k += NT) {
-            sL[k] = ops.L[k];
-            sM[k] = ops.M[k];
-        }
-        if (!bulk) {
-            for (int k = tid; k < ncl * NQ; k += NT) {
-                sQ[k] = __ldg(qsrc + k);
-                if (xsrc) sA[k] = xsrc[k];
-            }
-            if (split) {
-                for (int k = tid; k < ncl * NM; k += NT) sNrm[k] = __ldg(nsrc + k);
-                for (int k = tid; k < ncl * NJ; k += NT) sJac[k] = __ldg(jsrc + k);
-            } else {
-                for (int k = tid; k < ncl * ML::kSize; k += NT) sQf[k] = __ldg(msrc + k);
-            }
-        }
-        if (bulk && tid == 0 && !mbar_wait_bounded(&sBar, 0)) {
-            atomicOr(a.err, kErrStagingTimeout);  // the copies did not complete
-            sAbort = 1;
-            mbar_wait_bounded(&sBar, 0);
-        }
+    cp_async_wait_all();
+    if (tid == 0 && !mbar_wait_bounded(&sBar, 0)) {
+        atomicOr(a.err, kErrStagingTimeout);  // the copies did not complete
+        sAbort = 1;
+        mbar_wait_bounded(&sBar, 0);
     }
     __syncthreads();
     if (sAbort) return;
-    // lambda (first read two barriers on); the packed metric records, staged in
-    // sQf, are converted before phase A overwrites sQf
-    for (int k = tid; k < ncl * NQ; k += NT) sA[k] = a.xbar ? a.lam_scale * sA[k] : 0.0;
-    if (!split) {
-        for (int k = tid; k < ncl * ML::kSize; k += NT) {
-            const int c = k / ML::kSize, o = k - c * ML::kSize;
-            const double v = sQf[k];
-            if (o < NM) sNrm[c * NM + o] = v;
-            else if (o < NM + NN) sJac[c * NJ + (o - NM)] = v;
-        }
-        __syncthreads();
-    }
 
-    // ---- primal: flux-point states (phase A of the stage kernel) ----------------
-    for (int t = tid; t < ncl * 2 * N * 9; t += NT) {
-        const int v = t % 9, l = (t / 9) % N, f = (t / (9 * N)) % 2, c = t / (18 * N);
-        const double *q = sQ + c * NQ;
-        double qs[N];
+    const int q0 = c * QS + 9 * pt0, qstr = 9 * pts;  // the line's values in sQ and sA
+    // the interpolated state at flux point r
+    auto own_state = [&](int r, double (&q)[9]) {
+        int qi = q0;
+        asm volatile("" : "+r"(qi));  // read anew at every point
 #pragma unroll
-        for (int s = 0; s < N; s++) qs[s] = f == 0 ? q[v + 9 * (s + N * l)] : q[v + 9 * (l + N * s)];
-        double *o = sQf + c * kF + (f * N + l) * NP * 9 + v;
+        for (int k = 0; k < 9; k++) q[k] = 0.0;
 #pragma unroll
-        for (int r = 0; r < NP; r++) {
-            double acc = 0.0;
+        for (int s = 0; s < N; s++) {
+            const double L = ops.L[r * N + s];
 #pragma unroll
-            for (int s = 0; s < N; s++) acc = acc + qs[s] * ops.L[r * N + s];
-            o[r * 9] = acc;
+            for (int k = 0; k < 9; k++) q[k] = q[k] + sQ[qi + qstr * s + k] * L;
+        }
+    };
+    auto normal = [&](int r) { return *reinterpret_cast<const double2 *>(sMet + c * S::MS + ML::normal(fam, l, r)); };
+    // the other side's trace at the line's end r: 9 values N apart
+    auto other_at = [&](int r) { return sT + c * S::TS + ((r == 0 ? lf0 : lfN) - 1) * S::TFS + (N - 1 - (r == 0 ? np0 : npN)); };
+    auto is_pair = [](int kind) { return kind == kFaceLeft || kind == kFaceRight; };
+
+    // ---- primal: ghost traces, and the line's share of div B ---------------------------
+    if (act) {
+#pragma unroll 1
+        for (int r = 0; r <= N; r += N) {
+            const int kind = (r == 0 ? rec0 : recN).y & 0xff;
+            if (is_pair(kind)) continue;
+            double own[9], oth[9];
+            own_state(r, own);
+            const double2 n = normal(r);
+            vjp_ghost(kind, own, n.x, n.y, a.vismode, a.fs, oth);
+            double *tp = other_at(r);
+            for (int k = 0; k < 9; k++) tp[k * N] = oth[k];
+        }
+    }
+    double dvb[N];  // div B sums (nablaQsp of Bx in x and By in y)
+#pragma unroll
+    for (int i = 0; i < N; i++) dvb[i] = 0.0;
+    if (act && a.vismode == 1) {
+#pragma unroll
+        for (int r = 0; r <= N; r++) {
+            double bx = 0.0, by = 0.0;
+#pragma unroll
+            for (int s = 0; s < N; s++) {
+                bx += sQ[q0 + qstr * s + 5] * ops.L[r * N + s];
+                by += sQ[q0 + qstr * s + 6] * ops.L[r * N + s];
+            }
+            if (r == 0 || r == N) {
+                const double *tp = other_at(r);
+                bx = 0.5 * bx + 0.5 * tp[5 * N];
+                by = 0.5 * by + 0.5 * tp[6 * N];
+            }
+            const double2 n = normal(r);
+            const double bn = bx * n.x + by * n.y;
+#pragma unroll
+            for (int i = 0; i < N; i++) dvb[i] += bn * ops.M[r * N + i];
+        }
+#pragma unroll
+        for (int m = 0; m < NH; m++) {
+            const int i0 = 2 * m, i1 = 2 * m + 1 < N ? 2 * m + 1 : 2 * m;
+            if (2 * m + 1 < N || par) sBeta[c * NN + pt0 + pts * (2 * m + 1 - par)] = par ? dvb[i0] : dvb[i1];
         }
     }
     __syncthreads();
 
-    // ---- primal: neighbour / ghost traces and face-averaged Bx, By; on the ---------
-    // ---- other threads the partner's adjoint trace and the face normal -------------
-    for (int t2 = tid; t2 < 2 * ncl * 4 * N; t2 += NT) {
-        const bool part = t2 >= ncl * 4 * N;
-        const int t = part ? t2 - ncl * 4 * N : t2;
-        const int nfp = 1 + t % N, lf = 1 + (t / N) % 4, c = t / (4 * N);
-        int fam, line, r;
-        face_point<N>(lf, nfp, fam, line, r);
-        const int2 rec = a.faces[(size_t)(c0 + c) * 4 + (lf - 1)];
-        const int kind = rec.y & 0xff;
-        const bool own_right = kind == kFaceRight;
-        if (part) {
-            const double *onrm = sNrm + c * NM + ML::normal(fam, line, r);
-            double v[13] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, onrm[0], onrm[1]};
-            if (kind == kFaceLeft || own_right) {
-                const int pc = rec.x, plf = (rec.y >> 8) & 0xff;
-                int pfam, pline, pr;
-                face_point<N>(plf, N - nfp + 1, pfam, pline, pr);
-                if (own_right) {  // the flux is formed with the left (partner) cell's normal
-                    const double *pn = a.met + (size_t)pc * ML::kSize + ML::normal(pfam, pline, pr);
-                    v[11] = __ldg(pn);
-                    v[12] = __ldg(pn + 1);
+    // ---- per solution point: the source adjoint, -lambda/J, divB adjoint ----------------
+    double acc[N][9];  // the line's sums of the state adjoint; a finished point's start from its source adjoint
+#pragma unroll
+    for (int i = 0; i < N; i++)
+#pragma unroll
+        for (int k = 0; k < 9; k++) acc[i][k] = 0.0;
+    if (act) {
+#pragma unroll
+        for (int m = 0; m < NH; m++) {
+            const int i0 = 2 * m, i1 = 2 * m + 1 < N ? 2 * m + 1 : 2 * m;
+            if (!(2 * m + 1 < N) && par) continue;
+            const int pt = pt0 + pts * (2 * m + par);
+            const double rJ = 1.0 / sMet[c * S::MS + ML::kJac + pt];
+            const double divB = a.vismode == 1 ? (sBeta[c * NN + pt] + (par ? dvb[i1] : dvb[i0])) * rJ : 0.0;
+            const double *qs = sQ + c * QS + 9 * pt;
+            double *lp = sA + c * QS + 9 * pt;
+            double lam[9];
+#pragma unroll
+            for (int k = 0; k < 9; k++) lam[k] = a.xbar ? a.lam_scale * lp[k] : 0.0;
+            const double ri = 1.0 / qs[0], ux = qs[1] * ri, uy = qs[2] * ri, uz = qs[3] * ri;
+            const double Bx = qs[5], By = qs[6], Bz = qs[7];
+            double db = 0.0;
+            if (a.vismode == 1)
+                db = -(lam[1] * Bx + lam[2] * By + lam[3] * Bz + lam[4] * ((ux * Bx + uy * By) + uz * Bz) +
+                       lam[5] * ux + lam[6] * uy + lam[7] * uz);
+            // Powell and GLM sources (compresid.f90:60-78)
+            const double ub = -divB * (lam[4] * Bx + lam[5]);
+            const double vb = -divB * (lam[4] * By + lam[6]);
+            const double wb = -divB * (lam[4] * Bz + lam[7]);
+            double src[9];
+            src[0] = -(ub * ux + vb * uy + wb * uz) * ri;
+            src[1] = ub * ri;
+            src[2] = vb * ri;
+            src[3] = wb * ri;
+            src[4] = 0.0;
+            src[5] = -divB * (lam[1] + lam[4] * ux);
+            src[6] = -divB * (lam[2] + lam[4] * uy);
+            src[7] = -divB * (lam[3] + lam[4] * uz);
+            src[8] = -a.alpha * lam[8];
+#pragma unroll
+            for (int k = 0; k < 9; k++) {
+                lp[k] = -lam[k] * rJ;
+                if (i1 != i0) {
+                    acc[i0][k] = par ? 0.0 : src[k];
+                    acc[i1][k] = par ? src[k] : 0.0;
+                } else {
+                    acc[i0][k] = src[k];
                 }
-                // the partner's slot enters with sign_l * sign_r unless it is
-                // the left cell's
-                const int sign_l = own_right ? (pr == 0 ? -1 : 1) : (r == 0 ? -1 : 1);
-                const int sign_r = own_right ? (r == N ? -1 : 1) : (pr == N ? -1 : 1);
-                const double ps = own_right ? 1.0 : (double)(sign_l * sign_r);
-                if (a.xbar) {
-#pragma unroll
-                    for (int k = 0; k < 9; k++) v[k] = ps * a.at[adj_trace_at<N>(pc, plf, N - nfp, k)];
-                    if (a.vismode == 1) {
-                        v[9] = a.at[adj_trace_at<N>(pc, plf, N - nfp, 9)];
-                        v[10] = a.at[adj_trace_at<N>(pc, plf, N - nfp, 10)];
-                    }
-                }
             }
-            double *pa = sPa + c * kP + (t % (4 * N)) * 13;
-#pragma unroll
-            for (int k = 0; k < 13; k++) pa[k] = v[k];
-            continue;
-        }
-        const double *own = sQf + c * kF + ((fam * N + line) * NP + r) * 9;
-        double oth[9];
-        if (kind == kFaceLeft || own_right) {
-            const int pc = rec.x, plf = (rec.y >> 8) & 0xff;
-#pragma unroll
-            for (int k = 0; k < 9; k++) oth[k] = a.t_in[trace_at<N>(trace_stride<N, double>(), pc, plf, N - nfp, k)];
-        } else {
-            const double *nrm = sNrm + c * NM + ML::normal(fam, line, r);
-            bc_ghost<double, true>(kind, own, nrm[0], nrm[1], a.vismode, a.fs, oth);
-        }
-        double *so = sQo + c * kO + t % (4 * N) * 9;
-#pragma unroll
-        for (int k = 0; k < 9; k++) so[k] = oth[k];
-        double *vs = sVb + c * kV + ((fam * N + line) * NP + r) * 2;
-        const double *ql = own_right ? oth : own, *qr = own_right ? own : oth;
-        vs[0] = 0.5 * ql[5] + 0.5 * qr[5];
-        vs[1] = 0.5 * ql[6] + 0.5 * qr[6];
-    }
-    __syncthreads();
-
-    // ---- per solution point: divB, the source adjoint, -lambda/J, divB adjoint ------
-    for (int t = tid; t < ncl * NN; t += NT) {
-        const int i = t % N, j = (t / N) % N, c = t / NN;
-        const double rJ = 1.0 / sJac[c * NJ + i + N * j];
-        const double *met = sNrm + c * NM;
-        double divB = 0.0;
-        if (a.vismode == 1) {
-            // nablaQsp for Bx (x derivative) and By (y derivative)
-            auto V = [&](int f, int l, int r, int g) -> double {
-                return (r == 0 || r == N) ? sVb[c * kV + ((f * N + l) * NP + r) * 2 + g]
-                                          : sQf[c * kF + ((f * N + l) * NP + r) * 9 + 5 + g];
-            };
-            double ax = 0.0, bx = 0.0, ay = 0.0, by = 0.0;
-#pragma unroll
-            for (int r = 0; r < NP; r++) {
-                ax += V(0, j, r, 0) * sM[r * N + i] * met[ML::normal(0, j, r)];
-                bx += V(1, i, r, 0) * sM[r * N + j] * met[ML::normal(1, i, r)];
-                ay += V(0, j, r, 1) * sM[r * N + i] * met[ML::normal(0, j, r) + 1];
-                by += V(1, i, r, 1) * sM[r * N + j] * met[ML::normal(1, i, r) + 1];
-            }
-            divB = ((ax + bx) + (ay + by)) * rJ;
-        }
-        double *qs = sQ + c * NQ + 9 * (i + N * j);
-        double *lam = sA + c * NQ + 9 * (i + N * j);
-        const double rho = qs[0], ri = 1.0 / rho, ux = qs[1] * ri, uy = qs[2] * ri, uz = qs[3] * ri;
-        const double Bx = qs[5], By = qs[6], Bz = qs[7];
-        double db = 0.0;
-        if (a.vismode == 1)
-            db = -(lam[1] * Bx + lam[2] * By + lam[3] * Bz + lam[4] * ((ux * Bx + uy * By) + uz * Bz) +
-                   lam[5] * ux + lam[6] * uy + lam[7] * uz);
-        // Powell and GLM sources (compresid.f90:60-78)
-        const double ub = -divB * (lam[4] * Bx + lam[5]);
-        const double vb = -divB * (lam[4] * By + lam[6]);
-        const double wb = -divB * (lam[4] * Bz + lam[7]);
-        double src[9];
-        src[0] = -(ub * ux + vb * uy + wb * uz) * ri;
-        src[1] = ub * ri;
-        src[2] = vb * ri;
-        src[3] = wb * ri;
-        src[4] = 0.0;
-        src[5] = -divB * (lam[1] + lam[4] * ux);
-        src[6] = -divB * (lam[2] + lam[4] * uy);
-        src[7] = -divB * (lam[3] + lam[4] * uz);
-        src[8] = -a.alpha * lam[8];
-#pragma unroll
-        for (int k = 0; k < 9; k++) {
-            qs[k] = src[k];
-            lam[k] = -lam[k] * rJ;
-        }
-        sBeta[c * NN + i + N * j] = db * rJ;
-    }
-    __syncthreads();
-
-    // ---- transposed flux derivative and B gradient: adjoints at the flux points ------
-    for (int t = tid; t < ncl * 2 * N * 11; t += NT) {
-        const int v = t % 11, l = (t / 11) % N, f = (t / (11 * N)) % 2, c = t / (22 * N);
-        double x[N];
-#pragma unroll
-        for (int i = 0; i < N; i++) {
-            const int sp = f == 0 ? i + N * l : l + N * i;
-            x[i] = v < 9 ? sA[c * NQ + 9 * sp + v] : sBeta[c * NN + sp];
-        }
-#pragma unroll
-        for (int r = 0; r < NP; r++) {
-            double acc = 0.0;
-#pragma unroll
-            for (int i = 0; i < N; i++) acc += ops.M[r * N + i] * x[i];
-            if (v < 9) {
-                sFb[c * kF + ((f * N + l) * NP + r) * 9 + v] = acc;
-            } else {
-                const double n = sNrm[c * NM + ML::normal(f, l, r) + (v - 9)];
-                sVb[c * kV + ((f * N + l) * NP + r) * 2 + (v - 9)] = acc * n;
-            }
+            sBeta[c * NN + pt] = db * rJ;
         }
     }
     __syncthreads();
 
+    // ---- per flux point of the line: the point adjoint and its interpolation's share -----
     double cbar = 0.0, pb[6] = {0, 0, 0, 0, 0, 0};
-    // The point adjoints: face points on the first kFaceWarps warps, interior
-    // flux points on the others (adj_face_warps balances their rounds).  The
-    // interior warps then add the interior flux points' share of the
-    // transposed interpolation while the face warps finish.
-    constexpr int kFaceWarps = adj_face_warps(N, CPB);
-    const int wid = tid >> 5;
-    if (wid >= kFaceWarps) {
-        // ---- interior flux points ---------------------------------------------------
-        const int nth = NT - 32 * kFaceWarps, me = tid - 32 * kFaceWarps;
-        for (int t = me; t < ncl * 2 * N * (N - 1); t += nth) {
-            const int r = 1 + t % (N - 1), l = (t / (N - 1)) % N, f = (t / ((N - 1) * N)) % 2,
-                      c = t / (2 * N * (N - 1));
-            const int slot = (f * N + l) * NP + r;
-            const double *qf = sQf + c * kF + slot * 9;
-            double *fb = sFb + c * kF + slot * 9;
-            const double *nr = sNrm + c * NM + ML::normal(f, l, r);
-            double qb[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, um;
-            cbar += iflux_vjp(qf, a.c_h, nr[0], nr[1], fb, qb, um, nullptr);
-            if (a.vismode == 1) {
-                qb[5] += sVb[c * kV + slot * 2];
-                qb[6] += sVb[c * kV + slot * 2 + 1];
-            }
+    if (act) {
+        auto point = [&](int r) {
+            double q[9], fb[9], qb[9], bt = 0.0;
+            own_state(r, q);
+            {
+                int qi = q0, bi = c * NN + pt0;
+                asm volatile("" : "+r"(qi), "+r"(bi));  // read anew at every point
 #pragma unroll
-            for (int k = 0; k < 9; k++) fb[k] = qb[k];
-        }
-        // the interior warps' own barrier: their flux-point adjoints are all in
-        asm volatile("bar.sync 1, %0;" ::"r"(nth) : "memory");
-        for (int t = me; t < ncl * NQ; t += nth) {
-            const int v = t % 9, i = (t / 9) % N, j = (t / (9 * N)) % N, c = t / NQ;
-            const double *gx = sFb + c * kF + (0 * N + j) * NP * 9 + v;  // xi-line j
-            const double *gy = sFb + c * kF + (1 * N + i) * NP * 9 + v;  // eta-line i
-            double acc = sQ[t];
+                for (int k = 0; k < 9; k++) fb[k] = 0.0;
 #pragma unroll
-            for (int r = 1; r < N; r++) acc += sL[r * N + i] * gx[r * 9] + sL[r * N + j] * gy[r * 9];
-            sQ[t] = acc;
-        }
-    } else {
-        // ---- face points ------------------------------------------------------------
-        for (int t = tid; t < ncl * 4 * N; t += 32 * kFaceWarps) {
-            const int nfp = 1 + t % N, lf = 1 + (t / N) % 4, c = t / (4 * N);
-            int fam, line, r;
-            face_point<N>(lf, nfp, fam, line, r);
-            const int slot = (fam * N + line) * NP + r;
-            const double *own = sQf + c * kF + slot * 9;
-            const double *oth = sQo + c * kO + (t % (4 * N)) * 9;
-            double *fown = sFb + c * kF + slot * 9;
-            const int2 rec = a.faces[(size_t)(c0 + c) * 4 + (lf - 1)];
-            const int kind = rec.y & 0xff;
-            const bool pair = kind == kFaceLeft || kind == kFaceRight;
-            const bool own_right = kind == kFaceRight;
-            const double *pa = sPa + c * kP + (t % (4 * N)) * 13;
-            const double n0 = pa[11], n1 = pa[12];
-            int sign_l, sign_r;
-            double fbar[9], vbx = 0.0, vby = 0.0;
-            if (a.vismode == 1) {
-                vbx = sVb[c * kV + slot * 2];
-                vby = sVb[c * kV + slot * 2 + 1];
-            }
-            if (pair) {
-                const int plf = (rec.y >> 8) & 0xff;
-                int pfam, pline, pr;
-                face_point<N>(plf, N - nfp + 1, pfam, pline, pr);
-                sign_l = own_right ? (pr == 0 ? -1 : 1) : (r == 0 ? -1 : 1);
-                sign_r = own_right ? (r == N ? -1 : 1) : (pr == N ? -1 : 1);
-                const double ms = own_right ? (double)(sign_l * sign_r) : 1.0;
-                // the partner's share (staged signed, zero without xbar)
+                for (int s = 0; s < N; s++) {
+                    const double M = ops.M[r * N + s];
 #pragma unroll
-                for (int k = 0; k < 9; k++) fbar[k] = ms * fown[k] + pa[k];
-                if (a.vismode == 1) {
-                    vbx += pa[9];
-                    vby += pa[10];
-                }
-            } else {
-                sign_l = r == 0 ? -1 : 1;
-                sign_r = 1;
-#pragma unroll
-                for (int k = 0; k < 9; k++) fbar[k] = fown[k];
-                if (kind == kFaceWall) {  // the objective: force on the wall faces
-                    const double w = a.wq[line] * (double)sign_l;
-                    fbar[1] += a.sx * w;
-                    fbar[2] += a.sy * w;
+                    for (int k = 0; k < 9; k++) fb[k] += M * sA[qi + qstr * s + k];
+                    bt += M * sBeta[bi + pts * s];
                 }
             }
-            const double *ql = own_right ? oth : own, *qr = own_right ? own : oth;
-            double qown[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, eig, um;
-            // the face-averaged Bx, By feed the gradients of both cells
-            qown[5] = 0.5 * vbx;
-            qown[6] = 0.5 * vby;
-            // this cell's share of the c_h adjoint comes from its own flux
-            // slot (fown, weighted by the slot's sign)
-            double wdc;
-            if (pair) {
-                wdc = rusanov_vjp(ql, qr, n0, n1, sign_l, a.c_h, fbar, 0.0, 0.0, own_right ? nullptr : qown,
-                                  own_right ? qown : nullptr, eig, um, nullptr, fown);
-            } else {
-                double qgb[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-                qgb[5] = 0.5 * vbx;
-                qgb[6] = 0.5 * vby;
-                wdc = rusanov_vjp(own, oth, n0, n1, sign_l, a.c_h, fbar, 0.0, 0.0, qown, qgb, eig, um, nullptr, fown);
-                bc_ghost_vjp(kind, own, n0, n1, a.vismode, a.fs, qgb, qown, pb);
-            }
-            cbar += (own_right ? (double)(sign_l * sign_r) : 1.0) * wdc;
-
+            const double2 nn = normal(r);
+            double vbx = bt * nn.x, vby = bt * nn.y;  // adjoint of Bx, By there (zero unless vismode = 1)
 #pragma unroll
-            for (int k = 0; k < 9; k++) fown[k] = qown[k];
-        }
+            for (int k = 0; k < 9; k++) qb[k] = 0.0;
+            if (r > 0 && r < N) {
+                double um;
+                cbar += iflux_vjp(q, a.c_h, nn.x, nn.y, fb, qb, um, nullptr);
+                qb[5] += vbx;
+                qb[6] += vby;
+            } else {
+                const int2 rec = r == 0 ? rec0 : recN;
+                const int lf = r == 0 ? lf0 : lfN, np = r == 0 ? np0 : npN, kind = rec.y & 0xff;
+                const double *tp = other_at(r);
+                double oth[9], fbar[9];
+#pragma unroll
+                for (int k = 0; k < 9; k++) oth[k] = tp[k * N];
+                if (is_pair(kind)) {
+                    const int plf = (rec.y >> 8) & 0xff;
+                    const bool own_right = kind == kFaceRight, plow = plf == 1 || plf == 4;
+                    const double2 pn = own_right ? sP[(r == 0 ? 0 : NT) + tid] : nn;
+                    const int sign_l = own_right ? (plow ? -1 : 1) : (r == 0 ? -1 : 1);
+                    const int sign_r = own_right ? (r == N ? -1 : 1) : (plow ? 1 : -1);
+                    const double slr = (double)(sign_l * sign_r);
+                    // own slot's and the partner's share; a right cell's slot is
+                    // the left one's with both signs
+                    const double ms = own_right ? slr : 1.0, ps = own_right ? 1.0 : slr;
+                    const double *ap = sAT + c * S::AS + (lf - 1) * S::AF + (N - 1 - np);
+#pragma unroll
+                    for (int k = 0; k < 9; k++) fbar[k] = ms * fb[k] + (a.xbar ? ps * ap[k * N] : 0.0);
+                    if (a.xbar && a.vismode == 1) {
+                        vbx += ap[9 * N];
+                        vby += ap[10 * N];
+                    }
+                    // the face-averaged Bx, By feed the gradients of both cells
+                    qb[5] = 0.5 * vbx;
+                    qb[6] = 0.5 * vby;
+                    // the flux is the same with the roles swapped and the normal
+                    // reversed, so this cell is the left one here
+                    cbar += ms * rusanov_vjp_own(q, oth, pn.x, pn.y, own_right ? -sign_l : sign_l, a.c_h, fbar, fb, qb);
+                } else {
+                    const int sign_l = r == 0 ? -1 : 1;
+#pragma unroll
+                    for (int k = 0; k < 9; k++) fbar[k] = fb[k];
+                    if (kind == kFaceWall) {  // the objective: force on the wall faces
+                        const double w = a.wq[l] * (double)sign_l;
+                        fbar[1] += a.sx * w;
+                        fbar[2] += a.sy * w;
+                    }
+                    double qo[9], fo[9], ql[9], og[9], ff[9];  // the call's own copies
+                    for (int k = 0; k < 9; k++) {
+                        qo[k] = 0.0;
+                        fo[k] = fbar[k];
+                        ff[k] = fb[k];
+                        ql[k] = q[k];
+                        og[k] = oth[k];
+                    }
+                    qo[5] = 0.5 * vbx;
+                    qo[6] = 0.5 * vby;
+                    cbar += vjp_boundary(kind, ql, og, nn.x, nn.y, sign_l, a.vismode, a.fs, a.c_h, fo, ff, vbx, vby, qo, pb);
+                    for (int k = 0; k < 9; k++) qb[k] = qo[k];
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < N; i++) {
+                const double L = ops.L[r * N + i];
+#pragma unroll
+                for (int k = 0; k < 9; k++) acc[i][k] += L * qb[k];
+            }
+        };
+        point(0);
+#pragma unroll 1
+        for (int r = 1; r < N; r++) point(r);
+        point(N);
     }
-    __syncthreads();
+    __syncthreads();  // the traces, the states and -lambda/J are read
 
-    // the next stage's input state, for its adjoint traces, by a bulk copy into
-    // sQf (no longer read) that lands during the steps below
+    // the next stage's input state, for its adjoint traces, over -lambda/J
     const bool fuse = a.at_next != nullptr;  // uniform
     const double *qn = fuse ? a.q_next + (size_t)c0 * NQ : nullptr;
-    const bool qn_bulk = fuse && (((uintptr_t)qn | ((size_t)ncl * NQ * sizeof(double))) & 15) == 0;
-    __shared__ __align__(8) unsigned long long sBarN;
-    if (qn_bulk && tid == 0) {
-        fence_proxy_async();
-        mbar_init(&sBarN, 1);
-        mbar_expect_tx(&sBarN, (unsigned)(ncl * NQ * sizeof(double)));
-        bulk_g2s(sQf, qn, (unsigned)(ncl * NQ * sizeof(double)), &sBarN);
+    const bool qn_bulk = fuse && (((uintptr_t)qn | cbytes) & 15) == 0;
+    if (qn_bulk && tid < 32) {
+        if (tid == 0) {
+            fence_proxy_async();
+            mbar_expect_tx(&sBarN, (unsigned)(ncl * NQ * sizeof(double)));
+        }
+        __syncwarp();
+        if (tid < (S::kPad ? ncl : 1)) bulk_g2s(sA + tid * QS, qn + (size_t)tid * NQ, cbytes, &sBarN);
     }
 
-    // ---- transposed interpolation, the face points' share (the interior flux ---------
-    // ---- points' share is in): state adjoint at the solution points ------------------
-    for (int t = tid; t < ncl * NQ; t += NT) {
-        const int v = t % 9, i = (t / 9) % N, j = (t / (9 * N)) % N, c = t / NQ;
-        const double *gx = sFb + c * kF + (0 * N + j) * NP * 9 + v;  // xi-line j
-        const double *gy = sFb + c * kF + (1 * N + i) * NP * 9 + v;  // eta-line i
-        sQ[t] += (sL[i] * gx[0] + sL[j] * gy[0]) + (sL[N * N + i] * gx[N * 9] + sL[N * N + j] * gy[N * 9]);
+    // ---- the exchange: state adjoint at the solution points -----------------------------
+    if (act) {
+#pragma unroll
+        for (int m = 0; m < NH; m++) {
+            const int i0 = 2 * m, i1 = 2 * m + 1 < N ? 2 * m + 1 : 2 * m;
+            if (2 * m + 1 < N || par) {
+                double *o = sX + c * S::XS + (pt0 + pts * (2 * m + 1 - par)) * 9;
+#pragma unroll
+                for (int k = 0; k < 9; k++) o[k] = par ? acc[i0][k] : acc[i1][k];
+            }
+        }
+    }
+    __syncthreads();
+    if (act) {
+#pragma unroll
+        for (int m = 0; m < NH; m++) {
+            const int i0 = 2 * m, i1 = 2 * m + 1 < N ? 2 * m + 1 : 2 * m;
+            if (!(2 * m + 1 < N) && par) continue;
+            const int pt = pt0 + pts * (2 * m + par);
+            const double *x = sX + c * S::XS + pt * 9;
+            double *o = sQ + c * QS + 9 * pt;
+#pragma unroll
+            for (int k = 0; k < 9; k++) o[k] = (par ? acc[i1][k] : acc[i0][k]) + x[k];
+        }
     }
     __syncthreads();
 
@@ -740,7 +702,7 @@ __global__ void __launch_bounds__(adj_threads(N, CPB), 4) vjp_kernel(const VjpAr
     // the register reads of kU elements are issued before their use, so that
     // each thread keeps several loads in flight
     {
-        constexpr int kU = 4;
+        constexpr int kU = 6;
         const size_t g0 = (size_t)c0 * NQ;
         const int n = ncl * NQ;
         for (int e0 = tid; e0 < n; e0 += kU * NT) {
@@ -759,22 +721,27 @@ __global__ void __launch_bounds__(adj_threads(N, CPB), 4) vjp_kernel(const VjpAr
                 const int e = e0 + u * NT;
                 if (e >= n) break;
                 const size_t g = g0 + e;
+                const int cc = e / NQ;
+                double *x = sQ + cc * QS + (e - cc * NQ);
                 double o = 0.0;
                 if (a.ra) o = a.wa * va[u];
                 if (a.rb) o = o + a.wb * vb[u];
-                const double ov = o + sQ[e];
+                const double ov = o + *x;
                 a.out[g] = ov;
-                if (fuse) sQ[e] = ov;
+                if (fuse) *x = ov;
                 if (a.out2) a.out2[g] = (a.rc ? a.wc * vc[u] : 0.0) + a.wd * vx[u];
             }
         }
     }
 
     // ---- the next reverse stage's adjoint traces from out (adj_trace_kernel's ----------
-    // ---- arithmetic): -lambda/J and the divB adjoint per point, then per face point -----
+    // ---- arithmetic): -lambda/J and the divB adjoint per point, then per line end -------
     if (fuse) {
         if (!qn_bulk)
-            for (int k = tid; k < ncl * NQ; k += NT) sQf[k] = qn[k];
+            for (int k = tid; k < ncl * NQ; k += NT) {
+                const int cc = k / NQ;
+                sA[cc * QS + (k - cc * NQ)] = qn[k];
+            }
         else if (tid == 0 && !mbar_wait_bounded(&sBarN, 0)) {
             atomicOr(a.err, kErrStagingTimeout);  // the copy did not complete
             sAbort = 1;
@@ -783,45 +750,58 @@ __global__ void __launch_bounds__(adj_threads(N, CPB), 4) vjp_kernel(const VjpAr
         __syncthreads();
         if (sAbort) return;
         for (int k = tid; k < ncl * NN; k += NT) {
-            double *x = sQ + 9 * k;
+            const int cc = k / NN, pt = k - cc * NN;
+            double *x = sQ + cc * QS + 9 * pt;
             double db = 0.0;
             if (a.vismode == 1) {
-                const double *qq = sQf + 9 * k;
+                const double *qq = sA + cc * QS + 9 * pt;
                 const double ri = 1.0 / qq[0], ux = qq[1] * ri, uy = qq[2] * ri, uz = qq[3] * ri;
                 db = -a.scale_next * (x[1] * qq[5] + x[2] * qq[6] + x[3] * qq[7] +
                                       x[4] * ((ux * qq[5] + uy * qq[6]) + uz * qq[7]) + x[5] * ux + x[6] * uy +
                                       x[7] * uz);
             }
-            const int c = k / NN;
-            const double rJ = 1.0 / sJac[c * NJ + (k - c * NN)];
+            const double rJ = 1.0 / sMet[cc * S::MS + ML::kJac + pt];
             sBeta[k] = db * rJ;
 #pragma unroll
             for (int m = 0; m < 9; m++) x[m] = -(a.scale_next * x[m]) * rJ;
         }
         __syncthreads();
-        for (int t = tid; t < ncl * 4 * N; t += NT) {
-            const int c = t / (4 * N), f = t - c * 4 * N;
-            const int nfp = 1 + f % N, lf = 1 + f / N;
-            int fam, line, r;
-            face_point<N>(lf, nfp, fam, line, r);
-            double fb[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, bs = 0.0;
+        if (act) {
+            double f0[9], fN[9], b0 = 0.0, bN = 0.0;
+#pragma unroll
+            for (int k = 0; k < 9; k++) f0[k] = fN[k] = 0.0;
 #pragma unroll
             for (int i = 0; i < N; i++) {
-                const int sp = fam == 0 ? i + N * line : line + N * i;
-                const double m = sM[r * N + i];
-                const double *mu = sQ + c * NQ + 9 * sp;
+                const double m0 = ops.M[i], mN = ops.M[N * N + i];
+                const double *mu = sQ + q0 + qstr * i;
 #pragma unroll
-                for (int k = 0; k < 9; k++) fb[k] += m * mu[k];
-                bs += m * sBeta[c * NN + sp];
+                for (int k = 0; k < 9; k++) {
+                    f0[k] += m0 * mu[k];
+                    fN[k] += mN * mu[k];
+                }
+                const double b = sBeta[c * NN + pt0 + pts * i];
+                b0 += m0 * b;
+                bN += mN * b;
             }
-            const double *nr = sNrm + c * NM + ML::normal(fam, line, r);
-            double *o = a.at_next;
+            const double2 n0 = normal(0), nN = normal(N);
+            // collected over the neighbours' traces: sX's readers are done
+            double *o0 = sT + c * S::AS + (lf0 - 1) * S::AF + np0, *oN = sT + c * S::AS + (lfN - 1) * S::AF + npN;
 #pragma unroll
-            for (int k = 0; k < 9; k++) o[adj_trace_at<N>(c0 + c, lf, nfp - 1, k)] = fb[k];
-            o[adj_trace_at<N>(c0 + c, lf, nfp - 1, 9)] = bs * nr[0];
-            o[adj_trace_at<N>(c0 + c, lf, nfp - 1, 10)] = bs * nr[1];
-            o[adj_trace_at<N>(c0 + c, lf, nfp - 1, 11)] = 0.0;
+            for (int k = 0; k < 9; k++) {
+                o0[k * N] = f0[k];
+                oN[k * N] = fN[k];
+            }
+            o0[9 * N] = b0 * n0.x;
+            o0[10 * N] = b0 * n0.y;
+            o0[11 * N] = 0.0;
+            oN[9 * N] = bN * nN.x;
+            oN[10 * N] = bN * nN.y;
+            oN[11 * N] = 0.0;
         }
+        fence_proxy_async();
+        __syncthreads();
+        if (tid < ncl)
+            bulk_s2g(a.at_next + (size_t)(c0 + tid) * 4 * S::AF, sT + tid * S::AS, 4 * S::AF * sizeof(double));
     }
 
     // ---- per-CTA sums of the c_h and free-stream adjoints ------------------------------
@@ -843,6 +823,7 @@ __global__ void __launch_bounds__(adj_threads(N, CPB), 4) vjp_kernel(const VjpAr
             a.part[(size_t)tid * gridDim.x + blockIdx.x] = s;
         }
     }
+    if (tid < 32) bulk_wait_read();
 }
 
 // ---- per-stage reduction and the running-max adjoint --------------------------------

@@ -286,6 +286,57 @@ SDDC_HD double rusanov_vjp(const double *Ql, const double *Qr, double n0, double
     return wdc;
 }
 
+// rusanov_vjp for the left trace Qo alone, without the maxima's adjoints:
+// qb += (df/dQo)^T fb; returns wc . d f / d c_h.  The flux is the same with
+// the traces swapped and sign_l reversed, so Qo may be either side's.
+SDDC_HD double rusanov_vjp_own(const double *Qo, const double *Qx, double n0, double n1, int sign_l, double c,
+                               const double *fb, const double *wc, double *qb)
+{
+    const double n2 = n0 * n0 + n1 * n1, rm = Rsqrt(n2);
+    const double magnorm = n2 * rm;
+    const double sm = (double)sign_l * rm;
+    const double ux = n0 * sm, uy = n1 * sm;
+    const double K = 0.5 * magnorm * (double)sign_l;
+    RusSide O, X;
+    rus_side(Qo, ux, uy, O);
+    rus_side(Qx, ux, uy, X);
+    const double wdc = K * (wc[4] * (O.psi * O.Bn + X.psi * X.Bn) + (wc[5] * ux + wc[6] * uy) * (O.psi + X.psi) +
+                            wc[8] * (O.Bn + X.Bn));
+    const double Vn_s = O.Vn + X.Vn;
+    const double Bh[3] = {0.5 * (O.Bx + X.Bx), 0.5 * (O.By + X.By), 0.5 * (O.Bz + X.Bz)};
+    const double bn = Bh[0] * ux + Bh[1] * uy;
+    const double iS = 1.0 / (O.rho + X.rho);
+    const double ca = kGam * (O.p + X.p) * iS;
+    const double cd = 2.0 * ((Bh[0] * Bh[0] + Bh[1] * Bh[1]) + Bh[2] * Bh[2]) * iS;
+    const double cn = 2.0 * bn * bn * iS;
+    const double cad = ca + cd;
+    const double disc = cad * cad - 4.0 * ca * cn;
+    const double rct = disc > 0.0 ? Rsqrt(disc) : 0.0;
+    const double ct = disc > 0.0 ? disc * rct : Sqrt(disc);
+    const double xf = 0.5 * (cad + ct), rcf = Rsqrt(xf);
+    const double eig = 0.5 * Abs(Vn_s) + xf * rcf;
+    double g[9], ebar = 0.0;
+    for (int k = 0; k < 9; k++) {
+        g[k] = K * fb[k];
+        ebar -= g[k] * (Qx[k] - Qo[k]);
+    }
+    const double Vnb = 0.5 * sgn1(Vn_s) * ebar;
+    const double q4 = 0.25 * ebar * rcf;  // d eig / d cad = d eig / d ct
+    const double Db = 0.5 * q4 * rct;
+    const double cadb = q4 + 2.0 * cad * Db;
+    const double cab = -4.0 * cn * Db + cadb;
+    const double cnb = -4.0 * ca * Db;
+    const double pgb = cab * kGam * iS;
+    const double Sb = -(cab * ca + cadb * cd + cnb * cn) * iS;
+    const double bnb = 4.0 * cnb * bn * iS;
+    const double c4 = 2.0 * cadb * iS;  // half of d cd / d Bh
+    const double Bhalf[3] = {c4 * Bh[0] + 0.5 * bnb * ux, c4 * Bh[1] + 0.5 * bnb * uy, c4 * Bh[2]};
+    const double uvwb[3] = {0.0, 0.0, 0.0};
+    for (int k = 0; k < 9; k++) qb[k] += eig * g[k];
+    rus_side_vjp(O, c, ux, uy, g, Vnb, pgb, Bhalf, Sb, uvwb, qb);
+    return wdc;
+}
+
 // w . d f / d c_h of the Rusanov flux (f's c_h terms: k = 4, 5, 6, 8)
 SDDC_HD double rusanov_wdfdc(const double *Ql, const double *Qr, double n0, double n1, int sign_l, const double *w)
 {

@@ -108,6 +108,52 @@ def test_lines_match_oracle_over_several_waves(N, nx, ny):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("N", sorted(TILE))
+def test_vjp_lines_match_tangent_at_tile_edges(N):
+    """<Qbar, V> = <Rbar, R'(Q) V>, the bar of the VJP tests (1e-11)."""
+    for ncell in sorted({1, 2, TILE[N] - 1, TILE[N] + 1, 2 * TILE[N]}):
+        t, ph, Q, _ = _case(N, ncell)
+        rng = np.random.default_rng(ncell)
+        lam, V = rng.standard_normal(Q.shape), rng.standard_normal(Q.shape)
+        s = Solver(t, ph, precision="fp64_exact")
+        s.set_state(Q, 0.0, 3.0, 1.0)
+        Qbar, _ = s.vjp_resid(lam)
+        s.close()
+        T = O.Oracle(t, ph, tangent=True)
+        T.set_state(Q + 1e-30j * V, 0.0, 3.0, 1.0)
+        T.compresid()
+        jv = T.state()["resid"].imag / 1e-30
+        a, b = float(np.vdot(lam, jv)), float(np.vdot(Qbar, V))
+        assert abs(a - b) <= 1e-11 * np.vdot(np.abs(lam), np.abs(jv)), (ncell, a, b)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("N", [2, 3, 5, 6])
+def test_reverse_steps_in_any_grouping_are_the_same(N):
+    """A checkpoint at every step (each segment's first reverse stage takes its
+    adjoint traces from the trace launch) and none (all from the VJP's end)."""
+    c = cases.cylinder_case(5, 11, N, ms=0.5, noise=1e-3)
+    t = host.build_tables(c.mesh, N)
+    Q = c.initial_state(t)
+    dt = cases.cfl_dt(c.mesh, Q, N)
+    out = []
+    for every in (1, 100):
+        s = Solver(t, c.physics, precision="fp64_exact")
+        s.set_state(Q)
+        r = s.adjoint_run(dt, 4, 2, 4, checkpoint_every=every)
+        out.append((r["J"], r["Qbar0"], r["parbar"], s.state()["Q"].copy()))
+        s.rk_s5p3(dt, 1)  # the context goes on from the final state
+        out[-1] += (s.state()["Q"].copy(),)
+        s.close()
+    assert out[0][0] == out[1][0] and all(np.array_equal(a, b) for a, b in zip(out[0][1:], out[1][1:]))
+    s = Solver(t, c.physics, precision="fp64_exact")
+    s.set_state(Q)
+    s.rk_s5p3(dt, 5)
+    assert np.array_equal(s.state()["Q"], out[0][4])
+    s.close()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("form", ["fp64_exact", "fp64", "mixed"])
 def test_steps_in_any_grouping_are_the_same(form):
     """Single steps (eager, then a graph), a graph of several steps, and a dt
