@@ -29,23 +29,25 @@ NVCC_COMMON = ["-std=c++17", "-O3", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompi
                f"-I{INCLUDE}", f"-I{CSRC}"]
 CUDA_UNITS = {
     "stage_exact.cu": ["-fmad=false"],
-    "stage_fp64.cu": [],
-    # single-precision divide and square root of the mixed form's flux work
-    # to the hardware approximations (within 2 ulp); FP64 is unaffected
-    "stage_mixed.cu": ["-prec-div=false", "-prec-sqrt=false"],
     "context.cu": [],
     "noalloc.cu": [],
     "adjoint.cu": [],
     "adjoint_exact.cu": ["-fmad=false"],
     "output.cu": ["-fmad=false"],
 }
-# the line kernel's units: one object per N (0: the dispatch over N), with
-# the flags of the form's stage kernel
+# the units of the kernels by lines: one object per N (0: the dispatch over N)
+LINE_UNITS = {
+    "line_exact.cu": ["-fmad=false"],
+    "line_fp64.cu": [],
+    # single-precision divide and square root of the mixed form's flux work
+    # to the hardware approximations (within 2 ulp); FP64 is unaffected
+    "line_mixed.cu": ["-prec-div=false", "-prec-sqrt=false"],
+}
 LINE_N = (0, 2, 3, 4, 5, 6)
 OBJECTS = {name[:-3]: (name, flags) for name, flags in CUDA_UNITS.items()}
-for _form in ("exact", "fp64", "mixed"):
+for _unit, _flags in LINE_UNITS.items():
     for _n in LINE_N:
-        OBJECTS[f"line_{_form}_n{_n}"] = (f"line_{_form}.cu", [*CUDA_UNITS[f"stage_{_form}.cu"], f"-DSDDC_N={_n}"])
+        OBJECTS[f"{_unit[:-3]}_n{_n}"] = (_unit, [*_flags, f"-DSDDC_N={_n}"])
 
 
 def _nvcc() -> str:

@@ -360,7 +360,7 @@ int forward_steps(sddc_ctx *ctx, double dt, int step0, int nsteps, double *const
                 a.jac = nullptr;
                 a.jac_inv = 0;
             }
-            CKA(launch_stage_exact(ctx->N, ctx->cpb, false, a, ctx->ops, st));
+            CKA(launch_rk_exact(ctx, a, st));
         }
         const int n = step0 + m + 1;
         if (force && n >= n1 && n <= n2) CKA(wall_force(ctx, T[5 * (m + 1)], force + 2 * n));
@@ -404,7 +404,7 @@ extern "C" int sddc_vjp_resid(sddc_ctx *ctx, const double *Rbar, double *Qbar, d
     if (rc) return rc;
     AdjWs *w = ctx->adj;
     CKA(cudaMemcpyAsync(w->lam, Rbar, ctx->nq * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
-    CKA(launch_trace_exact(ctx->N, ctx->ncell, ctx->reg[0], w->tq, trace_stride(ctx->N, 8), ctx->ops, ctx->stream));
+    CKA(launch_trace_exact(ctx->N, ctx->ncell, ctx->reg[0], w->tq, trace_stride(ctx->N, 8), {ctx->err_flags}, ctx->ops, ctx->stream));
     CKA(cudaMemcpyAsync(w->host, ctx->maxima + 2 * ctx->slot, 2 * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
     CKA(cudaMemsetAsync(w->acc, 0, sizeof(AdjScalars), ctx->stream));
     CKA(cudaStreamSynchronize(ctx->stream));
@@ -523,7 +523,7 @@ extern "C" int sddc_adjoint_run(sddc_ctx *ctx, const sddc_adjoint_opts *o, doubl
     for (int s = 0; s < nseg; s++) {
         const int step0 = s * K, nst = std::min(K, ns - step0);
         CKA(cudaMemcpyAsync(S[0], ckpt[s], nq * sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream));
-        CKA(launch_trace_exact(ctx->N, ctx->ncell, S[0], T[0], trace_stride(ctx->N, 8), ctx->ops, ctx->stream));
+        CKA(launch_trace_exact(ctx->N, ctx->ncell, S[0], T[0], trace_stride(ctx->N, 8), {ctx->err_flags}, ctx->ops, ctx->stream));
         if (s == 0 && o->n1 == 0) CKA(wall_force(ctx, T[0], force));
         if ((rc = forward_steps(ctx, o->dt, step0, nst, S.data(), T.data(), hist, o->n1, o->n2, force, cmax,
                                 ctx->stream)))
@@ -614,7 +614,7 @@ extern "C" int sddc_adjoint_run(sddc_ctx *ctx, const sddc_adjoint_opts *o, doubl
         auto recompute = [&](int seg, int buf, cudaStream_t st) -> int {
             const int s0 = seg * K, n = std::min(K, ns - s0);
             CKA(cudaMemcpyAsync((*SS[buf])[0], ckpt[seg], nq * sizeof(double), cudaMemcpyDeviceToDevice, st));
-            CKA(launch_trace_exact(ctx->N, ctx->ncell, (*SS[buf])[0], (*TT[buf])[0], trace_stride(ctx->N, 8), ctx->ops, st));
+            CKA(launch_trace_exact(ctx->N, ctx->ncell, (*SS[buf])[0], (*TT[buf])[0], trace_stride(ctx->N, 8), {ctx->err_flags}, ctx->ops, st));
             return forward_steps(ctx, o->dt, s0, n, SS[buf]->data(), TT[buf]->data(), hist, 0, -1, nullptr, CM[buf], st);
         };
         for (int s = nseg - 1; s >= 0; s--) {

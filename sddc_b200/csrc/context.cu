@@ -166,7 +166,7 @@ static void free_all(sddc_ctx *ctx)
     for (auto &t : ctx->trace) cudaFree(t), t = nullptr;
     void *bufs[] = {ctx->met, ctx->nrm, ctx->jac, ctx->faces, ctx->maxima, ctx->sm_ind, ctx->muav, ctx->resid, ctx->grad,
                     ctx->mon_part, ctx->mon_out, ctx->int_part, ctx->wq,
-                    ctx->case_dev, ctx->tiles_rk, ctx->tiles_diag, ctx->visc_grad, ctx->visc_gt,
+                    ctx->case_dev, ctx->tiles, ctx->visc_grad, ctx->visc_gt,
                     ctx->visc_rv, ctx->met2, ctx->max_scratch, ctx->proc_cells};
     for (void *b : bufs) cudaFree(b);
     if (ctx->host_small) cudaFreeHost(ctx->host_small);
@@ -234,8 +234,7 @@ extern "C" int sddc_create(sddc_ctx **out, const sddc_params *p)
         if ((rc = alloc(ctx, &ctx->trace[r], ctx->trace_bytes, "face traces"))) return rc;
     }
     const size_t nc = p->ncell;
-    const int diag_grid = (p->ncell + kResidCpb - 1) / kResidCpb;
-    const int mon_blocks = std::max(ctx->grid, diag_grid);
+    const int mon_blocks = std::max(ctx->grid, resid_grid(ctx));
     ctx->nrm_double = p->precision != SDDC_MIXED;
     ctx->jac_inv = p->precision != SDDC_FP64_EXACT;
     const size_t n_nrm = nc * 4 * p->N * (p->N + 1), n_jac = nc * ((p->N * p->N + 1) & ~1);
@@ -468,9 +467,9 @@ static int refresh_traces(sddc_ctx *ctx)
 {
     cudaError_t e;
     switch (ctx->p.precision) {
-    case SDDC_FP64_EXACT: e = launch_trace_exact(ctx->N, ctx->ncell, ctx->reg[0], ctx->trace[0], ctx->tfs, ctx->ops, ctx->stream); break;
-    case SDDC_FP64: e = launch_trace_fp64(ctx->N, ctx->ncell, ctx->reg[0], ctx->trace[0], ctx->tfs, ctx->ops, ctx->stream); break;
-    default: e = launch_trace_mixed(ctx->N, ctx->ncell, ctx->reg[0], ctx->trace[0], ctx->tfs, ctx->ops, ctx->stream); break;
+    case SDDC_FP64_EXACT: e = launch_trace_exact(ctx->N, ctx->ncell, ctx->reg[0], ctx->trace[0], ctx->tfs, {ctx->err_flags}, ctx->ops, ctx->stream); break;
+    case SDDC_FP64: e = launch_trace_fp64(ctx->N, ctx->ncell, ctx->reg[0], ctx->trace[0], ctx->tfs, {ctx->err_flags}, ctx->ops, ctx->stream); break;
+    default: e = launch_trace_mixed(ctx->N, ctx->ncell, ctx->reg[0], ctx->trace[0], ctx->tfs, {ctx->err_flags}, ctx->ops, ctx->stream); break;
     }
     if (e != cudaSuccess) return cuda_err(ctx, e, "trace kernel");
     ctx->traces_stale = false;
@@ -549,6 +548,13 @@ static cudaError_t launch_visc(sddc_ctx *ctx, const double *q_in, const void *t_
     }
 }
 
+// a stage of the exact form, by the kernel that the context's tiles are for
+cudaError_t sddc::launch_rk_exact(sddc_ctx *ctx, const StageArgs &a, cudaStream_t st)
+{
+    return ctx->cpb == kTileCpb ? launch_tile_exact(ctx->N, a, ctx->ops, st)
+                                : launch_line_exact(ctx->N, a, ctx->ops, st);
+}
+
 static cudaError_t launch(sddc_ctx *ctx, bool diag, const StageArgs &a_in)
 {
     StageArgs a = a_in;
@@ -558,15 +564,15 @@ static cudaError_t launch(sddc_ctx *ctx, bool diag, const StageArgs &a_in)
         a.visc = ctx->visc_rv;
     }
     if (ctx->ncase) {  // a batch: one CTA per tile of the case-aligned tile table
-        a.tiles = diag ? ctx->tiles_diag : ctx->tiles_rk;
-        a.ntiles = diag ? ctx->ntiles_diag : ctx->ntiles_rk;
+        a.tiles = ctx->tiles;
+        a.ntiles = ctx->ntiles;
         a.cases = ctx->case_dev;
         a.persistent = ctx->persistent ? 1 : 0;
     }
     switch (ctx->p.precision) {
-    case SDDC_FP64_EXACT: return launch_stage_exact(ctx->N, ctx->cpb, diag, a, ctx->ops, ctx->stream);
-    case SDDC_FP64: return launch_stage_fp64(ctx->N, ctx->cpb, diag, a, ctx->ops, ctx->stream);
-    default: return launch_stage_mixed(ctx->N, ctx->cpb, diag, a, ctx->ops, ctx->stream);
+    case SDDC_FP64_EXACT: return diag ? launch_resid_exact(ctx->N, a, ctx->ops, ctx->stream) : launch_rk_exact(ctx, a, ctx->stream);
+    case SDDC_FP64: return diag ? launch_resid_fp64(ctx->N, a, ctx->ops, ctx->stream) : launch_line_fp64(ctx->N, a, ctx->ops, ctx->stream);
+    default: return diag ? launch_resid_mixed(ctx->N, a, ctx->ops, ctx->stream) : launch_line_mixed(ctx->N, a, ctx->ops, ctx->stream);
     }
 }
 
@@ -636,7 +642,7 @@ extern "C" int sddc_compresid(sddc_ctx *ctx)
     if ((rc = exchange(ctx, 0, a.slot_w))) return rc;
     ctx->slot = a.slot_w;
     ctx->sensor_stale = false;
-    ctx->mon_nblk = ctx->ncase ? ctx->ntiles_diag : (ctx->ncell + kResidCpb - 1) / kResidCpb;
+    ctx->mon_nblk = ctx->ncase ? ctx->ntiles : resid_grid(ctx);
     return check_flags(ctx);
 }
 
@@ -773,7 +779,7 @@ static int run_steps(sddc_ctx *ctx, double dt, int nsteps)
         s += n;
         ctx->stepped_dt = dt;
         ctx->sensor_stale = true;
-        ctx->mon_nblk = ctx->ncase ? ctx->ntiles_rk : ctx->grid;
+        ctx->mon_nblk = ctx->ncase ? ctx->ntiles : ctx->grid;
     }
     return check_flags(ctx);
 }
@@ -900,8 +906,9 @@ extern "C" int sddc_get_stream(sddc_ctx *ctx, void **stream)
 
 // ---------------------------------------------------------------- batches
 
-static int build_tiles(sddc_ctx *ctx, int cpb, int4 **dev, int *count)
+static int build_tiles(sddc_ctx *ctx)
 {
+    const int cpb = ctx->cpb;
     // persistent launches walk the table with a grid stride, largest case
     // first; otherwise the cases in their order
     std::vector<int> order(ctx->ncase);
@@ -915,12 +922,12 @@ static int build_tiles(sddc_ctx *ctx, int cpb, int4 **dev, int *count)
         for (int first = 0; first < k.ncell; first += cpb)
             tiles.push_back(make_int4(k.first_cell + first, std::min(cpb, k.ncell - first), c, first == 0 ? 1 : 0));
     }
-    cudaFree(*dev);
-    *dev = nullptr;
-    int rc = alloc(ctx, (void **)dev, tiles.size() * sizeof(int4), "tile table");
+    cudaFree(ctx->tiles);
+    ctx->tiles = nullptr;
+    int rc = alloc(ctx, (void **)&ctx->tiles, tiles.size() * sizeof(int4), "tile table");
     if (rc) return rc;
-    CK(cudaMemcpyAsync(*dev, tiles.data(), tiles.size() * sizeof(int4), cudaMemcpyHostToDevice, ctx->stream));
-    *count = (int)tiles.size();
+    CK(cudaMemcpyAsync(ctx->tiles, tiles.data(), tiles.size() * sizeof(int4), cudaMemcpyHostToDevice, ctx->stream));
+    ctx->ntiles = (int)tiles.size();
     return SDDC_OK;
 }
 
@@ -953,19 +960,17 @@ extern "C" int sddc_set_cases(sddc_ctx *ctx, int ncase, const sddc_case *cases)
     ctx->case_dev = nullptr;
     if ((rc = alloc(ctx, (void **)&ctx->case_dev, ncase * sizeof(CaseParams), "case table"))) return rc;
     CK(cudaMemcpyAsync(ctx->case_dev, cp.data(), ncase * sizeof(CaseParams), cudaMemcpyHostToDevice, ctx->stream));
-    if ((rc = build_tiles(ctx, ctx->cpb, &ctx->tiles_rk, &ctx->ntiles_rk))) return rc;
-    if ((rc = build_tiles(ctx, kResidCpb, &ctx->tiles_diag, &ctx->ntiles_diag))) return rc;
+    if ((rc = build_tiles(ctx))) return rc;
     // per-case running maxima and per-tile monitor partials
     cudaFree(ctx->maxima);
     cudaFree(ctx->mon_part);
     ctx->maxima = nullptr;
     ctx->mon_part = nullptr;
-    const int nmon = std::max(ctx->ntiles_rk, ctx->ntiles_diag);
     if ((rc = alloc(ctx, (void **)&ctx->maxima, (size_t)ncase * kSlots * 2 * sizeof(double), "maxima")) ||
-        (rc = alloc(ctx, (void **)&ctx->mon_part, (size_t)nmon * 2 * sizeof(double), "monitor")))
+        (rc = alloc(ctx, (void **)&ctx->mon_part, (size_t)ctx->ntiles * 2 * sizeof(double), "monitor")))
         return rc;
     CK(cudaMemsetAsync(ctx->maxima, 0, (size_t)ncase * kSlots * 2 * sizeof(double), ctx->stream));
-    CK(cudaMemsetAsync(ctx->mon_part, 0, (size_t)nmon * 2 * sizeof(double), ctx->stream));
+    CK(cudaMemsetAsync(ctx->mon_part, 0, (size_t)ctx->ntiles * 2 * sizeof(double), ctx->stream));
     drop_graphs(ctx);
     CK(cudaStreamSynchronize(ctx->stream));
     ctx->state = false;  // the maxima were reset: set the state again
@@ -977,11 +982,9 @@ extern "C" int sddc_set_persistent(sddc_ctx *ctx, int on)
 {
     if (!ctx) return SDDC_EINVAL;
     ctx->persistent = on != 0;
-    if (ctx->ncase) {  // the tile tables in the launch's order
-        int rc;
-        if ((rc = build_tiles(ctx, ctx->cpb, &ctx->tiles_rk, &ctx->ntiles_rk)) ||
-            (rc = build_tiles(ctx, kResidCpb, &ctx->tiles_diag, &ctx->ntiles_diag)))
-            return rc;
+    if (ctx->ncase) {  // the tile table in the launch's order
+        const int rc = build_tiles(ctx);
+        if (rc) return rc;
     }
     drop_graphs(ctx);
     CK(cudaStreamSynchronize(ctx->stream));

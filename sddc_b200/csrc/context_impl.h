@@ -16,12 +16,21 @@
 namespace sddc {
 struct AdjWs;
 struct Output;
-cudaError_t launch_stage_exact(int N, int cpb, bool diag, const StageArgs &a, const Ops &ops, cudaStream_t st);
-cudaError_t launch_stage_fp64(int N, int cpb, bool diag, const StageArgs &a, const Ops &ops, cudaStream_t st);
-cudaError_t launch_stage_mixed(int N, int cpb, bool diag, const StageArgs &a, const Ops &ops, cudaStream_t st);
-cudaError_t launch_trace_exact(int N, int ncell, const double *q, void *t, int tfs, const Ops &ops, cudaStream_t st);
-cudaError_t launch_trace_fp64(int N, int ncell, const double *q, void *t, int tfs, const Ops &ops, cudaStream_t st);
-cudaError_t launch_trace_mixed(int N, int ncell, const double *q, void *t, int tfs, const Ops &ops, cudaStream_t st);
+// RK stages by lines and (exact form, small meshes) by tiles; residual
+// evaluations; the face traces of a state
+cudaError_t launch_line_exact(int N, const StageArgs &a, const Ops &ops, cudaStream_t st);
+cudaError_t launch_line_fp64(int N, const StageArgs &a, const Ops &ops, cudaStream_t st);
+cudaError_t launch_line_mixed(int N, const StageArgs &a, const Ops &ops, cudaStream_t st);
+cudaError_t launch_tile_exact(int N, const StageArgs &a, const Ops &ops, cudaStream_t st);
+cudaError_t launch_resid_exact(int N, const StageArgs &a, const Ops &ops, cudaStream_t st);
+cudaError_t launch_resid_fp64(int N, const StageArgs &a, const Ops &ops, cudaStream_t st);
+cudaError_t launch_resid_mixed(int N, const StageArgs &a, const Ops &ops, cudaStream_t st);
+cudaError_t launch_trace_exact(int N, int ncell, const double *q, void *t, int tfs, const TraceInit &init,
+                               const Ops &ops, cudaStream_t st);
+cudaError_t launch_trace_fp64(int N, int ncell, const double *q, void *t, int tfs, const TraceInit &init,
+                              const Ops &ops, cudaStream_t st);
+cudaError_t launch_trace_mixed(int N, int ncell, const double *q, void *t, int tfs, const TraceInit &init,
+                               const Ops &ops, cudaStream_t st);
 struct ViscArgs;
 cudaError_t launch_visc_exact(int N, const ViscArgs &a, const Ops &ops, cudaStream_t st);
 cudaError_t launch_visc_fp64(int N, const ViscArgs &a, const Ops &ops, cudaStream_t st);
@@ -102,8 +111,8 @@ struct sddc_ctx {
     int ncase = 0;
     std::vector<sddc_case> cases;
     CaseParams *case_dev = nullptr;
-    int4 *tiles_rk = nullptr, *tiles_diag = nullptr;
-    int ntiles_rk = 0, ntiles_diag = 0;
+    int4 *tiles = nullptr;
+    int ntiles = 0;
     bool persistent = false;  // batch stages as grid-stride persistent launches
     // discrete adjoint work space (adjoint.cu), created on first use
     sddc::AdjWs *adj = nullptr;
@@ -133,7 +142,13 @@ SDDC_INTERNAL int alloc(sddc_ctx *ctx, void **p, size_t bytes, const char *what)
 SDDC_INTERNAL int ready(sddc_ctx *ctx);
 SDDC_INTERNAL int check_flags(sddc_ctx *ctx);  // synchronises the stream
 SDDC_INTERNAL unsigned take_flags(sddc_ctx *ctx);  // reads and clears, after a synchronisation
+SDDC_INTERNAL cudaError_t launch_rk_exact(sddc_ctx *ctx, const StageArgs &a, cudaStream_t st);
 SDDC_INTERNAL int met_size(int N);
+// CTAs of a residual evaluation of a single case
+inline int resid_grid(const sddc_ctx *ctx)
+{
+    return (ctx->ncell + line_tile_cells(ctx->N) - 1) / line_tile_cells(ctx->N);
+}
 SDDC_INTERNAL StageArgs base_args(sddc_ctx *ctx);
 SDDC_INTERNAL void adjoint_free(sddc_ctx *ctx);
 SDDC_INTERNAL void output_free(sddc_ctx *ctx);

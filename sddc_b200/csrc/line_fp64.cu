@@ -3,5 +3,7 @@
 #define SDDC_R double
 #define SDDC_EXACT_FORM false
 #define SDDC_LINE launch_line_fp64
+#define SDDC_RESID launch_resid_fp64
+#define SDDC_TRACE launch_trace_fp64
 #define SDDC_VISC launch_visc_fp64
 #include "line_launch.inc"

@@ -3,5 +3,7 @@
 #define SDDC_R float
 #define SDDC_EXACT_FORM false
 #define SDDC_LINE launch_line_mixed
+#define SDDC_RESID launch_resid_mixed
+#define SDDC_TRACE launch_trace_mixed
 #define SDDC_VISC launch_visc_mixed
 #include "line_launch.inc"

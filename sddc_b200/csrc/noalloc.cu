@@ -24,12 +24,15 @@
 #include "tables_pack.h"
 
 namespace sddc {
-cudaError_t launch_stage_exact(int N, int cpb, bool diag, const StageArgs &a, const Ops &ops, cudaStream_t st);
-cudaError_t launch_stage_fp64(int N, int cpb, bool diag, const StageArgs &a, const Ops &ops, cudaStream_t st);
-cudaError_t launch_stage_mixed(int N, int cpb, bool diag, const StageArgs &a, const Ops &ops, cudaStream_t st);
-cudaError_t launch_trace_exact(int N, int ncell, const double *q, void *t, int tfs, const Ops &ops, cudaStream_t st);
-cudaError_t launch_trace_fp64(int N, int ncell, const double *q, void *t, int tfs, const Ops &ops, cudaStream_t st);
-cudaError_t launch_trace_mixed(int N, int ncell, const double *q, void *t, int tfs, const Ops &ops, cudaStream_t st);
+cudaError_t launch_resid_exact(int N, const StageArgs &a, const Ops &ops, cudaStream_t st);
+cudaError_t launch_resid_fp64(int N, const StageArgs &a, const Ops &ops, cudaStream_t st);
+cudaError_t launch_resid_mixed(int N, const StageArgs &a, const Ops &ops, cudaStream_t st);
+cudaError_t launch_trace_exact(int N, int ncell, const double *q, void *t, int tfs, const TraceInit &init,
+                               const Ops &ops, cudaStream_t st);
+cudaError_t launch_trace_fp64(int N, int ncell, const double *q, void *t, int tfs, const TraceInit &init,
+                              const Ops &ops, cudaStream_t st);
+cudaError_t launch_trace_mixed(int N, int ncell, const double *q, void *t, int tfs, const TraceInit &init,
+                               const Ops &ops, cudaStream_t st);
 }  // namespace sddc
 
 using namespace sddc;
@@ -48,6 +51,7 @@ void *g_scratch_ptr[kMaxDevices] = {};  // device address of g_scratch, per devi
 // layout inside the scratch array (each part 256-byte aligned)
 struct ScratchLayout {
     size_t maxima, flags, sm_ind, trace, total;
+    int tfs;  // stride of a face's traces: whole 16-byte units where the array holds them
 };
 
 size_t up256(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -57,10 +61,12 @@ ScratchLayout layout(const sddc_params &p)
     ScratchLayout s;
     const size_t elem = p.precision == SDDC_MIXED ? sizeof(float) : sizeof(double);
     s.maxima = 0;                                               // [5][2] doubles
-    s.flags = up256(s.maxima + 10 * sizeof(double));            // unsigned
-    s.sm_ind = up256(s.flags + sizeof(unsigned));               // (2, NCELL) doubles
+    s.flags = s.maxima + 10 * sizeof(double);                   // unsigned, read back with the maxima
+    s.sm_ind = 512;                                             // (2, NCELL) doubles
     s.trace = up256(s.sm_ind + 2 * (size_t)p.ncell * sizeof(double));
-    s.total = s.trace + (size_t)p.ncell * 4 * p.N * 9 * elem;   // face traces
+    s.tfs = trace_stride(p.N, (int)elem);                       // face traces
+    if (s.trace + (size_t)p.ncell * 4 * s.tfs * elem > kScratchBytes) s.tfs = 9 * p.N;
+    s.total = s.trace + (size_t)p.ncell * 4 * s.tfs * elem;
     return s;
 }
 
@@ -162,23 +168,17 @@ extern "C" int sddc_compresid_noalloc(const sddc_params *p, const double *Lmat, 
     for (int s = 0; s < N; s++)
         for (int l = 0; l < NL; l++) ops.HL[s * NL + l] = lagrange(Xl, NL, l + 1, Xs[s]);
 
-    // clear what must start from zero; seed every running-max slot
+    // the face traces; the same launch seeds every running-max slot.  (The
+    // flags are zero when the library is loaded and cleared where one was read.)
     double *maxima = reinterpret_cast<double *>(scratch + L.maxima);
     unsigned *flags = reinterpret_cast<unsigned *>(scratch + L.flags);
-    double seed[10];
-    for (int s = 0; s < 5; s++) {
-        seed[2 * s] = eigvmax;
-        seed[2 * s + 1] = umax;
-    }
-    cudaError_t e = cudaMemcpyAsync(maxima, seed, sizeof(seed), cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(flags, 0, sizeof(unsigned), st);
-    if (e != cudaSuccess) return fail(SDDC_ECUDA, std::string("scratch set-up: ") + cudaGetErrorString(e));
-
+    const TraceInit init{flags, maxima, eigvmax, umax};
     void *trace = scratch + L.trace;
+    cudaError_t e;
     switch (p->precision) {
-    case SDDC_FP64_EXACT: e = launch_trace_exact(N, p->ncell, q_dev, trace, 9 * N, ops, st); break;
-    case SDDC_FP64: e = launch_trace_fp64(N, p->ncell, q_dev, trace, 9 * N, ops, st); break;
-    default: e = launch_trace_mixed(N, p->ncell, q_dev, trace, 9 * N, ops, st); break;
+    case SDDC_FP64_EXACT: e = launch_trace_exact(N, p->ncell, q_dev, trace, L.tfs, init, ops, st); break;
+    case SDDC_FP64: e = launch_trace_fp64(N, p->ncell, q_dev, trace, L.tfs, init, ops, st); break;
+    default: e = launch_trace_mixed(N, p->ncell, q_dev, trace, L.tfs, init, ops, st); break;
     }
     if (e != cudaSuccess) return fail(SDDC_ECUDA, std::string("trace kernel: ") + cudaGetErrorString(e));
 
@@ -191,7 +191,7 @@ extern "C" int sddc_compresid_noalloc(const sddc_params *p, const double *Lmat, 
     a.rk_kind = kRkNone;
     a.q_in = q_dev;
     a.t_in = trace;
-    a.tfs = 9 * N;
+    a.tfs = L.tfs;
     a.met = met_dev;
     a.faces = reinterpret_cast<const int2 *>(faces_dev);
     a.maxima = maxima;
@@ -203,23 +203,26 @@ extern "C" int sddc_compresid_noalloc(const sddc_params *p, const double *Lmat, 
     a.mon_part = nullptr;
     a.err_flags = flags;
     switch (p->precision) {
-    case SDDC_FP64_EXACT: e = launch_stage_exact(N, kResidCpb, true, a, ops, st); break;
-    case SDDC_FP64: e = launch_stage_fp64(N, kResidCpb, true, a, ops, st); break;
-    default: e = launch_stage_mixed(N, kResidCpb, true, a, ops, st); break;
+    case SDDC_FP64_EXACT: e = launch_resid_exact(N, a, ops, st); break;
+    case SDDC_FP64: e = launch_resid_fp64(N, a, ops, st); break;
+    default: e = launch_resid_mixed(N, a, ops, st); break;
     }
-    if (e != cudaSuccess) return fail(SDDC_ECUDA, std::string("stage kernel: ") + cudaGetErrorString(e));
+    if (e != cudaSuccess) return fail(SDDC_ECUDA, std::string("residual kernel: ") + cudaGetErrorString(e));
 
     // running maxima after the evaluation and the fault flags
-    double out[2];
-    unsigned f = 0;
-    e = cudaMemcpyAsync(out, maxima + 2, sizeof(out), cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&f, flags, sizeof(unsigned), cudaMemcpyDeviceToHost, st);
+    struct {
+        double maxima[10];
+        unsigned flags;
+    } out;
+    e = cudaMemcpyAsync(&out, maxima, L.flags + sizeof(unsigned), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return fail(SDDC_ECUDA, std::string("read-back: ") + cudaGetErrorString(e));
     if (maxima_out) {
-        maxima_out[0] = out[0];
-        maxima_out[1] = out[1];
+        maxima_out[0] = out.maxima[2];
+        maxima_out[1] = out.maxima[3];
     }
-    if (f) return fail(SDDC_ENUMERIC, "device numerics: non-positive density or non-finite wave speed");
+    if (out.flags && (e = cudaMemsetAsync(flags, 0, sizeof(unsigned), st)) != cudaSuccess)
+        return fail(SDDC_ECUDA, std::string("clearing the flags: ") + cudaGetErrorString(e));
+    if (out.flags) return fail(SDDC_ENUMERIC, "device numerics: non-positive density or non-finite wave speed");
     return SDDC_OK;
 }

@@ -192,7 +192,9 @@ template <typename R, bool EX>
 SDDC_HD void rusanov(const R *Qfl, const R *Qfr, R *Fnl, R *Fnr, R n0, R n1, int sign_l,
                                         int sign_r, R c_h, R &eigv_out, R &umax)
 {
-    const R magnorm = Sqrt(n0 * n0 + n1 * n1);
+    R magnorm;
+    if constexpr (EX) magnorm = Sqrt(n0 * n0 + n1 * n1);
+    else magnorm = Sqrt(fma(n0, n0, n1 * n1));  // one contraction in every kernel this is inlined into
     R unit_x, unit_y, ul, vl, wl, ur, vr, wr, pl, pr;
     const R Bxl = Qfl[5], Byl = Qfl[6], Bzl = Qfl[7], psil = Qfl[8];
     const R Bxr = Qfr[5], Byr = Qfr[6], Bzr = Qfr[7], psir = Qfr[8];

@@ -1,8 +1,43 @@
-// FP64 exact form of the stage kernel: the reference's operations in its
-// order, compiled with -fmad=false (no FMA contraction).
-#define SDDC_R double
-#define SDDC_EXACT_FORM true
-#define SDDC_LAUNCH launch_stage_exact
-#define SDDC_TRACE launch_trace_exact
-#define SDDC_LINE launch_line_exact
-#include "stage_launch.inc"
+// The exact form's RK stage by tiles, for small meshes: the reference's
+// operations in its order, compiled with -fmad=false (no FMA contraction).
+#include <algorithm>
+
+#include "stage_kernel.cuh"
+
+namespace sddc {
+
+namespace {
+
+template <int N> cudaError_t launch_n(const StageArgs &a, const Ops &ops, cudaStream_t st)
+{
+    auto kern = stage_kernel<N, kTileCpb>;
+    constexpr size_t smem = stage_smem_bytes<N, kTileCpb>();
+    static bool configured = false;  // per instantiation
+    if (!configured) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+        // the whole unified L1/shared array as shared memory, so that several
+        // CTAs fit on an SM
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+        if (e != cudaSuccess) return e;
+        configured = true;
+    }
+    kern<<<(a.ncell + kTileCpb - 1) / kTileCpb, stage_threads(N, kTileCpb), smem, st>>>(a, ops);
+    return cudaGetLastError();
+}
+
+}  // namespace
+
+cudaError_t launch_tile_exact(int N, const StageArgs &a, const Ops &ops, cudaStream_t st)
+{
+    switch (N) {
+    case 2: return launch_n<2>(a, ops, st);
+    case 3: return launch_n<3>(a, ops, st);
+    case 4: return launch_n<4>(a, ops, st);
+    case 5: return launch_n<5>(a, ops, st);
+    case 6: return launch_n<6>(a, ops, st);
+    default: return cudaErrorInvalidValue;
+    }
+}
+
+}  // namespace sddc

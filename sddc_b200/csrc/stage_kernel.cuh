@@ -1,38 +1,31 @@
-// The fused residual (+ RK stage) kernel of the SDDC drop-in, by tiles.
+// What the stage kernels share (their arguments, operators, TMA copies, face
+// traces), and the RK stage of the exact form by tiles, for small meshes
+// (small_exact_mesh).  Every other stage runs in line_kernel
+// (line_kernel.cuh), a residual evaluation in resid_kernel
+// (resid_kernel.cuh), both with a thread per line of solution points.
 //
 // One launch evaluates compresid (compresid.f90:1-80, compflux.f90:1-104,
 // interfaceflux_all.f90:1-112, cyclocflux_all.f90:1-112, bcflux.f90:1-377,
-// nablaQsp compflux.f90:107-157, the AV sensor AV.f90:1-142) for every cell.
-// It serves residual evaluations in every form, with the gradients of all
-// nine variables and the sensor, and the time step's stages of the exact
-// form on small meshes (small_exact_mesh), where it also applies the RK
-// stage update (iterations.f90:88-213).  All other stages run in line_kernel
-// (line_kernel.cuh), which keeps a line's values in registers.
+// nablaQsp compflux.f90:107-157) for every cell and applies the RK stage
+// update (iterations.f90:88-213).
 //
-// Work split: one CTA owns CPB consecutive cells and stages them in shared
-// memory.  Phases, separated by __syncthreads:
+// Work split: one CTA owns kTileCpb consecutive cells and stages them in
+// shared memory.  Phases, separated by __syncthreads:
 //   A  Lagrange interpolation of every line of solution points to its N+1
 //      flux points (one thread per cell x line index x variable: the xi-
-//      and eta-line of one index share the operator row, so their sums go
-//      through paired FMAs);
-//   B1 physical flux at the interior flux points (thread per point; the
-//      FP64 and mixed forms form F n0 + G n1 directly along the normal);
+//      and eta-line of one index share the operator row);
+//   B1 physical flux at the interior flux points (thread per point);
 //   B2 Rusanov flux at the 4N face points of each cell (thread per point).
 //      The neighbour's trace at the face point comes from the trace buffer
 //      (trace_at) that the stage producing the input published.  Each
 //      shared face is evaluated by both of its cells, each with the
 //      reference's left/right assignment, so both get the value the
-//      reference scatters to them.  Its loads from global memory are issued
-//      early in the FP64 and mixed forms: the face record before the
-//      staging wait, the neighbour's trace before B1 (all after B1 in the
-//      exact form);
-//   C  divergence of the flux, gradients from the face-averaged flux-point
-//      states, Powell and GLM sources (thread per solution point);
-//   D  the AV smoothness sensor per cell (residual evaluations only);
-//   E  in a time step, the RK stage update of each point by the thread of
-//      phase C: the RK register slice was staged by TMA with the state, the
+//      reference scatters to them;
+//   C  divergence of the flux, B gradients from the face-averaged flux-point
+//      states, Powell and GLM sources and the RK update (thread per solution
+//      point): the RK register slice was staged by TMA with the state, the
 //      output is formed in shared memory and stored by one TMA bulk copy
-//      while phase F runs; in a residual evaluation, the residual copy-out;
+//      while phase F runs;
 //   F  the face traces of the output state, published for the next stage.
 // Running maxima of the wave speed and of the velocity (the c_h input of
 // the next stage) go through atomicMax on five rotating slots, so that
@@ -52,14 +45,13 @@ constexpr int kMaxN = 6;
 // up to whole warps
 __host__ __device__ constexpr int stage_threads(int n, int cpb) { return (4 * n * cpb + 31) / 32 * 32; }
 
-// Cells per CTA of a time step's stages (line_kernel.cuh, 2N threads per
-// cell): one or two warps with few idle lanes.
+// Cells per CTA of the kernels by lines (2N threads per cell): one or two
+// warps with few idle lanes.
 __host__ __device__ constexpr int line_tile_cells(int n)
 {
     return n == 2 ? 8 : n == 3 ? 10 : n == 4 ? 8 : n == 5 ? 6 : 2;
 }
 
-constexpr int kResidCpb = 8;  // cells per CTA of a residual evaluation
 // Time steps of the exact form on meshes of fewer cells than this take the
 // tile kernel with kTileCpb cells per CTA: a line's 2N+2 dependent point
 // fluxes, in unfused operations, are a longer chain than the tile's phases,
@@ -143,10 +135,9 @@ struct StageArgs {
     const double *reg_c;
     const double *reg_d;
     double *resid_w;                   // residual copy (FiveStageRk stage 4 resid0)
-    const double *__restrict__ met;    // packed metrics, per cell
-    // the same metrics split for direct staging: normals in the arithmetic
-    // type [NCELL][4N(N+1)] and Jac [NCELL][MetLayout::kJacPad]; null: the
-    // kernel converts the packed record
+    const double *__restrict__ met;    // packed metrics, per cell (residual evaluations)
+    // the same metrics split for the stages: normals in the arithmetic type
+    // [NCELL][4N(N+1)] and Jac [NCELL][MetLayout::kJacPad]
     const void *__restrict__ nrm;
     const double *__restrict__ jac;
     int jac_inv;                       // jac holds 1/Jac (the forms other than the exact one)
@@ -162,6 +153,14 @@ struct StageArgs {
     double *__restrict__ cta_max;      // per-CTA (max eigv, max umax) of this stage, or null
     const double *__restrict__ visc;   // dFv + dGv (9,N,N,NCELL) of the viscous chain, or null (mu = eta0 = 0)
     unsigned *err_flags;
+};
+
+// beside the state and the traces, what a launch of the face traces takes: the
+// error flags and, where not null, the running-max slots it sets to a seed
+struct TraceInit {
+    unsigned *flags;
+    double *maxima = nullptr;
+    double eig = 0.0, um = 0.0;
 };
 
 // packed per-cell metric record: normals of both flux-point families, then Jac
@@ -240,13 +239,11 @@ __device__ __forceinline__ void bulk_prefetch_l2(const void *src, unsigned bytes
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
 }
 
-template <int N, typename R, bool DIAG> struct Smem {
+template <int N> struct Smem {
     static constexpr int NQ = 9 * N * N;
     static constexpr int NP = N + 1;
-    static constexpr int NG = DIAG ? 9 : 2;  // variables of the face-averaged state kept
-    static constexpr int kF = 2 * N * NP * 9;   // R per cell: state then flux at every flux point
-    static constexpr int kV = 2 * N * NP * NG;  // R per cell: face-averaged state at every flux point
-    static constexpr int kLow = 2 * (N - 1) * (N - 1);
+    static constexpr int kF = 2 * N * NP * 9;  // per cell: state then flux at every flux point
+    static constexpr int kV = 2 * N * NP * 2;  // per cell: face-averaged Bx, By at every flux point
 };
 
 // Lagrange coefficient access in the arithmetic type
@@ -309,7 +306,7 @@ __host__ __device__ __forceinline__ size_t trace_at(int tfs, size_t cell, int lf
 // the stride of a context's records in values of elem bytes: 9N rounded up to
 // whole 16-byte units, so that asynchronous copies move a face at a time
 // (6.7% more at N = 5 in the mixed form, none at N = 4).  The allocation-free
-// entry packs its records (stride 9N): its scratch array is fixed.
+// entry packs its records (stride 9N) where its fixed scratch array holds no more.
 __host__ __device__ constexpr int trace_stride(int n, int elem) { return (9 * n * elem + 15) / 16 * 16 / elem; }
 template <int N, typename R> __host__ __device__ constexpr int trace_stride() { return trace_stride(N, sizeof(R)); }
 
@@ -330,40 +327,35 @@ __device__ __forceinline__ double warp_sum(double v)
     return v;
 }
 
-template <int N, int CPB, typename R, bool DIAG> constexpr size_t stage_smem_bytes()
+template <int N, int CPB> constexpr size_t stage_smem_bytes()
 {
-    using S = Smem<N, R, DIAG>;
-    // sQ, sA, sJac, the AV operators; the sensor's sJz and sLow in residual
-    // evaluations only
-    size_t d = (size_t)CPB * (2 * S::NQ + MetLayout<N>::kJacPad + (DIAG ? N * N + S::kLow : 0)) + 4 * 32 + 2 * (N - 1) * N;
-    size_t r = (size_t)CPB * (S::kF + S::kV + 2 * MetLayout<N>::kFam) + 2 * (N + 1) * N;
-    return d * sizeof(double) + r * sizeof(R);
+    using S = Smem<N>;
+    return sizeof(double) * ((size_t)CPB * (2 * S::NQ + MetLayout<N>::kJacPad + S::kF + S::kV + 2 * MetLayout<N>::kFam) +
+                             4 * 32 + 2 * (N + 1) * N);
 }
 
 // CTAs per SM the kernel is compiled for: as many as the 228 KB of shared
 // memory per SM hold (1 KB per CTA is the driver's), but no fewer than 96
 // registers per thread, and at most 8
-template <int N, int CPB, typename R, bool DIAG> constexpr int stage_min_blocks()
+template <int N, int CPB> constexpr int stage_min_blocks()
 {
-    int b = (int)((228 * 1024) / (stage_smem_bytes<N, CPB, R, DIAG>() + 1024));
+    int b = (int)((228 * 1024) / (stage_smem_bytes<N, CPB>() + 1024));
     b = b < 1 ? 1 : (b > 8 ? 8 : b);
     while (b > 1 && 65536 / (stage_threads(N, CPB) * b) < 96) b--;
     return b;
 }
 
-// One tile (CPB consecutive cells, or an entry of a batch's tile table) by
-// the whole CTA; false if the staging copies timed out (the CTA stops).
-// EXACT instantiations are compiled without FMA contraction (-fmad=false) in
-// their own translation unit; they reproduce the reference's FP64 rounding.
-template <int N, int CPB, typename R, bool DIAG, bool EXACT>
-__device__ __forceinline__ bool stage_tile(const StageArgs &a, const Ops &ops, const int tile)
+// Compiled without FMA contraction (-fmad=false): the reference's operations
+// in its order.
+template <int N, int CPB>
+__global__ void __launch_bounds__(stage_threads(N, CPB), (stage_min_blocks<N, CPB>()))
+    stage_kernel(const StageArgs a, const Ops ops)
 {
-    constexpr bool EX = EXACT && (sizeof(R) == sizeof(double));
-    static_assert(DIAG || EX, "time steps of the other forms run in line_kernel");
-    using S = Smem<N, R, DIAG>;
+    using R = double;
+    using S = Smem<N>;
     using ML = MetLayout<N>;
     constexpr int NT = stage_threads(N, CPB);  // whole warps: the reductions use full-warp masks
-    constexpr int NQ = S::NQ, NP = S::NP, NG = S::NG;
+    constexpr int NQ = S::NQ, NP = S::NP, NG = 2;
     constexpr int NN = N * N;
 
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -371,15 +363,10 @@ __device__ __forceinline__ bool stage_tile(const StageArgs &a, const Ops &ops, c
     constexpr int NJ = ML::kJacPad;
     double *sQ = reinterpret_cast<double *>(smem_raw);          // [CPB][NQ]
     double *sJac = sQ + CPB * NQ;                                // [CPB][NJ]
-    double *sJz = sJac + CPB * NJ;                               // [CPB][NN]  Jz^2 for the sensor (DIAG)
-    double *sLow = sJz + (DIAG ? CPB * NN : 0);                  // [CPB][kLow] (DIAG)
     constexpr int NWR = 32;
-    double *sRed = sLow + (DIAG ? CPB * S::kLow : 0);            // [4][NWR] block reductions
-    // residual (DIAG); in a time step the RK register, then the output
-    double *sA = sRed + 4 * NWR;                                 // [CPB][NQ]
-    double *sOpH = sA + CPB * NQ;                                // [N-1][N]  AV projection
-    double *sOpHL = sOpH + (N - 1) * N;         // [N][N-1]  AV prolongation (DIAG)
-    R *sNrm = reinterpret_cast<R *>(sOpHL + N * (N - 1));  // [CPB][NM] flux-point normals
+    double *sRed = sJac + CPB * NJ;                              // [4][NWR] block reductions
+    double *sA = sRed + 4 * NWR;                                 // [CPB][NQ] the RK register, then the output
+    R *sNrm = sA + CPB * NQ;                                     // [CPB][NM] flux-point normals
     R *sF = sNrm + CPB * NM;                // [CPB][2][N][NP][9]
     R *sV = sF + CPB * S::kF;                                    // [CPB][2][N][NP][NG]
     // operators read with lane-dependent indices live in shared memory
@@ -387,69 +374,38 @@ __device__ __forceinline__ bool stage_tile(const StageArgs &a, const Ops &ops, c
     R *sOpL = sV + CPB * S::kV;                                  // [NP][N]
     R *sOpM = sOpL + NP * N;                                     // [NP][N]
 
-    const int tid = threadIdx.x;
-    int c0, ncl, cs;
-    bool first_tile;
-    if (a.tiles) {
-        const int4 tl = a.tiles[tile];
-        c0 = tl.x;
-        ncl = tl.y;
-        cs = tl.z;
-        first_tile = tl.w != 0;
-    } else {
-        c0 = tile * CPB;
-        ncl = min(CPB, a.ncell - c0);  // cells of this CTA
-        cs = 0;
-        first_tile = tile == 0;
-    }
-    // per-case data is read where it is used (kept out of registers)
-    double *maxima = a.maxima + 10 * cs;
-    // the face record of this thread's face point (a cell has 4N face points
-    // and at least 4N threads: one face point per thread at most), loaded
-    // before the staging wait (in the exact form with the rest of the face
-    // point's inputs, after B1: measured faster there); a thread has one face
-    // point at most
+    const int tid = threadIdx.x, tile = blockIdx.x;
+    const int c0 = tile * CPB, ncl = min(CPB, a.ncell - c0);  // cells of this CTA
+    double *maxima = a.maxima;
+    // a thread has one face point at most (a cell has 4N of them)
     const bool has_fp = tid < ncl * 4 * N;
-    int2 frec = make_int2(0, 0);
-    if (!EX && has_fp) frec = __ldg(a.faces + (size_t)c0 * 4 + tid / N);
 
     // ---- stage the state, the metrics and the operators ------------------------
     // The tile's state slice goes to sQ, its normals to sNrm and Jac to sJac
-    // (or, without the split metric arrays, its packed metric records to the
-    // flux buffer, free until phase A, for conversion) and, in a stage that
-    // reads one RK register, that register's slice to sA, by TMA bulk copies
-    // that one thread issues when every slice is 16-byte aligned; otherwise
-    // by batches of loads.
+    // and, in a stage that reads one RK register, that register's slice to sA,
+    // by TMA bulk copies that one thread issues when every slice is 16-byte
+    // aligned; otherwise by batches of loads.
     __shared__ __align__(8) unsigned long long sBar;
     __shared__ int sAbort;
-    double *sMetRaw = reinterpret_cast<double *>(sF);
-    const bool split = a.nrm != nullptr;  // uniform
-    const bool want_ra = !DIAG && (a.rk_kind == kRkTwoReg || a.rk_kind == kRkTwoRegT);
+    const bool want_ra = a.rk_kind == kRkTwoReg || a.rk_kind == kRkTwoRegT;
     const size_t qbytes = (size_t)ncl * NQ * sizeof(double);
-    const size_t mbytes = split ? 0 : (size_t)ncl * ML::kSize * sizeof(double);
-    const size_t nbytes = split ? (size_t)ncl * NM * sizeof(R) : 0;
-    const size_t jbytes = split ? (size_t)ncl * NJ * sizeof(double) : 0;
+    const size_t nbytes = (size_t)ncl * NM * sizeof(R);
+    const size_t jbytes = (size_t)ncl * NJ * sizeof(double);
     const double *qsrc = a.q_in + (size_t)c0 * NQ;
-    const double *msrc0 = a.met + (size_t)c0 * ML::kSize;
-    const R *nsrc = split ? reinterpret_cast<const R *>(a.nrm) + (size_t)c0 * NM : nullptr;
-    const double *jsrc = split ? a.jac + (size_t)c0 * NJ : nullptr;
+    const R *nsrc = reinterpret_cast<const R *>(a.nrm) + (size_t)c0 * NM;
+    const double *jsrc = a.jac + (size_t)c0 * NJ;
     const double *rsrc = want_ra ? a.reg_a + (size_t)c0 * NQ : nullptr;
     const bool bulk = ((uintptr_t)qsrc & 15) == 0 && (qbytes & 15) == 0 &&
-                      (split ? (((uintptr_t)nsrc | (uintptr_t)jsrc | nbytes | jbytes) & 15) == 0
-                             : (((uintptr_t)msrc0 | mbytes) & 15) == 0) &&
+                      (((uintptr_t)nsrc | (uintptr_t)jsrc | nbytes | jbytes) & 15) == 0 &&
                       (!want_ra || ((uintptr_t)rsrc & 15) == 0);  // uniform in the CTA
     if (tid == 0) {
         sAbort = 0;
         if (bulk) {
             mbar_init(&sBar, 1);
-            mbar_expect_tx(&sBar, (unsigned)(qbytes + mbytes + nbytes + jbytes + (want_ra ? qbytes : 0)));
+            mbar_expect_tx(&sBar, (unsigned)(qbytes + nbytes + jbytes + (want_ra ? qbytes : 0)));
             bulk_g2s(sQ, qsrc, (unsigned)qbytes, &sBar);
-            if (split) {
-                bulk_g2s(sNrm, nsrc, (unsigned)nbytes, &sBar);
-                bulk_g2s(sJac, jsrc, (unsigned)jbytes, &sBar);
-            } else {
-                bulk_g2s(sMetRaw, msrc0, (unsigned)mbytes, &sBar);
-            }
+            bulk_g2s(sNrm, nsrc, (unsigned)nbytes, &sBar);
+            bulk_g2s(sJac, jsrc, (unsigned)jbytes, &sBar);
             if (want_ra) bulk_g2s(sA, rsrc, (unsigned)qbytes, &sBar);
         }
     }
@@ -457,11 +413,6 @@ __device__ __forceinline__ bool stage_tile(const StageArgs &a, const Ops &ops, c
         sOpL[k] = opL<R>(ops, k);
         sOpM[k] = opM<R>(ops, k);
     }
-    if constexpr (DIAG)
-        for (int k = tid; k < (N - 1) * N; k += NT) {
-            sOpH[k] = ops.H[k];
-            sOpHL[k] = ops.HL[k];
-        }
     if (!bulk) {
         // batches of kU independent loads per thread before their stores, so
         // that each thread keeps several loads in flight
@@ -477,12 +428,8 @@ __device__ __forceinline__ bool stage_tile(const StageArgs &a, const Ops &ops, c
             }
         };
         stage_copy(sQ, qsrc, ncl * NQ);
-        if (split) {
-            stage_copy(sNrm, nsrc, ncl * NM);
-            stage_copy(sJac, jsrc, ncl * NJ);
-        } else {
-            stage_copy(sMetRaw, msrc0, ncl * ML::kSize);
-        }
+        stage_copy(sNrm, nsrc, ncl * NM);
+        stage_copy(sJac, jsrc, ncl * NJ);
         if (want_ra) stage_copy(sA, rsrc, ncl * NQ);
     }
     const double eig_r = maxima[2 * a.slot_r], um_r = maxima[2 * a.slot_r + 1];
@@ -496,18 +443,7 @@ __device__ __forceinline__ bool stage_tile(const StageArgs &a, const Ops &ops, c
         mbar_wait_bounded(&sBar, 0);
     }
     __syncthreads();
-    if (sAbort) return false;
-    if (!split) {
-        // the metric record: normals (rounded once to the arithmetic type) and Jac
-        for (int k = tid; k < ncl * ML::kSize; k += NT) {
-            const int c = k / ML::kSize, o = k - c * ML::kSize;
-            const double v = sMetRaw[k];
-            if (o < NM) sNrm[c * NM + o] = (R)v;
-            else if (o < NM + NN) sJac[c * NJ + (o - NM)] = v;
-        }
-        __syncthreads();
-    }
-
+    if (sAbort) return;
     // ---- A: interpolate every line to its flux points ---------------------------
     // one thread per (cell, line index l, variable): xi-line l and eta-line l
     // together, their sums paired (both use the same operator row)
@@ -536,61 +472,7 @@ __device__ __forceinline__ bool stage_tile(const StageArgs &a, const Ops &ops, c
     R eigmax = (R)0, umax = (R)0;
     unsigned err = 0;
 
-    // ---- B2's inputs from global memory (the neighbour's trace or the
-    // received remote trace, the normals).  The forms other than the exact
-    // one gather them before B1, so that their latency overlaps the interior
-    // fluxes (measured faster there; slower in the exact form, which gathers
-    // them after B1)
-    constexpr bool kGatherEarly = !EX;
-    R other[9];
-    R on0 = (R)0, on1 = (R)0, pn0 = (R)0, pn1 = (R)0;
-    auto gather = [&]() {
-        if (has_fp) {
-            if constexpr (EX) frec = __ldg(a.faces + (size_t)c0 * 4 + tid / N);
-            const int nfp = 1 + tid % N, lf = 1 + (tid / N) % 4, c = tid / (4 * N);
-            int fam, line, r;
-            face_point<N>(lf, nfp, fam, line, r);
-            const int kind = frec.y & 0xff;
-            const R *nrm = sNrm + c * NM + ML::normal(fam, line, r);
-            on0 = nrm[0]; on1 = nrm[1];
-            if (kind == kFaceProc) {
-                // the received trace, remote point N+1-nfp (procintflux_all.f90:83-99)
-                const R *rv = reinterpret_cast<const R *>(a.proc_recv) + ((size_t)frec.x * N + (N - nfp)) * 9;
-#pragma unroll
-                for (int k = 0; k < 9; k++) other[k] = rv[k];
-            } else if (kind == kFaceLeft || kind == kFaceRight) {
-                // partner point N-nfp+1 on the partner's local face; its trace was
-                // published by the stage that produced q_in
-                const int pc = frec.x, plf = (frec.y >> 8) & 0xff;
-                const R *tp = reinterpret_cast<const R *>(a.t_in);
-#pragma unroll
-                for (int k = 0; k < 9; k++) other[k] = tp[trace_at<N>(a.tfs, pc, plf, N - nfp, k)];
-                if (kind == kFaceRight) {
-                    // the left (partner) cell's normal, from the split array or
-                    // the packed record
-                    int pfam, pline, pr;
-                    face_point<N>(plf, N - nfp + 1, pfam, pline, pr);
-                    if (split) {
-                        const R *pn = reinterpret_cast<const R *>(a.nrm) + (size_t)pc * NM + ML::normal(pfam, pline, pr);
-                        pn0 = __ldg(pn);
-                        pn1 = __ldg(pn + 1);
-                    } else {
-                        const double *pn = a.met + (size_t)pc * ML::kSize + ML::normal(pfam, pline, pr);
-                        pn0 = (R)__ldg(pn);
-                        pn1 = (R)__ldg(pn + 1);
-                    }
-                }
-            }
-        }
-    };
-    if constexpr (kGatherEarly) gather();
-
     // ---- B1: interior flux points (inviscid_flux_interior) ---------------------
-    // the normal of family f, line l, flux point r of cell c
-    auto normal_at = [&](int c, int f, int l, int r, R &n0, R &n1) {
-        const R *nrm = sNrm + c * NM + ML::normal(f, l, r);
-        n0 = nrm[0]; n1 = nrm[1];
-    };
     for (int t = tid; t < ncl * 2 * N * (N - 1); t += NT) {
         const int r = 1 + t % (N - 1), l = (t / (N - 1)) % N, f = (t / ((N - 1) * N)) % 2,
                   c = t / (2 * N * (N - 1));
@@ -599,31 +481,17 @@ __device__ __forceinline__ bool stage_tile(const StageArgs &a, const Ops &ops, c
 #pragma unroll
         for (int k = 0; k < 9; k++) q[k] = slot[k];
         if (!(q[0] > (R)0)) err |= kErrNonPositiveDensity;
-        R n0, n1;
-        normal_at(c, f, l, r, n0, n1);
-        if constexpr (EX) {
-            // the reference's F and G, projected
-            R F[9], G[9];
-            iflux<R, EX>(q, c_h, umax, F, G);
+        const R *nrm = sNrm + c * NM + ML::normal(f, l, r);
+        const R n0 = nrm[0], n1 = nrm[1];
+        // the reference's F and G, projected
+        R F[9], G[9];
+        iflux<R, true>(q, c_h, umax, F, G);
 #pragma unroll
-            for (int k = 0; k < 9; k++) slot[k] = F[k] * n0 + G[k] * n1;
-        } else {
-            R Fn[9];
-            iflux_n<R>(q, c_h, n0, n1, umax, Fn);
-#pragma unroll
-            for (int k = 0; k < 9; k++) slot[k] = Fn[k];
-        }
+        for (int k = 0; k < 9; k++) slot[k] = F[k] * n0 + G[k] * n1;
         R *vs = sV + c * S::kV + ((f * N + l) * NP + r) * NG;
-        if constexpr (DIAG) {
-#pragma unroll
-            for (int k = 0; k < 9; k++) vs[k] = q[k];
-        } else {
-            vs[0] = q[5];
-            vs[1] = q[6];
-        }
+        vs[0] = q[5];
+        vs[1] = q[6];
     }
-
-    if constexpr (!kGatherEarly) gather();
 
     // ---- B2: face points (interfaceflux, CYCLOCFLUX, BCFLUX) -------------------
     if (has_fp) {
@@ -634,34 +502,40 @@ __device__ __forceinline__ bool stage_tile(const StageArgs &a, const Ops &ops, c
         R own[9], Fl[9], Fr[9];
 #pragma unroll
         for (int k = 0; k < 9; k++) own[k] = slot[k];
+        const int2 frec = __ldg(a.faces + (size_t)c0 * 4 + tid / N);
         const int kind = frec.y & 0xff;
-        R n0, n1;
-        int sign_l, sign_r;
         const bool pair = kind == kFaceLeft || kind == kFaceRight;
         const bool own_right = kind == kFaceRight;
+        const R *nrm = sNrm + c * NM + ML::normal(fam, line, r);
+        R n0 = nrm[0], n1 = nrm[1], other[9];
+        int sign_l = r == 0 ? -1 : 1, sign_r = 1;
         if (kind == kFaceProc) {
-            // PROCINTFLUX / CYCREMFLUX (procintflux_all.f90:104-151): this
-            // cell is the left cell, with its own normal and sign_r = 1
-            n0 = on0; n1 = on1;
-            sign_l = r == 0 ? -1 : 1;
-            sign_r = 1;
+            // PROCINTFLUX / CYCREMFLUX (procintflux_all.f90:83-151): this cell
+            // is the left cell; the received trace, remote point N+1-nfp
+            const R *rv = reinterpret_cast<const R *>(a.proc_recv) + ((size_t)frec.x * N + (N - nfp)) * 9;
+#pragma unroll
+            for (int k = 0; k < 9; k++) other[k] = rv[k];
         } else if (pair) {
+            // partner point N-nfp+1 on the partner's local face; its trace was
+            // published by the stage that produced q_in
+            const int pc = frec.x, plf = (frec.y >> 8) & 0xff;
+            const R *tp = reinterpret_cast<const R *>(a.t_in);
+#pragma unroll
+            for (int k = 0; k < 9; k++) other[k] = tp[trace_at<N>(a.tfs, pc, plf, N - nfp, k)];
             int pfam, pline, pr;
-            face_point<N>((frec.y >> 8) & 0xff, N - nfp + 1, pfam, pline, pr);
-            if (!own_right) {
-                n0 = on0; n1 = on1;
-                sign_l = r == 0 ? -1 : 1;
-                sign_r = pr == N ? -1 : 1;
-            } else {
-                n0 = pn0; n1 = pn1;
+            face_point<N>(plf, N - nfp + 1, pfam, pline, pr);
+            if (own_right) {
+                // the left (partner) cell's normal
+                const R *pn = reinterpret_cast<const R *>(a.nrm) + (size_t)pc * NM + ML::normal(pfam, pline, pr);
+                n0 = __ldg(pn);
+                n1 = __ldg(pn + 1);
                 sign_l = pr == 0 ? -1 : 1;
                 sign_r = r == N ? -1 : 1;
+            } else {
+                sign_r = pr == N ? -1 : 1;
             }
         } else {
-            n0 = on0; n1 = on1;
-            sign_l = r == 0 ? -1 : 1;
-            sign_r = 1;
-            bc_ghost<R, EX>(kind, own, n0, n1, a.vismode, a.cases ? a.cases[cs].fs : a.fs, other);
+            bc_ghost<R, true>(kind, own, n0, n1, a.vismode, a.fs, other);
         }
         // left and right states by element-wise selects (arrays picked
         // through a pointer would live in local memory)
@@ -673,19 +547,14 @@ __device__ __forceinline__ bool stage_tile(const StageArgs &a, const Ops &ops, c
         }
         if (!(Ql[0] > (R)0) || !(Qr[0] > (R)0)) err |= kErrNonPositiveDensity;
         R eig_face;
-        rusanov<R, EX>(Ql, Qr, Fl, Fr, n0, n1, sign_l, sign_r, c_h, eig_face, umax);
+        rusanov<R, true>(Ql, Qr, Fl, Fr, n0, n1, sign_l, sign_r, c_h, eig_face, umax);
         if (!(Abs(eig_face) < (R)INFINITY)) err |= kErrNonFiniteWaveSpeed;
         if (eig_face > eigmax) eigmax = eig_face;
 #pragma unroll
         for (int k = 0; k < 9; k++) slot[k] = own_right ? Fr[k] : Fl[k];
         R *vs = sV + c * S::kV + ((fam * N + line) * NP + r) * NG;
-        if constexpr (DIAG) {
-#pragma unroll
-            for (int k = 0; k < 9; k++) vs[k] = (R)0.5 * Ql[k] + (R)0.5 * Qr[k];
-        } else {
-            vs[0] = (R)0.5 * Ql[5] + (R)0.5 * Qr[5];
-            vs[1] = (R)0.5 * Ql[6] + (R)0.5 * Qr[6];
-        }
+        vs[0] = (R)0.5 * Ql[5] + (R)0.5 * Qr[5];
+        vs[1] = (R)0.5 * Ql[6] + (R)0.5 * Qr[6];
     }
     __syncthreads();
 
@@ -719,21 +588,14 @@ __device__ __forceinline__ bool stage_tile(const StageArgs &a, const Ops &ops, c
     // in a time step the RK coefficients of the stage (phase E runs here)
     // formed where used, from the kernel parameters (not held in registers
     // through the phase)
-    const double cdt = a.cases ? a.cases[cs].dt : a.dt;
+    const double cdt = a.dt;
     auto cf = [&](int i) -> double { return ((a.dt_mask >> i) & 1u) ? a.cb[i] * cdt : a.cb[i]; };
     double part_r = 0.0, part_d = 0.0;
     for (int t = tid; t < ncl * NN; t += NT) {
         const int i = t % N, j = (t / N) % N, c = t / NN;
         const int cell = c0 + c;
         const R *met = sNrm + c * NM;
-        // Jac, or its reciprocal when the split array holds reciprocals (the
-        // exact form divides by Jac, as the reference does; the others multiply
-        // by 1/Jac, rounded once, on the host or here)
-        const double Jv = sJac[c * NJ + i + N * j];
-        double J = Jv, rJ = Jv;
-        if constexpr (!EX) {
-            if (!a.jac_inv) rJ = 1.0 / Jv;
-        }
+        const double J = sJac[c * NJ + i + N * j];
         const R *Fx = sF + c * S::kF + (0 * N + j) * NP * 9;  // xi-line j
         const R *Fy = sF + c * S::kF + (1 * N + i) * NP * 9;  // eta-line i
         const R *Vx = sV + c * S::kV + (0 * N + j) * NP * NG;
@@ -742,12 +604,6 @@ __device__ __forceinline__ bool stage_tile(const StageArgs &a, const Ops &ops, c
         double gB[2][2] = {{0.0, 0.0}, {0.0, 0.0}};  // [Bx,By][x,y]
         // with vismode == 0 the reference never fills nablaQs; its divB
         // source then reads the zeros of the fresh allocation
-        if constexpr (DIAG) {
-            if (a.vismode != 1 && a.grad_out) {
-                double *go = a.grad_out + (size_t)cell * (18 * NN) + 18 * (i + N * j);
-                for (int k = 0; k < 18; k++) go[k] = 0.0;
-            }
-        }
 #pragma unroll
         for (int g = 0; g < NG; g++) {
             if (a.vismode != 1) break;
@@ -764,30 +620,10 @@ __device__ __forceinline__ bool stage_tile(const StageArgs &a, const Ops &ops, c
                 bx = bx + my * met[ML::normal(1, i, r)];
                 by = by + my * met[ML::normal(1, i, r) + 1];
             }
-            double gx, gy;
-            if constexpr (EX) {
-                gx = (double)(ax + bx) / J;
-                gy = (double)(ay + by) / J;
-            } else {
-                gx = (double)(ax + bx) * rJ;
-                gy = (double)(ay + by) * rJ;
-            }
-            const int var = DIAG ? g : g + 5;
-            if (var == 5) { gB[0][0] = gx; gB[0][1] = gy; }
-            if (var == 6) { gB[1][0] = gx; gB[1][1] = gy; }
-            if constexpr (DIAG) {
-                if (a.grad_out) {
-                    double *go = a.grad_out + (size_t)cell * (18 * NN) + 18 * (i + N * j);
-                    go[g] = gx;
-                    go[9 + g] = gy;
-                }
-            }
+            gB[g][0] = (double)(ax + bx) / J;
+            gB[g][1] = (double)(ay + by) / J;
         }
         const double divB = gB[0][0] + gB[1][1];
-        if constexpr (DIAG) {
-            const double d = gB[1][0] - gB[0][1];
-            sJz[c * NN + i + N * j] = d * d;
-        }
         // compresid.f90:12-51 divergence of the inviscid flux: the line sums
         // of phase C1 sit in point slot i of xi-line j and slot j of eta-line i
         double res[9];
@@ -796,32 +632,16 @@ __device__ __forceinline__ bool stage_tile(const StageArgs &a, const Ops &ops, c
             const R dF = Fx[i * 9 + k], dG = Fy[j * 9 + k];
             res[k] = (double)(-(dF + dG));
             // the viscous chain (compresid.f90:34-49); it adds exactly +0.0
-            // when mu == eta0 == 0, which only the exact form reproduces (it
-            // turns a -0.0 residual into +0.0)
-            if constexpr (EX) {
-                if (a.vismode == 1) res[k] = res[k] + (a.visc ? a.visc[(size_t)cell * NQ + 9 * (i + N * j) + k] : 0.0);
-            } else {
-                if (a.vismode == 1 && a.visc) res[k] = res[k] + a.visc[(size_t)cell * NQ + 9 * (i + N * j) + k];
-            }
+            // when mu == eta0 == 0 (which turns a -0.0 residual into +0.0)
+            if (a.vismode == 1) res[k] = res[k] + (a.visc ? a.visc[(size_t)cell * NQ + 9 * (i + N * j) + k] : 0.0);
         }
         // compresid.f90:53-78: 1/Jac, Powell 8-wave and GLM sources
         const double *q = sQ + c * NQ + 9 * (i + N * j);
-        if constexpr (EX) {
-            quotients<9>(res, J, res);
-        } else {
-#pragma unroll
-            for (int k = 0; k < 9; k++) res[k] = res[k] * rJ;
-        }
+        quotients<9>(res, J, res);
         const double Bx = q[5], By = q[6], Bz = q[7], psi = q[8];
-        double ux, uy, uz;
-        if constexpr (EX) {
-            double uu[3];
-            quotients<3>(q + 1, q[0], uu);
-            ux = uu[0]; uy = uu[1]; uz = uu[2];
-        } else {
-            const double ri = 1.0 / q[0];
-            ux = q[1] * ri; uy = q[2] * ri; uz = q[3] * ri;
-        }
+        double uu[3];
+        quotients<3>(q + 1, q[0], uu);
+        const double ux = uu[0], uy = uu[1], uz = uu[2];
         res[1] = res[1] - divB * Bx;
         res[2] = res[2] - divB * By;
         res[3] = res[3] - divB * Bz;
@@ -836,152 +656,50 @@ __device__ __forceinline__ bool stage_tile(const StageArgs &a, const Ops &ops, c
             part_d += divB * divB;
         }
         double *ap = sA + c * NQ + 9 * (i + N * j);
-        if constexpr (DIAG) {
-            // stage the residual for phase E's copy-out
+        // the RK stage update of this point (iterations.f90:88-213);
+        // the point's state and RK register slot are read by this thread
+        // only, so the output goes to the register slot in place
+        const size_t g = (size_t)cell * NQ + 9 * (i + N * j);
+        const int kind = a.rk_kind;
 #pragma unroll
-            for (int k = 0; k < 9; k++) ap[k] = res[k];
-        } else {
-            // ---- E: the RK stage update of this point (iterations.f90:88-213);
-            // the point's state and RK register slot are read by this thread
-            // only, so the output goes to the register slot in place
-            const size_t g = (size_t)cell * NQ + 9 * (i + N * j);
-            const int kind = a.rk_kind;
-#pragma unroll
-            for (int k = 0; k < 9; k++) {
-                const double qk = q[k], r = res[k];
-                double o;
-                switch (kind) {
-                case kRkAxpy: o = qk + cf(0) * r; break;
-                case kRkTwoReg: o = (cf(1) * ap[k] + cf(2) * qk) + cf(0) * r; break;
-                case kRkTwoRegT: o = (cf(1) * ap[k] + cf(2) * qk) + (cf(0) * r) * cf(3); break;
-                default:
-                    o = ((((cf(1) * a.reg_a[g + k] + cf(2) * a.reg_b[g + k]) + cf(3) * a.reg_c[g + k]) + cf(4) * qk) +
-                         cf(5) * a.reg_d[g + k]) +
-                        cf(0) * r;
-                    break;
-                }
-                ap[k] = o;
-                if (a.resid_w) a.resid_w[g + k] = r;
+        for (int k = 0; k < 9; k++) {
+            const double qk = q[k], r = res[k];
+            double o;
+            switch (kind) {
+            case kRkAxpy: o = qk + cf(0) * r; break;
+            case kRkTwoReg: o = (cf(1) * ap[k] + cf(2) * qk) + cf(0) * r; break;
+            case kRkTwoRegT: o = (cf(1) * ap[k] + cf(2) * qk) + (cf(0) * r) * cf(3); break;
+            default:
+                o = ((((cf(1) * a.reg_a[g + k] + cf(2) * a.reg_b[g + k]) + cf(3) * a.reg_c[g + k]) + cf(4) * qk) +
+                     cf(5) * a.reg_d[g + k]) +
+                    cf(0) * r;
+                break;
             }
-            fence_proxy_async();  // sA is the source of the bulk store below
+            ap[k] = o;
+            if (a.resid_w) a.resid_w[g + k] = r;
         }
+        fence_proxy_async();  // sA is the source of the bulk store below
     }
     __syncthreads();
 
-    // ---- D: AV smoothness sensor (comp_artificial_viscosity, AV.f90:14-83) ------
-    const bool av = DIAG && a.artiv == 1 && a.vismode == 1;
-    if constexpr (DIAG) if (av) {
-        constexpr int NL = N - 1;
-        // the sensed fields: density (v = 0) and Jz^2 (v = 1)
-        auto field = [&](int c, int v, int is, int js) -> double {
-            return v == 0 ? sQ[c * NQ + 9 * (is + N * js)] : sJz[c * NN + is + N * js];
-        };
-        // the flux buffer is free after phase C: it holds the separable
-        // projection's intermediate products
-        double *sTmp = reinterpret_cast<double *>(sF);  // [CPB][2][NL][N]
-        if constexpr (EX) {
-            // projection to the N-1 points with the reference's double sum
-            for (int t = tid; t < ncl * 2 * NL * NL; t += NT) {
-                const int isl = t % NL, jsl = (t / NL) % NL, v = (t / (NL * NL)) % 2, c = t / (2 * NL * NL);
-                double acc = 0.0;
-                for (int js = 0; js < N; js++)
-#pragma unroll
-                    for (int is = 0; is < N; is++)
-                        acc = acc + field(c, v, is, js) * sOpH[isl * N + is] * sOpH[jsl * N + js];
-                sLow[c * S::kLow + v * NL * NL + isl + NL * jsl] = acc;
-            }
-        } else {
-            // the same projection as two one-dimensional passes
-            for (int t = tid; t < ncl * 2 * NL * N; t += NT) {
-                const int isl = t % NL, js = (t / NL) % N, v = (t / (NL * N)) % 2, c = t / (2 * NL * N);
-                double acc = 0.0;
-#pragma unroll
-                for (int is = 0; is < N; is++) acc += field(c, v, is, js) * sOpH[isl * N + is];
-                sTmp[((c * 2 + v) * N + js) * NL + isl] = acc;
-            }
-            __syncthreads();
-            for (int t = tid; t < ncl * 2 * NL * NL; t += NT) {
-                const int isl = t % NL, jsl = (t / NL) % NL, v = (t / (NL * NL)) % 2, c = t / (2 * NL * NL);
-                double acc = 0.0;
-#pragma unroll
-                for (int js = 0; js < N; js++) acc += sTmp[((c * 2 + v) * N + js) * NL + isl] * sOpH[jsl * N + js];
-                sLow[c * S::kLow + v * NL * NL + isl + NL * jsl] = acc;
-            }
-        }
-        __syncthreads();
-        // projection back to the solution points and the terms of the sensor
-        // sum, one thread per (cell, variable, point); the face-state buffer
-        // is free after phase C and holds the terms
-        double *sTerm = reinterpret_cast<double *>(sV);  // [CPB][2][NN]
-        if constexpr (!EX) {
-            for (int t = tid; t < ncl * 2 * N * NL; t += NT) {
-                const int is = t % N, jsl = (t / N) % NL, v = (t / (N * NL)) % 2, c = t / (2 * N * NL);
-                const double *lo = sLow + c * S::kLow + v * NL * NL;
-                double acc = 0.0;
-#pragma unroll
-                for (int isl = 0; isl < NL; isl++) acc += lo[isl + NL * jsl] * sOpHL[is * NL + isl];
-                sTmp[((c * 2 + v) * NL + jsl) * N + is] = acc;
-            }
-            __syncthreads();
-        }
-        for (int t = tid; t < ncl * 2 * NN; t += NT) {
-            const int is = t % N, js = (t / N) % N, v = (t / NN) % 2, c = t / (2 * NN);
-            double hi = 0.0;
-            if constexpr (EX) {
-                const double *lo = sLow + c * S::kLow + v * NL * NL;
-                for (int jsl = 0; jsl < NL; jsl++)
-#pragma unroll
-                    for (int isl = 0; isl < NL; isl++)
-                        hi = hi + lo[isl + NL * jsl] * sOpHL[is * NL + isl] * sOpHL[js * NL + jsl];
-            } else {
-#pragma unroll
-                for (int jsl = 0; jsl < NL; jsl++) hi += sTmp[((c * 2 + v) * NL + jsl) * N + is] * sOpHL[js * NL + jsl];
-            }
-            const double x = field(c, v, is, js);
-            const double d = hi - x;
-            sTerm[(c * 2 + v) * NN + is + N * js] = d * d / (x * x);
-        }
-        __syncthreads();
-        // the sum in the reference's (js, is) order
-        for (int t = tid; t < ncl * 2; t += NT) {
-            const double *tm = sTerm + t * NN;
-            double se = 0.0;
-#pragma unroll
-            for (int k = 0; k < NN; k++) se = se + tm[k];
-            a.sm_ind[2 * (size_t)c0 + t] = log10(se);
-        }
-    }
-
-    // ---- E: residual copy-out (residual evaluation) or the output store ---------
-    const double *qout_src = nullptr;
-    bool out_bulk = false;
-    {
-        const size_t g0 = (size_t)c0 * NQ;
-        const int n = ncl * NQ;
-        if constexpr (DIAG) {
-            if (a.resid_out)
-                for (int e = tid; e < n; e += NT) a.resid_out[g0 + e] = sA[e];
-        } else {
-            // the output slice (formed in sA by phase C) to q_out: one bulk
-            // store issued by one thread, read from shared memory while phase
-            // F runs, or coalesced stores when the slice is not 16-byte aligned
-            double *dst = a.q_out + g0;
-            out_bulk = (((uintptr_t)dst | (size_t)n * sizeof(double)) & 15) == 0;
-            if (out_bulk) {
-                if (tid == 0) bulk_s2g(dst, sA, (unsigned)(n * sizeof(double)));
-            } else {
-                for (int e = tid; e < n; e += NT) dst[e] = sA[e];
-            }
-            qout_src = sA;
-        }
+    // ---- the output slice (formed in sA) to q_out: one bulk store issued by one
+    // thread, read from shared memory while phase F runs, or coalesced stores
+    // when the slice is not 16-byte aligned ----------------------------------------
+    double *dst = a.q_out + (size_t)c0 * NQ;
+    const int n = ncl * NQ;
+    const bool out_bulk = (((uintptr_t)dst | (size_t)n * sizeof(double)) & 15) == 0;
+    if (out_bulk) {
+        if (tid == 0) bulk_s2g(dst, sA, (unsigned)(n * sizeof(double)));
+    } else {
+        for (int e = tid; e < n; e += NT) dst[e] = sA[e];
     }
 
     // ---- F: face traces of the output state for the next stage's neighbours ---
     // (the barrier after phase C orders its output before these reads: in a
     // time step nothing between them writes shared memory)
-    if (!DIAG && a.t_out) {
+    if (a.t_out) {
         R *to = reinterpret_cast<R *>(a.t_out);
-        const R *qo = reinterpret_cast<const R *>(qout_src);
+        const R *qo = sA;
         // one thread per (cell, family, variable, line): the line's N values
         // give the traces at both of its ends (r = 0 and r = N), each summed
         // in order as phase A sums them
@@ -1012,16 +730,7 @@ __device__ __forceinline__ bool stage_tile(const StageArgs &a, const Ops &ops, c
     {
         const int lane = tid & 31, wid = tid >> 5;
         constexpr int NW = (NT + 31) / 32;
-        double em, um;
-        if constexpr (sizeof(R) == sizeof(float)) {
-            // the maxima are non-negative (never raised by NaN), and
-            // non-negative floats order as their bit patterns
-            em = (double)__uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(eigmax)));
-            um = (double)__uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(umax)));
-        } else {
-            em = warp_max((double)eigmax);
-            um = warp_max((double)umax);
-        }
+        const double em = warp_max(eigmax), um = warp_max(umax);
         unsigned e = __reduce_or_sync(0xffffffffu, err);
         double pr = 0.0, pd = 0.0;
         if (a.mon_part) {
@@ -1046,7 +755,7 @@ __device__ __forceinline__ bool stage_tile(const StageArgs &a, const Ops &ops, c
             }
             atomic_max_nonneg(&maxima[2 * a.slot_w], m0);
             atomic_max_nonneg(&maxima[2 * a.slot_w + 1], m1);
-            if (first_tile) {  // carry the previous stages' maxima forward
+            if (tile == 0) {  // carry the previous stages' maxima forward
                 // (re-read: slot_r is not written during the stage)
                 atomic_max_nonneg(&maxima[2 * a.slot_w], maxima[2 * a.slot_r]);
                 atomic_max_nonneg(&maxima[2 * a.slot_w + 1], maxima[2 * a.slot_r + 1]);
@@ -1064,37 +773,6 @@ __device__ __forceinline__ bool stage_tile(const StageArgs &a, const Ops &ops, c
             if (out_bulk) bulk_wait_read();
             if (bulk) mbar_inval(&sBar);
         }
-    }
-    return true;
-}
-
-template <int N, int CPB, typename R, bool DIAG, bool EXACT>
-__global__ void __launch_bounds__(stage_threads(N, CPB), (stage_min_blocks<N, CPB, R, DIAG>()))
-    stage_kernel(const StageArgs a, const Ops ops)
-{
-    stage_tile<N, CPB, R, DIAG, EXACT>(a, ops, blockIdx.x);
-}
-
-// Face traces of a state: T[trace_at(tfs, cell, lf, nfp, k)] = sum_s Q(k, line
-// points) * L(r, s) at the flux point of local face lf, face point nfp -- the
-// same interpolation, in the same order and type, as phase A and phase F.
-template <int N, typename R, bool EXACT>  // EXACT: compiled with -fmad=false, like phase A
-__global__ void trace_kernel(int ncell, const double *__restrict__ q, R *__restrict__ t, int tfs, const Ops ops)
-{
-    const size_t n = (size_t)ncell * 4 * N * 9;
-    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
-        const int nfp = 1 + (int)(e % N), k = (int)((e / N) % 9), lf = 1 + (int)((e / (9 * N)) % 4);
-        const size_t c = e / (36 * N);
-        int fam, line, r;
-        face_point<N>(lf, nfp, fam, line, r);
-        const double *qc = q + c * (9 * N * N);
-        R acc = (R)0;
-#pragma unroll
-        for (int s = 0; s < N; s++) {
-            const double x = fam == 0 ? qc[k + 9 * (s + N * line)] : qc[k + 9 * (line + N * s)];
-            acc = acc + (R)x * opL<R>(ops, r * N + s);
-        }
-        t[trace_at<N>(tfs, c, lf, nfp - 1, k)] = acc;
     }
 }
 

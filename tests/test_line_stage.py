@@ -12,6 +12,7 @@ import sddc_oracle as O
 from helpers import channel_physics, rel_l2, smooth_state
 from sddc_b200 import cases, host, mesh
 from sddc_b200.solver import Solver
+from test_gpu_parity import _sensor_close
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 NVCC = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
@@ -200,3 +201,82 @@ def test_both_exact_kernels_agree_with_zeros_and_fault(N):
         out.append(seen)
     for (fa, qa), (fb, qb) in zip(*out):
         assert fa == fb and np.array_equal(qa, qb, equal_nan=True)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("N", sorted(TILE))
+def test_residual_lines_match_oracle_at_tile_edges(N):
+    """The residual, all gradients and the sensor; two evaluations in a row, so
+    that the second has c_h > 0."""
+    for ncell in sorted({1, 2, TILE[N] - 1, TILE[N], TILE[N] + 1, 3 * TILE[N] + 1}):
+        if ncell < 1:
+            continue
+        t, ph, Q, _ = _case(N, ncell)
+        o = O.Oracle(t, ph)
+        o.set_state(Q)
+        o.compresid()
+        o.compresid()
+        ref, mo = o.state(), o.maxima()
+        # the flux's rounding enters the residual magnified by |M| |F| / (J |resid|),
+        # up to about 3e3 on these meshes: 3e3 eps (1.1e-16 and 6e-8)
+        for form, bar in (("fp64_exact", 0.0), ("fp64", 4e-13), ("mixed", 2e-4)):
+            s = Solver(t, ph, precision=form)
+            s.set_state(Q)
+            s.compresid()
+            s.compresid()
+            g = s.state(resid=True, nablaQs=True, sm_ind=True)
+            if not bar:
+                _sensor_close(g["sm_ind"], ref["sm_ind"])
+            for k in ("resid", "nablaQs"):
+                if bar:
+                    assert rel_l2(g[k], ref[k]) <= bar, (form, ncell, k)
+                else:
+                    assert np.array_equal(g[k], ref[k]), (ncell, k)
+            if not bar:
+                mg = s.maxima()
+                assert (mg["eigvmax"], mg["umax"]) == (mo["eigvmax"], mo["umax"])
+            s.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("form", [0, 1, 2])
+@pytest.mark.parametrize("N,nx,ny", [(5, 9, 7), (5, 100, 115), (4, 9, 7), (3, 31, 1)])
+def test_caller_held_memory_at_any_eight_byte_address(N, nx, ny, form):
+    """Arrays that no 16-byte copy can move (and, at 100x115 cells, traces packed
+    into the scratch array) give the bits that aligned ones give."""
+    import ctypes
+
+    import torch
+    import test_zz_no_alloc as Z
+
+    torch.cuda.init()
+    L = Z._bind()
+    m = mesh.channel_box(nx, ny, sides=("WALL", "OUTL", "FREE", "INLE"), seed=N)
+    t = host.build_tables(m, N)
+    ph = channel_physics()
+    Q = smooth_state(t, ph, seed=nx)
+    met, faces = Z._packed(L, t)
+    p, ops = Z._params(t, ph, form), [np.asfortranarray(x) for x in (t.Lmat, t.Mmat)]
+    got = []
+    for shift in (0, 1):
+        def at(a):  # a copy on the device, `shift` doubles past an allocation's start
+            d = torch.empty(a.size + shift, dtype=torch.float64, device="cuda")
+            d[shift:] = torch.from_numpy(np.ravel(a, order="K"))
+            return d[shift:]
+        q, met_d, res, grad = at(Q), at(met), at(np.zeros(Q.size)), at(np.zeros(2 * Q.size))
+        faces_d = torch.from_numpy(faces).cuda()
+        out = np.zeros(2)
+        torch.cuda.synchronize()
+        rc = L.sddc_compresid_noalloc(ctypes.byref(p), *[Z._p(x) for x in ops], q.data_ptr(), met_d.data_ptr(),
+                                      faces_d.data_ptr(), 3.0, 1.0, res.data_ptr(), grad.data_ptr(), Z._p(out), None)
+        assert rc == 0, L.sddc_noalloc_last_error()
+        got.append((res.cpu().numpy(), grad.cpu().numpy(), out))
+    for a, b in zip(*got):
+        assert np.array_equal(a, b)
+    s = Solver(t, ph, precision=form)
+    s.set_state(Q, 0.0, 3.0, 1.0)
+    s.compresid()
+    st = s.state(resid=True, nablaQs=True)
+    s.close()
+    for a, k in zip(got[0], ("resid", "nablaQs")):
+        assert np.array_equal(a, np.ravel(st[k], order="K"))
