@@ -105,7 +105,7 @@ __host__ __device__ constexpr bool line_use_wide(int tiles, int resident_held, i
 template <int N, typename R, bool WIDE> constexpr int line_warps()
 {
     if (sizeof(R) == 4) return N >= 6 ? 12 : N >= 4 ? 16 : N == 3 ? 20 : 24;
-    return N >= 4 ? (WIDE ? 12 : 8) : N == 3 ? 12 : 16;
+    return N >= 4 && !WIDE ? 8 : 12;
 }
 template <int N, int CPB, typename R, bool EX, bool WIDE> constexpr int line_min_blocks()
 {
@@ -155,7 +155,7 @@ __device__ __forceinline__ bool line_tile(const StageArgs &a, const Ops &ops, co
     P2<R> *sP = reinterpret_cast<P2<R> *>(sX + CPB * TS);  // [2][NT]
     __shared__ __align__(8) unsigned long long sBar;
     __shared__ int sAbort;
-    __shared__ double sRed[4 * (NT / 32)];
+    __shared__ double sRed[4 * (NT / 32)], sCarry[2];
 
     const int tid = threadIdx.x;
     int c0, ncl, cs;
@@ -267,6 +267,10 @@ __device__ __forceinline__ bool line_tile(const StageArgs &a, const Ops &ops, co
             if (want_ra) sA[o] = rsrc[k];
         }
 
+    if (tid == 0) {
+        sCarry[0] = eig_r;
+        sCarry[1] = um_r;
+    }
     // compflux.f90:6 -- running maxima of all previous stages
     const R c_h = (R)sqrt(eig_r * (eig_r - um_r));
     cp_async_wait_all();
@@ -466,7 +470,43 @@ __device__ __forceinline__ bool line_tile(const StageArgs &a, const Ops &ops, co
         if constexpr (kHold) flux_at(N, G, W, m);
         accumulate(N, G, W, m);
     }
+    // the tile's maxima, sent while its points are finished (every one of them
+    // is non-negative, so they order as their bit patterns)
+    const int lane = tid & 31, wid = tid >> 5;
+    constexpr int NW = NT / 32;
+    double em, um;
+    if constexpr (sizeof(R) == sizeof(float)) {
+        em = (double)__uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(eigmax)));
+        um = (double)__uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(umax)));
+    } else {
+        em = warp_max_nonneg((double)eigmax);
+        um = warp_max_nonneg((double)umax);
+    }
+    const unsigned eb = __reduce_or_sync(0xffffffffu, err);
+    if (lane == 0) {
+        sRed[wid] = em;
+        sRed[NW + wid] = um;
+        if (eb) atomicOr(a.err_flags, eb);
+    }
     __syncthreads();  // the neighbours' traces are read: sX is free
+    if (tid == 0) {
+        double m0 = 0.0, m1 = 0.0;
+#pragma unroll
+        for (int w = 0; w < NW; w++) {
+            m0 = sRed[w] > m0 ? sRed[w] : m0;
+            m1 = sRed[NW + w] > m1 ? sRed[NW + w] : m1;
+        }
+        if (a.cta_max) {
+            a.cta_max[2 * tile] = m0;
+            a.cta_max[2 * tile + 1] = m1;
+        }
+        if (first_tile) {  // carry the previous stages' maxima forward
+            m0 = sCarry[0] > m0 ? sCarry[0] : m0;
+            m1 = sCarry[1] > m1 ? sCarry[1] : m1;
+        }
+        atomic_max_nonneg(&maxima[2 * a.slot_w], m0);
+        atomic_max_nonneg(&maxima[2 * a.slot_w + 1], m1);
+    }
 
     // ---- 3: hand over the sums of the points the crossing line finishes ------------
     // point t of the line is finished by this thread if (t + l + fam) is even
@@ -694,29 +734,15 @@ __device__ __forceinline__ bool line_tile(const StageArgs &a, const Ops &ops, co
     }
     fence_proxy_async();
 
-    // ---- reductions ----------------------------------------------------------------
-    const int lane = tid & 31, wid = tid >> 5;
-    constexpr int NW = NT / 32;
-    double em, um;
-    if constexpr (sizeof(R) == sizeof(float)) {
-        em = (double)__uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(eigmax)));
-        um = (double)__uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(umax)));
-    } else {
-        em = warp_max((double)eigmax);
-        um = warp_max((double)umax);
-    }
-    const unsigned eb = __reduce_or_sync(0xffffffffu, err);
+    // ---- the monitors' sums, the traces' store ----------------------------------------
     double pr = 0.0, pd = 0.0;
     if (a.mon_part) {
         pr = warp_sum(part_r);
         pd = warp_sum(part_d);
     }
-    if (lane == 0) {
-        sRed[wid] = em;
-        sRed[NW + wid] = um;
+    if (a.mon_part && lane == 0) {
         sRed[2 * NW + wid] = pr;
         sRed[3 * NW + wid] = pd;
-        if (eb) atomicOr(a.err_flags, eb);
     }
     __syncthreads();
     if (tid < 32) {
@@ -725,27 +751,15 @@ __device__ __forceinline__ bool line_tile(const StageArgs &a, const Ops &ops, co
             bulk_s2g(reinterpret_cast<R *>(a.t_out) + (size_t)(c0 + tid) * 4 * TFS, sT + tid * TS,
                      (unsigned)(4 * TFS * sizeof(R)));
         if (tid == 0) {
-            double m0 = 0.0, m1 = 0.0, s0 = 0.0, s1 = 0.0;
-#pragma unroll
-            for (int w = 0; w < NW; w++) {
-                m0 = sRed[w] > m0 ? sRed[w] : m0;
-                m1 = sRed[NW + w] > m1 ? sRed[NW + w] : m1;
-                s0 += sRed[2 * NW + w];
-                s1 += sRed[3 * NW + w];
-            }
-            atomic_max_nonneg(&maxima[2 * a.slot_w], m0);
-            atomic_max_nonneg(&maxima[2 * a.slot_w + 1], m1);
-            if (first_tile) {  // carry the previous stages' maxima forward
-                atomic_max_nonneg(&maxima[2 * a.slot_w], maxima[2 * a.slot_r]);
-                atomic_max_nonneg(&maxima[2 * a.slot_w + 1], maxima[2 * a.slot_r + 1]);
-            }
             if (a.mon_part) {
+                double s0 = 0.0, s1 = 0.0;
+#pragma unroll
+                for (int w = 0; w < NW; w++) {
+                    s0 += sRed[2 * NW + w];
+                    s1 += sRed[3 * NW + w];
+                }
                 a.mon_part[2 * tile] = s0;
                 a.mon_part[2 * tile + 1] = s1;
-            }
-            if (a.cta_max) {
-                a.cta_max[2 * tile] = m0;
-                a.cta_max[2 * tile + 1] = m1;
             }
             mbar_inval(&sBar);
         }

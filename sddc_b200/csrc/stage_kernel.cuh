@@ -320,6 +320,14 @@ template <typename T> __device__ __forceinline__ T warp_max(T v)
     return v;
 }
 
+// the same of non-negative doubles, which order as their bit patterns
+__device__ __forceinline__ double warp_max_nonneg(double v)
+{
+    const unsigned hi = (unsigned)__double2hiint(v), top = __reduce_max_sync(0xffffffffu, hi);
+    const unsigned lo = __reduce_max_sync(0xffffffffu, hi == top ? (unsigned)__double2loint(v) : 0u);
+    return __hiloint2double((int)top, (int)lo);
+}
+
 __device__ __forceinline__ double warp_sum(double v)
 {
 #pragma unroll
