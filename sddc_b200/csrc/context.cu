@@ -214,9 +214,9 @@ extern "C" int sddc_create(sddc_ctx **out, const sddc_params *p)
         return bad("cells_per_cta must be 0, 4, 6, 8 or 16");
     ctx->N = p->N;
     ctx->ncell = p->ncell;
-    // time steps run by lines, or (exact form) by tiles: see small_exact_mesh
+    // time steps run by lines, or (exact form) by tiles: see exact_by_tiles
     const bool tiles = p->precision == SDDC_FP64_EXACT &&
-                       (p->cells_per_cta ? p->cells_per_cta == kTileCpb : small_exact_mesh(p->N, p->ncell));
+                       (p->cells_per_cta ? p->cells_per_cta == kTileCpb : exact_by_tiles(p->N, p->ncell));
     ctx->cpb = tiles ? kTileCpb : line_tile_cells(p->N);
     if (!ctx->p.ncellglob) ctx->p.ncellglob = p->ncell;
     ctx->msize = met_size(p->N);

@@ -1,6 +1,6 @@
 // What the stage kernels share (their arguments, operators, TMA copies, face
 // traces), and the RK stage of the exact form by tiles, for small meshes
-// (small_exact_mesh).  Every other stage runs in line_kernel
+// (exact_by_tiles).  Every other stage runs in line_kernel
 // (line_kernel.cuh), a residual evaluation in resid_kernel
 // (resid_kernel.cuh), both with a thread per line of solution points.
 //
@@ -52,16 +52,32 @@ __host__ __device__ constexpr int line_tile_cells(int n)
     return n == 2 ? 8 : n == 3 ? 10 : n == 4 ? 8 : n == 5 ? 6 : 2;
 }
 
-// Time steps of the exact form on meshes of fewer cells than this take the
-// tile kernel with kTileCpb cells per CTA: a line's 2N+2 dependent point
-// fluxes, in unfused operations, are a longer chain than the tile's phases,
-// which shows while the mesh leaves SMs idle.  us per step, tile kernel and
-// line kernel: N = 4, 48^2 cells 58 and 66, 64^2 cells 76 and 74; N = 5,
-// 64^2 cells 152 and 169, 96^2 cells 299 and 290; N = 6, 32^2 cells 78 and 88,
-// 48^2 cells 146 and 103.  (The FP64 and mixed forms are no slower by lines at
-// 8^2 cells: 41 and 41, 38 and 31 at N = 4.)
+// Time steps of the exact form run by tiles of kTileCpb cells where that is
+// the faster of the two: a line's 2N+2 dependent point fluxes, in unfused
+// operations, are a longer chain than the tile's phases, which shows while the
+// mesh leaves SMs idle, and so is a last wave of CTAs by lines that is mostly
+// empty.  spare: the cells that would fill it.  us per stage, by tiles and by
+// lines: N = 3, 4096 cells 11.8 and 13.5, 4900 17.2 and 15.9, 9409 23.3 and
+// 28.8; N = 4, 2500 11.8 and 14.8, 7056 23.3 and 21.6, 8100 24.5 and 27.9, 9409
+// 29.4 and 27.6, 32400 96 and 86; N = 5, 4096 26.7 and 33.9, 7056 42.8 and 41.3,
+// 8100 44.6 and 53.1, 32400 178 and 165; N = 6, 1600 16.3 and 21.5, 4900 43.4
+// and 54.2, 9409 82.9 and 79.4.  (The FP64 and mixed forms always run by lines.)
 constexpr int kTileCpb = 4;
-__host__ __device__ constexpr bool small_exact_mesh(int n, int ncell) { return ncell < (n == 5 ? 5000 : n == 6 ? 1500 : 3500); }
+__host__ __device__ constexpr bool exact_by_tiles(int n, int ncell)
+{
+    // cells of a wave by lines: 12 warps per SM at N = 2, 3 and (line_has_wide) 4,
+    // else 8
+    const int wave = 148 * line_tile_cells(n) * (n == 2 ? 12 : n == 3 || n == 4 ? 6 : n == 6 ? 8 : 4);
+    const long spare = (wave - ncell % wave) % wave;
+    switch (n) {
+    case 2: return ncell < 4000;
+    case 3: return 2L * ncell < 3 * spare - 6000;
+    case 4:  // (up to 4736 cells, and near 9472, waves of 8 warps per SM serve, at 0.7 of the time)
+        return ncell <= 4736 || (ncell > wave && (ncell < 8800 || ncell > 9472) && ncell < 4 * spare);
+    case 5: return 2L * ncell < 13 * spare + 9800;
+    default: return 5L * ncell < 3 * spare + 37500;
+    }
+}
 
 // operators in kernel parameter space (row-major)
 struct Ops {
