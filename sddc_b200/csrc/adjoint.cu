@@ -50,6 +50,7 @@ struct AdjWs {
     int nwall = 0;
     double wq[kMaxN] = {};   // quadrature weights of the solution points
     double *host = nullptr;  // pinned read-back
+    cudaEvent_t maxima = nullptr;  // sddc_vjp_resid: the running maxima are on the host
     size_t bytes = 0;
 };
 
@@ -60,6 +61,7 @@ void adjoint_free(sddc_ctx *ctx)
     void *b[] = {w->at, w->at2, w->part, w->acc, w->recs, w->rec_n, w->lam, w->qbar, w->tq, w->wall};
     for (void *p : b) cudaFree(p);
     if (w->host) cudaFreeHost(w->host);
+    if (w->maxima) cudaEventDestroy(w->maxima);
     delete w;
     ctx->adj = nullptr;
 }
@@ -403,24 +405,31 @@ extern "C" int sddc_vjp_resid(sddc_ctx *ctx, const double *Rbar, double *Qbar, d
     int rc = check_adjoint_ctx(ctx);
     if (rc) return rc;
     AdjWs *w = ctx->adj;
-    CKA(cudaMemcpyAsync(w->lam, Rbar, ctx->nq * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
-    CKA(launch_trace_exact(ctx->N, ctx->ncell, ctx->reg[0], w->tq, trace_stride(ctx->N, 8), {ctx->err_flags}, ctx->ops, ctx->stream));
+    // the maxima that the launch arguments need arrive while Rbar travels
+    if (!w->maxima) CKA(cudaEventCreateWithFlags(&w->maxima, cudaEventDisableTiming));
     CKA(cudaMemcpyAsync(w->host, ctx->maxima + 2 * ctx->slot, 2 * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+    CKA(cudaEventRecord(w->maxima, ctx->stream));
+    CKA(cudaMemcpyAsync(w->lam, Rbar, ctx->nq * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
+    // the state's traces in the exact form's rounding: an exact context keeps them
+    const bool own = ctx->p.precision == SDDC_FP64_EXACT;
+    if (!own)
+        CKA(launch_trace_exact(ctx->N, ctx->ncell, ctx->reg[0], w->tq, trace_stride(ctx->N, 8), {ctx->err_flags},
+                               ctx->ops, ctx->stream));
     CKA(cudaMemsetAsync(w->acc, 0, sizeof(AdjScalars), ctx->stream));
-    CKA(cudaStreamSynchronize(ctx->stream));
+    CKA(cudaEventSynchronize(w->maxima));
     w->at_ready = false;
     RevStage s;
     s.q = ctx->reg[0];
-    s.t = w->tq;
+    s.t = own ? static_cast<const double *>(ctx->trace[0]) : w->tq;
     s.xbar = w->lam;
     s.scale = 1.0;
     s.out = w->qbar;
     s.L = s.Lnext = w->host[0];
     s.U = s.Unext = w->host[1];
     if ((rc = reverse_stage(ctx, s))) return rc;
-    CKA(cudaMemcpyAsync(Qbar, w->qbar, ctx->nq * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
     AdjScalars acc;
     CKA(cudaMemcpyAsync(w->host, w->acc, sizeof(AdjScalars), cudaMemcpyDeviceToHost, ctx->stream));
+    CKA(cudaMemcpyAsync(Qbar, w->qbar, ctx->nq * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
     CKA(cudaStreamSynchronize(ctx->stream));
     std::memcpy(&acc, w->host, sizeof(AdjScalars));
     if (parbar) {
