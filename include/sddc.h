@@ -60,10 +60,9 @@ typedef struct sddc_params {
     int artiv;      /* ARTIV: 1 computes the AV sensor                         */
     int k_stage;    /* 3: RK_S5P3, 5: FiveStageRk                              */
     int precision;  /* SDDC_FP64_EXACT, SDDC_FP64 or SDDC_MIXED                */
-    int cells_per_cta; /* 0, or 4, 6, 8 or 16.  The exact form has two stage kernels: 4
-                          asks for the one by tiles of 4 cells, another value for the
-                          one by lines, 0 leaves it to the mesh size.  The other
-                          forms and batches always step by lines, with a tile set by N */
+    int cells_per_cta; /* 0, or 4, 6, 8 or 16: accepted as a hint that no kernel needs
+                          any more.  Each form's kernel and tile follow from N and the
+                          mesh size */
     double mu, eta0;   /* viscosity and resistivity (QUAD.INP), >= 0            */
     double dxcycl, dycycl;
     double rinf, pinf, uinf, vinf, bxinf, byinf; /* free stream (QUAD.INP) */

@@ -215,9 +215,8 @@ extern "C" int sddc_create(sddc_ctx **out, const sddc_params *p)
     ctx->N = p->N;
     ctx->ncell = p->ncell;
     // time steps run by lines, or (exact form) by tiles: see exact_by_tiles
-    const bool tiles = p->precision == SDDC_FP64_EXACT &&
-                       (p->cells_per_cta ? p->cells_per_cta == kTileCpb : exact_by_tiles(p->N, p->ncell));
-    ctx->cpb = tiles ? kTileCpb : line_tile_cells(p->N);
+    ctx->by_tiles = p->precision == SDDC_FP64_EXACT && exact_by_tiles(p->N, p->ncell);
+    ctx->cpb = ctx->by_tiles ? tile_cells(p->N, p->ncell) : line_tile_cells(p->N);
     if (!ctx->p.ncellglob) ctx->p.ncellglob = p->ncell;
     ctx->msize = met_size(p->N);
     ctx->nq = (size_t)9 * p->N * p->N * p->ncell;
@@ -551,8 +550,8 @@ static cudaError_t launch_visc(sddc_ctx *ctx, const double *q_in, const void *t_
 // a stage of the exact form, by the kernel that the context's tiles are for
 cudaError_t sddc::launch_rk_exact(sddc_ctx *ctx, const StageArgs &a, cudaStream_t st)
 {
-    return ctx->cpb == kTileCpb ? launch_tile_exact(ctx->N, a, ctx->ops, st)
-                                : launch_line_exact(ctx->N, a, ctx->ops, st);
+    return ctx->by_tiles ? launch_tile_exact(ctx->N, ctx->cpb, a, ctx->ops, st)
+                         : launch_line_exact(ctx->N, a, ctx->ops, st);
 }
 
 static cudaError_t launch(sddc_ctx *ctx, bool diag, const StageArgs &a_in)
@@ -945,7 +944,8 @@ extern "C" int sddc_set_cases(sddc_ctx *ctx, int ncase, const sddc_case *cases)
         next += cases[c].ncell;
     }
     if (next != ctx->ncell) return set_err(ctx, SDDC_EINVAL, "the cases do not cover the context's cells");
-    ctx->cpb = line_tile_cells(ctx->N);  // batches run by lines
+    ctx->by_tiles = false;  // batches run by lines
+    ctx->cpb = line_tile_cells(ctx->N);
     ctx->ncase = ncase;
     ctx->cases.assign(cases, cases + ncase);
     std::vector<CaseParams> cp(ncase);

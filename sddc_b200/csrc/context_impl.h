@@ -16,12 +16,12 @@
 namespace sddc {
 struct AdjWs;
 struct Output;
-// RK stages by lines and (exact form, small meshes) by tiles; residual
+// RK stages by lines and (exact form) by tiles; residual
 // evaluations; the face traces of a state
 cudaError_t launch_line_exact(int N, const StageArgs &a, const Ops &ops, cudaStream_t st);
 cudaError_t launch_line_fp64(int N, const StageArgs &a, const Ops &ops, cudaStream_t st);
 cudaError_t launch_line_mixed(int N, const StageArgs &a, const Ops &ops, cudaStream_t st);
-cudaError_t launch_tile_exact(int N, const StageArgs &a, const Ops &ops, cudaStream_t st);
+cudaError_t launch_tile_exact(int N, int cpb, const StageArgs &a, const Ops &ops, cudaStream_t st);
 cudaError_t launch_resid_exact(int N, const StageArgs &a, const Ops &ops, cudaStream_t st);
 cudaError_t launch_resid_fp64(int N, const StageArgs &a, const Ops &ops, cudaStream_t st);
 cudaError_t launch_resid_mixed(int N, const StageArgs &a, const Ops &ops, cudaStream_t st);
@@ -65,6 +65,7 @@ struct sddc_ctx {
     using CaseParams = sddc::CaseParams;
     sddc_params p{};
     int N = 0, ncell = 0, cpb = 8, msize = 0, grid = 0;
+    bool by_tiles = false;  // exact form: stages by tiles (exact_by_tiles)
     size_t nq = 0;  // doubles per state
     cudaStream_t stream = nullptr;
     std::string err;

@@ -79,13 +79,14 @@ template <int N, int CPB, typename R, bool EX> __host__ __device__ constexpr siz
 
 // Whether a thread holds its line's states in registers beside the sums.  In
 // double at N = 6 they do not fit (exact form, 121x87 cells: 638 us a step
-// with spills, 465 read from shared memory), and at N = 4 there is a second
+// with spills, 465 read from shared memory), in the exact form not at N = 5 either
+// (300x300 cells 428 us a stage with spills, 402), and at N = 4 there is a second
 // kernel without them (WIDE): 168 registers instead of 240 let a scheduler
 // hold 3 warps instead of 2.  (At N = 5 the sums alone leave no third warp: 363
 // us a stage held, 423 read.)
-template <int N, typename R, bool WIDE> __host__ __device__ constexpr bool line_hold()
+template <int N, typename R, bool EX, bool WIDE> __host__ __device__ constexpr bool line_hold()
 {
-    return sizeof(R) == sizeof(float) || (N <= 5 && !WIDE);
+    return sizeof(R) == sizeof(float) || (N <= (EX ? 4 : 5) && !WIDE);
 }
 __host__ __device__ constexpr bool line_has_wide(int n, int elem) { return n == 4 && elem == 8; }
 // Which of the two takes a stage of the given tiles, by the waves it needs
@@ -310,7 +311,7 @@ __device__ __forceinline__ bool line_tile(const StageArgs &a, const Ops &ops, co
         // the line's states: in registers, or read from shared memory at every
         // flux point (line_hold); then both ends' fluxes are formed first, while
         // the sums' registers are still free
-        constexpr bool kHold = line_hold<N, R, WIDE>();
+        constexpr bool kHold = line_hold<N, R, EX, WIDE>();
         P2<R> q2[kHold ? N : 1][K2];
         R q8[kHold ? N : 1];
         const int q0 = c * QS + (fam == 0 ? 9 * N * l : 9 * l);

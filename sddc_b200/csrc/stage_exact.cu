@@ -1,4 +1,4 @@
-// The exact form's RK stage by tiles, for small meshes: the reference's
+// The exact form's RK stage by tiles: the reference's
 // operations in its order, compiled with -fmad=false (no FMA contraction).
 #include <algorithm>
 
@@ -8,10 +8,10 @@ namespace sddc {
 
 namespace {
 
-template <int N> cudaError_t launch_n(const StageArgs &a, const Ops &ops, cudaStream_t st)
+template <int N, int CPB> cudaError_t launch_n(const StageArgs &a, const Ops &ops, cudaStream_t st)
 {
-    auto kern = stage_kernel<N, kTileCpb>;
-    constexpr size_t smem = stage_smem_bytes<N, kTileCpb>();
+    auto kern = stage_kernel<N, CPB>;
+    constexpr size_t smem = stage_smem_bytes<N, CPB>();
     static bool configured = false;  // per instantiation
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -22,20 +22,20 @@ template <int N> cudaError_t launch_n(const StageArgs &a, const Ops &ops, cudaSt
         if (e != cudaSuccess) return e;
         configured = true;
     }
-    kern<<<(a.ncell + kTileCpb - 1) / kTileCpb, stage_threads(N, kTileCpb), smem, st>>>(a, ops);
+    kern<<<(a.ncell + CPB - 1) / CPB, stage_threads(N, CPB), smem, st>>>(a, ops);
     return cudaGetLastError();
 }
 
 }  // namespace
 
-cudaError_t launch_tile_exact(int N, const StageArgs &a, const Ops &ops, cudaStream_t st)
+cudaError_t launch_tile_exact(int N, int cpb, const StageArgs &a, const Ops &ops, cudaStream_t st)
 {
     switch (N) {
-    case 2: return launch_n<2>(a, ops, st);
-    case 3: return launch_n<3>(a, ops, st);
-    case 4: return launch_n<4>(a, ops, st);
-    case 5: return launch_n<5>(a, ops, st);
-    case 6: return launch_n<6>(a, ops, st);
+    case 2: return launch_n<2, 8>(a, ops, st);
+    case 3: return launch_n<3, 4>(a, ops, st);
+    case 4: return launch_n<4, 8>(a, ops, st);
+    case 5: return launch_n<5, 4>(a, ops, st);
+    case 6: return cpb == 4 ? launch_n<6, 4>(a, ops, st) : launch_n<6, 8>(a, ops, st);
     default: return cudaErrorInvalidValue;
     }
 }

@@ -1,6 +1,6 @@
 // What the stage kernels share (their arguments, operators, TMA copies, face
-// traces), and the RK stage of the exact form by tiles, for small meshes
-// (exact_by_tiles).  Every other stage runs in line_kernel
+// traces), and the RK stage of the exact form by tiles, for the meshes on
+// which that is faster (exact_by_tiles).  Every other stage runs in line_kernel
 // (line_kernel.cuh), a residual evaluation in resid_kernel
 // (resid_kernel.cuh), both with a thread per line of solution points.
 //
@@ -9,7 +9,7 @@
 // nablaQsp compflux.f90:107-157) for every cell and applies the RK stage
 // update (iterations.f90:88-213).
 //
-// Work split: one CTA owns kTileCpb consecutive cells and stages them in
+// Work split: one CTA owns CPB consecutive cells (tile_cells) and stages them in
 // shared memory.  Phases, separated by __syncthreads:
 //   A  Lagrange interpolation of every line of solution points to its N+1
 //      flux points (one thread per cell x line index x variable: the xi-
@@ -52,31 +52,39 @@ __host__ __device__ constexpr int line_tile_cells(int n)
     return n == 2 ? 8 : n == 3 ? 10 : n == 4 ? 8 : n == 5 ? 6 : 2;
 }
 
-// Time steps of the exact form run by tiles of kTileCpb cells where that is
-// the faster of the two: a line's 2N+2 dependent point fluxes, in unfused
-// operations, are a longer chain than the tile's phases, which shows while the
-// mesh leaves SMs idle, and so is a last wave of CTAs by lines that is mostly
-// empty.  spare: the cells that would fill it.  us per stage, by tiles and by
-// lines: N = 3, 4096 cells 11.8 and 13.5, 4900 17.2 and 15.9, 9409 23.3 and
-// 28.8; N = 4, 2500 11.8 and 14.8, 7056 23.3 and 21.6, 8100 24.5 and 27.9, 9409
-// 29.4 and 27.6, 32400 96 and 86; N = 5, 4096 26.7 and 33.9, 7056 42.8 and 41.3,
-// 8100 44.6 and 53.1, 32400 178 and 165; N = 6, 1600 16.3 and 21.5, 4900 43.4
-// and 54.2, 9409 82.9 and 79.4.  (The FP64 and mixed forms always run by lines.)
-constexpr int kTileCpb = 4;
+// Time steps of the exact form run by tiles where that is the faster of the
+// two: a line's 2N+2 dependent point fluxes, in unfused operations, are a
+// longer chain than the tile's phases, which shows while the mesh leaves SMs
+// idle, and so is a last wave of CTAs by lines that is mostly empty.  spare: the
+// cells that would fill it.  At N = 6 the line's sums leave no registers for
+// its states, and tiles are the faster at every size.  us per stage, by tiles
+// and by lines: N = 2, 8100 cells 11.5 and 12.1, 32400 37.6 and 32.6; N = 3, 4096
+// 11.9 and 13.5, 8100 22.1 and 17.5, 9409 23.3 and 28.8; N = 4, 8100 23.7 and 28.0,
+// 9409 28 and 27.6, 14400 43.7 and 50.0, 32400 91 and 86; N = 5, 4096 26.5 and 33.2,
+// 8100 44.7 and 50.6, 32400 178 and 157; N = 6, 4096 33.9 and 38.8, 32400 232 and
+// 247.  (The FP64 and mixed forms always run by lines.)
 __host__ __device__ constexpr bool exact_by_tiles(int n, int ncell)
 {
     // cells of a wave by lines: 12 warps per SM at N = 2, 3 and (line_has_wide) 4,
     // else 8
-    const int wave = 148 * line_tile_cells(n) * (n == 2 ? 12 : n == 3 || n == 4 ? 6 : n == 6 ? 8 : 4);
+    const int wave = 148 * line_tile_cells(n) * (n == 2 ? 12 : n == 3 || n == 4 ? 6 : 4);
     const long spare = (wave - ncell % wave) % wave;
     switch (n) {
-    case 2: return ncell < 4000;
+    case 2: return ncell < 9472;  // (a wave by tiles)
     case 3: return 2L * ncell < 3 * spare - 6000;
     case 4:  // (up to 4736 cells, and near 9472, waves of 8 warps per SM serve, at 0.7 of the time)
-        return ncell <= 4736 || (ncell > wave && (ncell < 8800 || ncell > 9472) && ncell < 4 * spare);
-    case 5: return 2L * ncell < 13 * spare + 9800;
-    default: return 5L * ncell < 3 * spare + 37500;
+        return ncell <= 4736 || (ncell > wave && (ncell < 8800 || ncell > 9472) && ncell < 4 * spare + 6000);
+    case 5: return ncell < 5 * spare + 3000;
+    default: return true;
     }
+}
+// Cells per CTA there.  us per stage with 4 and 8 (6 is nowhere the best by more
+// than 3%): N = 2, 8100 cells 12.0 and 11.5; N = 3, 4096 11.9 and 13.2; N = 4, 14400
+// 45.7 and 43.7; N = 5, 8100 44.7 and 51.5; N = 6, 8100 70.6 and 61.8, but 576
+// (too few CTAs) 12.6 and 14.4
+__host__ __device__ constexpr int tile_cells(int n, int ncell)
+{
+    return n == 2 || n == 4 || (n == 6 && ncell >= 148 * 8) ? 8 : 4;
 }
 
 // operators in kernel parameter space (row-major)

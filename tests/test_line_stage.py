@@ -39,6 +39,14 @@ def _case(N, ncell):
     return t, ph, smooth_state(t, ph, seed=ncell), 0.2 * m.min_edge() / N
 
 
+def _by_lines(t, ph, dt, form, **kw):
+    """A context whose stages run by lines in every form: a batch of one case."""
+    s = Solver(t, ph, precision=form, **kw)
+    s.set_cases([dict(first_cell=0, ncell=t.ncell, dt=dt, rinf=ph.rinf, pinf=ph.pinf, uinf=ph.uinf, vinf=ph.vinf,
+                      bxinf=ph.bxinf, byinf=ph.byinf)])
+    return s
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("N", sorted(TILE))
 @pytest.mark.parametrize("k_stage", [3, 5])
@@ -54,16 +62,20 @@ def test_lines_match_oracle_at_tile_edges(N, k_stage):
         mo = o.maxima()
         # the bars of the parity tests: exact bit for bit, FP64 1e-12, mixed 1e-6
         for form, bar in (("fp64_exact", 0.0), ("fp64", 1e-12), ("mixed", 1e-6)):
-            s = Solver(t, ph, precision=form, k_stage=k_stage, cells_per_cta=8)
+            s = _by_lines(t, ph, dt, form, k_stage=k_stage)
             s.set_state(Q)
-            s.rk_s5p3(dt, 2)
+            s.step_cases(2)
             g = s.state()["Q"]
             if bar:
                 assert rel_l2(g, ref) <= bar, (form, ncell)
             else:
                 assert np.array_equal(g, ref), ncell
-                mg = s.maxima()
-                assert (mg["eigvmax"], mg["umax"]) == (mo["eigvmax"], mo["umax"])
+                assert s.case_maxima(0) == (mo["eigvmax"], mo["umax"])
+            s.close()
+            s = Solver(t, ph, precision=form, k_stage=k_stage)
+            s.set_state(Q)
+            s.rk_s5p3(dt, 2)
+            assert np.array_equal(s.state()["Q"], g), (form, ncell)
             s.close()
 
 
@@ -78,7 +90,7 @@ def test_viscous_lines_match_oracle_at_tile_edges(N):
         o.rk_s5p3(0.2 * dt, 1)
         ref = o.state()["Q"]
         for form, bar in (("fp64_exact", 0.0), ("fp64", 1e-12), ("mixed", 1e-6)):
-            s = Solver(t, ph, precision=form, cells_per_cta=8)
+            s = Solver(t, ph, precision=form)
             s.set_state(Q)
             s.rk_s5p3(0.2 * dt, 1)
             g = s.state()["Q"]
@@ -87,20 +99,24 @@ def test_viscous_lines_match_oracle_at_tile_edges(N):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("N,nx,ny", [(4, 76, 75), (4, 64, 65), (6, 37, 41)])
-def test_lines_match_oracle_over_several_waves(N, nx, ny):
+@pytest.mark.parametrize("N,nx,ny,mu", [(4, 76, 75, 0.0), (4, 64, 75, 0.02), (4, 64, 65, 0.0), (5, 101, 69, 0.0), (6, 37, 41, 0.0),
+                                        (6, 15, 7, 0.0)])
+def test_stages_match_oracle_over_several_waves(N, nx, ny, mu):
     """More tiles than CTAs are resident: at N = 4 in double 713 tiles take the
-    kernel of three warps per scheduler, 520 the other one."""
+    kernel of three warps per scheduler, 520 the other one (the exact form by
+    tiles).  The exact form at N = 5, 6969 cells, runs by lines; at N = 6 by tiles
+    of 8, and of 4 cells on the smallest meshes."""
     m = mesh.channel_box(nx, ny, sides=("SYMP", "OUTL", "WALL", "INLE"), jitter=0.2, seed=N)
     t = host.build_tables(m, N)
     ph = channel_physics()
-    Q, dt = smooth_state(t, ph, seed=nx), 0.2 * m.min_edge() / N
+    ph = dataclasses.replace(ph, mu=mu, eta0=mu)
+    Q, dt = smooth_state(t, ph, seed=nx), 0.2 * m.min_edge() / N * (0.2 if mu else 1.0)
     o = O.Oracle(t, ph)
     o.set_state(Q)
     o.rk_s5p3(dt, 1)
     ref = o.state()["Q"]
     for form, bar in (("fp64_exact", 0.0), ("fp64", 1e-12), ("mixed", 1e-6)):
-        s = Solver(t, ph, precision=form, cells_per_cta=8)
+        s = Solver(t, ph, precision=form)
         s.set_state(Q)
         s.rk_s5p3(dt, 1)
         g = s.state()["Q"]
@@ -186,13 +202,13 @@ def test_both_exact_kernels_agree_with_zeros_and_fault(N):
     Q = c.initial_state(t)
     dt = cases.cfl_dt(c.mesh, Q, N)
     out = []
-    for cpb in (4, 8):
-        s = Solver(t, c.physics, precision="fp64_exact", cells_per_cta=cpb)
+    for lines in (False, True):
+        s = _by_lines(t, c.physics, dt, "fp64_exact") if lines else Solver(t, c.physics, precision="fp64_exact")
         s.set_state(Q)
         seen = []
         for _ in range(12):
             try:
-                s.rk_s5p3(dt, 1)
+                s.step_cases(1) if lines else s.rk_s5p3(dt, 1)
                 fault = False
             except RuntimeError:
                 fault = True
