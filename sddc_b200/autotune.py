@@ -1,10 +1,9 @@
-"""Element-tile autotuner: picks the cells per CTA of the stage kernel.
+"""Tile autotuner: picks ``cells_per_cta`` for a context.
 
-The fused stage kernel stages ``cells_per_cta`` cells in shared memory; the
-best tile depends on N, the arithmetic form and the mesh size (occupancy
-against barrier stalls and the tail of the grid).  ``tune`` times each
-candidate on the caller's own case for a few RK3 steps and keeps the
-fastest; results are cached per (GPU, N, form, size class) in
+The kernels and their tiles now follow from the form, N and the mesh, so the
+candidates differ by noise only; the tuner remains for its callers.  ``tune``
+times each candidate on the caller's own case for a few RK3 steps and keeps
+the fastest; results are cached per (GPU, N, form, size class) in
 ``sddc_b200/lib/autotune.json``.
 """
 from __future__ import annotations

@@ -29,14 +29,12 @@
 // Running maxima go through atomicMax on rotating slots, as there.
 //
 // What bounds it: latency.  At N = 5 in the mixed form (6 cells, 64 threads,
-// 128 registers, 7 CTAs per SM) a scheduler holds 3.2 warps and issues in 45%
-// of its cycles, with 39% of DRAM bandwidth and the L1 pipe 58% busy (the tile
-// kernel: 87%); in the FP64 form (254 registers) it holds 1.9 warps, issues
-// in 33% and keeps the FP64 pipe 31% busy.  Why this split: a stage moves 10
-// KB per cell through shared memory instead of 26 KB.  us per RK_S5P3 step,
-// tile kernel and this one: 256x512 cells, N = 5, mixed 1408 and 1144, FP64
-// 2277 and 1820; 512x512 cells, N = 4, mixed 1810 and 1376; 121x87 cells, N = 6,
-// exact 676 and 465.
+// 128 registers) a scheduler holds 3.3 warps and issues in 48% of its cycles,
+// with 40% of DRAM bandwidth and the L1 pipe 62% busy (the tile kernel: 87%); in
+// the FP64 form (252 registers) it holds 1.9 warps and issues in 37%.  Why this
+// split: a stage moves 10 KB per cell through shared memory instead of 26 KB.
+// us per RK_S5P3 step, tile kernel and this one: 256x512 cells, N = 5, mixed 1373
+// and 1070, FP64 2267 and 1685; 512x512 cells, N = 4, mixed 1810 and 1290.
 #pragma once
 
 #include "stage_kernel.cuh"

@@ -34,8 +34,8 @@ cudaError_t launch_tile_exact(int N, int cpb, const StageArgs &a, const Ops &ops
     case 2: return launch_n<2, 8>(a, ops, st);
     case 3: return launch_n<3, 4>(a, ops, st);
     case 4: return launch_n<4, 8>(a, ops, st);
-    case 5: return launch_n<5, 4>(a, ops, st);
-    case 6: return cpb == 4 ? launch_n<6, 4>(a, ops, st) : launch_n<6, 8>(a, ops, st);
+    case 5: return launch_n<5, 6>(a, ops, st);
+    case 6: return cpb == 6 ? launch_n<6, 6>(a, ops, st) : launch_n<6, 8>(a, ops, st);
     default: return cudaErrorInvalidValue;
     }
 }

@@ -41,9 +41,12 @@ namespace sddc {
 
 constexpr int kMaxN = 6;
 
-// threads of a CTA owning cpb cells: one per face point (4N a cell), rounded
-// up to whole warps
-__host__ __device__ constexpr int stage_threads(int n, int cpb) { return (4 * n * cpb + 31) / 32 * 32; }
+// threads of a CTA of the kernel by tiles: one per face point (4N a cell), in
+// the 6-cell tile of N >= 5 one per solution point; whole warps
+__host__ __device__ constexpr int stage_threads(int n, int cpb)
+{
+    return ((cpb == 6 && n >= 5 ? n * n : 4 * n) * cpb + 31) / 32 * 32;
+}
 
 // Cells per CTA of the kernels by lines (2N threads per cell): one or two
 // warps with few idle lanes.
@@ -56,35 +59,32 @@ __host__ __device__ constexpr int line_tile_cells(int n)
 // two: a line's 2N+2 dependent point fluxes, in unfused operations, are a
 // longer chain than the tile's phases, which shows while the mesh leaves SMs
 // idle, and so is a last wave of CTAs by lines that is mostly empty.  spare: the
-// cells that would fill it.  At N = 6 the line's sums leave no registers for
-// its states, and tiles are the faster at every size.  us per stage, by tiles
-// and by lines: N = 2, 8100 cells 11.5 and 12.1, 32400 37.6 and 32.6; N = 3, 4096
-// 11.9 and 13.5, 8100 22.1 and 17.5, 9409 23.3 and 28.8; N = 4, 8100 23.7 and 28.0,
-// 9409 28 and 27.6, 14400 43.7 and 50.0, 32400 91 and 86; N = 5, 4096 26.5 and 33.2,
-// 8100 44.7 and 50.6, 32400 178 and 157; N = 6, 4096 33.9 and 38.8, 32400 232 and
-// 247.  (The FP64 and mixed forms always run by lines.)
+// cells that would fill it.  At N = 5 and 6 the line's sums leave no registers
+// for its states, and tiles are the faster at every size.  us per stage, by
+// tiles and by lines: N = 2, 8100 cells 11.5 and 12.1, 32400 37.6 and 32.6; N = 3,
+// 4096 11.9 and 13.5, 8100 22.1 and 17.5, 9409 23.3 and 28.8; N = 4, 8100 23.7 and
+// 28.0, 9409 28 and 27.6, 14400 43.7 and 50.0, 32400 91 and 86; N = 5, 4096 21.8 and
+// 33.2, 90000 401 and 402; N = 6, 4096 33.9 and 38.8, 32400 232 and 247.  (The FP64
+// and mixed forms, and batches, always run by lines.)
 __host__ __device__ constexpr bool exact_by_tiles(int n, int ncell)
 {
-    // cells of a wave by lines: 12 warps per SM at N = 2, 3 and (line_has_wide) 4,
-    // else 8
-    const int wave = 148 * line_tile_cells(n) * (n == 2 ? 12 : n == 3 || n == 4 ? 6 : 4);
+    // cells of a wave by lines: 12 warps per SM, at N = 4 with line_has_wide
+    const int wave = 148 * line_tile_cells(n) * (n == 2 ? 12 : 6);
     const long spare = (wave - ncell % wave) % wave;
     switch (n) {
     case 2: return ncell < 9472;  // (a wave by tiles)
     case 3: return 2L * ncell < 3 * spare - 6000;
     case 4:  // (up to 4736 cells, and near 9472, waves of 8 warps per SM serve, at 0.7 of the time)
         return ncell <= 4736 || (ncell > wave && (ncell < 8800 || ncell > 9472) && ncell < 4 * spare + 6000);
-    case 5: return ncell < 5 * spare + 3000;
     default: return true;
     }
 }
-// Cells per CTA there.  us per stage with 4 and 8 (6 is nowhere the best by more
-// than 3%): N = 2, 8100 cells 12.0 and 11.5; N = 3, 4096 11.9 and 13.2; N = 4, 14400
-// 45.7 and 43.7; N = 5, 8100 44.7 and 51.5; N = 6, 8100 70.6 and 61.8, but 576
-// (too few CTAs) 12.6 and 14.4
+// Cells per CTA there.  us per stage with 4, 6 and 8: N = 2, 8100 cells 12.0, 16.8,
+// 11.5; N = 3, 4096 11.9, 13.2, 13.2; N = 4, 14400 45.7, 47.3, 43.7; N = 5, 576 11.3,
+// 9.7, 12.8, 14400 80, 71, 92; N = 6, 576 12.6, 11.4, 14.4, 8100 71, 65, 62
 __host__ __device__ constexpr int tile_cells(int n, int ncell)
 {
-    return n == 2 || n == 4 || (n == 6 && ncell >= 148 * 8) ? 8 : 4;
+    return n == 3 ? 4 : n == 5 || (n == 6 && ncell < 148 * 8) ? 6 : 8;
 }
 
 // operators in kernel parameter space (row-major)

@@ -104,8 +104,8 @@ def test_viscous_lines_match_oracle_at_tile_edges(N):
 def test_stages_match_oracle_over_several_waves(N, nx, ny, mu):
     """More tiles than CTAs are resident: at N = 4 in double 713 tiles take the
     kernel of three warps per scheduler, 520 the other one (the exact form by
-    tiles).  The exact form at N = 5, 6969 cells, runs by lines; at N = 6 by tiles
-    of 8, and of 4 cells on the smallest meshes."""
+    tiles).  The exact form runs by tiles of 6 cells at N = 5, at N = 6 of 8, and of
+    6 on the smallest meshes."""
     m = mesh.channel_box(nx, ny, sides=("SYMP", "OUTL", "WALL", "INLE"), jitter=0.2, seed=N)
     t = host.build_tables(m, N)
     ph = channel_physics()
