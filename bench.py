@@ -328,7 +328,7 @@ def run_ours(args):
                      "traffic_note": "mean DRAM bytes per stage launch over the 5 stages of a step (ncu, "
                                      "profiles/traffic.json); algorithmic bytes per launch: "
                                      f"{dof * bpd:.4g}",
-                     "bytes_per_dof_stage": bpd, "kernel": f"stage_kernel<{c.N},{TILES['mixed']['cells_per_cta']},float> (mixed)",
+                     "bytes_per_dof_stage": bpd, "kernel": f"line_kernel<{c.N},float> (mixed)",
                      "fp64_side": {"ref_ops_per_dof_stage": REF_OPS_PER_DOF_STAGE_N5,
                                    "ref_ops_per_byte": REF_OPS_PER_DOF_STAGE_N5 / bpd,
                                    "fp64_form_ref_ops_per_s": val["fp64"] * REF_OPS_PER_DOF_STAGE_N5,

@@ -942,7 +942,7 @@ __device__ void locate_tile(const LocateArgs &a, const Ops &ops, int tile, bool 
     using ML = MetLayout<N>;
     constexpr int NQ = 9 * N * N, NP = N + 1;
     const int c0 = tile * a.cpb, ncl = min(a.cpb, a.ncell - c0);
-    // flux-point state of line (fam, line) at point r, as phase A computes it
+    // flux-point state of line (fam, line) at point r, as the forward form computes it
     auto interp = [&](int cell, int fam, int line, int r, double *qf) {
         const double *qc = a.q + (size_t)cell * NQ;
         for (int v = 0; v < 9; v++) {

@@ -617,9 +617,8 @@ __global__ void __launch_bounds__(stage_threads(N, CPB), (stage_min_blocks<N, CP
     __syncthreads();
 
     // ---- C: B gradient, sources and the residual per solution point ------------
-    // in a time step the RK coefficients of the stage (phase E runs here)
-    // formed where used, from the kernel parameters (not held in registers
-    // through the phase)
+    // the RK coefficients of the stage, formed where used from the kernel
+    // parameters (not held in registers through the phase)
     const double cdt = a.dt;
     auto cf = [&](int i) -> double { return ((a.dt_mask >> i) & 1u) ? a.cb[i] * cdt : a.cb[i]; };
     double part_r = 0.0, part_d = 0.0;
