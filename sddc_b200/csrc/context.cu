@@ -963,9 +963,12 @@ extern "C" int sddc_set_cases(sddc_ctx *ctx, int ncase, const sddc_case *cases)
     if ((rc = build_tiles(ctx))) return rc;
     // per-case running maxima and per-tile monitor partials
     cudaFree(ctx->maxima);
+    cudaFree(ctx->max_scratch);  // sized by the cases: the next sensor read allocates it anew
     cudaFree(ctx->mon_part);
     ctx->maxima = nullptr;
+    ctx->max_scratch = nullptr;
     ctx->mon_part = nullptr;
+    ctx->sensor_stale = false;
     if ((rc = alloc(ctx, (void **)&ctx->maxima, (size_t)ncase * kSlots * 2 * sizeof(double), "maxima")) ||
         (rc = alloc(ctx, (void **)&ctx->mon_part, (size_t)ctx->ntiles * 2 * sizeof(double), "monitor")))
         return rc;

@@ -1,0 +1,87 @@
+"""The host runtime of the drop-in (csrc/context.cu, adjoint.cu, noalloc.cu,
+line_launch.inc) against a stand-in of the CUDA runtime, tests/native/
+fake_cudart.cpp: sizes of copies, order of work on streams, attributes of
+launches, device memory, failing allocations.  Nothing is computed and no GPU
+is used: the library is loaded in a child process in which the stand-in is
+its libcudart."""
+import os
+import shutil
+import subprocess
+import sys
+import textwrap
+
+import pytest
+
+from sddc_b200 import _native
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+ROOT = os.path.dirname(HERE)
+NVCC = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+
+pytestmark = pytest.mark.skipif(not os.path.exists(NVCC) or not os.path.exists(_native.GPU_LIB),
+                                reason="nvcc or libsddc_b200.so not there (python -m sddc_b200.build)")
+
+PRELUDE = """
+import ctypes, sys
+sys.path[:0] = [{root!r}, {here!r}]
+import numpy as np
+from helpers import *
+from sddc_b200 import _native
+from sddc_b200.solver import AdjointOpts, Params, Solver, SddcError, lib
+F = ctypes.CDLL("libcudart.so.12")
+F.fake_message.restype = ctypes.c_char_p
+for f in ("fake_live", "fake_peak"):
+    getattr(F, f).restype = ctypes.c_size_t
+F.fake_launches.restype = ctypes.c_long
+F.fake_fail_alloc.argtypes = [ctypes.c_long]
+
+def clean():
+    assert F.fake_violations() == 0, F.fake_message()
+
+def launches(part):
+    return F.fake_launches(part.encode())
+"""
+
+
+@pytest.fixture(scope="module")
+def runtime(tmp_path_factory):
+    """A directory with the stand-in as libcudart.so.12."""
+    d = tmp_path_factory.mktemp("cudart")
+    (d / "versions.map").write_text("libcudart.so.12 { global: *; };\n")
+    subprocess.run([NVCC, "-std=c++17", "-O1", "-gencode", "arch=compute_100a,code=sm_100a", "-Xcompiler", "-fPIC",
+                    "-shared", "-cudart", "none", f"-I{os.path.join(ROOT, 'sddc_b200', 'csrc')}",
+                    os.path.join(HERE, "native", "fake_cudart.cpp"), os.path.join(HERE, "native", "fake_args.cu"),
+                    "-o", str(d / "libcudart.so.12"), "-Xlinker", f"--version-script={d / 'versions.map'}", "-Xlinker",
+                    "-soname=libcudart.so.12"], check=True, capture_output=True)
+    return str(d)
+
+
+def _run(runtime, body):
+    code = PRELUDE.format(root=ROOT, here=HERE) + textwrap.dedent(body)
+    env = dict(os.environ, LD_LIBRARY_PATH=runtime)
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, env=env, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
+def test_sensor_read_after_a_larger_batch_is_set(runtime):
+    """The copy of the running maxima that a sensor read takes has the size of
+    the batch now set, not of the one at the first read."""
+    _run(runtime, """
+        m, t, ph, Q = case_periodic(6, 3)
+
+        def set_cases(s, n):
+            edges = np.linspace(0, t.ncell, n + 1).astype(int)
+            s.set_cases([dict(first_cell=int(a), ncell=int(b - a), dt=1e-3, rinf=1., pinf=1., uinf=.1, vinf=0., bxinf=0.,
+                              byinf=0.) for a, b in zip(edges[:-1], edges[1:])])
+            s.set_state(Q)
+            s.step_cases(2)
+
+        s = Solver(t, ph, precision="fp64")
+        s.set_state(Q)
+        s.rk_s5p3(1e-3, 1)
+        s.state(sm_ind=True)
+        for n in (2, 12, 3, 40):
+            set_cases(s, n)
+            s.state(sm_ind=True)
+        clean()
+        """)
