@@ -2,3 +2,4 @@
 #include "stage_kernel.cuh"
 
 unsigned *stage_flags(const void *stage_args) { return static_cast<const sddc::StageArgs *>(stage_args)->err_flags; }
+unsigned *trace_flags(const void *trace_init) { return static_cast<const sddc::TraceInit *>(trace_init)->flags; }

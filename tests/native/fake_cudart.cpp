@@ -15,8 +15,10 @@
 
 #include <cuda_runtime_api.h>
 
-// in fake_args.cu: the fault flags that a residual launch got
+// in fake_args.cu: the fault flags that a residual launch, a launch of the face
+// traces got
 unsigned *stage_flags(const void *stage_args);
+unsigned *trace_flags(const void *trace_init);
 
 namespace {
 
@@ -28,8 +30,9 @@ std::map<char *, Alloc> mem;
 size_t live = 0, peak = 0;  // device bytes
 long fail_in = -1;          // device allocations until one fails (-1: none does)
 int device = 0;
-bool faulty = false;  // residual launches flag a non-positive density
+std::string faulty, failing;  // kernels whose launches set a fault flag, return an error
 int violations = 0;
+cudaError_t last = cudaSuccess;
 std::string message;
 std::map<std::string, long> launches;
 
@@ -117,8 +120,9 @@ cudaError_t launch(const void *f, dim3 grid, size_t smem, cudaStream_t st, void 
                   " bytes of shared memory");
         return cudaErrorInvalidValue;
     }
-    if (faulty && fn.name.find("resid_kernel") != std::string::npos) {
-        unsigned *flags = stage_flags(args[0]);
+    if (!failing.empty() && fn.name.find(failing) != std::string::npos) return last = cudaErrorLaunchFailure;
+    if (!faulty.empty() && fn.name.find(faulty) != std::string::npos) {
+        unsigned *flags = faulty == "trace_kernel" ? trace_flags(args[4]) : stage_flags(args[0]);
         put(at(st), [flags] { *flags |= 1u; });
     }
     return cudaSuccess;
@@ -148,7 +152,8 @@ extern "C" {
 // ---- the tests' side --------------------------------------------------------------
 int fake_violations() { return violations; }
 const char *fake_message() { return message.c_str(); }
-void fake_set_fault(int on) { faulty = on != 0; }
+void fake_fault(const char *kernel) { faulty = kernel; }
+void fake_fail(const char *kernel) { failing = kernel; }
 void fake_fail_alloc(long n) { fail_in = n; }
 size_t fake_live() { return live; }
 size_t fake_peak() { return peak; }
@@ -164,7 +169,12 @@ long fake_launches(const char *part)
 // ---- the runtime's ------------------------------------------------------------------
 cudaError_t cudaSetDevice(int d) { device = d; return cudaSuccess; }
 cudaError_t cudaGetDevice(int *d) { *d = device; return cudaSuccess; }
-cudaError_t cudaGetLastError() { return cudaSuccess; }
+cudaError_t cudaGetLastError()
+{
+    const cudaError_t e = last;
+    last = cudaSuccess;
+    return e;
+}
 const char *cudaGetErrorString(cudaError_t) { return "stand-in error"; }
 cudaError_t cudaDeviceGetAttribute(int *v, cudaDeviceAttr a, int)
 {

@@ -85,3 +85,25 @@ def test_sensor_read_after_a_larger_batch_is_set(runtime):
             s.state(sm_ind=True)
         clean()
         """)
+
+
+def test_an_error_of_a_launch_is_reported_once(runtime):
+    """A stage launch that failed is its own call's error, not also the next
+    call's."""
+    _run(runtime, """
+        m, t, ph, Q = case_cylinder()
+        for kernel, call in ((b"line_kernel", lambda s: s.rk_s5p3(1e-3, 1)), (b"resid_kernel", lambda s: s.compresid())):
+            s = Solver(t, ph, precision="fp64")
+            s.set_state(Q)
+            F.fake_fail(kernel)
+            try:
+                call(s)
+                assert False
+            except SddcError as e:
+                assert e.code == -2
+            F.fake_fail(b"")
+            s.set_state(Q)
+            call(s)
+            s.close()
+        clean()
+        """)
