@@ -168,19 +168,29 @@ extern "C" int sddc_compresid_noalloc(const sddc_params *p, const double *Lmat, 
     for (int s = 0; s < N; s++)
         for (int l = 0; l < NL; l++) ops.HL[s * NL + l] = lagrange(Xl, NL, l + 1, Xs[s]);
 
-    // the face traces; the same launch seeds every running-max slot.  (The
-    // flags are zero when the library is loaded and cleared where one was read.)
+    // the face traces; the same launch seeds every running-max slot.  The
+    // flags are zero when the library is loaded, and a call that may have set
+    // one clears them, in its stream, before it returns: the next call may come
+    // on another stream.
     double *maxima = reinterpret_cast<double *>(scratch + L.maxima);
     unsigned *flags = reinterpret_cast<unsigned *>(scratch + L.flags);
     const TraceInit init{flags, maxima, eigvmax, umax};
     void *trace = scratch + L.trace;
     cudaError_t e;
+    auto clear_flags = [&]() {
+        const cudaError_t m = cudaMemsetAsync(flags, 0, sizeof(unsigned), st);
+        return m == cudaSuccess ? cudaStreamSynchronize(st) : m;
+    };
+    auto fail_cuda = [&](const char *what) {
+        clear_flags();
+        return fail(SDDC_ECUDA, std::string(what) + ": " + cudaGetErrorString(e));
+    };
     switch (p->precision) {
     case SDDC_FP64_EXACT: e = launch_trace_exact(N, p->ncell, q_dev, trace, L.tfs, init, ops, st); break;
     case SDDC_FP64: e = launch_trace_fp64(N, p->ncell, q_dev, trace, L.tfs, init, ops, st); break;
     default: e = launch_trace_mixed(N, p->ncell, q_dev, trace, L.tfs, init, ops, st); break;
     }
-    if (e != cudaSuccess) return fail(SDDC_ECUDA, std::string("trace kernel: ") + cudaGetErrorString(e));
+    if (e != cudaSuccess) return fail_cuda("trace kernel");
 
     StageArgs a{};
     a.ncell = p->ncell;
@@ -207,7 +217,7 @@ extern "C" int sddc_compresid_noalloc(const sddc_params *p, const double *Lmat, 
     case SDDC_FP64: e = launch_resid_fp64(N, a, ops, st); break;
     default: e = launch_resid_mixed(N, a, ops, st); break;
     }
-    if (e != cudaSuccess) return fail(SDDC_ECUDA, std::string("residual kernel: ") + cudaGetErrorString(e));
+    if (e != cudaSuccess) return fail_cuda("residual kernel");
 
     // running maxima after the evaluation and the fault flags
     struct {
@@ -216,12 +226,12 @@ extern "C" int sddc_compresid_noalloc(const sddc_params *p, const double *Lmat, 
     } out;
     e = cudaMemcpyAsync(&out, maxima, L.flags + sizeof(unsigned), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) return fail(SDDC_ECUDA, std::string("read-back: ") + cudaGetErrorString(e));
+    if (e != cudaSuccess) return fail_cuda("read-back");
     if (maxima_out) {
         maxima_out[0] = out.maxima[2];
         maxima_out[1] = out.maxima[3];
     }
-    if (out.flags && (e = cudaMemsetAsync(flags, 0, sizeof(unsigned), st)) != cudaSuccess)
+    if (out.flags && (e = clear_flags()) != cudaSuccess)
         return fail(SDDC_ECUDA, std::string("clearing the flags: ") + cudaGetErrorString(e));
     if (out.flags) return fail(SDDC_ENUMERIC, "device numerics: non-positive density or non-finite wave speed");
     return SDDC_OK;

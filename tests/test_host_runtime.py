@@ -107,3 +107,56 @@ def test_an_error_of_a_launch_is_reported_once(runtime):
             s.close()
         clean()
         """)
+
+
+NOALLOC = """
+        import test_zz_no_alloc as Z
+        L = Z._bind()
+        m, t, ph, Q = case_cylinder()
+        met, faces = Z._packed(L, t)
+
+        def device(a):
+            p = ctypes.c_void_p()
+            assert F.cudaMalloc(ctypes.byref(p), ctypes.c_size_t(a.nbytes)) == 0
+            return p
+
+        def stream():
+            p = ctypes.c_void_p()
+            assert F.cudaStreamCreateWithFlags(ctypes.byref(p), 1) == 0
+            return p
+
+        p, ops, out = Z._params(t, ph, 1), [np.asfortranarray(x) for x in (t.Lmat, t.Mmat)], np.zeros(2)
+        dev = [device(a) for a in (Q, met, faces, Q, np.zeros(2 * Q.size))]
+
+        def call(st):
+            return L.sddc_compresid_noalloc(ctypes.byref(p), *[Z._p(x) for x in ops], *dev[:3], 0.0, 0.0, *dev[3:],
+                                            Z._p(out), st)
+"""
+
+
+def test_allocation_free_call_after_a_fault_on_another_stream(runtime):
+    """A fault belongs to the call that found it: nothing orders the next
+    call's stream after what that one left in its own."""
+    _run(runtime, NOALLOC + """
+        a, b = stream(), stream()
+        for good in (b, a, b):
+            F.fake_fault(b"resid_kernel")
+            assert call(a) == -4
+            F.fake_fault(b"")
+            assert call(good) == 0, L.sddc_noalloc_last_error()
+        clean()
+        """)
+
+
+def test_allocation_free_call_after_one_that_broke_off(runtime):
+    """A call that could not launch its residual leaves no flag behind."""
+    _run(runtime, NOALLOC + """
+        a, b = stream(), stream()
+        F.fake_fault(b"trace_kernel")
+        F.fake_fail(b"resid_kernel")
+        assert call(a) == -2
+        F.fake_fault(b"")
+        F.fake_fail(b"")
+        assert call(b) == 0, L.sddc_noalloc_last_error()
+        clean()
+        """)
