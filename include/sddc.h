@@ -163,7 +163,11 @@ int sddc_set_exchange(sddc_ctx *ctx, sddc_exchange_fn fn, void *user, void *send
                       double *maxima_dev);
 
 /* Device pointer of the state (9,N,N,NCELL), valid until the next call;
-   for callers that keep their data on the GPU. */
+   for callers that keep their data on the GPU.  For steps and residual
+   evaluations it is read only: they take the neighbours' values from the
+   face traces kept beside the state, which only sddc_set_state renews.
+   sddc_vjp_resid and sddc_adjoint_run form their traces from the state as
+   they find it. */
 int sddc_state_device_ptr(sddc_ctx *ctx, double **q_dev);
 
 /* The CUDA stream (cudaStream_t) every launch of the context goes to; for

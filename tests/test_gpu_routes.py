@@ -34,3 +34,25 @@ def test_sensor_of_a_batch_set_after_a_smaller_one():
         s = Solver(t, ph, precision="fp64")
         assert np.array_equal(sensor(s, n), g, equal_nan=True), n
         s.close()
+
+
+@pytest.mark.parametrize("form", ["fp64_exact", "fp64", "mixed"])
+def test_vjp_of_a_state_written_on_the_device(form):
+    """The VJP is that of the state now in device memory, neighbours' traces
+    included, also where a caller wrote it there."""
+    import torch
+
+    m, t, ph, Q = case_cylinder()
+    Q2 = np.asfortranarray(Q * (1 + 0.01 * np.random.default_rng(3).uniform(-1, 1, Q.shape[::-1]).T))
+    lam = np.asfortranarray(np.random.default_rng(4).standard_normal(Q.shape[::-1]).T)
+    s = Solver(t, ph, precision=form)
+    s.set_state(Q2, 0.0, 3.0, 1.0)
+    want = s.vjp_resid(lam)
+    s.set_state(Q, 0.0, 3.0, 1.0)
+    owner = type("Q", (), {"__cuda_array_interface__": dict(shape=(Q.size,), typestr="<f8", version=2,
+                                                            data=(s.device_state_ptr(), False))})()
+    torch.as_tensor(owner, device="cuda").copy_(torch.from_numpy(Q2.ravel(order="K")))
+    torch.cuda.synchronize()
+    got = s.vjp_resid(lam)
+    s.close()
+    assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
