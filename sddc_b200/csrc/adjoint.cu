@@ -30,6 +30,7 @@
 
 #include "adjoint_kernel.cuh"
 #include "context_impl.h"
+#include "per_device.h"
 
 using namespace sddc;
 
@@ -99,13 +100,13 @@ template <int N> cudaError_t launch_vjp_n(sddc_ctx *ctx, const VjpArgs &a)
 {
     constexpr int CPB = VjpSmem<N>::CPB;
     constexpr size_t smem = VjpSmem<N>::kBytes;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(vjp_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(vjp_kernel<N>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-        if (e != cudaSuccess) return e;
-        configured = true;
-    }
+    static PerDevice configured;
+    int set = 0;
+    const cudaError_t e = configured.get(&set, [&](int, int *out) {
+        *out = 1;
+        return set_smem(vjp_kernel<N>, smem);
+    });
+    if (e != cudaSuccess) return e;
     vjp_kernel<N><<<(ctx->ncell + CPB - 1) / CPB, line_threads(N, CPB), smem, ctx->stream>>>(a, ctx->ops);
     return cudaGetLastError();
 }

@@ -2,6 +2,7 @@
 // operations in its order, compiled with -fmad=false (no FMA contraction).
 #include <algorithm>
 
+#include "per_device.h"
 #include "stage_kernel.cuh"
 
 namespace sddc {
@@ -12,16 +13,13 @@ template <int N, int CPB> cudaError_t launch_n(const StageArgs &a, const Ops &op
 {
     auto kern = stage_kernel<N, CPB>;
     constexpr size_t smem = stage_smem_bytes<N, CPB>();
-    static bool configured = false;  // per instantiation
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        // the whole unified L1/shared array as shared memory, so that several
-        // CTAs fit on an SM
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-        if (e != cudaSuccess) return e;
-        configured = true;
-    }
+    static PerDevice configured;  // per instantiation
+    int set = 0;
+    const cudaError_t e = configured.get(&set, [&](int, int *out) {
+        *out = 1;
+        return set_smem(kern, smem);
+    });
+    if (e != cudaSuccess) return e;
     kern<<<(a.ncell + CPB - 1) / CPB, stage_threads(N, CPB), smem, st>>>(a, ops);
     return cudaGetLastError();
 }

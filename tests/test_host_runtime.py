@@ -160,3 +160,40 @@ def test_allocation_free_call_after_one_that_broke_off(runtime):
         assert call(b) == 0, L.sddc_noalloc_last_error()
         clean()
         """)
+
+
+def test_every_kernel_has_its_attributes_on_every_gpu(runtime):
+    """Kernels ask for more shared memory than a device gives without being
+    told: on each GPU of a process, in every form and at every N."""
+    _run(runtime, """
+        for device in (0, 1, 0, 2):
+            F.cudaSetDevice(device)
+            for N in (2, 3, 4, 5, 6):
+                m, t, ph, Q = case_cylinder(3, 8, N)
+                big = case_cylinder(24, 32, N)
+                for form in ("fp64_exact", "fp64", "mixed"):
+                    s = Solver(t, ph, precision=form)
+                    s.set_state(Q)
+                    s.compresid()
+                    s.rk_s5p3(1e-3, 2)
+                    s.vjp_resid(Q)
+                    s.adjoint_run(1e-3, 2, 1, 2)
+                    for k in (False, True):
+                        s.set_cases([dict(first_cell=0, ncell=t.ncell, dt=1e-3, rinf=1., pinf=1., uinf=.1, vinf=0.,
+                                          bxinf=0., byinf=0.)])
+                        s.set_persistent(k)
+                        s.set_state(Q)
+                        s.step_cases(1)
+                    s.close()
+                    s = Solver(big[1], big[2], precision=form, k_stage=5)
+                    s.set_state(big[3])
+                    s.rk_s5p3(1e-3, 1)
+                    s.close()
+                    ph.mu = 0.01
+                    s = Solver(t, ph, precision=form)
+                    ph.mu = 0.0
+                    s.set_state(Q)
+                    s.rk_s5p3(1e-3, 1)
+                    s.close()
+        clean()
+        """)
