@@ -307,7 +307,7 @@ int reverse_stage(sddc_ctx *ctx, const RevStage &s)
 int adjoint_flags(sddc_ctx *ctx)
 {
     CKA(cudaStreamSynchronize(ctx->stream));
-    const unsigned f = *(volatile unsigned *)ctx->err_flags;
+    const unsigned f = *(volatile unsigned *)ctx->err_flags.host;
     if (f & (kErrAdjointMaxLost | kErrAdjointRecords)) {
         take_flags(ctx);
         if (f & kErrAdjointRecords) return set_err(ctx, SDDC_ENUMERIC, "adjoint: more points attain a running maximum than the record buffer holds");
@@ -413,7 +413,7 @@ extern "C" int sddc_vjp_resid(sddc_ctx *ctx, const double *Rbar, double *Qbar, d
     // the state's traces in the exact form's rounding, from the state as it is
     // now: a caller may have written it through sddc_state_device_ptr.  Ahead
     // of Rbar's copy, whose first bytes the host stages meanwhile.
-    CKA(launch_trace_exact(ctx->N, ctx->ncell, ctx->reg[0], w->tq, trace_stride(ctx->N, 8), {ctx->err_flags}, ctx->ops,
+    CKA(launch_trace_exact(ctx->N, ctx->ncell, ctx->reg[0], w->tq, trace_stride(ctx->N, 8), TraceInit{ctx->err_flags}, ctx->ops,
                            ctx->stream));
     CKA(cudaMemcpyAsync(w->lam, Rbar, ctx->nq * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
     CKA(cudaMemsetAsync(w->acc, 0, sizeof(AdjScalars), ctx->stream));
@@ -533,7 +533,7 @@ extern "C" int sddc_adjoint_run(sddc_ctx *ctx, const sddc_adjoint_opts *o, doubl
     for (int s = 0; s < nseg; s++) {
         const int step0 = s * K, nst = std::min(K, ns - step0);
         CKA(cudaMemcpyAsync(S[0], ckpt[s], nq * sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream));
-        CKA(launch_trace_exact(ctx->N, ctx->ncell, S[0], T[0], trace_stride(ctx->N, 8), {ctx->err_flags}, ctx->ops, ctx->stream));
+        CKA(launch_trace_exact(ctx->N, ctx->ncell, S[0], T[0], trace_stride(ctx->N, 8), TraceInit{ctx->err_flags}, ctx->ops, ctx->stream));
         if (s == 0 && o->n1 == 0) CKA(wall_force(ctx, T[0], force));
         if ((rc = forward_steps(ctx, o->dt, step0, nst, S.data(), T.data(), hist, o->n1, o->n2, force, cmax,
                                 ctx->stream)))
@@ -624,7 +624,7 @@ extern "C" int sddc_adjoint_run(sddc_ctx *ctx, const sddc_adjoint_opts *o, doubl
         auto recompute = [&](int seg, int buf, cudaStream_t st) -> int {
             const int s0 = seg * K, n = std::min(K, ns - s0);
             CKA(cudaMemcpyAsync((*SS[buf])[0], ckpt[seg], nq * sizeof(double), cudaMemcpyDeviceToDevice, st));
-            CKA(launch_trace_exact(ctx->N, ctx->ncell, (*SS[buf])[0], (*TT[buf])[0], trace_stride(ctx->N, 8), {ctx->err_flags}, ctx->ops, st));
+            CKA(launch_trace_exact(ctx->N, ctx->ncell, (*SS[buf])[0], (*TT[buf])[0], trace_stride(ctx->N, 8), TraceInit{ctx->err_flags}, ctx->ops, st));
             return forward_steps(ctx, o->dt, s0, n, SS[buf]->data(), TT[buf]->data(), hist, 0, -1, nullptr, CM[buf], st);
         };
         for (int s = nseg - 1; s >= 0; s--) {

@@ -78,7 +78,7 @@ struct VjpArgs {
     double sx, sy;
     double wq[kMaxN];
     double *part;  // [8][CTAs]: cbar, pbar[6], 0
-    unsigned *err;
+    FaultFlags err;
     // the next reverse stage's adjoint traces, formed from out (the adjoint of
     // that stage's output) in the epilogue: its input state and lam_scale, and
     // the trace buffer (null: its own trace launch forms them)
@@ -234,7 +234,7 @@ struct RecSink {
     int cap;
     int *n;
     int *cnt;
-    unsigned *err;
+    FaultFlags err;
 };
 
 static __device__ __noinline__ void adj_record(RecSink rs, int cell, int slot, int kind, int counted, const double *d,
@@ -250,7 +250,7 @@ static __device__ __noinline__ void adj_record(RecSink rs, int cell, int slot, i
         for (int m = 0; m < 9; m++) R.d[m] = d[m];
         for (int m = 0; m < 6; m++) R.p[m] = p ? p[m] : 0.0;
     } else {
-        atomicOr(rs.err, kErrAdjointRecords);
+        raise_fault(rs.err, kErrAdjointRecords);
     }
     if (counted) atomicAdd(rs.cnt + kind, 1);
 }
@@ -439,7 +439,7 @@ __global__ void __launch_bounds__(line_threads(N, VjpSmem<N>::CPB), (vjp_min_blo
         }
     cp_async_wait_all();
     if (tid == 0 && !mbar_wait_bounded(&sBar, 0)) {
-        atomicOr(a.err, kErrStagingTimeout);  // the copies did not complete
+        raise_fault(a.err, kErrStagingTimeout);  // the copies did not complete
         sAbort = 1;
         mbar_wait_bounded(&sBar, 0);
     }
@@ -743,7 +743,7 @@ __global__ void __launch_bounds__(line_threads(N, VjpSmem<N>::CPB), (vjp_min_blo
                 sA[cc * QS + (k - cc * NQ)] = qn[k];
             }
         else if (tid == 0 && !mbar_wait_bounded(&sBarN, 0)) {
-            atomicOr(a.err, kErrStagingTimeout);  // the copy did not complete
+            raise_fault(a.err, kErrStagingTimeout);  // the copy did not complete
             sAbort = 1;
             mbar_wait_bounded(&sBarN, 0);
         }
@@ -848,7 +848,7 @@ static __global__ void __launch_bounds__(kRedThreads) adj_reduce_kernel(int nblk
                                                                  double dc_dl, double dc_du,
                                                                  const AdjRec *__restrict__ recs, int *rec_n,
                                                                  int *rec_cnt, int rec_cap, double *out,
-                                                                 const Ops ops, unsigned *err, NextTraces next)
+                                                                 const Ops ops, FaultFlags err, NextTraces next)
 {
     __shared__ double s[7][kRedThreads / 32];
     __shared__ double w[2];
@@ -870,7 +870,7 @@ static __global__ void __launch_bounds__(kRedThreads) adj_reduce_kernel(int nblk
         const int ce = rec_cnt[0], cu = rec_cnt[1];
         w[0] = (owner_eig && ce > 0) ? acc->lam_eig / ce : 0.0;
         w[1] = (owner_um && cu > 0) ? acc->lam_um / cu : 0.0;
-        if ((owner_eig && ce == 0) || (owner_um && cu == 0)) atomicOr(err, kErrAdjointMaxLost);
+        if ((owner_eig && ce == 0) || (owner_um && cu == 0)) raise_fault(err, kErrAdjointMaxLost);
     }
     __syncthreads();
     const int nrec = min(*rec_n, rec_cap);

@@ -165,7 +165,7 @@ static void free_all(sddc_ctx *ctx)
     for (auto &r : ctx->reg) cudaFree(r), r = nullptr;
     for (auto &t : ctx->trace) cudaFree(t), t = nullptr;
     void *bufs[] = {ctx->met, ctx->nrm, ctx->jac, ctx->faces, ctx->maxima, ctx->sm_ind, ctx->muav, ctx->resid, ctx->grad,
-                    ctx->mon_part, ctx->mon_out, ctx->int_part, ctx->wq,
+                    ctx->mon_part, ctx->mon_out, ctx->int_part, ctx->wq, ctx->err_flags.dev,
                     ctx->case_dev, ctx->tiles, ctx->visc_grad, ctx->visc_gt,
                     ctx->visc_rv, ctx->met2, ctx->max_scratch, ctx->proc_cells};
     for (void *b : bufs) cudaFree(b);
@@ -247,7 +247,8 @@ extern "C" int sddc_create(sddc_ctx **out, const sddc_params *p)
         (rc = alloc(ctx, (void **)&ctx->mon_part, (size_t)mon_blocks * 2 * sizeof(double), "monitor")) ||
         (rc = alloc(ctx, (void **)&ctx->mon_out, 4 * sizeof(double), "monitor")) ||
         (rc = alloc(ctx, (void **)&ctx->int_part, 1024 * 2 * sizeof(double), "integrals")) ||
-        (rc = alloc(ctx, (void **)&ctx->wq, kMaxN * sizeof(double), "weights")))
+        (rc = alloc(ctx, (void **)&ctx->wq, kMaxN * sizeof(double), "weights")) ||
+        (rc = alloc(ctx, (void **)&ctx->err_flags.dev, sizeof(unsigned), "flags")))
         return rc;
     // the viscous chain runs only with vismode = 1 (compflux.f90:36)
     ctx->visc = p->vismode == 1 && (p->mu != 0.0 || p->eta0 != 0.0);
@@ -259,8 +260,9 @@ extern "C" int sddc_create(sddc_ctx **out, const sddc_params *p)
             return rc;
     }
     CK(cudaMallocHost((void **)&ctx->host_small, 65 * sizeof(double)));
-    ctx->err_flags = reinterpret_cast<unsigned *>(ctx->host_small + 64);
-    *ctx->err_flags = 0;
+    ctx->err_flags.host = reinterpret_cast<unsigned *>(ctx->host_small + 64);
+    *ctx->err_flags.host = 0;
+    CK(cudaMemsetAsync(ctx->err_flags.dev, 0, sizeof(unsigned), ctx->stream));
     CK(cudaMemsetAsync(ctx->maxima, 0, kSlots * 2 * sizeof(double), ctx->stream));
     CK(cudaMemsetAsync(ctx->sm_ind, 0, nc * 2 * sizeof(double), ctx->stream));
     CK(cudaMemsetAsync(ctx->mon_part, 0, (size_t)mon_blocks * 2 * sizeof(double), ctx->stream));
@@ -466,9 +468,9 @@ static int refresh_traces(sddc_ctx *ctx)
 {
     cudaError_t e;
     switch (ctx->p.precision) {
-    case SDDC_FP64_EXACT: e = launch_trace_exact(ctx->N, ctx->ncell, ctx->reg[0], ctx->trace[0], ctx->tfs, {ctx->err_flags}, ctx->ops, ctx->stream); break;
-    case SDDC_FP64: e = launch_trace_fp64(ctx->N, ctx->ncell, ctx->reg[0], ctx->trace[0], ctx->tfs, {ctx->err_flags}, ctx->ops, ctx->stream); break;
-    default: e = launch_trace_mixed(ctx->N, ctx->ncell, ctx->reg[0], ctx->trace[0], ctx->tfs, {ctx->err_flags}, ctx->ops, ctx->stream); break;
+    case SDDC_FP64_EXACT: e = launch_trace_exact(ctx->N, ctx->ncell, ctx->reg[0], ctx->trace[0], ctx->tfs, TraceInit{ctx->err_flags}, ctx->ops, ctx->stream); break;
+    case SDDC_FP64: e = launch_trace_fp64(ctx->N, ctx->ncell, ctx->reg[0], ctx->trace[0], ctx->tfs, TraceInit{ctx->err_flags}, ctx->ops, ctx->stream); break;
+    default: e = launch_trace_mixed(ctx->N, ctx->ncell, ctx->reg[0], ctx->trace[0], ctx->tfs, TraceInit{ctx->err_flags}, ctx->ops, ctx->stream); break;
     }
     if (e != cudaSuccess) return cuda_err(ctx, e, "trace kernel");
     ctx->traces_stale = false;
@@ -597,8 +599,12 @@ static int proc_ready(sddc_ctx *ctx)
 
 unsigned sddc::take_flags(sddc_ctx *ctx)
 {
-    const unsigned f = *(volatile unsigned *)ctx->err_flags;
-    if (f) *ctx->err_flags = 0;
+    const unsigned f = *(volatile unsigned *)ctx->err_flags.host;
+    // both words, and before the next launch, on whatever stream it goes; where
+    // that fails the host's word stays, for the next call to report
+    if (f && cudaMemsetAsync(ctx->err_flags.dev, 0, sizeof(unsigned), ctx->stream) == cudaSuccess &&
+        cudaStreamSynchronize(ctx->stream) == cudaSuccess)
+        *ctx->err_flags.host = 0;
     return f;
 }
 

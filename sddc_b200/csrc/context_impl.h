@@ -63,6 +63,7 @@ constexpr double F11 = 0.39175222700392, F21 = 0.44437049406734, F22 = 0.5556295
 struct sddc_ctx {
     using Ops = sddc::Ops;
     using CaseParams = sddc::CaseParams;
+    using FaultFlags = sddc::FaultFlags;
     sddc_params p{};
     int N = 0, ncell = 0, cpb = 8, msize = 0, grid = 0;
     bool by_tiles = false;  // exact form: stages by tiles (exact_by_tiles)
@@ -84,9 +85,8 @@ struct sddc_ctx {
     double *maxima = nullptr;  // [sddc::kSlots][2]
     double *sm_ind = nullptr, *muav = nullptr, *resid = nullptr, *grad = nullptr;
     double *mon_part = nullptr, *mon_out = nullptr, *int_part = nullptr, *wq = nullptr;
-    // numerical faults, OR-ed by the kernels: pinned host memory behind
-    // host_small, so that the host reads them after a synchronisation without a copy
-    unsigned *err_flags = nullptr;
+    // numerical faults; the host's word lies behind host_small
+    FaultFlags err_flags{};
     double *host_small = nullptr;  // pinned scratch for small read-backs
     Ops ops{};
     int slot = 0;  // slot holding the running maxima after the last evaluation

@@ -274,7 +274,7 @@ __device__ __forceinline__ bool line_tile(const StageArgs &a, const Ops &ops, co
     const R c_h = (R)sqrt(eig_r * (eig_r - um_r));
     cp_async_wait_all();
     if (tid == 0 && !mbar_wait_bounded(&sBar, 0)) {
-        atomicOr(a.err_flags, kErrStagingTimeout);
+        raise_fault(a.err_flags, kErrStagingTimeout);
         sAbort = 1;
         mbar_wait_bounded(&sBar, 0);
     }
@@ -485,7 +485,7 @@ __device__ __forceinline__ bool line_tile(const StageArgs &a, const Ops &ops, co
     if (lane == 0) {
         sRed[wid] = em;
         sRed[NW + wid] = um;
-        if (eb) atomicOr(a.err_flags, eb);
+        if (eb) raise_fault(a.err_flags, eb);
     }
     __syncthreads();  // the neighbours' traces are read: sX is free
     if (tid == 0) {

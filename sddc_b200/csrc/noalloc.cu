@@ -174,7 +174,7 @@ extern "C" int sddc_compresid_noalloc(const sddc_params *p, const double *Lmat, 
     // on another stream.
     double *maxima = reinterpret_cast<double *>(scratch + L.maxima);
     unsigned *flags = reinterpret_cast<unsigned *>(scratch + L.flags);
-    const TraceInit init{flags, maxima, eigvmax, umax};
+    const TraceInit init{{flags, nullptr}, maxima, eigvmax, umax};
     void *trace = scratch + L.trace;
     cudaError_t e;
     auto clear_flags = [&]() {
@@ -211,7 +211,7 @@ extern "C" int sddc_compresid_noalloc(const sddc_params *p, const double *Lmat, 
     a.resid_out = resid_dev;
     a.grad_out = nablaqs_dev;
     a.mon_part = nullptr;
-    a.err_flags = flags;
+    a.err_flags = {flags, nullptr};
     switch (p->precision) {
     case SDDC_FP64_EXACT: e = launch_resid_exact(N, a, ops, st); break;
     case SDDC_FP64: e = launch_resid_fp64(N, a, ops, st); break;

@@ -186,7 +186,7 @@ __global__ void __launch_bounds__(line_threads(N, ResidSmem<N, R>::CPB), (resid_
     const R c_h = (R)sqrt(eig_r * (eig_r - um_r));
     cp_async_wait_all();
     if (bulk && tid == 0 && !mbar_wait_bounded(&sBar, 0)) {
-        atomicOr(a.err_flags, kErrStagingTimeout);
+        raise_fault(a.err_flags, kErrStagingTimeout);
         sAbort = 1;
         mbar_wait_bounded(&sBar, 0);
     }
@@ -666,7 +666,7 @@ __global__ void __launch_bounds__(line_threads(N, ResidSmem<N, R>::CPB), (resid_
         sRed[32 + wid] = um;
         sRed[64 + wid] = pr;
         sRed[96 + wid] = pd;
-        if (eb) atomicOr(a.err_flags, eb);
+        if (eb) raise_fault(a.err_flags, eb);
     }
     __syncthreads();
     if (tid == 0) {
@@ -735,7 +735,7 @@ __global__ void __launch_bounds__(line_threads(N, TraceSmem<N, R>::CPB))
             __syncwarp();
             if (tid < (QS != NQ ? ncl : 1)) bulk_g2s(sQ + tid * QS, qsrc + (size_t)tid * NQ, cbytes, &sBar);
             if (tid == 0 && !mbar_wait_bounded(&sBar, 0)) {
-                atomicOr(init.flags, kErrStagingTimeout);
+                raise_fault(init.flags, kErrStagingTimeout);
                 sAbort = 1;
                 mbar_wait_bounded(&sBar, 0);
             }

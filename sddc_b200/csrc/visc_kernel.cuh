@@ -56,7 +56,7 @@ struct ViscArgs {
     double *grad;  // nablaQs (9,2,N,N,NCELL)
     double *gt;    // gradient traces [cell][lf][18][nfp]: (9 x-derivatives, 9 y-derivatives)
     double *rv;    // dFv + dGv (9,N,N,NCELL)
-    unsigned *err_flags;
+    FaultFlags err_flags;
 };
 
 // o[k-1] = Fv(k) n0 + Gv(k) n1, k = 1..7, of getVfluxvectors
@@ -286,7 +286,7 @@ template <int N, int CPB, typename T> struct ViscTile {
             }
         cp_async_wait_all();
         if (tid == 0 && !mbar_wait_bounded(&sBar, 0)) {
-            atomicOr(a.err_flags, kErrStagingTimeout);
+            raise_fault(a.err_flags, kErrStagingTimeout);
             sAbort = 1;
             mbar_wait_bounded(&sBar, 0);
         }

@@ -1,5 +1,12 @@
 // What the stand-in runtime (fake_cudart.cpp) reads of a launch's arguments.
 #include "stage_kernel.cuh"
 
-unsigned *stage_flags(const void *stage_args) { return static_cast<const sddc::StageArgs *>(stage_args)->err_flags; }
-unsigned *trace_flags(const void *trace_init) { return static_cast<const sddc::TraceInit *>(trace_init)->flags; }
+static void raise(const sddc::FaultFlags &f)
+{
+    *f.dev |= sddc::kErrNonPositiveDensity;
+    if (f.host) *f.host |= sddc::kErrNonPositiveDensity;
+}
+void raise_stage(const void *stage_args) { raise(static_cast<const sddc::StageArgs *>(stage_args)->err_flags); }
+void raise_trace(const void *trace_init) { raise(static_cast<const sddc::TraceInit *>(trace_init)->flags); }
+size_t stage_args_bytes() { return sizeof(sddc::StageArgs); }
+size_t trace_init_bytes() { return sizeof(sddc::TraceInit); }

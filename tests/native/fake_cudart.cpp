@@ -15,10 +15,12 @@
 
 #include <cuda_runtime_api.h>
 
-// in fake_args.cu: the fault flags that a residual launch, a launch of the face
-// traces got
-unsigned *stage_flags(const void *stage_args);
-unsigned *trace_flags(const void *trace_init);
+// in fake_args.cu: sets a fault bit as a stage or residual launch, a launch of
+// the face traces with these arguments would
+void raise_stage(const void *stage_args);
+void raise_trace(const void *trace_init);
+size_t stage_args_bytes();
+size_t trace_init_bytes();
 
 namespace {
 
@@ -122,8 +124,10 @@ cudaError_t launch(const void *f, dim3 grid, size_t smem, cudaStream_t st, void 
     }
     if (!failing.empty() && fn.name.find(failing) != std::string::npos) return last = cudaErrorLaunchFailure;
     if (!faulty.empty() && fn.name.find(faulty) != std::string::npos) {
-        unsigned *flags = faulty == "trace_kernel" ? trace_flags(args[4]) : stage_flags(args[0]);
-        put(at(st), [flags] { *flags |= 1u; });
+        const bool trace = faulty == "trace_kernel";
+        const char *arg = static_cast<const char *>(args[trace ? 4 : 0]);
+        const std::vector<char> v(arg, arg + (trace ? trace_init_bytes() : stage_args_bytes()));
+        put(at(st), [trace, v] { trace ? raise_trace(v.data()) : raise_stage(v.data()); });
     }
     return cudaSuccess;
 }
