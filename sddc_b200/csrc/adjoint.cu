@@ -157,9 +157,8 @@ cudaError_t wall_force(sddc_ctx *ctx, const double *t, double *out)
                              ctx->stream);
 }
 
-int ensure_ws(sddc_ctx *ctx)
+int make_ws(sddc_ctx *ctx)
 {
-    if (ctx->adj) return SDDC_OK;
     auto *w = new AdjWs();
     ctx->adj = w;
     const size_t nc = ctx->ncell, N = ctx->N;
@@ -196,6 +195,14 @@ int ensure_ws(sddc_ctx *ctx)
         CKA(cudaMemcpyAsync(w->wall, wl.data(), wl.size() * sizeof(int2), cudaMemcpyHostToDevice, ctx->stream));
     CKA(cudaStreamSynchronize(ctx->stream));
     return SDDC_OK;
+}
+
+int ensure_ws(sddc_ctx *ctx)
+{
+    if (ctx->adj) return SDDC_OK;
+    const int rc = make_ws(ctx);
+    if (rc) adjoint_free(ctx);  // no part of it: the next call starts anew
+    return rc;
 }
 
 int check_adjoint_ctx(sddc_ctx *ctx)

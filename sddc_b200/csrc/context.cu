@@ -626,13 +626,8 @@ extern "C" int sddc_compresid(sddc_ctx *ctx)
     int rc = ready(ctx);
     if (!rc) rc = proc_ready(ctx);
     if (rc) return rc;
-    const size_t nc = ctx->ncell;
-    if (!ctx->resid) {
-        if ((rc = alloc(ctx, (void **)&ctx->resid, ctx->nq * sizeof(double), "resid")) ||
-            (rc = alloc(ctx, (void **)&ctx->grad, 2 * ctx->nq * sizeof(double), "nablaQs")))
-            return rc;
-    }
-    (void)nc;
+    if (!ctx->grad && (rc = alloc(ctx, (void **)&ctx->grad, 2 * ctx->nq * sizeof(double), "nablaQs"))) return rc;
+    if (!ctx->resid && (rc = alloc(ctx, (void **)&ctx->resid, ctx->nq * sizeof(double), "resid"))) return rc;
     StageArgs a = base_args(ctx);
     a.rk_kind = kRkNone;
     a.q_in = ctx->reg[0];
@@ -911,28 +906,38 @@ extern "C" int sddc_get_stream(sddc_ctx *ctx, void **stream)
 
 // ---------------------------------------------------------------- batches
 
-static int build_tiles(sddc_ctx *ctx)
+// device memory that is its owner's until given to the context
+struct Held {
+    void *p = nullptr;
+    ~Held() { cudaFree(p); }
+    template <typename T> void give(T *&to)  // in place of what the context held
+    {
+        cudaFree(to);
+        to = static_cast<T *>(p);
+        p = nullptr;
+    }
+};
+
+// the tile table of cases for launches of the given kind
+static int build_tiles(sddc_ctx *ctx, const std::vector<sddc_case> &cases, bool persistent, Held *out, int *count)
 {
-    const int cpb = ctx->cpb;
+    const int cpb = line_tile_cells(ctx->N);
     // persistent launches walk the table with a grid stride, largest case
     // first; otherwise the cases in their order
-    std::vector<int> order(ctx->ncase);
-    for (int c = 0; c < ctx->ncase; c++) order[c] = c;
-    if (ctx->persistent)
-        std::stable_sort(order.begin(), order.end(),
-                         [&](int x, int y) { return ctx->cases[x].ncell > ctx->cases[y].ncell; });
+    std::vector<int> order(cases.size());
+    for (size_t c = 0; c < cases.size(); c++) order[c] = (int)c;
+    if (persistent)
+        std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return cases[x].ncell > cases[y].ncell; });
     std::vector<int4> tiles;
     for (int c : order) {
-        const sddc_case &k = ctx->cases[c];
+        const sddc_case &k = cases[c];
         for (int first = 0; first < k.ncell; first += cpb)
             tiles.push_back(make_int4(k.first_cell + first, std::min(cpb, k.ncell - first), c, first == 0 ? 1 : 0));
     }
-    cudaFree(ctx->tiles);
-    ctx->tiles = nullptr;
-    int rc = alloc(ctx, (void **)&ctx->tiles, tiles.size() * sizeof(int4), "tile table");
+    int rc = alloc(ctx, &out->p, tiles.size() * sizeof(int4), "tile table");
     if (rc) return rc;
-    CK(cudaMemcpyAsync(ctx->tiles, tiles.data(), tiles.size() * sizeof(int4), cudaMemcpyHostToDevice, ctx->stream));
-    ctx->ntiles = (int)tiles.size();
+    CK(cudaMemcpyAsync(out->p, tiles.data(), tiles.size() * sizeof(int4), cudaMemcpyHostToDevice, ctx->stream));
+    *count = (int)tiles.size();
     return SDDC_OK;
 }
 
@@ -950,10 +955,8 @@ extern "C" int sddc_set_cases(sddc_ctx *ctx, int ncase, const sddc_case *cases)
         next += cases[c].ncell;
     }
     if (next != ctx->ncell) return set_err(ctx, SDDC_EINVAL, "the cases do not cover the context's cells");
-    ctx->by_tiles = false;  // batches run by lines
-    ctx->cpb = line_tile_cells(ctx->N);
-    ctx->ncase = ncase;
-    ctx->cases.assign(cases, cases + ncase);
+    // everything new first: where an allocation fails the context stays as it was
+    const std::vector<sddc_case> cs(cases, cases + ncase);
     std::vector<CaseParams> cp(ncase);
     for (int c = 0; c < ncase; c++) {
         const sddc_case &k = cases[c];
@@ -961,27 +964,30 @@ extern "C" int sddc_set_cases(sddc_ctx *ctx, int ncase, const sddc_case *cases)
         cp[c].dt = k.dt;
         cp[c].pad = 0.0;
     }
-    int rc;
-    cudaFree(ctx->case_dev);
-    ctx->case_dev = nullptr;
-    if ((rc = alloc(ctx, (void **)&ctx->case_dev, ncase * sizeof(CaseParams), "case table"))) return rc;
-    CK(cudaMemcpyAsync(ctx->case_dev, cp.data(), ncase * sizeof(CaseParams), cudaMemcpyHostToDevice, ctx->stream));
-    if ((rc = build_tiles(ctx))) return rc;
-    // per-case running maxima and per-tile monitor partials
-    cudaFree(ctx->maxima);
-    cudaFree(ctx->max_scratch);  // sized by the cases: the next sensor read allocates it anew
-    cudaFree(ctx->mon_part);
-    ctx->maxima = nullptr;
-    ctx->max_scratch = nullptr;
-    ctx->mon_part = nullptr;
-    ctx->sensor_stale = false;
-    if ((rc = alloc(ctx, (void **)&ctx->maxima, (size_t)ncase * kSlots * 2 * sizeof(double), "maxima")) ||
-        (rc = alloc(ctx, (void **)&ctx->mon_part, (size_t)ctx->ntiles * 2 * sizeof(double), "monitor")))
+    Held case_dev, tiles, maxima, mon_part;  // per case: parameters, running maxima; per tile: monitor partials
+    int rc, ntiles = 0;
+    if ((rc = alloc(ctx, &case_dev.p, ncase * sizeof(CaseParams), "case table")) ||
+        (rc = build_tiles(ctx, cs, ctx->persistent, &tiles, &ntiles)) ||
+        (rc = alloc(ctx, &maxima.p, (size_t)ncase * kSlots * 2 * sizeof(double), "maxima")) ||
+        (rc = alloc(ctx, &mon_part.p, (size_t)ntiles * 2 * sizeof(double), "monitor")))
         return rc;
-    CK(cudaMemsetAsync(ctx->maxima, 0, (size_t)ncase * kSlots * 2 * sizeof(double), ctx->stream));
-    CK(cudaMemsetAsync(ctx->mon_part, 0, (size_t)ctx->ntiles * 2 * sizeof(double), ctx->stream));
-    drop_graphs(ctx);
+    CK(cudaMemcpyAsync(case_dev.p, cp.data(), ncase * sizeof(CaseParams), cudaMemcpyHostToDevice, ctx->stream));
+    CK(cudaMemsetAsync(maxima.p, 0, (size_t)ncase * kSlots * 2 * sizeof(double), ctx->stream));
+    CK(cudaMemsetAsync(mon_part.p, 0, (size_t)ntiles * 2 * sizeof(double), ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
+    drop_graphs(ctx);
+    case_dev.give(ctx->case_dev);
+    tiles.give(ctx->tiles);
+    maxima.give(ctx->maxima);
+    mon_part.give(ctx->mon_part);
+    cudaFree(ctx->max_scratch);  // sized by the cases: the next sensor read allocates it anew
+    ctx->max_scratch = nullptr;
+    ctx->sensor_stale = false;
+    ctx->by_tiles = false;  // batches run by lines
+    ctx->cpb = line_tile_cells(ctx->N);
+    ctx->ncase = ncase;
+    ctx->cases = cs;
+    ctx->ntiles = ntiles;
     ctx->state = false;  // the maxima were reset: set the state again
     ctx->mon_nblk = 0;
     return SDDC_OK;
@@ -990,13 +996,18 @@ extern "C" int sddc_set_cases(sddc_ctx *ctx, int ncase, const sddc_case *cases)
 extern "C" int sddc_set_persistent(sddc_ctx *ctx, int on)
 {
     if (!ctx) return SDDC_EINVAL;
-    ctx->persistent = on != 0;
     if (ctx->ncase) {  // the tile table in the launch's order
-        const int rc = build_tiles(ctx);
+        Held tiles;
+        int ntiles = 0;
+        const int rc = build_tiles(ctx, ctx->cases, on != 0, &tiles, &ntiles);
         if (rc) return rc;
+        CK(cudaStreamSynchronize(ctx->stream));
+        drop_graphs(ctx);
+        tiles.give(ctx->tiles);
+        ctx->ntiles = ntiles;
     }
     drop_graphs(ctx);
-    CK(cudaStreamSynchronize(ctx->stream));
+    ctx->persistent = on != 0;
     return SDDC_OK;
 }
 

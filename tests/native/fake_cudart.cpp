@@ -53,6 +53,7 @@ struct Event {
     Stream *stream = nullptr;
 };
 Stream null_stream;
+std::vector<Stream *> streams{&null_stream};
 Stream &at(cudaStream_t s) { return s ? *reinterpret_cast<Stream *>(s) : null_stream; }
 void put(Stream &s, Work w) { (s.capture ? *s.capture : s.queue).push_back(std::move(w)); }
 void drain(Stream &s)
@@ -196,9 +197,14 @@ cudaError_t cudaMalloc(void **p, size_t n)
     *p = get(n, true);
     return cudaSuccess;
 }
-cudaError_t cudaFree(void *p) { release(p); return cudaSuccess; }
+cudaError_t cudaFree(void *p)  // waits for the device
+{
+    for (Stream *s : streams) drain(*s);
+    release(p);
+    return cudaSuccess;
+}
 cudaError_t cudaMallocHost(void **p, size_t n) { *p = get(n, false); return cudaSuccess; }
-cudaError_t cudaFreeHost(void *p) { release(p); return cudaSuccess; }
+cudaError_t cudaFreeHost(void *p) { return cudaFree(p); }
 cudaError_t cudaGetSymbolAddress(void **p, const void *sym)
 {
     Var &v = vars[sym];
@@ -227,7 +233,7 @@ cudaError_t cudaMemsetAsync(void *d, int v, size_t n, cudaStream_t st)
     return cudaSuccess;
 }
 
-cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned) { *s = reinterpret_cast<cudaStream_t>(new Stream); return cudaSuccess; }
+cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned) { streams.push_back(new Stream); *s = reinterpret_cast<cudaStream_t>(streams.back()); return cudaSuccess; }
 cudaError_t cudaStreamCreateWithPriority(cudaStream_t *s, unsigned f, int) { return cudaStreamCreateWithFlags(s, f); }
 cudaError_t cudaStreamDestroy(cudaStream_t s) { drain(at(s)); return cudaSuccess; }
 cudaError_t cudaStreamSynchronize(cudaStream_t s) { drain(at(s)); return cudaSuccess; }

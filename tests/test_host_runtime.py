@@ -197,3 +197,67 @@ def test_every_kernel_has_its_attributes_on_every_gpu(runtime):
                     s.close()
         clean()
         """)
+
+
+def test_calls_after_a_failed_allocation(runtime):
+    """Whichever allocation of a call fails: the call says so, and what follows
+    finds the context as it was or whole, never half of what was to be made."""
+    _run(runtime, """
+        m, t, ph, Q = case_periodic(6, 3)
+        def records(n):
+            edges = np.linspace(0, t.ncell, n + 1).astype(int)
+            return [dict(first_cell=int(a), ncell=int(b - a), dt=1e-3, rinf=1., pinf=1., uinf=.1, vinf=0., bxinf=0.,
+                         byinf=0.) for a, b in zip(edges[:-1], edges[1:])]
+
+        def fails(call, k):
+            F.fake_fail_alloc(k)
+            try:
+                call()
+                return False
+            except SddcError as e:
+                assert e.code == -5, e
+                return True
+            finally:
+                F.fake_fail_alloc(-1)
+
+        # the VJP's work space and the residual's arrays
+        for call in (lambda s: s.vjp_resid(Q), lambda s: s.compresid()):
+            k = 0
+            while True:
+                s = Solver(t, ph, precision="fp64")
+                s.set_state(Q)
+                failed = fails(lambda: call(s), k)
+                call(s)
+                s.compresid()
+                s.state(resid=True, nablaQs=True)
+                s.close()
+                if not failed:
+                    break
+                k += 1
+            assert k > 1, k
+        # a batch: the one that was set, or none, stays in force
+        for before in (0, 3):
+            for k in range(4):
+                s = Solver(t, ph, precision="fp64")
+                if before:
+                    s.set_cases(records(before))
+                s.set_state(Q)
+                step = (lambda: s.step_cases(1)) if before else (lambda: s.rk_s5p3(1e-3, 1))
+                step()
+                assert fails(lambda: s.set_cases(records(20)), k)
+                step()
+                s.compresid()
+                s.monitor()
+                s.state(sm_ind=True)
+                if before:
+                    assert fails(lambda: s.set_persistent(True), 0)
+                    n = launches("persistent")
+                    step()
+                    assert launches("persistent") == n
+                s.set_cases(records(20))
+                s.set_state(Q)
+                s.step_cases(1)
+                s.monitor()
+                s.close()
+        clean()
+        """)
