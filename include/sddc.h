@@ -105,8 +105,8 @@ int sddc_set_state(sddc_ctx *ctx, const double *Q, double ctime, double eigvmax,
 int sddc_compresid(sddc_ctx *ctx);
 
 /* nsteps time steps of size dt with the scheme of k_stage (RK_S5P3 or
-   FiveStageRk), 5 residual evaluations per step.  Launches are captured in a
-   CUDA graph after the first step.  Returns SDDC_ENUMERIC if any stage saw a
+   FiveStageRk), 5 residual evaluations per step.  Launches are captured in
+   CUDA graphs where enough steps of one dt come.  Returns SDDC_ENUMERIC if any stage saw a
    non-positive density or a non-finite wave speed (the state is still
    advanced, as the reference would). */
 int sddc_rk_step(sddc_ctx *ctx, double dt, int nsteps);

@@ -156,6 +156,7 @@ static void drop_graphs(sddc_ctx *ctx)
             g = {};
         }
     ctx->stepped_dt = -1.0;
+    ctx->dt_steps = 0;
 }
 
 static void free_all(sddc_ctx *ctx)
@@ -740,15 +741,22 @@ static int run_steps(sddc_ctx *ctx, double dt, int nsteps)
         CK(cudaStreamSynchronize(ctx->stream));
         return check_flags(ctx);
     }
-    // Steps replay a graph of 1 or of kGraphSteps steps.  The first step with a
-    // dt runs eagerly (kernel attributes, warm-up; a dt that changes from call
-    // to call never pays for a capture); a graph is captured when its steps
-    // come a second time, in the same call or in a later one.
-    const double seen = ctx->stepped_dt;
+    // Steps replay a graph of 1 or of kGraphSteps steps with their dt, captured
+    // where the steps run and those still to come pay for it, as far as they
+    // are known: dt may be another in the next call.  A call's first step runs
+    // eagerly (kernel attributes, warm-up) until kGraphSteps have come with its
+    // dt, the later ones as a graph at once; the longer graph waits for
+    // kGraphPays.  On a small mesh (576 cells, mixed, us) an eager step takes
+    // 45, one by a graph 39, in the longer graph 33; the captures take about
+    // 100 and 250.  us per call of 10 and of 33 steps with a dt of its own: no
+    // longer graph in the first 480 and 1322, one in both 577 and 1210.
+    if (ctx->stepped_dt != dt) ctx->dt_steps = 0;
     for (int s = 0; s < nsteps;) {
         const int s0 = ctx->slot;
-        const bool warm = s > 0 || seen == dt;
-        const int many = warm && nsteps - s >= kGraphSteps ? 1 : 0;
+        const bool warm = s > 0 || ctx->dt_steps >= kGraphSteps;
+        const auto &longer = ctx->graph[s0][1];
+        const bool paid = (longer.exec && longer.dt == dt) || ctx->dt_steps + (nsteps - s) >= kGraphPays;
+        const int many = warm && nsteps - s >= kGraphSteps && paid ? 1 : 0;
         const int n = many ? kGraphSteps : 1;
         sddc_ctx::StepGraph &g = ctx->graph[s0][many];
         if (g.exec && g.dt != dt) {
@@ -778,6 +786,7 @@ static int run_steps(sddc_ctx *ctx, double dt, int nsteps)
         for (int k = 0; k < n; k++) ctx->ctime += dt;
         s += n;
         ctx->stepped_dt = dt;
+        ctx->dt_steps = std::min(ctx->dt_steps + n, kGraphPays);
         ctx->sensor_stale = true;
         ctx->mon_nblk = ctx->ncase ? ctx->ntiles : ctx->grid;
     }

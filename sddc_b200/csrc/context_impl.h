@@ -41,7 +41,9 @@ cudaError_t launch_visc_mixed(int N, const ViscArgs &a, const Ops &ops, cudaStre
 namespace sddc {
 
 constexpr int kSlots = 5;     // rotating running-max slots
-constexpr int kGraphSteps = 8;  // time steps of the longer graph (a small mesh's step takes about 35 us)
+// time steps of the longer graph (a small mesh's step takes about 35 us), and
+// how many with one dt pay for its capture
+constexpr int kGraphSteps = 8, kGraphPays = 32;
 constexpr int kRegs = 6;      // RK registers (FiveStageRk needs six)
 constexpr int kMonThreads = 256;
 
@@ -108,6 +110,7 @@ struct sddc_ctx {
     };
     StepGraph graph[sddc::kSlots][2];  // by the slot a step starts from: one step, kGraphSteps steps
     double stepped_dt = -1.0;          // dt of the last step run (-1: none since the graphs were dropped)
+    int dt_steps = 0;                  // steps run with it
     // batch of independent cases (sddc_set_cases); ncase == 0 for one case
     int ncase = 0;
     std::vector<sddc_case> cases;

@@ -99,3 +99,20 @@ def test_steps_of_a_diverged_mesh(form):
     # (measured per stage 1.1 to 1.6 times; 100 to 130 with every warp's OR
     # across the host link)
     assert diverged < 10 * max(sound, again), (sound, diverged, again)
+
+
+@pytest.mark.parametrize("form", ["fp64_exact", "fp64", "mixed"])
+def test_steps_of_long_and_short_calls_are_the_same(form):
+    """Eager steps, graphs of one step and of several: the same bits and time."""
+    m, t, ph, Q = case_channel(9, 7, 4)
+    dt = 0.1 * m.min_edge() / 4
+    out = []
+    for groups in ([1] * 50, [50], [20, 1, 29], [9] * 5 + [5]):
+        s = Solver(t, ph, precision=form)
+        s.set_state(Q)
+        for n in groups:
+            s.rk_s5p3(dt, n)
+        out.append((s.state()["Q"].copy(), s.maxima()))
+        s.close()
+    for q, mx in out[1:]:
+        assert np.array_equal(q, out[0][0]) and mx == out[0][1]

@@ -261,3 +261,31 @@ def test_calls_after_a_failed_allocation(runtime):
                 s.close()
         clean()
         """)
+
+
+def test_graphs_are_captured_where_their_steps_pay(runtime):
+    """A dt that changes from call to call (an adaptive step) pays for no more
+    captures than its steps win back; a constant dt gets its graphs."""
+    _run(runtime, """
+        m, t, ph, Q = case_cylinder()
+        s = Solver(t, ph, precision="fp64")
+        s.set_state(Q)
+
+        def graphs(calls):
+            a, b = launches("graph instantiation"), launches("graph launch")
+            for dt, n in calls:
+                s.rk_s5p3(dt, n)
+            return launches("graph instantiation") - a, launches("graph launch") - b
+
+        # ten steps with a dt each: the graph of a single step, no longer one
+        assert graphs([(1e-3 * (1 + 1e-6 * k), 10) for k in range(1, 6)]) == (5, 45)
+        # a dt for two single steps each: none
+        assert graphs([(2e-3 * (1 + 1e-6 * (k // 2)), 1) for k in range(10)]) == (0, 0)
+        # one dt: a graph after some single steps; the longer one in a long call
+        # and, from many calls, after as many steps
+        assert graphs([(3e-3, 1)] * 20) == (1, 12)
+        assert graphs([(3e-3, 8)]) == (0, 8)
+        assert graphs([(3e-3, 8)] * 2) == (1, 2)
+        assert graphs([(4e-3, 41)]) == (1, 5)
+        clean()
+        """)
