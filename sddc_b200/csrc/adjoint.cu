@@ -314,7 +314,7 @@ int reverse_stage(sddc_ctx *ctx, const RevStage &s)
 int adjoint_flags(sddc_ctx *ctx)
 {
     CKA(cudaStreamSynchronize(ctx->stream));
-    const unsigned f = *(volatile unsigned *)ctx->err_flags.host;
+    const unsigned f = *(volatile unsigned *)ctx->err_host;
     if (f & (kErrAdjointMaxLost | kErrAdjointRecords)) {
         take_flags(ctx);
         if (f & kErrAdjointRecords) return set_err(ctx, SDDC_ENUMERIC, "adjoint: more points attain a running maximum than the record buffer holds");

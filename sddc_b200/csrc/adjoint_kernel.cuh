@@ -78,7 +78,7 @@ struct VjpArgs {
     double sx, sy;
     double wq[kMaxN];
     double *part;  // [8][CTAs]: cbar, pbar[6], 0
-    FaultFlags err;
+    FaultFlags *err;
     // the next reverse stage's adjoint traces, formed from out (the adjoint of
     // that stage's output) in the epilogue: its input state and lam_scale, and
     // the trace buffer (null: its own trace launch forms them)
@@ -234,7 +234,7 @@ struct RecSink {
     int cap;
     int *n;
     int *cnt;
-    FaultFlags err;
+    FaultFlags *err;
 };
 
 static __device__ __noinline__ void adj_record(RecSink rs, int cell, int slot, int kind, int counted, const double *d,
@@ -848,7 +848,7 @@ static __global__ void __launch_bounds__(kRedThreads) adj_reduce_kernel(int nblk
                                                                  double dc_dl, double dc_du,
                                                                  const AdjRec *__restrict__ recs, int *rec_n,
                                                                  int *rec_cnt, int rec_cap, double *out,
-                                                                 const Ops ops, FaultFlags err, NextTraces next)
+                                                                 const Ops ops, FaultFlags *err, NextTraces next)
 {
     __shared__ double s[7][kRedThreads / 32];
     __shared__ double w[2];

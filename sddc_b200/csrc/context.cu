@@ -166,7 +166,7 @@ static void free_all(sddc_ctx *ctx)
     for (auto &r : ctx->reg) cudaFree(r), r = nullptr;
     for (auto &t : ctx->trace) cudaFree(t), t = nullptr;
     void *bufs[] = {ctx->met, ctx->nrm, ctx->jac, ctx->faces, ctx->maxima, ctx->sm_ind, ctx->muav, ctx->resid, ctx->grad,
-                    ctx->mon_part, ctx->mon_out, ctx->int_part, ctx->wq, ctx->err_flags.dev,
+                    ctx->mon_part, ctx->mon_out, ctx->int_part, ctx->wq, ctx->err_flags,
                     ctx->case_dev, ctx->tiles, ctx->visc_grad, ctx->visc_gt,
                     ctx->visc_rv, ctx->met2, ctx->max_scratch, ctx->proc_cells};
     for (void *b : bufs) cudaFree(b);
@@ -249,7 +249,7 @@ extern "C" int sddc_create(sddc_ctx **out, const sddc_params *p)
         (rc = alloc(ctx, (void **)&ctx->mon_out, 4 * sizeof(double), "monitor")) ||
         (rc = alloc(ctx, (void **)&ctx->int_part, 1024 * 2 * sizeof(double), "integrals")) ||
         (rc = alloc(ctx, (void **)&ctx->wq, kMaxN * sizeof(double), "weights")) ||
-        (rc = alloc(ctx, (void **)&ctx->err_flags.dev, sizeof(unsigned), "flags")))
+        (rc = alloc(ctx, (void **)&ctx->err_flags, sizeof(FaultFlags), "flags")))
         return rc;
     // the viscous chain runs only with vismode = 1 (compflux.f90:36)
     ctx->visc = p->vismode == 1 && (p->mu != 0.0 || p->eta0 != 0.0);
@@ -261,9 +261,10 @@ extern "C" int sddc_create(sddc_ctx **out, const sddc_params *p)
             return rc;
     }
     CK(cudaMallocHost((void **)&ctx->host_small, 65 * sizeof(double)));
-    ctx->err_flags.host = reinterpret_cast<unsigned *>(ctx->host_small + 64);
-    *ctx->err_flags.host = 0;
-    CK(cudaMemsetAsync(ctx->err_flags.dev, 0, sizeof(unsigned), ctx->stream));
+    ctx->err_host = reinterpret_cast<unsigned *>(ctx->host_small + 64);
+    *ctx->err_host = 0;
+    const FaultFlags flags{0, 0, ctx->err_host};
+    CK(cudaMemcpyAsync(ctx->err_flags, &flags, sizeof(flags), cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemsetAsync(ctx->maxima, 0, kSlots * 2 * sizeof(double), ctx->stream));
     CK(cudaMemsetAsync(ctx->sm_ind, 0, nc * 2 * sizeof(double), ctx->stream));
     CK(cudaMemsetAsync(ctx->mon_part, 0, (size_t)mon_blocks * 2 * sizeof(double), ctx->stream));
@@ -600,12 +601,12 @@ static int proc_ready(sddc_ctx *ctx)
 
 unsigned sddc::take_flags(sddc_ctx *ctx)
 {
-    const unsigned f = *(volatile unsigned *)ctx->err_flags.host;
+    const unsigned f = *(volatile unsigned *)ctx->err_host;
     // both words, and before the next launch, on whatever stream it goes; where
     // that fails the host's word stays, for the next call to report
-    if (f && cudaMemsetAsync(ctx->err_flags.dev, 0, sizeof(unsigned), ctx->stream) == cudaSuccess &&
+    if (f && cudaMemsetAsync(&ctx->err_flags->bits, 0, sizeof(unsigned), ctx->stream) == cudaSuccess &&
         cudaStreamSynchronize(ctx->stream) == cudaSuccess)
-        *ctx->err_flags.host = 0;
+        *ctx->err_host = 0;
     return f;
 }
 

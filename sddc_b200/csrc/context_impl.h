@@ -87,8 +87,9 @@ struct sddc_ctx {
     double *maxima = nullptr;  // [sddc::kSlots][2]
     double *sm_ind = nullptr, *muav = nullptr, *resid = nullptr, *grad = nullptr;
     double *mon_part = nullptr, *mon_out = nullptr, *int_part = nullptr, *wq = nullptr;
-    // numerical faults; the host's word lies behind host_small
-    FaultFlags err_flags{};
+    // numerical faults, and the host's word of them behind host_small
+    FaultFlags *err_flags = nullptr;
+    unsigned *err_host = nullptr;
     double *host_small = nullptr;  // pinned scratch for small read-backs
     Ops ops{};
     int slot = 0;  // slot holding the running maxima after the last evaluation

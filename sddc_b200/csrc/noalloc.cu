@@ -61,7 +61,7 @@ ScratchLayout layout(const sddc_params &p)
     ScratchLayout s;
     const size_t elem = p.precision == SDDC_MIXED ? sizeof(float) : sizeof(double);
     s.maxima = 0;                                               // [5][2] doubles
-    s.flags = s.maxima + 10 * sizeof(double);                   // unsigned, read back with the maxima
+    s.flags = s.maxima + 10 * sizeof(double);                   // FaultFlags, its bits read back with the maxima
     s.sm_ind = 512;                                             // (2, NCELL) doubles
     s.trace = up256(s.sm_ind + 2 * (size_t)p.ncell * sizeof(double));
     s.tfs = trace_stride(p.N, (int)elem);                       // face traces
@@ -173,12 +173,12 @@ extern "C" int sddc_compresid_noalloc(const sddc_params *p, const double *Lmat, 
     // one clears them, in its stream, before it returns: the next call may come
     // on another stream.
     double *maxima = reinterpret_cast<double *>(scratch + L.maxima);
-    unsigned *flags = reinterpret_cast<unsigned *>(scratch + L.flags);
-    const TraceInit init{{flags, nullptr}, maxima, eigvmax, umax};
+    FaultFlags *flags = reinterpret_cast<FaultFlags *>(scratch + L.flags);  // (its host word stays null)
+    const TraceInit init{flags, maxima, eigvmax, umax};
     void *trace = scratch + L.trace;
     cudaError_t e;
     auto clear_flags = [&]() {
-        const cudaError_t m = cudaMemsetAsync(flags, 0, sizeof(unsigned), st);
+        const cudaError_t m = cudaMemsetAsync(&flags->bits, 0, sizeof(unsigned), st);
         return m == cudaSuccess ? cudaStreamSynchronize(st) : m;
     };
     auto fail_cuda = [&](const char *what) {
@@ -211,7 +211,7 @@ extern "C" int sddc_compresid_noalloc(const sddc_params *p, const double *Lmat, 
     a.resid_out = resid_dev;
     a.grad_out = nablaqs_dev;
     a.mon_part = nullptr;
-    a.err_flags = {flags, nullptr};
+    a.err_flags = flags;
     switch (p->precision) {
     case SDDC_FP64_EXACT: e = launch_resid_exact(N, a, ops, st); break;
     case SDDC_FP64: e = launch_resid_fp64(N, a, ops, st); break;

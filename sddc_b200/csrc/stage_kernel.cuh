@@ -119,19 +119,20 @@ enum RkKind : int {
     kRkFive = 4      // out = ((((c1*a + c2*b) + c3*c) + c4*q) + c5*d) + c0*r   FiveStageRk stage 5
 };
 
-// Where kernels leave fault bits: OR-ed into a word in device memory and, by the
-// launch that first finds a bit missing there, into the host's word (pinned;
-// null where the caller copies the device word), which is read after a
+// Where kernels leave fault bits, in device memory: OR-ed into its word and, by the
+// warp that first finds a bit missing there, into the host's (pinned; null
+// where the caller copies the device word), which is read after a
 // synchronisation without a copy.  A diverged mesh faults in every warp of every
 // stage: with all of them OR-ed across the host link a stage of 131072 cells
 // (N = 5, FP64) took 41.7 ms, so 0.39 (0.34 without a fault).
 struct FaultFlags {
-    unsigned *dev, *host;
+    unsigned bits, pad;
+    unsigned *host;
 };
-__device__ __forceinline__ void raise_fault(const FaultFlags &f, unsigned bits)
+__device__ __forceinline__ void raise_fault(FaultFlags *f, unsigned bits)
 {
-    const unsigned seen = atomicOr(f.dev, bits);
-    if (f.host && (bits & ~seen)) atomicOr(f.host, bits);
+    const unsigned seen = atomicOr(&f->bits, bits);
+    if ((bits & ~seen) && f->host) atomicOr(f->host, bits);
 }
 
 // per-case data of a batch of independent cases sharing one launch
@@ -191,13 +192,13 @@ struct StageArgs {
     double *__restrict__ mon_part;     // per-CTA (sum resid^2, sum divB^2), or null
     double *__restrict__ cta_max;      // per-CTA (max eigv, max umax) of this stage, or null
     const double *__restrict__ visc;   // dFv + dGv (9,N,N,NCELL) of the viscous chain, or null (mu = eta0 = 0)
-    FaultFlags err_flags;
+    FaultFlags *err_flags;
 };
 
 // beside the state and the traces, what a launch of the face traces takes: the
 // fault flags and, where not null, the running-max slots it sets to a seed
 struct TraceInit {
-    FaultFlags flags;
+    FaultFlags *flags;
     double *maxima = nullptr;
     double eig = 0.0, um = 0.0;
 };

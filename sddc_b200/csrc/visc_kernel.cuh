@@ -56,7 +56,7 @@ struct ViscArgs {
     double *grad;  // nablaQs (9,2,N,N,NCELL)
     double *gt;    // gradient traces [cell][lf][18][nfp]: (9 x-derivatives, 9 y-derivatives)
     double *rv;    // dFv + dGv (9,N,N,NCELL)
-    FaultFlags err_flags;
+    FaultFlags *err_flags;
 };
 
 // o[k-1] = Fv(k) n0 + Gv(k) n1, k = 1..7, of getVfluxvectors
