@@ -285,7 +285,7 @@ int reverse_stage(sddc_ctx *ctx, const RevStage &s)
         LocateArgs l{};
         l.ncell = ctx->ncell;
         l.vismode = ctx->p.vismode;
-        l.cpb = ctx->cpb;
+        l.cpb = ctx->ex_cpb;
         l.c_h = c_h;
         l.fs = a.fs;
         l.q = s.q;
@@ -298,7 +298,7 @@ int reverse_stage(sddc_ctx *ctx, const RevStage &s)
         l.eig_max = s.Lnext;
         l.um_max = s.Unext;
         l.rs = RecSink{w->recs, w->rec_cap, w->rec_n, w->rec_n + 1, ctx->err_flags};
-        CKA(launch_adj_locate(ctx->N, (ctx->ncell + ctx->cpb - 1) / ctx->cpb, l, ctx->ops, ctx->stream));
+        CKA(launch_adj_locate(ctx->N, ceil_div(ctx->ncell, ctx->ex_cpb), l, ctx->ops, ctx->stream));
     }
     if (!s.reduce) return SDDC_OK;
     double dl = 0.0, du = 0.0;
@@ -341,7 +341,7 @@ const FwdStage kS5P3[5] = {{kRkAxpy, 0, 1, -1, {B10, 0, 0}},
 int forward_steps(sddc_ctx *ctx, double dt, int step0, int nsteps, double *const *S, double *const *T, double *hist,
                   int n1, int n2, double *force, double *cmax, cudaStream_t st)
 {
-    const size_t fgrid = (ctx->ncell + ctx->cpb - 1) / ctx->cpb;
+    const size_t fgrid = ceil_div(ctx->ncell, ctx->ex_cpb);
     for (int m = 0; m < nsteps; m++) {
         for (int k = 0; k < 5; k++) {
             const FwdStage &f = kS5P3[k];
@@ -474,7 +474,7 @@ extern "C" int sddc_adjoint_run(sddc_ctx *ctx, const sddc_adjoint_opts *o, doubl
     RunBufs rb;
     std::vector<double *> ckpt(nseg), S(5 * segmax + 1), T(5 * segmax + 1);
     double *hist = nullptr, *force = nullptr, *cmax = nullptr, *fin = nullptr, *A[6] = {};
-    const size_t ncmax = (size_t)5 * segmax * 2 * ((ctx->ncell + ctx->cpb - 1) / ctx->cpb);
+    const size_t ncmax = (size_t)5 * segmax * 2 * (ceil_div(ctx->ncell, ctx->ex_cpb));
     for (auto &c : ckpt) rb.name(&c, nq);
     for (int i = 0; i <= 5 * segmax; i++) {
         rb.name(&S[i], nq);
@@ -646,7 +646,7 @@ extern "C" int sddc_adjoint_run(sddc_ctx *ctx, const sddc_adjoint_opts *o, doubl
             double *cmax_ = CM[cur];
             for (int m = nst - 1; m >= 0; m--) {
                 const int n = step0 + m, i = 5 * m;
-                const size_t fgrid = (ctx->ncell + ctx->cpb - 1) / ctx->cpb;
+                const size_t fgrid = ceil_div(ctx->ncell, ctx->ex_cpb);
                 auto maxima = [&](RevStage &r, int k) {
                     const size_t g = (size_t)5 * n + k;
                     r.cta_max = cmax_ + (size_t)(5 * m + k) * 2 * fgrid;

@@ -167,7 +167,7 @@ static void free_all(sddc_ctx *ctx)
     for (auto &t : ctx->trace) cudaFree(t), t = nullptr;
     void *bufs[] = {ctx->met, ctx->nrm, ctx->jac, ctx->faces, ctx->maxima, ctx->sm_ind, ctx->muav, ctx->resid, ctx->grad,
                     ctx->mon_part, ctx->mon_out, ctx->int_part, ctx->wq, ctx->err_flags,
-                    ctx->case_dev, ctx->tiles, ctx->visc_grad, ctx->visc_gt,
+                    ctx->case_dev, ctx->tiles, ctx->tiles_resid, ctx->visc_grad, ctx->visc_gt,
                     ctx->visc_rv, ctx->met2, ctx->max_scratch, ctx->proc_cells};
     for (void *b : bufs) cudaFree(b);
     if (ctx->host_small) cudaFreeHost(ctx->host_small);
@@ -193,6 +193,50 @@ int sddc::alloc(sddc_ctx *ctx, void **p, size_t bytes, const char *what)
     return SDDC_OK;
 }
 
+// us of a stage of the exact form from the waves its CTAs make on the device:
+// base once, full per wave that fills it, start for a last wave and the rest of
+// full in proportion to the places it takes
+struct WaveCost {
+    double base, start, full;
+};
+static double stage_us(int tiles, int resident, const WaveCost &c)
+{
+    const int rest = tiles % resident;
+    return c.base + tiles / resident * c.full + (rest ? c.start + (c.full - c.start) * rest / resident : 0.0);
+}
+
+// Whether stages of the exact form run by tiles (stage_kernel.cuh) or by lines
+// (line_kernel.cuh), given the CTAs of either.  A line's 2N+2 dependent point
+// fluxes, in unfused operations, are a longer chain than the tile's phases: a wave
+// of lines takes longer to start, and less per cell once full.  At N = 6 the
+// line's sums leave no registers for its states, and tiles are faster at every
+// size; at N = 5 up to 90000 cells (401 us, 402 by lines), and general (batches,
+// metrics from the packed records) to about five waves.  Fitted to sweeps of 8
+// to 62500 cells and to batches of 512 to 32768 in 8 and 16 cases, where the choice
+// is within 2.3% of the faster one.  A persistent launch of several waves evens
+// them out by lines, not by tiles (16 cases of 506 cells: N = 2, 11.1 and 12.1; N = 4,
+// 25.3 and 26.5; N = 5 50.8 and 45.8).  us per stage, by tiles and by lines: N = 2,
+// 9409 cells 11.7 and 12.2, 10000 16.6 and 12.2; N = 3, 4489 12.2 and 15.4, 8100 22.3
+// and 16.8, 9409 23.1 and 28.0; N = 4, 4096 13.5 and 14.8, 6400 21.5 and 20.3, 8100
+// 23.7 and 27.3, 14400 42.3 and 49.3, 32400 88.6 and 86.3; N = 5, 4096 21.8 and 31.8,
+// 16 cases of 2025 180 and 170; N = 6, 32400 220 and 246.
+static cudaError_t exact_by_tiles(int N, bool general, bool persistent, int tiles, int lines, bool *out)
+{
+    *out = true;
+    if (N == 6 || (N == 5 && !general)) return cudaSuccess;
+    static const WaveCost by_tile[] = {{2.3, 5.0, 9.3}, {2.2, 4.4, 10.5}, {0.7, 7.4, 12.5}, {1.4, 8.2, 14.0}};
+    static const WaveCost by_line[] = {{1.7, 7.2, 11.5}, {1.5, 10.2, 16.5}, {0.8, 11.8, 13.7}, {4.6, 10.4, 17.4}};
+    static const WaveCost by_wide = {4.4, 9.9, 17.2};
+    int rt = 0, held = 0, wide = 0;
+    cudaError_t e = tile_residency_exact(N, &rt);
+    if (e == cudaSuccess) e = line_residency_exact(N, &held, &wide);
+    if (e != cudaSuccess) return e;
+    const double us = wide && line_use_wide(lines, held, wide) ? stage_us(lines, wide, by_wide)
+                                                               : stage_us(lines, held, by_line[N - 2]);
+    *out = stage_us(tiles, rt, by_tile[N - 2]) <= us && !(persistent && N <= 4 && tiles > rt);
+    return cudaSuccess;
+}
+
 extern "C" int sddc_create(sddc_ctx **out, const sddc_params *p)
 {
     if (!out || !p) return SDDC_EINVAL;
@@ -215,14 +259,16 @@ extern "C" int sddc_create(sddc_ctx **out, const sddc_params *p)
         return bad("cells_per_cta must be 0, 4, 6, 8 or 16");
     ctx->N = p->N;
     ctx->ncell = p->ncell;
-    // time steps run by lines, or (exact form) by tiles: see exact_by_tiles
-    ctx->by_tiles = p->precision == SDDC_FP64_EXACT && exact_by_tiles(p->N, p->ncell);
-    ctx->cpb = ctx->by_tiles ? tile_cells(p->N, p->ncell) : line_tile_cells(p->N);
     if (!ctx->p.ncellglob) ctx->p.ncellglob = p->ncell;
     ctx->msize = met_size(p->N);
     ctx->nq = (size_t)9 * p->N * p->N * p->ncell;
-    ctx->grid = (p->ncell + ctx->cpb - 1) / ctx->cpb;
     *out = ctx;
+    const int exact_cpb = tile_cells(p->N, p->ncell);
+    CK(exact_by_tiles(p->N, p->precision != SDDC_FP64_EXACT, false, ceil_div(p->ncell, exact_cpb), resid_grid(ctx),
+                      &ctx->by_tiles));
+    ctx->ex_cpb = ctx->by_tiles ? exact_cpb : line_tile_cells(p->N);
+    ctx->cpb = p->precision == SDDC_FP64_EXACT ? ctx->ex_cpb : line_tile_cells(p->N);
+    ctx->grid = ceil_div(p->ncell, ctx->cpb);
     CK(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
     const int nreg = p->k_stage == 5 ? 6 : 4;
     int rc;
@@ -554,7 +600,7 @@ static cudaError_t launch_visc(sddc_ctx *ctx, const double *q_in, const void *t_
 // a stage of the exact form, by the kernel that the context's tiles are for
 cudaError_t sddc::launch_rk_exact(sddc_ctx *ctx, const StageArgs &a, cudaStream_t st)
 {
-    return ctx->by_tiles ? launch_tile_exact(ctx->N, ctx->cpb, a, ctx->ops, st)
+    return ctx->by_tiles ? launch_tile_exact(ctx->N, ctx->ex_cpb, a, ctx->ops, st)
                          : launch_line_exact(ctx->N, a, ctx->ops, st);
 }
 
@@ -567,8 +613,8 @@ static cudaError_t launch(sddc_ctx *ctx, bool diag, const StageArgs &a_in)
         a.visc = ctx->visc_rv;
     }
     if (ctx->ncase) {  // a batch: one CTA per tile of the case-aligned tile table
-        a.tiles = ctx->tiles;
-        a.ntiles = ctx->ntiles;
+        a.tiles = diag ? ctx->tiles_resid : ctx->tiles;
+        a.ntiles = diag ? ctx->ntiles_resid : ctx->ntiles;
         a.cases = ctx->case_dev;
         a.persistent = ctx->persistent ? 1 : 0;
     }
@@ -644,7 +690,7 @@ extern "C" int sddc_compresid(sddc_ctx *ctx)
     if ((rc = exchange(ctx, 0, a.slot_w))) return rc;
     ctx->slot = a.slot_w;
     ctx->sensor_stale = false;
-    ctx->mon_nblk = ctx->ncase ? ctx->ntiles : resid_grid(ctx);
+    ctx->mon_nblk = ctx->ncase ? ctx->ntiles_resid : resid_grid(ctx);
     return check_flags(ctx);
 }
 
@@ -749,8 +795,8 @@ static int run_steps(sddc_ctx *ctx, double dt, int nsteps)
     // dt, the later ones as a graph at once; the longer graph waits for
     // kGraphPays.  On a small mesh (576 cells, mixed, us) an eager step takes
     // 45, one by a graph 39, in the longer graph 33; the captures take about
-    // 100 and 250.  us per call of 10 and of 33 steps with a dt of its own: no
-    // longer graph in the first 480 and 1322, one in both 577 and 1210.
+    // 100 and 250 (a call of 10 steps with a dt of its own: 480 without the
+    // longer graph, 577 with it).
     if (ctx->stepped_dt != dt) ctx->dt_steps = 0;
     for (int s = 0; s < nsteps;) {
         const int s0 = ctx->slot;
@@ -928,10 +974,16 @@ struct Held {
     }
 };
 
-// the tile table of cases for launches of the given kind
-static int build_tiles(sddc_ctx *ctx, const std::vector<sddc_case> &cases, bool persistent, Held *out, int *count)
+static int tile_count(const std::vector<sddc_case> &cases, int cpb)
 {
-    const int cpb = line_tile_cells(ctx->N);
+    int n = 0;
+    for (const sddc_case &k : cases) n += ceil_div(k.ncell, cpb);
+    return n;
+}
+
+// the table of cases in tiles of cpb cells, for launches of the given kind
+static int build_tiles(sddc_ctx *ctx, const std::vector<sddc_case> &cases, int cpb, bool persistent, Held *out, int *count)
+{
     // persistent launches walk the table with a grid stride, largest case
     // first; otherwise the cases in their order
     std::vector<int> order(cases.size());
@@ -950,6 +1002,35 @@ static int build_tiles(sddc_ctx *ctx, const std::vector<sddc_case> &cases, bool 
     *count = (int)tiles.size();
     return SDDC_OK;
 }
+
+// how the stages of a batch run: by tiles or by lines (exact form), and the tile
+// tables of the stages and of residual evaluations
+struct BatchPlan {
+    bool by_tiles = false;
+    int cpb = 0, ex_cpb = 0, ntiles = 0, ntiles_resid = 0, most = 0;  // most: monitor partials of any plan
+    Held tiles, tiles_resid;
+    int make(sddc_ctx *ctx, const std::vector<sddc_case> &cases, bool persistent)
+    {
+        const int N = ctx->N, lines = line_tile_cells(N), exact = tile_cells(N, ctx->ncell);
+        CK(exact_by_tiles(N, true, persistent, tile_count(cases, exact), tile_count(cases, lines), &by_tiles));
+        ex_cpb = by_tiles ? exact : lines;
+        cpb = ctx->p.precision == SDDC_FP64_EXACT ? ex_cpb : lines;
+        most = std::max(tile_count(cases, exact), tile_count(cases, lines));
+        int rc = build_tiles(ctx, cases, cpb, persistent, &tiles, &ntiles);
+        if (!rc) rc = build_tiles(ctx, cases, lines, persistent, &tiles_resid, &ntiles_resid);
+        return rc;
+    }
+    void give(sddc_ctx *ctx)
+    {
+        ctx->by_tiles = by_tiles;
+        ctx->cpb = cpb;
+        ctx->ex_cpb = ex_cpb;
+        ctx->ntiles = ntiles;
+        ctx->ntiles_resid = ntiles_resid;
+        tiles.give(ctx->tiles);
+        tiles_resid.give(ctx->tiles_resid);
+    }
+};
 
 extern "C" int sddc_set_cases(sddc_ctx *ctx, int ncase, const sddc_case *cases)
 {
@@ -974,30 +1055,28 @@ extern "C" int sddc_set_cases(sddc_ctx *ctx, int ncase, const sddc_case *cases)
         cp[c].dt = k.dt;
         cp[c].pad = 0.0;
     }
-    Held case_dev, tiles, maxima, mon_part;  // per case: parameters, running maxima; per tile: monitor partials
-    int rc, ntiles = 0;
+    Held case_dev, maxima, mon_part;  // per case: parameters, running maxima; per tile: monitor partials
+    BatchPlan plan;
+    int rc;
     if ((rc = alloc(ctx, &case_dev.p, ncase * sizeof(CaseParams), "case table")) ||
-        (rc = build_tiles(ctx, cs, ctx->persistent, &tiles, &ntiles)) ||
+        (rc = plan.make(ctx, cs, ctx->persistent)) ||
         (rc = alloc(ctx, &maxima.p, (size_t)ncase * kSlots * 2 * sizeof(double), "maxima")) ||
-        (rc = alloc(ctx, &mon_part.p, (size_t)ntiles * 2 * sizeof(double), "monitor")))
+        (rc = alloc(ctx, &mon_part.p, (size_t)plan.most * 2 * sizeof(double), "monitor")))
         return rc;
     CK(cudaMemcpyAsync(case_dev.p, cp.data(), ncase * sizeof(CaseParams), cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemsetAsync(maxima.p, 0, (size_t)ncase * kSlots * 2 * sizeof(double), ctx->stream));
-    CK(cudaMemsetAsync(mon_part.p, 0, (size_t)ntiles * 2 * sizeof(double), ctx->stream));
+    CK(cudaMemsetAsync(mon_part.p, 0, (size_t)plan.most * 2 * sizeof(double), ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     drop_graphs(ctx);
     case_dev.give(ctx->case_dev);
-    tiles.give(ctx->tiles);
+    plan.give(ctx);
     maxima.give(ctx->maxima);
     mon_part.give(ctx->mon_part);
     cudaFree(ctx->max_scratch);  // sized by the cases: the next sensor read allocates it anew
     ctx->max_scratch = nullptr;
     ctx->sensor_stale = false;
-    ctx->by_tiles = false;  // batches run by lines
-    ctx->cpb = line_tile_cells(ctx->N);
     ctx->ncase = ncase;
     ctx->cases = cs;
-    ctx->ntiles = ntiles;
     ctx->state = false;  // the maxima were reset: set the state again
     ctx->mon_nblk = 0;
     return SDDC_OK;
@@ -1006,15 +1085,12 @@ extern "C" int sddc_set_cases(sddc_ctx *ctx, int ncase, const sddc_case *cases)
 extern "C" int sddc_set_persistent(sddc_ctx *ctx, int on)
 {
     if (!ctx) return SDDC_EINVAL;
-    if (ctx->ncase) {  // the tile table in the launch's order
-        Held tiles;
-        int ntiles = 0;
-        const int rc = build_tiles(ctx, ctx->cases, on != 0, &tiles, &ntiles);
+    if (ctx->ncase) {  // the tile tables in the launch's order
+        BatchPlan plan;
+        const int rc = plan.make(ctx, ctx->cases, on != 0);
         if (rc) return rc;
         CK(cudaStreamSynchronize(ctx->stream));
-        drop_graphs(ctx);
-        tiles.give(ctx->tiles);
-        ctx->ntiles = ntiles;
+        plan.give(ctx);
     }
     drop_graphs(ctx);
     ctx->persistent = on != 0;

@@ -22,6 +22,9 @@ cudaError_t launch_line_exact(int N, const StageArgs &a, const Ops &ops, cudaStr
 cudaError_t launch_line_fp64(int N, const StageArgs &a, const Ops &ops, cudaStream_t st);
 cudaError_t launch_line_mixed(int N, const StageArgs &a, const Ops &ops, cudaStream_t st);
 cudaError_t launch_tile_exact(int N, int cpb, const StageArgs &a, const Ops &ops, cudaStream_t st);
+// CTAs of an exact stage resident at once, by tiles and by lines (N = 2..5)
+cudaError_t tile_residency_exact(int N, int *resident);
+cudaError_t line_residency_exact(int N, int *held, int *wide);
 cudaError_t launch_resid_exact(int N, const StageArgs &a, const Ops &ops, cudaStream_t st);
 cudaError_t launch_resid_fp64(int N, const StageArgs &a, const Ops &ops, cudaStream_t st);
 cudaError_t launch_resid_mixed(int N, const StageArgs &a, const Ops &ops, cudaStream_t st);
@@ -67,8 +70,12 @@ struct sddc_ctx {
     using CaseParams = sddc::CaseParams;
     using FaultFlags = sddc::FaultFlags;
     sddc_params p{};
-    int N = 0, ncell = 0, cpb = 8, msize = 0, grid = 0;
-    bool by_tiles = false;  // exact form: stages by tiles (exact_by_tiles)
+    int N = 0, ncell = 0, msize = 0;
+    int cpb = 8, grid = 0;  // cells per CTA of the form's stages, their CTAs
+    // how exact stages run, in this form or for the adjoint of another: by tiles
+    // or by lines (exact_by_tiles), and their cells per CTA
+    bool by_tiles = false;
+    int ex_cpb = 8;
     size_t nq = 0;  // doubles per state
     cudaStream_t stream = nullptr;
     std::string err;
@@ -116,8 +123,8 @@ struct sddc_ctx {
     int ncase = 0;
     std::vector<sddc_case> cases;
     CaseParams *case_dev = nullptr;
-    int4 *tiles = nullptr;
-    int ntiles = 0;
+    int4 *tiles = nullptr, *tiles_resid = nullptr;  // of the stages, of residual evaluations
+    int ntiles = 0, ntiles_resid = 0;
     bool persistent = false;  // batch stages as grid-stride persistent launches
     // discrete adjoint work space (adjoint.cu), created on first use
     sddc::AdjWs *adj = nullptr;
@@ -149,10 +156,11 @@ SDDC_INTERNAL int check_flags(sddc_ctx *ctx);  // synchronises the stream
 SDDC_INTERNAL unsigned take_flags(sddc_ctx *ctx);  // reads and clears, after a synchronisation
 SDDC_INTERNAL cudaError_t launch_rk_exact(sddc_ctx *ctx, const StageArgs &a, cudaStream_t st);
 SDDC_INTERNAL int met_size(int N);
+inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 // CTAs of a residual evaluation of a single case
 inline int resid_grid(const sddc_ctx *ctx)
 {
-    return (ctx->ncell + line_tile_cells(ctx->N) - 1) / line_tile_cells(ctx->N);
+    return ceil_div(ctx->ncell, line_tile_cells(ctx->N));
 }
 SDDC_INTERNAL StageArgs base_args(sddc_ctx *ctx);
 SDDC_INTERNAL void adjoint_free(sddc_ctx *ctx);

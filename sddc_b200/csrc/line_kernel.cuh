@@ -76,7 +76,7 @@ template <int N, int CPB, typename R, bool EX> __host__ __device__ constexpr siz
 }
 
 // Whether a thread holds its line's states in registers beside the sums.  In
-// double at N = 6 they do not fit (exact form, 121x87 cells: 638 us a step
+// double at N = 6 they do not fit (121x87 cells in exact operations: 638 us a step
 // with spills, 465 read from shared memory), in the exact form not at N = 5 either
 // (300x300 cells 428 us a stage with spills, 402), and at N = 4 there is a second
 // kernel without them (WIDE): 168 registers instead of 240 let a scheduler

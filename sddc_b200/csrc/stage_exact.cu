@@ -9,31 +9,66 @@ namespace sddc {
 
 namespace {
 
-template <int N, int CPB> cudaError_t launch_n(const StageArgs &a, const Ops &ops, cudaStream_t st)
-{
-    auto kern = stage_kernel<N, CPB>;
-    constexpr size_t smem = stage_smem_bytes<N, CPB>();
-    static PerDevice configured;  // per instantiation
-    int set = 0;
-    const cudaError_t e = configured.get(&set, [&](int, int *out) {
-        *out = 1;
-        return set_smem(kern, smem);
-    });
-    if (e != cudaSuccess) return e;
-    kern<<<(a.ncell + CPB - 1) / CPB, stage_threads(N, CPB), smem, st>>>(a, ops);
-    return cudaGetLastError();
-}
+template <int N, int CPB> struct TileLaunch {
+    using Kern = void (*)(const StageArgs, const Ops);
+    static constexpr size_t kSmem = stage_smem_bytes<N, CPB>();
+    static constexpr int kThreads = stage_threads(N, CPB);
+
+    // the kernels of a plain case, of batches and packed metrics, and of a
+    // persistent batch
+    static Kern kernel(int w)
+    {
+        static const Kern kerns[3] = {stage_kernel<N, CPB, false>, stage_kernel<N, CPB, true>,
+                                      stage_kernel_persistent<N, CPB>};
+        return kerns[w];
+    }
+    // CTAs of kernel w resident at once (its attributes are set on the way)
+    static cudaError_t residency(int w, int *out)
+    {
+        static PerDevice resident[3];
+        return resident[w].get(out, [&](int dev, int *n) {
+            cudaError_t e = set_smem(kernel(w), kSmem);
+            int sms = 0, per_sm = 0;
+            if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+            if (e == cudaSuccess)
+                e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel(w), kThreads, kSmem);
+            *n = std::max(1, sms * per_sm);
+            return e;
+        });
+    }
+    static cudaError_t run(const StageArgs &a, const Ops &ops, cudaStream_t st)
+    {
+        const int w = a.tiles && a.persistent ? 2 : a.tiles || !a.nrm ? 1 : 0;
+        int resident = 0;
+        const cudaError_t e = residency(w, &resident);
+        if (e != cudaSuccess) return e;
+        const int tiles = a.tiles ? a.ntiles : (a.ncell + CPB - 1) / CPB;
+        kernel(w)<<<w == 2 ? std::min(tiles, resident) : tiles, kThreads, kSmem, st>>>(a, ops);
+        return cudaGetLastError();
+    }
+};
 
 }  // namespace
 
 cudaError_t launch_tile_exact(int N, int cpb, const StageArgs &a, const Ops &ops, cudaStream_t st)
 {
     switch (N) {
-    case 2: return launch_n<2, 8>(a, ops, st);
-    case 3: return launch_n<3, 4>(a, ops, st);
-    case 4: return launch_n<4, 8>(a, ops, st);
-    case 5: return launch_n<5, 6>(a, ops, st);
-    case 6: return cpb == 6 ? launch_n<6, 6>(a, ops, st) : launch_n<6, 8>(a, ops, st);
+    case 2: return TileLaunch<2, 8>::run(a, ops, st);
+    case 3: return TileLaunch<3, 4>::run(a, ops, st);
+    case 4: return TileLaunch<4, 8>::run(a, ops, st);
+    case 5: return TileLaunch<5, 6>::run(a, ops, st);
+    case 6: return cpb == 6 ? TileLaunch<6, 6>::run(a, ops, st) : TileLaunch<6, 8>::run(a, ops, st);
+    default: return cudaErrorInvalidValue;
+    }
+}
+
+cudaError_t tile_residency_exact(int N, int *resident)
+{
+    switch (N) {
+    case 2: return TileLaunch<2, 8>::residency(0, resident);
+    case 3: return TileLaunch<3, 4>::residency(0, resident);
+    case 4: return TileLaunch<4, 8>::residency(0, resident);
+    case 5: return TileLaunch<5, 6>::residency(1, resident);
     default: return cudaErrorInvalidValue;
     }
 }

@@ -1,6 +1,6 @@
 // What the stage kernels share (their arguments, operators, TMA copies, face
-// traces), and the RK stage of the exact form by tiles, for the meshes on
-// which that is faster (exact_by_tiles).  Every other stage runs in line_kernel
+// traces), and the RK stage of the exact form by tiles, for the meshes and
+// batches on which that is faster (exact_by_tiles).  Every other stage runs in line_kernel
 // (line_kernel.cuh), a residual evaluation in resid_kernel
 // (resid_kernel.cuh), both with a thread per line of solution points.
 //
@@ -55,31 +55,7 @@ __host__ __device__ constexpr int line_tile_cells(int n)
     return n == 2 ? 8 : n == 3 ? 10 : n == 4 ? 8 : n == 5 ? 6 : 2;
 }
 
-// Time steps of the exact form run by tiles where that is the faster of the
-// two: a line's 2N+2 dependent point fluxes, in unfused operations, are a
-// longer chain than the tile's phases, which shows while the mesh leaves SMs
-// idle, and so is a last wave of CTAs by lines that is mostly empty.  spare: the
-// cells that would fill it.  At N = 5 and 6 the line's sums leave no registers
-// for its states, and tiles are the faster at every size.  us per stage, by
-// tiles and by lines: N = 2, 8100 cells 11.5 and 12.1, 32400 37.6 and 32.6; N = 3,
-// 4096 11.9 and 13.5, 8100 22.1 and 17.5, 9409 23.3 and 28.8; N = 4, 8100 23.7 and
-// 28.0, 9409 28 and 27.6, 14400 43.7 and 50.0, 32400 91 and 86; N = 5, 4096 21.8 and
-// 33.2, 90000 401 and 402; N = 6, 4096 33.9 and 38.8, 32400 232 and 247.  (The FP64
-// and mixed forms, and batches, always run by lines.)
-__host__ __device__ constexpr bool exact_by_tiles(int n, int ncell)
-{
-    // cells of a wave by lines: 12 warps per SM, at N = 4 with line_has_wide
-    const int wave = 148 * line_tile_cells(n) * (n == 2 ? 12 : 6);
-    const long spare = (wave - ncell % wave) % wave;
-    switch (n) {
-    case 2: return ncell < 9472;  // (a wave by tiles)
-    case 3: return 2L * ncell < 3 * spare - 6000;
-    case 4:  // (up to 4736 cells, and near 9472, waves of 8 warps per SM serve, at 0.7 of the time)
-        return ncell <= 4736 || (ncell > wave && (ncell < 8800 || ncell > 9472) && ncell < 4 * spare + 6000);
-    default: return true;
-    }
-}
-// Cells per CTA there.  us per stage with 4, 6 and 8: N = 2, 8100 cells 12.0, 16.8,
+// Cells per CTA of the kernel by tiles.  us per stage with 4, 6 and 8: N = 2, 8100 cells 12.0, 16.8,
 // 11.5; N = 3, 4096 11.9, 13.2, 13.2; N = 4, 14400 45.7, 47.3, 43.7; N = 5, 576 11.3,
 // 9.7, 12.8, 14400 80, 71, 92; N = 6, 576 12.6, 11.4, 14.4, 8100 71, 65, 62
 __host__ __device__ constexpr int tile_cells(int n, int ncell)
@@ -394,10 +370,12 @@ template <int N, int CPB> constexpr int stage_min_blocks()
 }
 
 // Compiled without FMA contraction (-fmad=false): the reference's operations
-// in its order.
-template <int N, int CPB>
-__global__ void __launch_bounds__(stage_threads(N, CPB), (stage_min_blocks<N, CPB>()))
-    stage_kernel(const StageArgs a, const Ops ops)
+// in its order.  GEN: also the tiles of a batch, with their cases' data, and
+// metrics from the packed records (a.nrm null: contexts of another form); a
+// kernel of its own, so that a plain case does not carry them.  False if the
+// staging copies did not arrive.
+template <int N, int CPB, bool GEN>
+__device__ __forceinline__ bool stage_tile(const StageArgs &a, const Ops &ops, const int tile)
 {
     using R = double;
     using S = Smem<N>;
@@ -422,40 +400,56 @@ __global__ void __launch_bounds__(stage_threads(N, CPB), (stage_min_blocks<N, CP
     R *sOpL = sV + CPB * S::kV;                                  // [NP][N]
     R *sOpM = sOpL + NP * N;                                     // [NP][N]
 
-    const int tid = threadIdx.x, tile = blockIdx.x;
-    const int c0 = tile * CPB, ncl = min(CPB, a.ncell - c0);  // cells of this CTA
-    double *maxima = a.maxima;
+    const int tid = threadIdx.x;
+    int c0 = tile * CPB, ncl = min(CPB, a.ncell - c0), cs = 0;  // cells of this tile, their case
+    bool first_tile = tile == 0;
+    if (GEN && a.tiles) {
+        const int4 tl = a.tiles[tile];
+        c0 = tl.x;
+        ncl = tl.y;
+        cs = tl.z;
+        first_tile = tl.w != 0;
+    }
+    double *maxima = a.maxima + 10 * cs;
     // a thread has one face point at most (a cell has 4N of them)
     const bool has_fp = tid < ncl * 4 * N;
 
     // ---- stage the state, the metrics and the operators ------------------------
     // The tile's state slice goes to sQ, its normals to sNrm and Jac to sJac
     // and, in a stage that reads one RK register, that register's slice to sA,
-    // by TMA bulk copies that one thread issues when every slice is 16-byte
-    // aligned; otherwise by batches of loads.
+    // by TMA bulk copies that one thread issues.  Where the state slices are no
+    // whole 16-byte units (odd N, an odd first cell or count) they come by
+    // batches of loads.
     __shared__ __align__(8) unsigned long long sBar;
     __shared__ int sAbort;
     const bool want_ra = a.rk_kind == kRkTwoReg || a.rk_kind == kRkTwoRegT;
     const size_t qbytes = (size_t)ncl * NQ * sizeof(double);
-    const size_t nbytes = (size_t)ncl * NM * sizeof(R);
-    const size_t jbytes = (size_t)ncl * NJ * sizeof(double);
+    // normals and Jac from their own arrays, or both from the packed records
+    // (where they lie one behind the other, as they do here per cell)
+    const bool split = !GEN || a.nrm != nullptr;  // uniform
+    static_assert(ML::kJac == NM && ML::kSize == NM + NJ && NM % 2 == 0 && NJ % 2 == 0,
+                  "a record is a cell's normals, then its Jac, both whole 16-byte units");
+    const R *nbase = split ? reinterpret_cast<const R *>(a.nrm) : a.met;
+    const int nstride = split ? NM : ML::kSize;
     const double *qsrc = a.q_in + (size_t)c0 * NQ;
-    const R *nsrc = reinterpret_cast<const R *>(a.nrm) + (size_t)c0 * NM;
-    const double *jsrc = a.jac + (size_t)c0 * NJ;
     const double *rsrc = want_ra ? a.reg_a + (size_t)c0 * NQ : nullptr;
-    const bool bulk = ((uintptr_t)qsrc & 15) == 0 && (qbytes & 15) == 0 &&
-                      (((uintptr_t)nsrc | (uintptr_t)jsrc | nbytes | jbytes) & 15) == 0 &&
-                      (!want_ra || ((uintptr_t)rsrc & 15) == 0);  // uniform in the CTA
+    const bool bulk = (((uintptr_t)qsrc | (uintptr_t)rsrc | qbytes) & 15) == 0;  // uniform in the CTA
     if (tid == 0) {
         sAbort = 0;
-        if (bulk) {
-            mbar_init(&sBar, 1);
-            mbar_expect_tx(&sBar, (unsigned)(qbytes + nbytes + jbytes + (want_ra ? qbytes : 0)));
-            bulk_g2s(sQ, qsrc, (unsigned)qbytes, &sBar);
-            bulk_g2s(sNrm, nsrc, (unsigned)nbytes, &sBar);
-            bulk_g2s(sJac, jsrc, (unsigned)jbytes, &sBar);
-            if (want_ra) bulk_g2s(sA, rsrc, (unsigned)qbytes, &sBar);
+        mbar_init(&sBar, 1);
+        mbar_expect_tx(&sBar, (unsigned)(ncl * (NM + NJ) * sizeof(double) + (bulk ? qbytes * (want_ra ? 2 : 1) : 0)));
+        if (bulk) bulk_g2s(sQ, qsrc, (unsigned)qbytes, &sBar);
+        if (split) {
+            bulk_g2s(sNrm, nbase + (size_t)c0 * NM, (unsigned)(ncl * NM * sizeof(R)), &sBar);
+            bulk_g2s(sJac, a.jac + (size_t)c0 * NJ, (unsigned)(ncl * NJ * sizeof(double)), &sBar);
+        } else {
+            for (int c = 0; c < ncl; c++) {
+                const double *rec = a.met + (size_t)(c0 + c) * ML::kSize;
+                bulk_g2s(sNrm + c * NM, rec, NM * sizeof(R), &sBar);
+                bulk_g2s(sJac + c * NJ, rec + ML::kJac, NJ * sizeof(double), &sBar);
+            }
         }
+        if (bulk && want_ra) bulk_g2s(sA, rsrc, (unsigned)qbytes, &sBar);
     }
     for (int k = tid; k < NP * N; k += NT) {
         sOpL[k] = opL<R>(ops, k);
@@ -464,26 +458,25 @@ __global__ void __launch_bounds__(stage_threads(N, CPB), (stage_min_blocks<N, CP
     if (!bulk) {
         // batches of kU independent loads per thread before their stores, so
         // that each thread keeps several loads in flight
-        auto stage_copy = [&](auto *dst, const auto *src, int n) {
-            constexpr int kU = 4;
+        auto stage_copy = [&](double *dst, const double *src) {
+            constexpr int kU = 8;
+            const int n = ncl * NQ;
             for (int k0 = tid; k0 < n; k0 += kU * NT) {
-                decltype(+src[0]) v[kU];
+                double v[kU];
 #pragma unroll
-                for (int u = 0; u < kU; u++) v[u] = k0 + u * NT < n ? __ldg(src + k0 + u * NT) : decltype(+src[0])(0);
+                for (int u = 0; u < kU; u++) v[u] = k0 + u * NT < n ? __ldg(src + k0 + u * NT) : 0.0;
 #pragma unroll
                 for (int u = 0; u < kU; u++)
                     if (k0 + u * NT < n) dst[k0 + u * NT] = v[u];
             }
         };
-        stage_copy(sQ, qsrc, ncl * NQ);
-        stage_copy(sNrm, nsrc, ncl * NM);
-        stage_copy(sJac, jsrc, ncl * NJ);
-        if (want_ra) stage_copy(sA, rsrc, ncl * NQ);
+        stage_copy(sQ, qsrc);
+        if (want_ra) stage_copy(sA, rsrc);
     }
     const double eig_r = maxima[2 * a.slot_r], um_r = maxima[2 * a.slot_r + 1];
     // compflux.f90:6 -- running maxima of all previous stages
     const R c_h = (R)sqrt(eig_r * (eig_r - um_r));
-    if (bulk && tid == 0 && !mbar_wait_bounded(&sBar, 0)) {
+    if (tid == 0 && !mbar_wait_bounded(&sBar, 0)) {
         // the copies did not complete: flag it, give them time to land in
         // this CTA's shared memory, and leave (every thread, below)
         raise_fault(a.err_flags, kErrStagingTimeout);
@@ -491,7 +484,7 @@ __global__ void __launch_bounds__(stage_threads(N, CPB), (stage_min_blocks<N, CP
         mbar_wait_bounded(&sBar, 0);
     }
     __syncthreads();
-    if (sAbort) return;
+    if (sAbort) return false;
     // ---- A: interpolate every line to its flux points ---------------------------
     // one thread per (cell, line index l, variable): xi-line l and eta-line l
     // together, their sums paired (both use the same operator row)
@@ -574,7 +567,7 @@ __global__ void __launch_bounds__(stage_threads(N, CPB), (stage_min_blocks<N, CP
             face_point<N>(plf, N - nfp + 1, pfam, pline, pr);
             if (own_right) {
                 // the left (partner) cell's normal
-                const R *pn = reinterpret_cast<const R *>(a.nrm) + (size_t)pc * NM + ML::normal(pfam, pline, pr);
+                const R *pn = nbase + (size_t)pc * nstride + ML::normal(pfam, pline, pr);
                 n0 = __ldg(pn);
                 n1 = __ldg(pn + 1);
                 sign_l = pr == 0 ? -1 : 1;
@@ -583,7 +576,7 @@ __global__ void __launch_bounds__(stage_threads(N, CPB), (stage_min_blocks<N, CP
                 sign_r = pr == N ? -1 : 1;
             }
         } else {
-            bc_ghost<R, true>(kind, own, n0, n1, a.vismode, a.fs, other);
+            bc_ghost<R, true>(kind, own, n0, n1, a.vismode, GEN && a.cases ? a.cases[cs].fs : a.fs, other);
         }
         // left and right states by element-wise selects (arrays picked
         // through a pointer would live in local memory)
@@ -635,7 +628,7 @@ __global__ void __launch_bounds__(stage_threads(N, CPB), (stage_min_blocks<N, CP
     // ---- C: B gradient, sources and the residual per solution point ------------
     // the RK coefficients of the stage, formed where used from the kernel
     // parameters (not held in registers through the phase)
-    const double cdt = a.dt;
+    const double cdt = GEN && a.cases ? a.cases[cs].dt : a.dt;
     auto cf = [&](int i) -> double { return ((a.dt_mask >> i) & 1u) ? a.cb[i] * cdt : a.cb[i]; };
     double part_r = 0.0, part_d = 0.0;
     for (int t = tid; t < ncl * NN; t += NT) {
@@ -802,7 +795,7 @@ __global__ void __launch_bounds__(stage_threads(N, CPB), (stage_min_blocks<N, CP
             }
             atomic_max_nonneg(&maxima[2 * a.slot_w], m0);
             atomic_max_nonneg(&maxima[2 * a.slot_w + 1], m1);
-            if (tile == 0) {  // carry the previous stages' maxima forward
+            if (first_tile) {  // carry the previous stages' maxima forward
                 // (re-read: slot_r is not written during the stage)
                 atomic_max_nonneg(&maxima[2 * a.slot_w], maxima[2 * a.slot_r]);
                 atomic_max_nonneg(&maxima[2 * a.slot_w + 1], maxima[2 * a.slot_r + 1]);
@@ -818,8 +811,29 @@ __global__ void __launch_bounds__(stage_threads(N, CPB), (stage_min_blocks<N, CP
             // the bulk store must have read sA before the CTA's shared memory
             // goes or the next tile reuses it; the staging barrier is free
             if (out_bulk) bulk_wait_read();
-            if (bulk) mbar_inval(&sBar);
+            mbar_inval(&sBar);
         }
+    }
+    return true;
+}
+
+template <int N, int CPB, bool GEN>
+__global__ void __launch_bounds__(stage_threads(N, CPB), (stage_min_blocks<N, CPB>()))
+    stage_kernel(const StageArgs a, const Ops ops)
+{
+    stage_tile<N, CPB, GEN>(a, ops, blockIdx.x);
+}
+
+// a batch's stage as a persistent launch: each CTA walks the tile table with a
+// grid stride
+template <int N, int CPB>
+__global__ void __launch_bounds__(stage_threads(N, CPB), (stage_min_blocks<N, CPB>()))
+    stage_kernel_persistent(const StageArgs a, const Ops ops)
+{
+    for (int t = blockIdx.x; t < a.ntiles; t += gridDim.x) {
+        if (!stage_tile<N, CPB, true>(a, ops, t)) return;
+        fence_proxy_async();  // what this thread wrote, before the next tile's copies
+        __syncthreads();      // tile t's last shared-memory reads before tile t + grid stages
     }
 }
 

@@ -116,3 +116,71 @@ def test_steps_of_long_and_short_calls_are_the_same(form):
         s.close()
     for q, mx in out[1:]:
         assert np.array_equal(q, out[0][0]) and mx == out[0][1]
+
+
+@pytest.mark.parametrize("persistent", [False, True])
+@pytest.mark.parametrize("form", ["fp64_exact", "fp64", "mixed"])
+@pytest.mark.parametrize("N,sizes", [(2, [(11, 9), (7, 3), (31, 33)]), (3, [(11, 9), (5, 7), (23, 21)]),
+                                     (4, [(9, 9), (3, 5), (13, 11)]), (5, [(7, 9), (5, 5), (17, 13)]),
+                                     (6, [(7, 5), (3, 3), (9, 11)])])
+def test_batch_of_odd_cases_equals_separate_runs(N, sizes, form, persistent):
+    """Cases of odd cell counts, so that tiles begin at odd cells: their state
+    slices are no whole 16-byte units at odd N.  States, maxima and the
+    residual, bit for bit those of each case in its own context."""
+    cl = [cases.cylinder_case(a, b, N, ms=0.2 + 0.03 * k, ma=2.0, seed=k, noise=1e-4) for k, (a, b) in enumerate(sizes)]
+    members = ensemble.build_members(cl)
+    b = ensemble.Batch(members, precision=form, persistent=persistent)
+    b.reset()
+    b.step(2)
+    b.solver.compresid()
+    g = b.solver.state(resid=True)
+    for k, m in enumerate(members):
+        s = Solver(m.tables, m.case.physics, precision=form)
+        s.set_state(m.Q0)
+        s.rk_s5p3(m.dt, 2)
+        s.compresid()
+        w, mx = s.state(resid=True), s.maxima()
+        s.close()
+        assert np.array_equal(b.member_state(g["Q"], k), w["Q"]), k
+        assert np.array_equal(b.member_state(g["resid"], k), w["resid"]), k
+        assert b.solver.case_maxima(k) == (mx["eigvmax"], mx["umax"]), k
+    b.close()
+
+
+@pytest.mark.parametrize("persistent", [False, True])
+@pytest.mark.parametrize("form", ["fp64_exact", "fp64"])
+@pytest.mark.parametrize("N,count,a,b", [(3, 5, 45, 45), (5, 5, 35, 33), (5, 9, 45, 45), (6, 3, 33, 31)])
+def test_batch_over_several_waves_equals_separate_runs(N, count, a, b, form, persistent):
+    """More tiles than are resident at once, from odd cells on: the exact form
+    by tiles and (N = 3; N = 5 in the larger batch) by lines."""
+    members = ensemble.build_members([cases.cylinder_case(a, b, N, ms=0.25, ma=2.0, seed=1, noise=1e-4)] * count)
+    one = members[0]
+    bt = ensemble.Batch(members, precision=form, persistent=persistent)
+    bt.reset()
+    bt.step(2)
+    g = bt.solver.state()["Q"]
+    s = Solver(one.tables, one.case.physics, precision=form)
+    s.set_state(one.Q0)
+    s.rk_s5p3(one.dt, 2)
+    w = s.state()["Q"]
+    s.close()
+    for k in range(count):
+        assert np.array_equal(bt.member_state(g, k), w), k
+    bt.close()
+
+
+@pytest.mark.parametrize("N", [2, 3, 4, 5, 6])
+def test_adjoint_of_every_form_is_the_exact_one(N):
+    """The adjoint runs the exact form's stages whatever the context's form:
+    by the same kernels, from metrics in another layout."""
+    m, t, ph, Q = case_cylinder(9, 16, N)
+    dt = 0.1 * cases.cfl_dt(m, Q, N)
+    out = []
+    for form in ("fp64_exact", "fp64", "mixed"):
+        s = Solver(t, ph, precision=form)
+        s.set_state(Q)
+        r = s.adjoint_run(dt, 6, 2, 6, checkpoint_every=3)
+        out.append((r["J"], r["Qbar0"], r["parbar"], s.state()["Q"].copy()))
+        s.close()
+    for r in out[1:]:
+        assert r[0] == out[0][0] and all(np.array_equal(x, y) for x, y in zip(r[1:], out[0][1:]))

@@ -237,7 +237,7 @@ def test_calls_after_a_failed_allocation(runtime):
             assert k > 1, k
         # a batch: the one that was set, or none, stays in force
         for before in (0, 3):
-            for k in range(4):
+            for k in range(5):
                 s = Solver(t, ph, precision="fp64")
                 if before:
                     s.set_cases(records(before))
@@ -250,7 +250,7 @@ def test_calls_after_a_failed_allocation(runtime):
                 s.monitor()
                 s.state(sm_ind=True)
                 if before:
-                    assert fails(lambda: s.set_persistent(True), 0)
+                    assert fails(lambda: s.set_persistent(True), k % 2)
                     n = launches("persistent")
                     step()
                     assert launches("persistent") == n
