@@ -725,6 +725,7 @@ static cudaError_t enqueue_step(sddc_ctx *ctx, double dt, int s0, int *xrc = nul
         st[4] = {kRkFive, 4, 0, 0, 2, 3, 5, -1, {F56, F51, F52, F53, F54, F55}, 1u | 32u};
     }
     a.artiv = 0;  // the sensor is evaluated on request (sensor_stale)
+    a.kinds = ctx->p.k_stage == 3 ? 2 : 4;
     ctx->last_in = st[4].in;
     for (int k = 0; k < 5; k++) {
         a.rk_kind = st[k].kind;

@@ -129,6 +129,7 @@ struct StageArgs {
     // is set, else cb[i] (the products round as the host's would)
     double cb[8];
     unsigned dt_mask;
+    int kinds;                         // how many different RkKinds a step's stages have
     double dt;                         // single case
     Freestream fs;                     // single case
     // batch: one tile per CTA (first cell, cells, case, 1 if the case's

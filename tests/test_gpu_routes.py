@@ -184,3 +184,29 @@ def test_adjoint_of_every_form_is_the_exact_one(N):
         s.close()
     for r in out[1:]:
         assert r[0] == out[0][0] and all(np.array_equal(x, y) for x, y in zip(r[1:], out[0][1:]))
+
+
+@pytest.mark.parametrize("N,nx,ny", [(2, 5, 3), (3, 33, 31), (4, 76, 75), (5, 9, 7), (5, 101, 69), (6, 41, 37)])
+def test_five_stage_scheme_matches_oracle(N, nx, ny):
+    """FiveStageRk on meshes of one wave (one kernel for all its stages) and of
+    several (a kernel for each kind; at N = 4 in double without held states)."""
+    m, t, ph, Q = case_channel(nx, ny, N)
+    dt = 0.1 * m.min_edge() / N
+    o = O.Oracle(t, ph)
+    o.set_state(Q)
+    o.five_stage_rk(dt, 2)
+    ref = o.state()["Q"]
+    for form, bar in (("fp64_exact", 0.0), ("fp64", 1e-12), ("mixed", 1e-6)):
+        s = Solver(t, ph, precision=form, k_stage=5)
+        s.set_state(Q)
+        s.rk_s5p3(dt, 2)
+        g = s.state()["Q"]
+        s.close()
+        assert np.array_equal(g, ref) if not bar else rel_l2(g, ref) <= bar, form
+    s = Solver(t, ph, precision="fp64", k_stage=5)  # one case as a persistent batch
+    s.set_cases(_records(t.ncell, 1, ph, dt))
+    s.set_persistent(True)
+    s.set_state(Q)
+    s.step_cases(2)
+    assert rel_l2(s.state()["Q"], ref) <= 1e-12
+    s.close()
