@@ -28,11 +28,11 @@
 // which are zero.  Every sum keeps the reference's order; the exact
 // instantiation is compiled without FMA.
 //
-// What bounds them: latency at 1.4 to 1.8 warps per scheduler (232 and 224
+// What bounds them: latency at 1.4 to 1.8 warps per scheduler (up to 255
 // registers at N = 4 hold the sums of 18 and 7 values per point of the line;
 // the states and gradients are read from shared memory at every flux point,
 // which keeps the L1 pipe 59% and 49% busy).  At 128x128 cells, N = 4, FP64,
-// they take 38 and 58 us cold; one thread per point and variable, with every
+// they take 37 and 52 us cold; one thread per point and variable, with every
 // operand from shared memory and an IEEE division per quotient, took about
 // 215 together (a step of the chain: 1253 us then, 725 now).
 #pragma once
@@ -165,7 +165,8 @@ template <int N, int CPB, typename T> struct ViscSmem {
     static_assert(NX * NN <= GTS, "the exchanged sums fit the gradient traces' region");
 };
 // cells per CTA: the stage's (at N = 4, 8 cells leave 6 warps per SM and 4
-// cells 7, but with twice the bank conflicts: 38 and 41 us, 58 and 60)
+// cells 7, but with twice the bank conflicts: 38 and 41 us, 58 and 60 with the
+// ends peeled)
 __host__ __device__ constexpr int visc_cells(int n) { return line_tile_cells(n); }
 template <int N, int CPB, size_t SMEM> constexpr int visc_min_blocks()
 {
@@ -337,10 +338,32 @@ template <int N, int CPB, typename T> struct ViscTile {
     __device__ __forceinline__ int parity() const { return (l ^ fam) & 1; }
 };
 
+// f(r) at every flux point of the line.  ROLLED: one body for the ends and the
+// points between them.  The chain's three kernels with the ends peeled do not fit
+// the instruction cache together, and each launch fetches its own again: us per
+// stage of the chain, peeled and rolled, exact, 8100 cells, N = 4 103 and 83, N = 5
+// 168 and 152; FP64, 14400 cells, N = 4 127 and 121.  Where the sums fit the
+// registers of three warps anyway (N = 2 and 3 outside the exact form) that
+// shows on meshes of one wave only (64 cells, N = 3 24 and 22; 8100 cells 46 and 47),
+// and at N = 6 the peeled ends give more than they cost (FP64, 14400 cells 315 and
+// 331).
+template <int N, bool ROLLED, typename F> __device__ __forceinline__ void along_line(F f)
+{
+    if constexpr (!ROLLED) {
+        f(0);
+#pragma unroll 1
+        for (int r = 1; r < N; r++) f(r);
+        f(N);
+    } else {
+#pragma unroll 1
+        for (int r = 0; r <= N; r++) f(r);
+    }
+}
+
 // ---- gradients at the solution points and their face traces ------------------------
 // T: the trace type of the form (EX and T keep the instantiations of the
 // translation units apart)
-template <int N, bool EX, typename T, int CPB>
+template <int N, bool EX, typename T, int CPB, bool ROLLED>
 __global__ void __launch_bounds__(line_threads(N, CPB), (visc_min_blocks<N, CPB, ViscSmem<N, CPB, T>::kGradBytes>()))
     visc_grad_kernel(const ViscArgs a, const Ops ops)
 {
@@ -376,10 +399,7 @@ __global__ void __launch_bounds__(line_threads(N, CPB), (visc_min_blocks<N, CPB,
                 }
             }
         };
-        add(0);
-#pragma unroll 1
-        for (int r = 1; r < N; r++) add(r);
-        add(N);
+        along_line<N, ROLLED>(add);
     }
     const int par = t.parity();
     if (t.act) {
@@ -460,7 +480,7 @@ __global__ void __launch_bounds__(line_threads(N, CPB), (visc_min_blocks<N, CPB,
 }
 
 // ---- the viscous flux and its divergence ---------------------------------------------
-template <int N, bool EX, typename T, int CPB>
+template <int N, bool EX, typename T, int CPB, bool ROLLED>
 __global__ void __launch_bounds__(line_threads(N, CPB), (visc_min_blocks<N, CPB, ViscSmem<N, CPB, T>::kFluxBytes>()))
     visc_flux_kernel(const ViscArgs a, const Ops ops)
 {
@@ -583,10 +603,7 @@ __global__ void __launch_bounds__(line_threads(N, CPB), (visc_min_blocks<N, CPB,
                 for (int k = 0; k < NX; k++) d[i][k] = d[i][k] + o[k] * M;
             }
         };
-        add(0);
-#pragma unroll 1
-        for (int r = 1; r < N; r++) add(r);
-        add(N);
+        along_line<N, ROLLED>(add);
     }
     __syncthreads();  // the gradient traces and the states are read
     const int par = t.parity();

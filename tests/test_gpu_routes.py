@@ -210,3 +210,25 @@ def test_five_stage_scheme_matches_oracle(N, nx, ny):
     s.step_cases(2)
     assert rel_l2(s.state()["Q"], ref) <= 1e-12
     s.close()
+
+
+@pytest.mark.parametrize("N,nx,ny", [(2, 9, 7), (2, 141, 139), (3, 9, 7), (3, 97, 95), (5, 61, 59)])
+def test_viscous_chain_matches_oracle_on_one_and_several_waves(N, nx, ny):
+    """Below and above the CTAs resident at once: launches in order or begun
+    early, and at N = 2 and 3 outside the exact form two kernels each."""
+    import dataclasses
+
+    m, t, ph, Q = case_channel(nx, ny, N, sides=("WALL", "OUTL", "SYMP", "INLE"))
+    ph = dataclasses.replace(ph, mu=0.02, eta0=0.015)
+    dt = min(0.02 * m.min_edge() / N, 0.02 * (m.min_edge() / N) ** 2 / ph.mu)
+    o = O.Oracle(t, ph)
+    o.set_state(Q)
+    o.rk_s5p3(dt, 1)
+    ref = o.state()["Q"]
+    for form, bar in (("fp64_exact", 0.0), ("fp64", 1e-12), ("mixed", 1e-6)):
+        s = Solver(t, ph, precision=form)
+        s.set_state(Q)
+        s.rk_s5p3(dt, 1)
+        g = s.state()["Q"]
+        s.close()
+        assert np.array_equal(g, ref) if not bar else rel_l2(g, ref) <= bar, form
