@@ -492,7 +492,6 @@ extern "C" int sddc_adjoint_run(sddc_ctx *ctx, const sddc_adjoint_opts *o, doubl
     std::vector<double *> S2(overlap ? 5 * segmax + 1 : 0), T2(overlap ? 5 * segmax + 1 : 0);
     double *cmax2 = nullptr;
     if (overlap) {
-        rb.name(&fin, nq);  // the final state: the sweep overwrites the stores
         for (int i = 0; i <= 5 * segmax; i++) {
             rb.name(&S2[i], nq);
             rb.name(&T2[i], tr);
@@ -551,10 +550,8 @@ extern "C" int sddc_adjoint_run(sddc_ctx *ctx, const sddc_adjoint_opts *o, doubl
     CKA(cudaEventRecord(ev[1], ctx->stream));
     {
         double *last = S[5 * (ns - (nseg - 1) * K)];
-        if (overlap)
-            CKA(cudaMemcpyAsync(fin, last, nq * sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream));
-        else
-            fin = last;
+        fin = overlap ? ctx->reg[1] : last;  // the sweep overwrites the stores; no stage of the run uses the register
+        if (overlap) CKA(cudaMemcpyAsync(fin, last, nq * sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream));
     }
     std::vector<double> H(2 * ((size_t)5 * ns + 1)), Fh(2 * ((size_t)ns + 1));
     CKA(cudaMemcpyAsync(H.data(), hist, H.size() * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));

@@ -289,3 +289,24 @@ def test_graphs_are_captured_where_their_steps_pay(runtime):
         assert graphs([(4e-3, 41)]) == (1, 5)
         clean()
         """)
+
+
+def test_device_memory_of_an_adjoint_run(runtime):
+    """What include/sddc.h says a run holds, and no state more: the checkpoints,
+    two stores of stage states and traces, six adjoint registers."""
+    _run(runtime, """
+        m, t, ph, Q = case_cylinder(8, 16, 4)
+        s = Solver(t, ph, precision="fp64_exact")
+        s.set_state(Q)
+        s.vjp_resid(Q)  # the work space is there
+        state, traces, tiles = Q.size * 8, t.ncell * 4 * 36 * 8, t.ncell // 8
+        for steps, every, stores in ((4, 4, 1), (4, 2, 2), (6, 2, 2)):
+            live = F.fake_live()
+            F.fake_reset_peak()
+            s.adjoint_run(1e-3, steps, 1, steps, checkpoint_every=every)
+            run = F.fake_peak() - live
+            assert F.fake_live() == live
+            want = (steps // every + 6) * state + stores * ((5 * every + 1) * (state + traces) + 5 * every * 2 * tiles * 8)
+            assert want <= run < want + state // 2, (steps, every, run, want)
+        clean()
+        """)
