@@ -48,7 +48,27 @@ template <int n, typename R> SDDC_HD void quotients(const R *a, R b, R *q)
 #pragma unroll
     for (int i = 0; i < n; i++) q[i] = a[i] / b;
 }
+// the first n by b, the next h by b / 2
+template <int n, int h, typename R> SDDC_HD void quotients_by_half(const R *a, R b, R *q)
+{
+#pragma unroll
+    for (int i = 0; i < n + h; i++) q[i] = i < n ? a[i] / b : a[i] / ((R)0.5 * b);
+}
 #ifdef __CUDA_ARCH__
+template <int n, int h> __device__ __forceinline__ void quotients_by_half(const double *a, double b, double *q)
+{
+    bool ok = mid_range(__double2hiint(b));
+#pragma unroll
+    for (int i = 0; i < n + h; i++) ok = ok && (mid_range(__double2hiint(a[i])) || a[i] == 0.0);
+    if (ok) {  // (far from the format's ends doubling a quotient is exact)
+        const double y = __drcp_rn(b);
+#pragma unroll
+        for (int i = 0; i < n + h; i++) q[i] = (i < n ? 1.0 : 2.0) * quotient_from(a[i], b, y);
+    } else {
+#pragma unroll
+        for (int i = 0; i < n + h; i++) q[i] = i < n ? a[i] / b : a[i] / (0.5 * b);
+    }
+}
 template <int n> __device__ __forceinline__ void quotients(const double *a, double b, double *q)
 {
     bool ok = mid_range(__double2hiint(b));
@@ -236,11 +256,9 @@ SDDC_HD void rusanov(const R *Qfl, const R *Qfr, R *Fnl, R *Fnr, R n0, R n1, int
     const R bn = Bx * unit_x + By * unit_y;
     R c_a, c_d, c_n;
     if constexpr (EX) {
-        const R rs = Qfl[0] + Qfr[0];
-        // by rs, and twice by rs / 2: doubling the numerators instead is exact
-        const R num[3] = {(R)kGam * (pgl + pgr), (R)2 * ((Bx * Bx + By * By) + Bz * Bz), (R)2 * (bn * bn)};
+        const R num[3] = {(R)kGam * (pgl + pgr), (Bx * Bx + By * By) + Bz * Bz, bn * bn};
         R c[3];
-        quotients<3>(num, rs, c);
+        quotients_by_half<1, 2>(num, Qfl[0] + Qfr[0], c);
         c_a = c[0];
         c_d = c[1];
         c_n = c[2];
