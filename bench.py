@@ -471,16 +471,7 @@ def ensemble_run(torch, gpu_index=None, ncase=64, steps=1000, warmup=3, seed=0):
         e1.synchronize()
         return e0.elapsed_time(e1) / 1e3
 
-    # tile for the batch (untimed tuning on the batch itself)
-    best, best_t = 4, None
-    for cpb in autotune.CANDIDATES:
-        b = ensemble.Batch(members, precision="mixed", cells_per_cta=cpb)
-        b.reset()
-        b.step(2)
-        tt = timed(lambda: b.step(3), b.solver.stream_handle())
-        if best_t is None or tt < best_t:
-            best, best_t = cpb, tt
-        b.close()
+    best = autotune.CANDIDATES[0]  # no launch depends on it
     launches = {}
     clocks = {}
     for mode in ("per_tile", "persistent"):
