@@ -418,17 +418,20 @@ extern "C" int sddc_vjp_resid(sddc_ctx *ctx, const double *Rbar, double *Qbar, d
     CKA(cudaMemcpyAsync(w->host, ctx->maxima + 2 * ctx->slot, 2 * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
     CKA(cudaEventRecord(w->maxima, ctx->stream));
     // the state's traces in the exact form's rounding, from the state as it is
-    // now: a caller may have written it through sddc_state_device_ptr.  Ahead
-    // of Rbar's copy, whose first bytes the host stages meanwhile.
-    CKA(launch_trace_exact(ctx->N, ctx->ncell, ctx->reg[0], w->tq, trace_stride(ctx->N, 8), TraceInit{ctx->err_flags}, ctx->ops,
-                           ctx->stream));
+    // now.  An exact context keeps them beside the state, which holds as long as
+    // no caller was given the state's address to write to.  Ahead of Rbar's
+    // copy, whose first bytes the host stages meanwhile.
+    const bool kept = ctx->p.precision == SDDC_FP64_EXACT && !ctx->state_shared;
+    if (!kept)
+        CKA(launch_trace_exact(ctx->N, ctx->ncell, ctx->reg[0], w->tq, trace_stride(ctx->N, 8),
+                               TraceInit{ctx->err_flags}, ctx->ops, ctx->stream));
     CKA(cudaMemcpyAsync(w->lam, Rbar, ctx->nq * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
     CKA(cudaMemsetAsync(w->acc, 0, sizeof(AdjScalars), ctx->stream));
     CKA(cudaEventSynchronize(w->maxima));
     w->at_ready = false;
     RevStage s;
     s.q = ctx->reg[0];
-    s.t = w->tq;
+    s.t = kept ? static_cast<const double *>(ctx->trace[0]) : w->tq;
     s.xbar = w->lam;
     s.scale = 1.0;
     s.out = w->qbar;

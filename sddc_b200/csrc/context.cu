@@ -950,6 +950,7 @@ extern "C" int sddc_get_maxima(sddc_ctx *ctx, double *eigvmax, double *umax, dou
 extern "C" int sddc_state_device_ptr(sddc_ctx *ctx, double **q_dev)
 {
     if (!ctx || !q_dev) return SDDC_EINVAL;
+    ctx->state_shared = true;
     *q_dev = ctx->reg[0];
     return SDDC_OK;
 }

@@ -111,6 +111,7 @@ struct sddc_ctx {
     int mon_nblk = 0;  // CTAs of the last launch that wrote monitor partials
     bool tables = false, state = false;
     bool traces_stale = true;  // trace[0] does not match reg[0] yet
+    bool state_shared = false;  // a caller has the address of reg[0] and may write there
     double ctime = 0.0;
     struct StepGraph {
         cudaGraphExec_t exec = nullptr;
