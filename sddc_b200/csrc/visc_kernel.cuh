@@ -170,8 +170,10 @@ template <int N, int CPB, typename T> struct ViscSmem {
 __host__ __device__ constexpr int visc_cells(int n) { return line_tile_cells(n); }
 template <int N, int CPB, size_t SMEM> constexpr int visc_min_blocks()
 {
-    // 8 warps of 255 registers per SM, more where fewer registers hold a line
-    const int w = (N >= 4 ? 8 : N == 3 ? 12 : 16) / (line_threads(N, CPB) / 32), m = (int)(228 * 1024 / (SMEM + 1280));
+    // 8 warps of 255 registers per SM, 12 of 168 where those hold a line (at N = 2
+    // 16 of 128 left 92 bytes of spills: us per stage of the chain, exact, 64 cells
+    // 20.8 and 20.3 so, 14400 cells 50.3 and 49.1)
+    const int w = (N >= 4 ? 8 : 12) / (line_threads(N, CPB) / 32), m = (int)(228 * 1024 / (SMEM + 1280));
     const int b = w < m ? w : m;
     return b < 1 ? 1 : b;
 }
