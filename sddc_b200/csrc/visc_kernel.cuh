@@ -34,7 +34,7 @@
 // which keeps the L1 pipe 59% and 49% busy).  At 128x128 cells, N = 4, FP64,
 // they take 37 and 52 us cold; one thread per point and variable, with every
 // operand from shared memory and an IEEE division per quotient, took about
-// 215 together (a step of the chain: 1253 us then, 725 now).
+// 215 together (a step of the chain: 1253 us then, 678 now).
 #pragma once
 
 #include "line_kernel.cuh"
