@@ -252,7 +252,7 @@ int sddc_set_persistent(sddc_ctx *ctx, int on);
    is rejected with SDDC_EINVAL.  All calls share the array: calls that
    overlap on the GPU (several host threads, several streams) race; the
    array keeps the last call's contents and each call rewrites what it
-   reads.  The first call on a device looks up the array's device address
+   reads (fault flags are cleared by the call that set them).  The first call on a device looks up the array's device address
    (cudaGetSymbolAddress); make it before any stream capture on that device. */
 #define SDDC_NOALLOC_SCRATCH_BYTES ((size_t)16 << 20)
 

@@ -159,6 +159,10 @@ cudaError_t wall_force(sddc_ctx *ctx, const double *t, double *out)
 
 int make_ws(sddc_ctx *ctx)
 {
+    if (ctx->p.precision != SDDC_FP64_EXACT) {
+        const int rc = plan_exact(ctx);
+        if (rc) return rc;
+    }
     auto *w = new AdjWs();
     ctx->adj = w;
     const size_t nc = ctx->ncell, N = ctx->N;

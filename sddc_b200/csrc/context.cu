@@ -237,6 +237,17 @@ static cudaError_t exact_by_tiles(int N, bool general, bool persistent, int tile
     return cudaSuccess;
 }
 
+// how the exact stages of a single case run (of a context of another form: when
+// its adjoint needs them, so that only then their kernels are loaded)
+int sddc::plan_exact(sddc_ctx *ctx)
+{
+    const int cpb = tile_cells(ctx->N, ctx->ncell);
+    CK(exact_by_tiles(ctx->N, ctx->p.precision != SDDC_FP64_EXACT, false, ceil_div(ctx->ncell, cpb), resid_grid(ctx),
+                      &ctx->by_tiles));
+    ctx->ex_cpb = ctx->by_tiles ? cpb : line_tile_cells(ctx->N);
+    return SDDC_OK;
+}
+
 extern "C" int sddc_create(sddc_ctx **out, const sddc_params *p)
 {
     if (!out || !p) return SDDC_EINVAL;
@@ -263,11 +274,12 @@ extern "C" int sddc_create(sddc_ctx **out, const sddc_params *p)
     ctx->msize = met_size(p->N);
     ctx->nq = (size_t)9 * p->N * p->N * p->ncell;
     *out = ctx;
-    const int exact_cpb = tile_cells(p->N, p->ncell);
-    CK(exact_by_tiles(p->N, p->precision != SDDC_FP64_EXACT, false, ceil_div(p->ncell, exact_cpb), resid_grid(ctx),
-                      &ctx->by_tiles));
-    ctx->ex_cpb = ctx->by_tiles ? exact_cpb : line_tile_cells(p->N);
-    ctx->cpb = p->precision == SDDC_FP64_EXACT ? ctx->ex_cpb : line_tile_cells(p->N);
+    ctx->cpb = line_tile_cells(p->N);
+    if (p->precision == SDDC_FP64_EXACT) {
+        const int rc = plan_exact(ctx);
+        if (rc) return rc;
+        ctx->cpb = ctx->ex_cpb;
+    }
     ctx->grid = ceil_div(p->ncell, ctx->cpb);
     CK(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
     const int nreg = p->k_stage == 5 ? 6 : 4;
@@ -1009,14 +1021,14 @@ static int build_tiles(sddc_ctx *ctx, const std::vector<sddc_case> &cases, int c
 // tables of the stages and of residual evaluations
 struct BatchPlan {
     bool by_tiles = false;
-    int cpb = 0, ex_cpb = 0, ntiles = 0, ntiles_resid = 0, most = 0;  // most: monitor partials of any plan
+    int cpb = 0, ntiles = 0, ntiles_resid = 0, most = 0;  // most: monitor partials of any plan
     Held tiles, tiles_resid;
     int make(sddc_ctx *ctx, const std::vector<sddc_case> &cases, bool persistent)
     {
         const int N = ctx->N, lines = line_tile_cells(N), exact = tile_cells(N, ctx->ncell);
-        CK(exact_by_tiles(N, true, persistent, tile_count(cases, exact), tile_count(cases, lines), &by_tiles));
-        ex_cpb = by_tiles ? exact : lines;
-        cpb = ctx->p.precision == SDDC_FP64_EXACT ? ex_cpb : lines;
+        if (ctx->p.precision == SDDC_FP64_EXACT)
+            CK(exact_by_tiles(N, true, persistent, tile_count(cases, exact), tile_count(cases, lines), &by_tiles));
+        cpb = by_tiles ? exact : lines;
         most = std::max(tile_count(cases, exact), tile_count(cases, lines));
         int rc = build_tiles(ctx, cases, cpb, persistent, &tiles, &ntiles);
         if (!rc) rc = build_tiles(ctx, cases, lines, persistent, &tiles_resid, &ntiles_resid);
@@ -1025,8 +1037,7 @@ struct BatchPlan {
     void give(sddc_ctx *ctx)
     {
         ctx->by_tiles = by_tiles;
-        ctx->cpb = cpb;
-        ctx->ex_cpb = ex_cpb;
+        ctx->cpb = ctx->ex_cpb = cpb;
         ctx->ntiles = ntiles;
         ctx->ntiles_resid = ntiles_resid;
         tiles.give(ctx->tiles);

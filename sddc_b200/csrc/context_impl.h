@@ -157,6 +157,7 @@ SDDC_INTERNAL int check_flags(sddc_ctx *ctx);  // synchronises the stream
 SDDC_INTERNAL unsigned take_flags(sddc_ctx *ctx);  // reads and clears, after a synchronisation
 SDDC_INTERNAL cudaError_t launch_rk_exact(sddc_ctx *ctx, const StageArgs &a, cudaStream_t st);
 SDDC_INTERNAL int met_size(int N);
+SDDC_INTERNAL int plan_exact(sddc_ctx *ctx);
 inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 // CTAs of a residual evaluation of a single case
 inline int resid_grid(const sddc_ctx *ctx)
