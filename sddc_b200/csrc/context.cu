@@ -205,6 +205,17 @@ static double stage_us(int tiles, int resident, const WaveCost &c)
     return c.base + tiles / resident * c.full + (rest ? c.start + (c.full - c.start) * rest / resident : 0.0);
 }
 
+// CTAs per SM of the exact form's kernels
+struct ExactCtas {
+    int tile, held, wide;  // by tiles; by lines with held states, without (0: no such kernel)
+};
+template <int N> constexpr ExactCtas exact_ctas()
+{
+    constexpr int cpb = line_tile_cells(N);
+    return {stage_min_blocks<N, tile_cells(N, 0)>(), line_min_blocks<N, cpb, double, true, false>(),
+            line_has_wide(N, sizeof(double)) ? line_min_blocks<N, cpb, double, true, true>() : 0};
+}
+
 // Whether stages of the exact form run by tiles (stage_kernel.cuh) or by lines
 // (line_kernel.cuh), given the CTAs of either.  A line's 2N+2 dependent point
 // fluxes, in unfused operations, are a longer chain than the tile's phases: a wave
@@ -227,18 +238,23 @@ static cudaError_t exact_by_tiles(int N, bool general, bool persistent, int tile
     static const WaveCost by_tile[] = {{2.3, 5.0, 9.3}, {2.2, 4.4, 10.5}, {0.7, 7.4, 12.5}, {1.4, 8.2, 14.0}};
     static const WaveCost by_line[] = {{1.7, 7.2, 11.5}, {1.5, 10.2, 16.5}, {0.8, 11.8, 13.7}, {4.6, 10.4, 17.4}};
     static const WaveCost by_wide = {4.4, 9.9, 17.2};
-    int rt = 0, held = 0, wide = 0;
-    cudaError_t e = tile_residency_exact(N, &rt);
-    if (e == cudaSuccess) e = line_residency_exact(N, &held, &wide);
+    // the CTAs each kernel is compiled for, on every SM (asking the device what it
+    // holds would load kernels that may not run)
+    static const ExactCtas per_sm[] = {exact_ctas<2>(), exact_ctas<3>(), exact_ctas<4>(), exact_ctas<5>()};
+    int dev = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return e;
+    const ExactCtas &c = per_sm[N - 2];
+    const int rt = sms * c.tile, held = sms * c.held, wide = sms * c.wide;
     const double us = wide && line_use_wide(lines, held, wide) ? stage_us(lines, wide, by_wide)
                                                                : stage_us(lines, held, by_line[N - 2]);
     *out = stage_us(tiles, rt, by_tile[N - 2]) <= us && !(persistent && N <= 4 && tiles > rt);
     return cudaSuccess;
 }
 
-// how the exact stages of a single case run (of a context of another form: when
-// its adjoint needs them, so that only then their kernels are loaded)
+// how the exact stages of a single case run (in a context of another form: its
+// adjoint's)
 int sddc::plan_exact(sddc_ctx *ctx)
 {
     const int cpb = tile_cells(ctx->N, ctx->ncell);

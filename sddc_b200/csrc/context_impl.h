@@ -22,9 +22,6 @@ cudaError_t launch_line_exact(int N, const StageArgs &a, const Ops &ops, cudaStr
 cudaError_t launch_line_fp64(int N, const StageArgs &a, const Ops &ops, cudaStream_t st);
 cudaError_t launch_line_mixed(int N, const StageArgs &a, const Ops &ops, cudaStream_t st);
 cudaError_t launch_tile_exact(int N, int cpb, const StageArgs &a, const Ops &ops, cudaStream_t st);
-// CTAs of an exact stage resident at once, by tiles and by lines (N = 2..5)
-cudaError_t tile_residency_exact(int N, int *resident);
-cudaError_t line_residency_exact(int N, int *held, int *wide);
 cudaError_t launch_resid_exact(int N, const StageArgs &a, const Ops &ops, cudaStream_t st);
 cudaError_t launch_resid_fp64(int N, const StageArgs &a, const Ops &ops, cudaStream_t st);
 cudaError_t launch_resid_mixed(int N, const StageArgs &a, const Ops &ops, cudaStream_t st);

@@ -6,5 +6,4 @@
 #define SDDC_RESID launch_resid_exact
 #define SDDC_TRACE launch_trace_exact
 #define SDDC_VISC launch_visc_exact
-#define SDDC_RESIDENT line_residency_exact
 #include "line_launch.inc"

@@ -37,4 +37,15 @@ template <typename K> cudaError_t set_smem(K kern, size_t bytes)
     return e != cudaSuccess ? e : cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
 }
 
+// CTAs of a kernel resident at once on a device; sets its attributes on the way
+template <typename K> cudaError_t resident_ctas(K kern, int threads, size_t smem, int dev, int *n)
+{
+    int sms = 0, per_sm = 0;
+    cudaError_t e = set_smem(kern, smem);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem);
+    *n = sms * per_sm > 1 ? sms * per_sm : 1;
+    return e;
+}
+
 }  // namespace sddc

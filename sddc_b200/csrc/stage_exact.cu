@@ -26,15 +26,7 @@ template <int N, int CPB> struct TileLaunch {
     static cudaError_t residency(int w, int *out)
     {
         static PerDevice resident[3];
-        return resident[w].get(out, [&](int dev, int *n) {
-            cudaError_t e = set_smem(kernel(w), kSmem);
-            int sms = 0, per_sm = 0;
-            if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-            if (e == cudaSuccess)
-                e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel(w), kThreads, kSmem);
-            *n = std::max(1, sms * per_sm);
-            return e;
-        });
+        return resident[w].get(out, [&](int dev, int *n) { return resident_ctas(kernel(w), kThreads, kSmem, dev, n); });
     }
     static cudaError_t run(const StageArgs &a, const Ops &ops, cudaStream_t st)
     {
@@ -58,17 +50,6 @@ cudaError_t launch_tile_exact(int N, int cpb, const StageArgs &a, const Ops &ops
     case 4: return TileLaunch<4, 8>::run(a, ops, st);
     case 5: return TileLaunch<5, 6>::run(a, ops, st);
     case 6: return cpb == 6 ? TileLaunch<6, 6>::run(a, ops, st) : TileLaunch<6, 8>::run(a, ops, st);
-    default: return cudaErrorInvalidValue;
-    }
-}
-
-cudaError_t tile_residency_exact(int N, int *resident)
-{
-    switch (N) {
-    case 2: return TileLaunch<2, 8>::residency(0, resident);
-    case 3: return TileLaunch<3, 4>::residency(0, resident);
-    case 4: return TileLaunch<4, 8>::residency(0, resident);
-    case 5: return TileLaunch<5, 6>::residency(1, resident);
     default: return cudaErrorInvalidValue;
     }
 }
