@@ -235,8 +235,8 @@ static cudaError_t exact_by_tiles(int N, bool general, bool persistent, int tile
 {
     *out = true;
     if (N == 6 || (N == 5 && !general)) return cudaSuccess;
-    static const WaveCost by_tile[] = {{2.3, 5.0, 9.3}, {2.2, 4.4, 10.5}, {0.7, 7.4, 12.5}, {1.4, 8.2, 14.0}};
-    static const WaveCost by_line[] = {{1.7, 7.2, 11.5}, {1.5, 10.2, 16.5}, {0.8, 11.8, 13.7}, {4.6, 10.4, 17.4}};
+    static const WaveCost by_tile[] = {{2.3, 5.0, 9.3}, {2.2, 4.4, 10.5}, {0.7, 7.4, 12.5}, {4.5, 4.0, 13.3}};
+    static const WaveCost by_line[] = {{1.7, 7.2, 11.5}, {1.5, 10.2, 16.5}, {0.8, 11.8, 13.7}, {4.6, 10.4, 16.8}};
     static const WaveCost by_wide = {4.4, 9.9, 17.2};
     // the CTAs each kernel is compiled for, on every SM (asking the device what it
     // holds would load kernels that may not run)

@@ -271,7 +271,9 @@ __device__ __forceinline__ bool line_tile(const StageArgs &a, const Ops &ops, co
     // in whole lines of memory (point by point in step 4, with 36 loads 72 bytes
     // apart, a stage of FiveStageRk took on average 97.7 us instead of 81.3 at
     // 32400 cells, N = 5, mixed, 125 instead of 116 in FP64)
-    if (kind == kRkFive) {
+    // (the persistent kernel, KIND -2, does so: the pass beside its loop costs
+    // every stage 6%)
+    if (KIND != -2 && kind == kRkFive) {
         // a thread's share in two batches, three where it has the float form's
         // registers
         constexpr int per = (CPB * NQ + NT - 1) / NT, kU = sizeof(R) == 8 ? (per + 1) / 2 : (per + 2) / 3;
@@ -675,9 +677,15 @@ __device__ __forceinline__ bool line_tile(const StageArgs &a, const Ops &ops, co
             } else if (kind == kRkTwoRegT) {
 #pragma unroll
                 for (int k = 0; k < 9; k++) o[k] = (k1 * ap[k] + k2 * qv[k]) + (k0 * res[k]) * cf(3);
-            } else {  // kRkFive: its other terms lie in ap
+            } else if constexpr (KIND != -2) {  // kRkFive: its other terms lie in ap
 #pragma unroll
                 for (int k = 0; k < 9; k++) o[k] = ap[k] + k0 * res[k];
+            } else {
+#pragma unroll
+                for (int k = 0; k < 9; k++)
+                    o[k] = ((((k1 * a.reg_a[g + k] + k2 * a.reg_b[g + k]) + cf(3) * a.reg_c[g + k]) + cf(4) * qv[k]) +
+                            cf(5) * a.reg_d[g + k]) +
+                           k0 * res[k];
             }
 #pragma unroll
             for (int k = 0; k < 9; k++) ap[k] = o[k];
@@ -798,7 +806,8 @@ __device__ __forceinline__ bool line_tile(const StageArgs &a, const Ops &ops, co
     return true;
 }
 
-// KIND: the stage's RkKind, or -1 for any (read from the arguments)
+// KIND: the stage's RkKind, or -1 for any (read from the arguments; -2 in the
+// persistent kernel)
 template <int N, int CPB, typename R, bool EXACT, int KIND, bool WIDE>
 __global__ void __launch_bounds__(line_threads(N, CPB), (line_min_blocks<N, CPB, R, EXACT, WIDE>()))
     line_kernel(const StageArgs a, const Ops ops)
@@ -813,7 +822,7 @@ __global__ void __launch_bounds__(line_threads(N, CPB), (line_min_blocks<N, CPB,
     line_kernel_persistent(const StageArgs a, const Ops ops)
 {
     for (int t = blockIdx.x; t < a.ntiles; t += gridDim.x) {
-        if (!line_tile<N, CPB, R, EXACT, -1, WIDE>(a, ops, t)) return;
+        if (!line_tile<N, CPB, R, EXACT, -2, WIDE>(a, ops, t)) return;
         __syncthreads();  // tile t's last shared-memory reads before tile t+grid stages
     }
 }
