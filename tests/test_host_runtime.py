@@ -310,3 +310,50 @@ def test_device_memory_of_an_adjoint_run(runtime):
             assert want <= run < want + state // 2, (steps, every, run, want)
         clean()
         """)
+
+
+def test_exact_stages_take_the_kernel_that_the_waves_favour(runtime):
+    """148 SMs: sizes at which a sweep put one kernel at least 5% ahead, single
+    and in batches (the launches recorded, not run)."""
+    _run(runtime, """
+        def route(s, step):
+            a, b = launches("stage_kernel"), launches("line_kernel")
+            step(s)
+            a, b = launches("stage_kernel") - a, launches("line_kernel") - b
+            assert sorted((a, b)) == [0, 5], (a, b)
+            return "tiles" if a else "lines"
+
+        def single(N, nx, ny):
+            m = mesh.periodic_box(nx, ny)
+            t = host.build_tables(m, N)
+            s = Solver(t, channel_physics(), precision="fp64_exact")
+            s.set_state(np.ones((9, N, N, t.ncell), order="F"))
+            r = route(s, lambda s: s.rk_s5p3(1e-3, 1))
+            s.close()
+            return r
+
+        def batch(N, nx, ny, count, persistent=False):
+            m = mesh.periodic_box(nx, ny * count)
+            t = host.build_tables(m, N)
+            s = Solver(t, channel_physics(), precision="fp64_exact")
+            s.set_cases([dict(first_cell=k * nx * ny, ncell=nx * ny, dt=1e-3, rinf=1., pinf=1., uinf=.1, vinf=0.,
+                              bxinf=0., byinf=0.) for k in range(count)])
+            s.set_persistent(persistent)
+            s.set_state(np.ones((9, N, N, t.ncell), order="F"))
+            r = route(s, lambda s: s.step_cases(1))
+            s.close()
+            return r
+
+        for N, nx, ny, want in ((2, 8, 8, "tiles"), (2, 64, 64, "tiles"), (2, 100, 100, "lines"), (2, 180, 180, "lines"),
+                                (3, 8, 8, "tiles"), (3, 67, 67, "tiles"), (3, 74, 74, "lines"), (3, 90, 90, "lines"),
+                                (3, 97, 97, "tiles"), (3, 127, 127, "lines"), (4, 8, 8, "tiles"), (4, 67, 67, "tiles"),
+                                (4, 80, 80, "lines"), (4, 90, 90, "tiles"), (4, 120, 120, "tiles"), (4, 220, 220, "lines"),
+                                (5, 8, 8, "tiles"), (5, 120, 120, "tiles"), (6, 90, 90, "tiles")):
+            assert single(N, nx, ny) == want, (N, nx, ny)
+        for N, nx, ny, count, want in ((3, 8, 8, 8, "tiles"), (3, 22, 23, 16, "lines"), (4, 8, 8, 8, "tiles"),
+                                       (4, 22, 23, 16, "tiles"), (5, 22, 23, 8, "tiles"), (5, 22, 23, 16, "tiles"),
+                                       (5, 45, 45, 16, "lines"), (6, 22, 23, 16, "tiles")):
+            assert batch(N, nx, ny, count) == want, (N, nx, ny, count)
+        assert batch(4, 22, 23, 16, True) == "lines" and batch(4, 8, 8, 8, True) == "tiles"
+        clean()
+        """)
